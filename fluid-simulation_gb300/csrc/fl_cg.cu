@@ -13,95 +13,124 @@
 //   phase 2   p += alpha d, r -= alpha q (cg_update.wgsl); r.r partials
 //   exchange  beta and the convergence test (cg_beta.wgsl); the loop exits.
 //
-// Exchange = grid barrier and reduction in one step.  Every partial is
-// published as one 64-bit word {tag, value}, a block's words stored together
-// by one warp (on the block's own 128-byte lines in the line layouts); each
-// block polls all partials until every word carries the exchange's tag, then
-// reduces them itself.  No counter, no second read of the partials, no
-// broadcast: seeing the tags is the barrier, and all blocks
-// evaluate the same reduction in the same order.  Tags are unique per solve
-// (a per-area epoch advanced by k_cg_plan), so words left by earlier solves
-// never match.  Exchange B publishes with release semantics and polls with
-// acquire loads: a block's release covers all of its vector writes of the
-// update phase and the phase before, which is what the next direction +
+// A warp takes whole 256-cell chunks (the 256-wide workgroups of
+// cg_reduce.wgsl).  Lane l holds the quads (four consecutive cells) l and
+// l + 32 of the chunk, so the first level of the chunk's reduction tree is in
+// the lane, the next five are shuffles and the last two are shuffles between
+// the lanes that hold a quad's components: the same pairing as the 256-thread
+// tree, with no shared memory and no block barrier inside a phase.  The x
+// neighbours come from the neighbouring lanes by shuffle; the y and z rows
+// load as float4.  Cells that are not liquid hold zero in d and r, so nothing
+// branches per lane.  Two forms, chosen by each block from its chunk count:
+//
+//   register form   one chunk per warp (up to CG_WARPS chunks): d, r and the
+//                   stencil words stay in registers for the whole solve, p, q
+//                   and a copy of the neighbours' d in shared memory; only the
+//                   neighbours' r is loaded.
+//   general form    chunks in turn, {d, r, q, p} of as many half chunks as the
+//                   pool holds in shared memory, the rest in global memory.
+//
+// What bounds it: up to one chunk per warp, the latency of the two exchanges
+// (2,000-4,000 cycles each: publication, L2 round trip, trees) and of one L2
+// load, then instruction issue (about 300 instructions per warp and phase 1);
+// beyond, L2 throughput and the same latencies per round of chunks.  Solves of
+// 40 / 179 / 200 / 200 iterations on 32^3 / 64^3 / 128^3 (2.0 M particles) /
+// 256^3 (18.3 M): 179 / 867 / 1,315 / 6,580 us against 224 / 1,123 / 1,558 /
+// 7,197 for the earlier kernel (1,024 threads over listed cells or quads, chunk
+// trees from shared memory, every block reading every chunk partial).
+//
+// Two things to keep: a warp index that the compiler knows to be uniform (the
+// shuffle trees took 1,600 cycles instead of 560 without), and no spilled
+// registers in the loops (the acquire of exchange B empties the L1, so each
+// reload is an L2 round trip: phase 1 took 5,500 cycles instead of 3,000).
+//
+// Exchange = grid barrier and reduction in one step.  Partials are published
+// as 64-bit words {tag, value}; readers poll until every word carries the
+// exchange's tag.  No counter, no broadcast: seeing the tags is the barrier,
+// and all blocks evaluate the same reduction in the same order.  Tags are
+// unique per solve (a per-area epoch advanced by k_cg_plan), so words left by
+// earlier solves never match.  Exchange B publishes with release semantics and
+// polls with acquire loads: a block's release covers all of its vector writes
+// of the update phase and the phase before, which is what the next direction +
 // SpMV phase's neighbour loads need.  Exchange A carries only its partials
 // (relaxed).
 //
 // Only 256-cell chunks holding a liquid cell are visited (the rest are zero in
-// every vector).  k_cg_plan lists them once per solve, grouped by residue
-// chunk mod 256 and ascending within a group: segment li holds exactly the
-// nonzero terms that thread li of cg_reduce_final.wgsl adds in sequence (the
-// skipped terms are +0, and acc + 0 == acc for an accumulator that starts at
-// +0).  It also splits the plan into one contiguous range per block with equal
-// liquid-cell weight.  FL_CG_F32: a warp evaluates a chunk's 256-wide
-// cg_reduce.wgsl tree (same pairing, same order); every block stages all chunk
-// partials, sums its segments and evaluates the cg_reduce_final.wgsl tree, so
-// the scalars are the reference's f32 arithmetic exactly.  FL_CG_F64: see Df.
-// Each block lists its liquid cells with their stencil masks (k_grid_prep's
-// cinfo) in shared memory once per solve; an iteration then touches liquid
-// cells only and issues no dependent loads for topology.
+// every vector).  Segment li = active chunks li, li + 256, ... in ascending
+// order: the nonzero terms that thread li of cg_reduce_final.wgsl adds in
+// sequence (the skipped terms are +0, and acc + 0 == acc for an accumulator
+// that starts at +0).  k_cg_plan gives the blocks their chunks once per solve:
+//
+//   heads and tails  a block owns the first chunks of its segments and
+//                    publishes their partial sums; chunks beyond T of a segment
+//                    go to other blocks and are published one by one.  Every
+//                    block adds the tails to the heads itself: one hop.
+//   split segments   (more chunks than that is good for) ranges of equal weight;
+//                    all chunk partials are published, one warp per segment adds
+//                    them and publishes the segment sum: two hops.
+//
+// Every block then evaluates the 256-wide tree of cg_reduce_final.wgsl over the
+// segment sums, so in FL_CG_F32 the scalars are the reference's f32 arithmetic
+// exactly.  The extended-precision forms publish one float-float or double
+// partial per block instead.
 #include <cstddef>
 
 #include "fl_device.cuh"
 
 namespace fl {
 
+constexpr int CG_THREADS = 512;
 constexpr int CG_WARPS = CG_THREADS / 32;
-constexpr uint32_t KT = 2 * CG_WARPS;    // chunks per tree pass: two chunk trees per warp
-constexpr uint32_t CELL_CAP = 16384;     // liquid cells listed per block
-constexpr uint32_t QCAP = CELL_CAP / 2;  // quads listed per block (8 bytes each, in the same array)
-constexpr uint32_t KCH = 2048;           // chunk ids cached per block
-constexpr uint32_t VAL_CAP = 16384;      // chunk partials staged per window
-constexpr uint32_t MAX_PASS = KCH / KT;  // cached tree passes
-// Resident operands: when a block's listed cells fit one pass of at most two
-// cells per thread and the exchange window needs at most half of `vals`, each
-// listed cell keeps {d, r, q, p} in the upper half of `vals` for the whole
-// solve (16 B per cell; the half holds 2 * CG_THREADS cells).
-constexpr uint32_t VALS_HALF = (VAL_CAP + VAL_CAP / 32) / 2;
-constexpr uint32_t RES_MAX_A = VALS_HALF - VALS_HALF / 33;  // vpos(A - 1) < VALS_HALF
+constexpr uint32_t KCH = 512;            // chunks a block keeps a table of
+constexpr uint32_t OWNER_WARPS = 4;      // warps of a block that add split segments
+constexpr uint32_t RAW_MAX = 1024;       // tail partials read by every block
 constexpr uint32_t TAG_SPAN_MAX = 1u << 30;
-constexpr int STAGE_BATCH = 8;
-// Words in flight per thread when staging the blocks' slot lines (one window:
-// at 128^3 about 2.4 words per thread, so a smaller batch frees registers).
-constexpr int LINE_BATCH = 4;
-constexpr uint32_t MAX_CG_BLOCKS = 1024;
-// Per-chunk cost in liquid-cell units for the block split (each chunk adds a
-// tree and, when sparsely filled, cells that share few cache lines).  Kept
-// small: a block above 2 * CG_THREADS listed cells needs a second, serial
-// round of the cell loop, which costs more than the chunk overhead (measured
-// on the 128^3 dam break; 128 pushed dense blocks past that threshold).
-constexpr uint32_t CHUNK_WEIGHT = 32;
+constexpr uint32_t MAX_CG_BLOCKS = 256;
+// Per-chunk cost in liquid-cell units for ranges of equal weight: a warp takes a
+// chunk at once, so a sparsely filled one costs it nearly as much as a full one
+// (with 32, the slowest block's phase 1 at 256^3 took 38,000 cycles against
+// 26,000; with 256, 29,500); solvers that list cells use 32.
+constexpr uint32_t CHUNK_WEIGHT = 256, CELL_CHUNK_WEIGHT = 32;
+// What the pool leaves of the 228 KB serves as L1 for the neighbours' rows: 140 KB
+// against 200 KB and 100 KB on the full-depth 128^3 dam (FL_CG_F64): 2,073, 2,094
+// and 2,206 us per solve; 256^3 within 1 %.
+constexpr uint32_t POOL_BYTES = 140 * 1024;
+constexpr uint32_t HALF_BYTES = 32 * 4 * 16;  // a resident half chunk: float4 d, r, q, p of 32 quads
 
 struct CgShared {
-    float tree[KT][CHUNK];     // per-chunk products of one pass, tree slot = cell in chunk
-    float vals[VAL_CAP + VAL_CAP / 32];  // staged partials of one exchange window (positions vpos)
-    uint32_t cell[CELL_CAP];   // listed liquid cells: bits 0-9 stencil mask, 10-17 cell in chunk, 18-31 chunk
-    uint32_t chunk[KCH];       // this block's chunk ids (plan order)
-    uint32_t off[CHUNK + 1];   // plan segment offsets
-    uint32_t pass_off[MAX_PASS + 1];
+    // Per half chunk (32 quads, one per lane).  Register form: float4 p and the
+    // neighbours' d.  Otherwise: operands of the resident halves, then the
+    // stencil words of all (4 B per quad).
+    alignas(16) unsigned char pool[POOL_BYTES];
+    union {
+        float stage[OWNER_WARPS][CHUNK];   // partials of a split segment
+        float raw[RAW_MAX];                // tail partials
+        struct {
+            double dpart[CG_THREADS];      // FL_CG_F64_IEEE: thread partials
+            float words[2 * MAX_CG_BLOCKS];  // extended forms: the blocks' partials
+        };
+    };
+    uint4 tab[KCH];            // the block's chunks: id, active quads (two masks), first half's index
+    float part[KCH];           // chunk partials of one phase
+    uint32_t off[CHUNK + 1];   // plan entries of the segments' heads
+    uint32_t toff[CHUNK + 1];  // and of their tails
     float seg[CHUNK];          // segment sums (cg_reduce_final.wgsl thread accumulators)
-    float red[2 * CG_WARPS];   // F64: float-float warp partials; F32: one pass of chunk trees
-    uint32_t wcnt[CG_WARPS];
+    float red[2 * CG_THREADS / 32];   // extended forms: warp partials
     float scal[4];             // scalars of an exchange, broadcast by warp 0
-    uint32_t layout, nslot;              // exchange slot layout (0 plan order, 1 lines, 2 one line per block), slots used
-    float thr_f;                         // f32 stopping threshold on r.r
-    float thr_dh, thr_dl;                // FL_CG_F64 stopping threshold on r.r (float-float)
-    double rs_d, thr_d;                  // FL_CG_F64_IEEE: r.r of the last exchange, stopping threshold
-    float rs_hi, rs_lo;                  // r.r of the last exchange (rs_old); FL_CG_F32 uses rs_hi
-    // Block-uniform loop bounds, read from shared memory where used (the cell
-    // loops sit at the 64-register limit of a 1024-thread block).
-    uint32_t u_s0, u_m, u_mc, u_npc, u_ncell, u_res, u_quad, u_lb;
-    uint32_t bstart[MAX_CG_BLOCKS + 1];  // first plan entry of every block
-    uint32_t spos[MAX_CG_BLOCKS + 1];    // first exchange slot of every block
-    uint16_t lineblk[VAL_CAP / 16 + MAX_CG_BLOCKS];  // line of the slot area -> owning block
+    unsigned long long* area[6];  // exchange areas (see k_cg)
+    // Block-uniform values read where they are used: the cell loops are at the
+    // 128-register limit of a 512-thread block, and a spilled register costs an
+    // L2 round trip after every exchange (the acquire empties the L1).
+    uint32_t nh, s0, m, mres, HL, nheads, ah;
+    uint64_t limit;            // of every wait, in ns
+    float one;                 // 1.0f (see addp2)
+    float thr_f;               // f32 stopping threshold on r.r
+    float thr_dh, thr_dl;      // FL_CG_F64 stopping threshold on r.r (float-float)
+    double rs_d, thr_d;        // FL_CG_F64_IEEE: r.r of the last exchange, stopping threshold
+    float rs_hi, rs_lo;        // r.r of the last exchange (rs_old); FL_CG_F32 uses rs_hi
 };
+static_assert(CG_WARPS * 2 * 6 * 32 * 16 <= POOL_BYTES, "register form: six quads per lane and half in the pool");
 static_assert(sizeof(CgShared) <= 227 * 1024, "CG shared memory exceeds the 227 KB per-block limit");
-static_assert(offsetof(CgShared, vals) % 16 == 0 && (VALS_HALF * 4) % 16 == 0, "resident operands are float4");
-static_assert(offsetof(CgShared, tree) % 16 == 0 && offsetof(CgShared, cell) % 8 == 0,
-              "quad layout: float4 tree slots, 8-byte quad entries");
-static_assert(offsetof(CgShared, tree) % 8 == 0 && sizeof(CgShared::tree) >= 8 * CG_THREADS,
-              "the IEEE-double form stages its thread partials in the tree buffer");
-static_assert(VALS_HALF + 4 * 2 * CG_THREADS <= VAL_CAP + VAL_CAP / 32, "resident operands fit the upper half");
 
 // ---------------------------------------------------------------------------
 // Tagged words
@@ -139,93 +168,84 @@ __device__ __forceinline__ unsigned long long ld_tag(const unsigned long long* p
     return acq ? ld_acquire_u64(p) : ld_relaxed_u64(p);
 }
 
-// Polls *p until it carries `tag` and returns the word.  Bounded: after the
-// settings' wait limit (2 s by default), or once another block recorded an
-// error, it records FL_TIMEOUT and returns a word without the tag.
+// Polls *p until it carries `tag` and returns the word.  Bounded: after `limit`
+// ns, or once another block recorded an error, it records FL_TIMEOUT and returns
+// a word without the tag.  The clock is read on the first re-poll and then
+// every 64 polls (so a limit below one poll's latency expires at the first
+// miss); the status word, a global load, every 64 polls only.
 __device__ __noinline__ unsigned long long wait_tag(const unsigned long long* p, uint32_t tag, DevStats* st, bool acq,
-                                                    const DevParams* prm) {
-    const uint64_t t0 = global_ns(), limit = wait_limit_ns(prm);
-    uint32_t spins = 0;
-    unsigned long long w = ld_tag(p, acq);
-    while ((uint32_t)(w >> 32) != tag) {
-        // The clock is read on the first re-poll and then every 64 polls (so
-        // a limit below one poll's latency expires at the first miss); the
-        // status word, a global load, every 64 polls only.
-        ++spins;
+                                                    const uint64_t* limit) {
+    const uint64_t t0 = global_ns();
+    for (uint32_t spins = 1;; spins++) {
+        const unsigned long long w = ld_tag(p, acq);
+        if ((uint32_t)(w >> 32) == tag) return w;
         const bool slow = (spins & 63u) == 0u;
         if (slow && *(volatile uint32_t*)&st->status != 0u) return 0ull;
-        if ((slow || spins == 1u) && global_ns() - t0 > limit) {
+        if ((slow || spins == 1u) && global_ns() - t0 > *limit) {
             atomicCAS(&st->status, 0u, 5u /* FL_TIMEOUT */);
             return 0ull;
         }
-        w = ld_tag(p, acq);
     }
-    return w;
-}
-
-// Stages tagged words: for each virtual index v < nvirt, addr(v) is the word
-// (nullptr: unused index) and dst(v) its slot in vals.  A thread issues up to
-// STAGE_BATCH loads at once, then waits for its unpublished words one at a
-// time (one poll in flight per thread keeps the traffic on the shared lines
-// low; measured faster than re-polling all pending words together).
-// Returns false on abort.
-template <class AddrF, class DstF>
-__device__ __forceinline__ bool stage_words(uint32_t nvirt, uint32_t tag, bool acq, DevStats* st,
-                                            const DevParams* prm, float* vals, AddrF addr, DstF dst) {
-    bool ok = true;
-    for (uint32_t v0 = threadIdx.x; v0 < nvirt; v0 += STAGE_BATCH * CG_THREADS) {
-        unsigned long long w[STAGE_BATCH];
-#pragma unroll
-        for (int k = 0; k < STAGE_BATCH; k++) {
-            const uint32_t v = v0 + k * CG_THREADS;
-            const unsigned long long* a = v < nvirt ? addr(v) : nullptr;
-            w[k] = a ? ld_tag(a, acq) : 0ull;
-        }
-#pragma unroll
-        for (int k = 0; k < STAGE_BATCH; k++) {
-            const uint32_t v = v0 + k * CG_THREADS;
-            const unsigned long long* a = v < nvirt ? addr(v) : nullptr;
-            if (a && ok) {
-                if ((uint32_t)(w[k] >> 32) != tag) {
-                    w[k] = wait_tag(a, tag, st, acq, prm);
-                    ok = (uint32_t)(w[k] >> 32) == tag;
-                }
-                vals[dst(v)] = __uint_as_float((uint32_t)w[k]);
-            }
-        }
-    }
-    return ok;
 }
 
 // ---------------------------------------------------------------------------
 // Reductions
 
-// Staging position of entry e of an exchange window: one pad word every 32
-// entries.  Thread li sums its segment's entries in sequence; segments of
-// equal length 16 (a common case) would start on two banks only, so
-// without the pad the segment sums ran 16-way bank conflicted (0.85 vs
-// 0.47 us per exchange at 128^3).
-__device__ __forceinline__ uint32_t vpos(uint32_t e) { return e + (e >> 5); }
-
-// float4 access to the CG vectors in the quad layout (16-byte aligned quads)
-__device__ __forceinline__ float4 ld_f4(const float* a) { return *reinterpret_cast<const float4*>(a); }
-__device__ __forceinline__ void st_f4(float* a, float4 v) { *reinterpret_cast<float4*>(a) = v; }
-__device__ __forceinline__ float f4_at(const float4& v, int k) { return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w; }
-__device__ __forceinline__ void f4_set(float4& v, int k, float x) {
-    if (k == 0) v.x = x;
-    else if (k == 1) v.y = x;
-    else if (k == 2) v.z = x;
-    else v.w = x;
+// A block-uniform value read from shared memory at its use (not kept in a register).
+template <class T>
+__device__ __forceinline__ T vld(const T& x) {
+    return *(const volatile T*)&x;
 }
 
-// A block-uniform value read from shared memory at its use (not kept in a register).
-__device__ __forceinline__ uint32_t vld(const uint32_t& x) { return *(const volatile uint32_t*)&x; }
+// A quad of f32 values as two register pairs, for the packed f32x2
+// instructions: each half rounds like the scalar operation, and a phase, which
+// is bound by instruction issue, takes half as many.
+struct __align__(16) Quad {
+    unsigned long long a, b;
+};
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+    unsigned long long v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(x), "f"(y));
+    return v;
+}
+__device__ __forceinline__ float lo2(unsigned long long v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float hi2(unsigned long long v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ unsigned long long mul2(unsigned long long x, unsigned long long y) {
+    unsigned long long v;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(x), "l"(y));
+    return v;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long x, unsigned long long y) {
+    unsigned long long v;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(x), "l"(y));
+    return v;
+}
+// prod * one + y with `one` a pair of ones that the assembler cannot see
+// through.  An add.rn.f32x2 of a mul.rn.f32x2's result comes out as one fused
+// multiply-add (one rounding instead of two), so every product is added with
+// this.
+__device__ __forceinline__ unsigned long long addp2(unsigned long long prod, unsigned long long one, unsigned long long y) {
+    unsigned long long v;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(prod), "l"(one), "l"(y));
+    return v;
+}
+__device__ __forceinline__ Quad qmul(Quad x, Quad y) { return {mul2(x.a, y.a), mul2(x.b, y.b)}; }
+__device__ __forceinline__ Quad qadd(Quad x, Quad y) { return {add2(x.a, y.a), add2(x.b, y.b)}; }
+__device__ __forceinline__ Quad qaddp(Quad prod, Quad one, Quad y) { return {addp2(prod.a, one.a, y.a), addp2(prod.b, one.a, y.b)}; }
+// y - x, by way of -x * one: the same single rounding
+__device__ __forceinline__ Quad qsubp(Quad x, Quad one, Quad y) {
+    return {addp2(x.a, one.b, y.a), addp2(x.b, one.b, y.b)};
+}
+__device__ __forceinline__ Quad qall(float x) { return {pack2(x, x), pack2(x, x)}; }
+__device__ __forceinline__ Quad quad(float x, float y, float z, float w) { return {pack2(x, y), pack2(z, w)}; }
+__device__ __forceinline__ Quad ld_quad(const float* a) { return *reinterpret_cast<const Quad*>(a); }
+__device__ __forceinline__ void st_quad(float* a, Quad v) { *reinterpret_cast<Quad*>(a) = v; }
 
 // cg_reduce.wgsl:38-49 over s[0..255], evaluated by one warp: lane l forms the
 // level-128 sums of indices l, l+32, l+64, l+96, the level-64 sums of l and
-// l+32, the level-32 sum of l, then the same shuffle steps 16..1.  Operand
+// l+32, the level-32 sum of l, then the shuffle steps 16..1.  Operand
 // order and pairing equal the 256-thread tree's.  Valid in lane 0.
-__device__ __forceinline__ float chunk_tree(const float* s, uint32_t lane) {
+__device__ __forceinline__ float tree256(const float* s, uint32_t lane) {
     const float a0 = __fadd_rn(s[lane], s[lane + 128]);
     const float a1 = __fadd_rn(s[lane + 32], s[lane + 160]);
     const float a2 = __fadd_rn(s[lane + 64], s[lane + 192]);
@@ -234,6 +254,34 @@ __device__ __forceinline__ float chunk_tree(const float* s, uint32_t lane) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = __fadd_rn(v, __shfl_down_sync(0xffffffffu, v, o));
     return v;
+}
+
+// The same tree over a chunk whose products sit in the warp's registers: a
+// and b are the products of the lane's quads l and l + 32 (tree slots 4l..4l+3
+// and 128 + 4l..).  Level 128 adds them; at levels 64 and 32 a lane keeps half
+// of its components and hands the partner lane the other half, so that from
+// then on it carries one component (2*bit4 + bit3 of the lane) of the quads
+// that share its low three bits; levels 16..4 add quads, levels 2 and 1
+// components.  f32 addition commutes, so every lane ends with the same bits.
+template <bool VEC>
+__device__ __forceinline__ float tree256_quads(Quad a, Quad b, Quad one, uint32_t lane) {
+    const Quad t = qaddp(a, one, b);
+    const float x = lo2(t.a), y = hi2(t.a), z = lo2(t.b), w = hi2(t.b);
+    if (!VEC) {  // components 32 apart: levels 64 and 32 in the lane, then the shuffle steps
+        float v = __fadd_rn(__fadd_rn(x, z), __fadd_rn(y, w));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, o));
+        return v;
+    }
+    const bool h4 = (lane & 16u) != 0u, h3 = (lane & 8u) != 0u;
+    const float u0 = __fadd_rn(h4 ? z : x, __shfl_xor_sync(0xffffffffu, h4 ? x : z, 16));
+    const float u1 = __fadd_rn(h4 ? w : y, __shfl_xor_sync(0xffffffffu, h4 ? y : w, 16));
+    float v = __fadd_rn(h3 ? u1 : u0, __shfl_xor_sync(0xffffffffu, h3 ? u0 : u1, 8));
+    v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 4));
+    v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 2));
+    v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 1));
+    v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 16));
+    return __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 8));
 }
 
 // Per-thread inner-product accumulator of the extended-precision forms:
@@ -266,124 +314,177 @@ __device__ __forceinline__ float d_lo(double v) { return __int_as_float(__double
 __device__ __forceinline__ float d_hi(double v) { return __int_as_float(__double2hiint(v)); }
 __device__ __forceinline__ double d_of(float lo, float hi) { return __hiloint2double(__float_as_int(hi), __float_as_int(lo)); }
 
-// FL_CG_F64: inner products accumulated in float-float (fl_device.cuh) by each
-// thread, across its block and across blocks; alpha and beta are float-float
-// quotients rounded to f32, and the stopping test compares float-float values.
-
-// a / b rounded to f32: the f32 quotient plus one float-float correction.
-
 // ---------------------------------------------------------------------------
 // Plan
 
-// One block of 256 threads.  Lists the active chunks by residue (segment li =
-// chunks li, li+256, ... ascending), splits the list into G contiguous ranges
-// of equal weight (liquid cells + CHUNK_WEIGHT per chunk), and reserves this solve's
-// tag range.  When the 32-bit epoch would wrap, the exchange words are
-// cleared first, so no stale word can carry a tag of a later solve.
-__global__ void __launch_bounds__(CHUNK) k_cg_plan(DevBufs b, uint32_t G) {
-    __shared__ uint32_t s_wc[CHUNK / 32], s_ww[CHUNK / 32];
+// Plan header (cg_off): the offsets of the segments' heads [CHUNK + 1], tag
+// base, form, first plan entry of every block [G + 1], blocks that own chunks,
+// blocks that own heads, exchange word of every segment [CHUNK], offsets of the
+// tails [CHUNK + 1].
+enum { PLAN_F32, PLAN_EXTENDED, PLAN_RANGES };
+constexpr uint32_t H_TAG = CHUNK + 1, H_FORM = CHUNK + 2, H_START = CHUNK + 3;
+
+// One block of 256 threads.  Lists the active chunks, gives each block a
+// contiguous range of the list, and reserves this solve's tag range.  When the
+// 32-bit epoch would wrap, the exchange words are cleared first, so no stale
+// word can carry a tag of a later solve.
+//
+// Heads and tails: a block takes at most T chunks, a multiple of its warps (or
+// half of them where that leaves no tails: a small solve with more SMs at work).
+// A segment's first T chunks are its head; heads are packed in order, whole;
+// what is left of the segments goes to blocks of its own, T chunks each.  The
+// smallest T of 32 (one per lane) is taken that needs no more than G blocks and
+// leaves at most RAW_MAX tail chunks.  At 128^3 every warp then has one chunk:
+// segments of 17 chunks kept whole gave some warps two (1,546 against 1,385 us).
+//
+// Split segments, when that needs more than one more round of CG_WARPS chunks:
+// ranges of equal weight (liquid cells + CHUNK_WEIGHT per chunk) of the list in
+// segment order; with at least 9 chunks per block on average no range is empty.
+//
+// form: PLAN_EXTENDED (no segment sums) takes heads and tails only where each
+// warp gets one chunk; PLAN_RANGES the G ranges of equal weight, for solvers
+// that use just those.
+__global__ void __launch_bounds__(CHUNK) k_cg_plan(DevBufs b, uint32_t G, int form) {
+    const bool ranges_only = form == PLAN_RANGES;
+    const uint32_t per_chunk = ranges_only ? CELL_CHUNK_WEIGHT : CHUNK_WEIGHT;
+    __shared__ uint32_t s_wc[CHUNK / 32], s_ww[CHUNK / 32], s_wa[CHUNK / 32], s_wh[CHUNK / 32];
+    __shared__ uint32_t s_cnt[CHUNK];
+    __shared__ uint16_t s_blk[CHUNK][32];  // block of segment i's head under lane l's T
+    __shared__ uint16_t s_first[MAX_CG_BLOCKS];
+    __shared__ uint32_t s_sel, s_T, s_nblk;
     __shared__ int s_wrap;
     const DevParams& P = *b.prm;
     const uint32_t nchunks = P.nchunks;
     const uint32_t li = threadIdx.x, lane = li & 31, warp = li >> 5;
     uint32_t* hdr = b.cg_off;
-    uint32_t* start = hdr + CHUNK + 3;
-    uint32_t* spos = start + G + 1;
+    uint32_t* start = hdr + H_START;
+    uint32_t* segslot = start + G + 3;
+    uint32_t* toffs = segslot + CHUNK;
     uint32_t cnt = 0, wsum = 0;
     for (uint32_t c = li; c < nchunks; c += CHUNK) {
         const uint32_t f = b.chunk_flag[c];
         if (f) {
             cnt++;
-            wsum += f + CHUNK_WEIGHT;
+            wsum += f + per_chunk;
         }
     }
-    uint32_t x = cnt, y = wsum;
+    const uint32_t has = __ballot_sync(0xffffffffu, cnt != 0u);
+    auto scan = [&](uint32_t v) {  // inclusive, within the warp
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t xa = __shfl_up_sync(0xffffffffu, x, o), ya = __shfl_up_sync(0xffffffffu, y, o);
-        if (lane >= (uint32_t)o) {
-            x += xa;
-            y += ya;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= (uint32_t)o) v += t;
         }
-    }
+        return v;
+    };
+    const uint32_t x = scan(cnt), y = scan(wsum);
+    s_cnt[li] = cnt;
     if (lane == 31) {
         s_wc[warp] = x;
         s_ww[warp] = y;
+        s_wa[warp] = (uint32_t)__popc(has);
     }
     __syncthreads();
-    uint32_t base = 0, wbase = 0, A = 0, W = 0;
+    uint32_t base = 0, wbase = 0, A = 0, W = 0, act = (uint32_t)__popc(has & ((1u << lane) - 1u));
     for (uint32_t w = 0; w < CHUNK / 32; w++) {
         if (w < warp) {
             base += s_wc[w];
             wbase += s_ww[w];
+            act += s_wa[w];
         }
         A += s_wc[w];
         W += s_ww[w];
     }
-    const uint32_t off = base + x - cnt;
-    hdr[li] = off;
-    if (li == CHUNK - 1) hdr[CHUNK] = off + cnt;
-    uint32_t pos = off;
-    uint64_t XG = (uint64_t)(wbase + y - wsum) * G;  // G x the weight of all plan entries before `pos`
-    // Blocks bb with X*G < bb*W <= X1*G start after the entry spanning
+    if (!ranges_only && warp == 0) {
+        const uint32_t T = lane ? CG_WARPS * lane : CG_WARPS / 2;
+        uint32_t blk = 0xffffffffu, cur = T, tails = 0;
+#pragma unroll 16
+        for (uint32_t i = 0; i < (uint32_t)CHUNK; i++) {
+            const uint32_t c = s_cnt[i], h = c < T ? c : T;
+            tails += c - h;
+            if (h && cur + h > T) {
+                blk++;
+                cur = 0;
+            }
+            cur += h;
+            s_blk[i][lane] = (uint16_t)blk;
+        }
+        const uint32_t nb = blk + 1u + (tails + T - 1) / T;
+        const uint32_t fits = __ballot_sync(0xffffffffu, nb <= G && tails <= (lane ? RAW_MAX : 0u) && T <= KCH);
+        const uint32_t sel = fits ? (uint32_t)__ffs(fits) - 1u : 31u;
+        if (lane == sel) {
+            s_sel = sel;
+            s_T = fits ? T : 0u;
+            s_nblk = blk + 1u;
+        }
+    }
+    __syncthreads();
+    uint32_t Gs = G, T = 0;
+    if (!ranges_only) {
+        Gs = A / 9u < 1u ? 1u : (A / 9u < G ? A / 9u : G);
+        const uint32_t per = (A + Gs - 1) / Gs;
+        const uint32_t rounds = (s_T + CG_WARPS - 1) / CG_WARPS;
+        if (s_T && (form == PLAN_F32 || rounds == 1) && rounds <= (per + CG_WARPS - 1) / CG_WARPS + 1) T = s_T;
+    }
+    // head and tail of segment li, their places in the list
+    const uint32_t nh = T && cnt > T ? T : cnt;
+    const uint32_t xh = scan(nh);
+    if (lane == 31) s_wh[warp] = xh;
+    __syncthreads();
+    uint32_t hoff = xh - nh, Ah = 0;
+    for (uint32_t w = 0; w < CHUNK / 32; w++) {
+        if (w < warp) hoff += s_wh[w];
+        Ah += s_wh[w];
+    }
+    const uint32_t toff = base + x - cnt - hoff;
+    hdr[li] = hoff;
+    if (li == CHUNK - 1) hdr[CHUNK] = hoff + nh;
+    const uint32_t nheads = T ? s_nblk : Gs, ntails = T ? (A - Ah + T - 1) / T : 0u;
+    const uint32_t nact = A == 0 ? 1u : nheads + ntails;
+    uint64_t XG = (uint64_t)(wbase + y - wsum) * Gs;  // Gs x the weight of all entries before this segment
+    // Blocks bb with X*Gs < bb*W <= X1*Gs start after the entry spanning
     // weights [X, X1).  X only grows along this thread's entries, so the
     // next such block is tracked incrementally from one division.
     uint64_t bb_next = W ? XG / W + 1 : 0, bbW = bb_next * W;
+    uint32_t k = 0;
     for (uint32_t c = li; c < nchunks; c += CHUNK) {
         const uint32_t f = b.chunk_flag[c];
         if (!f) continue;
-        b.cg_chunk[pos] = c;
-        XG += (uint64_t)(f + CHUNK_WEIGHT) * G;
-        for (; bbW <= XG; bb_next++, bbW += W) start[bb_next] = pos + 1;
-        pos++;
+        b.cg_chunk[k < nh ? hoff + k : Ah + toff + (k - nh)] = c;
+        k++;
+        if (!T) {
+            XG += (uint64_t)(f + per_chunk) * Gs;
+            for (; bbW <= XG; bb_next++, bbW += W) start[bb_next] = hoff + k;
+        }
     }
-    if (A == 0)
-        for (uint32_t bb = li; bb <= G; bb += CHUNK) start[bb] = 0;
-    else if (li == 0)
-        start[0] = 0;
-    __syncthreads();
-    // Slot layout: block bb's chunk partials at spos[bb] + j, each block's
-    // range rounded up to whole 128-byte lines (16 words) and packed in block
-    // order (a reader maps a line back to its block); used when all chunk
-    // partials fit one staging window.  Else densely at plan entry s_bb + j
-    // (spos[bb] = s_bb).  hdr[CHUNK + 2] = 1 for the line layout.
-    const bool lines = A > 0 && A <= VAL_CAP;
-    {
-        const uint32_t per = (G + CHUNK - 1) / CHUNK;
-        const uint32_t b0 = li * per < G ? li * per : G, b1 = b0 + per < G ? b0 + per : G;
-        uint32_t mine = 0;
-        for (uint32_t bb = b0; bb < b1; bb++) {
-            const uint32_t mb = start[bb + 1] - start[bb];
-            mine += lines ? (mb + 15u) & ~15u : mb;
+    uint32_t slot = li;
+    if (T && A) {  // each block's words start on a 128-byte line
+        const uint32_t blk = s_blk[li][s_sel];
+        if (cnt && (li == 0 || s_blk[li - 1][s_sel] != blk)) {
+            s_first[blk] = (uint16_t)act;
+            start[blk] = hoff;
         }
-        uint32_t xs = mine;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(0xffffffffu, xs, o);
-            if (lane >= (uint32_t)o) xs += t;
-        }
-        if (lane == 31) s_wc[warp] = xs;
         __syncthreads();
-        uint32_t run = xs - mine;
-        for (uint32_t w = 0; w < warp; w++) run += s_wc[w];
-        for (uint32_t bb = b0; bb < b1; bb++) {
-            spos[bb] = run;
-            const uint32_t mb = start[bb + 1] - start[bb];
-            run += lines ? (mb + 15u) & ~15u : mb;
+        if (cnt) {
+            const uint32_t first = s_first[blk];
+            slot = 16u * blk + (first & ~15u) + (act - first);
         }
-        if (b0 < b1 && b1 == G) spos[G] = run;
-        if (G == 0 && li == 0) spos[0] = 0;
+        for (uint32_t t = li; t < ntails; t += CHUNK) start[nheads + t] = Ah + t * T;
     }
-    // 2: every block owns 1..16 chunks, so block bb's line is simply line bb
-    uint32_t mmin = 0xffffffffu, mmax = 0;
-    for (uint32_t bb = li; bb < G; bb += CHUNK) {
-        const uint32_t mb = start[bb + 1] - start[bb];
-        mmin = mb < mmin ? mb : mmin;
-        mmax = mb > mmax ? mb : mmax;
+    if (li == 0 && (!T || A == 0)) start[0] = 0;
+    for (uint32_t bb = nact + li; bb <= G; bb += CHUNK)
+        if (T || bb > Gs || A == 0) start[bb] = A;
+    if (!ranges_only) {
+        segslot[li] = slot;
+        toffs[li] = toff;
+        if (li == CHUNK - 1) toffs[CHUNK] = A - Ah;
     }
-    const int one_line = __syncthreads_and(mmin >= 1u && mmax <= 16u);
-    if (li == 0) hdr[CHUNK + 2] = lines ? (one_line ? 2u : 1u) : 0u;
     if (li == 0) {
+        hdr[H_FORM] = T ? 1u : 0u;
+        if (!ranges_only) {
+            start[G + 1] = nact;
+            start[G + 2] = nheads;
+        }
         const uint32_t span = 2u * (P.iters < TAG_SPAN_MAX ? P.iters : TAG_SPAN_MAX) + 4u;
         uint32_t e0 = (uint32_t)b.cg_x[0];
         int wrap = 0;
@@ -392,7 +493,7 @@ __global__ void __launch_bounds__(CHUNK) k_cg_plan(DevBufs b, uint32_t G) {
             e0 = 0;
         }
         b.cg_x[0] = (unsigned long long)(e0 + span);
-        hdr[CHUNK + 1] = e0;
+        hdr[H_TAG] = e0;
         s_wrap = wrap;
     }
     __syncthreads();
@@ -405,7 +506,14 @@ __global__ void __launch_bounds__(CHUNK) k_cg_plan(DevBufs b, uint32_t G) {
 // ---------------------------------------------------------------------------
 // The solve
 
-template <int PREC>
+// VEC: rows are a multiple of four cells and the vectors 16-byte aligned, so a
+// quad and its +-y and +-z rows load as float4.  Otherwise a lane's four cells
+// of a half are 32 apart, so that its scalar loads are coalesced whatever the
+// rows' alignment (consecutive cells made each load touch four times the lines:
+// 121 x 112 x 110, 60 iterations, a whole fl_solve_pressure call: 1,520 us
+// against 1,289).  Either way component k of a
+// lane's quad is the cell at CSTEP * k from its first.
+template <int PREC, bool VEC>
 __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     CgShared& sh = *reinterpret_cast<CgShared*>(smem_raw);
@@ -413,175 +521,199 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
     const DevParams& P = *b.prm;
     const uint32_t C = P.C, iters = P.iters < TAG_SPAN_MAX ? P.iters : TAG_SPAN_MAX, nchunks = P.nchunks;
     const uint32_t nx = P.nx, nxy = P.nx * P.ny;  // grids hold at most 2^30 cells
+    constexpr uint32_t CSTEP = VEC ? 1u : 32u, LSTEP = VEC ? 4u : 1u;  // between a lane's cells, between lanes
     constexpr bool f64 = PREC != FL_CG_F32;       // no chunk trees: per-thread accumulators
     constexpr bool ieee = PREC == FL_CG_F64_IEEE;
     using Acc = typename AccT<PREC>::type;
-    const float tol_sq = P.tol_sq;
-    const double tol_sq_d = P.tol_sq_d;
     // Stopping test enabled: evaluated once (a double compare in the loop
     // would run on the FP64 pipe in every warp of every iteration).
     const bool stop_on = f64 ? P.tol_sq_d > 0.0 : P.tol_sq > 0.0f;
     DevStats* st = b.st;
-    const uint32_t G = gridDim.x, tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    float* __restrict__ r = b.r;
-    float* __restrict__ p = b.p;
-    float* __restrict__ q = b.q;
-    const uint16_t* __restrict__ cinfo = b.cinfo;
-    const uint32_t* __restrict__ plan = b.cg_chunk;
+    const uint32_t G = gridDim.x, tid = threadIdx.x, lane = tid & 31u;
+    const uint32_t warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // known to be uniform
     const uint32_t* hdr = b.cg_off;
-    for (uint32_t i = tid; i <= CHUNK; i += CG_THREADS) sh.off[i] = hdr[i];
-    const uint32_t tag_base = hdr[CHUNK + 1];
-    // Block-uniform values read only by the exchanges live in shared memory
-    // (sh.layout, sh.nslot, sh.off[CHUNK]) rather than in registers: the cell
-    // loops are at the 64-register limit of a 1024-thread block.
-    if (tid == 0) sh.layout = hdr[CHUNK + 2];
-    const uint32_t* bstart = hdr + CHUNK + 3;
-    const uint32_t* spos = bstart + G + 1;
-    for (uint32_t i = tid; i <= G; i += CG_THREADS) {
-        sh.bstart[i] = bstart[i];
-        sh.spos[i] = spos[i];
+    const uint32_t* start = hdr + H_START;
+    const uint32_t nact = start[G + 1];
+    if (blockIdx.x >= nact) return;  // only blocks that own chunks take part
+    float* r = b.r;
+    float* p = b.p;
+    float* q = b.q;
+    const uint16_t* __restrict__ cinfo = b.cinfo;
+    const uint32_t s0 = start[blockIdx.x], m = start[blockIdx.x + 1] - s0;  // plan entries [s0, s0 + m)
+    const uint32_t* __restrict__ plan = b.cg_chunk + s0;
+    const bool whole = hdr[H_FORM] != 0u;  // heads and tails
+    const uint32_t tag_base = hdr[H_TAG];
+    {
+        const uint32_t* segslot = start + G + 3;
+        const uint32_t* toffs = segslot + CHUNK;
+        for (uint32_t i = tid; i <= (uint32_t)CHUNK; i += CG_THREADS) {
+            sh.off[i] = hdr[i];
+            sh.toff[i] = toffs[i];
+        }
     }
-    const uint32_t s0 = bstart[blockIdx.x], s1 = bstart[blockIdx.x + 1];
-    const uint32_t m = s1 - s0;  // this block's chunks: plan entries [s0, s1)
-    if (tid == 0) sh.nslot = spos[G];
-    __syncthreads();
-    if (sh.layout != 0u)  // line -> owning block
-        for (uint32_t bb = tid; bb < G; bb += CG_THREADS)
-            for (uint32_t L = sh.spos[bb] >> 4; L < sh.spos[bb + 1] >> 4; L++) sh.lineblk[L] = (uint16_t)bb;
+    const uint32_t segslot = tid < (uint32_t)CHUNK && hdr[tid] != hdr[tid + 1] ? start[G + 3 + tid] : 0xffffffffu;
     // Every exchange area starts on a 128-byte line (the pool is 256-byte
-    // aligned): a block's slot line must not share a physical line with a
+    // aligned): a block's line must not share a physical line with a
     // neighbour's (measured 8-11 % of the solve at 128^3 when it did).
-    const size_t nslot = (((size_t)nchunks + 15) & ~(size_t)15) + 16 * (size_t)G;
-    unsigned long long* slotA = b.cg_x + 16;       // d.q chunk partials
-    unsigned long long* slotB = slotA + nslot;     // r.r chunk partials
-    unsigned long long* wordA = slotB + nslot;     // FL_CG_F64: {hi, lo} of block b at 16*b
-    unsigned long long* wordB = wordA + 16 * (size_t)G;
-    unsigned long long* segA = wordB + 16 * (size_t)G;  // two-hop exchanges: 256 segment sums each
-    unsigned long long* segB = segA + CHUNK;
-    const uint32_t mch = m < KCH ? m : KCH;
-    for (uint32_t j = tid; j < mch; j += CG_THREADS) sh.chunk[j] = plan[s0 + j];
-    for (uint32_t i = tid; i < KT * CHUNK; i += CG_THREADS) (&sh.tree[0][0])[i] = 0.0f;
-    __syncthreads();
-    const uint32_t A = sh.off[CHUNK];
-
-    // Quad layout: when rows are a multiple of four cells and the vectors are
-    // 16-byte aligned, every aligned run of four cells (a quad) and its +-y
-    // and +-z rows load as float4, so the cell loops issue one load per four
-    // cells per vector instead of one per cell.  The listing then holds the
-    // quads with a liquid cell (QCAP of them), each with its four cells'
-    // stencil words; otherwise the liquid cells one by one (CELL_CAP).
-    //
-    // A block whose cells qualify for the resident operands (one pass, at
-    // most 2 * CG_THREADS liquid cells: chunk_flag counts them, saturated at
-    // 255, so 256 bounds a full chunk) lists cells: with every operand in
-    // shared memory the cell form was faster (CG stage at 128^3 1.69 vs
-    // 1.75 ms per substep); larger blocks take quads (256^3 8.01 vs 8.72 ms).
-    uint32_t liq_bound = 0;
-    if (warp == 0 && m <= KT) {
-        for (uint32_t j = lane; j < m; j += 32) {
-            const uint32_t f = b.chunk_flag[sh.chunk[j]];
-            liq_bound += f == 255u ? 256u : f;
-        }
-        liq_bound = __reduce_add_sync(0xffffffffu, liq_bound);
-        if (lane == 0) sh.u_lb = liq_bound;
-    }
-    __syncthreads();
-    const bool res_fit = m <= KT && sh.u_lb <= 2u * CG_THREADS && A <= RES_MAX_A;
-    __syncthreads();
-    const bool quads = !res_fit && (nx & 3u) == 0u &&
-                       (((uintptr_t)p | (uintptr_t)r | (uintptr_t)q | (uintptr_t)b.dA | (uintptr_t)b.dB) & 15u) == 0u &&
-                       ((uintptr_t)cinfo & 7u) == 0u;
-    uint2* const qlist = reinterpret_cast<uint2*>(sh.cell);
-    uint32_t ncell = 0, mc = 0;
-    if (quads) {
-        // 16 chunks (64 quads each) per round, in (chunk, quad) order; entry
-        // x = stencil words of cells 0..2 (10 bits each), y = cell 3's word |
-        // quad << 10 | chunk slot << 16.
-        const uint32_t lt_mask = (1u << lane) - 1u;
-        for (uint32_t j0 = 0; j0 < mch; j0 += 16) {
-            if ((j0 % KT) == 0 && tid == 0) sh.pass_off[j0 / KT] = ncell;
-            const uint32_t j = j0 + (tid >> 6), qd = tid & 63u;
-            uint2 info = make_uint2(0u, 0u);
-            if (j < mch) {
-                const uint32_t c0 = sh.chunk[j] * CHUNK + 4u * qd;
-                if (c0 < C) info = *reinterpret_cast<const uint2*>(cinfo + c0);  // C is a multiple of 4
-            }
-            const uint32_t w0 = info.x & 1023u, w1 = (info.x >> 16) & 1023u, w2 = info.y & 1023u,
-                           w3 = (info.y >> 16) & 1023u;
-            const bool liq = ((w0 | w1 | w2 | w3) & 1u) != 0u;
-            const uint32_t bal = __ballot_sync(0xffffffffu, liq);
-            if (lane == 0) sh.wcnt[warp] = (uint32_t)__popc(bal);
-            __syncthreads();
-            uint32_t before = 0, total = 0;
-            for (uint32_t w = 0; w < (uint32_t)CG_WARPS; w++) {
-                const uint32_t n = sh.wcnt[w];
-                if (w < warp) before += n;
-                total += n;
-            }
-            __syncthreads();
-            if (ncell + total > QCAP) break;  // uniform: every thread sees the same totals
-            if (liq) qlist[ncell + before + __popc(bal & lt_mask)] = make_uint2(w0 | (w1 << 10) | (w2 << 20), w3 | (qd << 10) | (j << 16));
-            ncell += total;
-            mc = j0 + 16 < mch ? j0 + 16 : mch;
-        }
-    } else {
-        // List the liquid cells of chunks [0, mc), four chunks per round, in
-        // (chunk, cell) order; stop before CELL_CAP would be exceeded.
-        const uint32_t lt_mask = (1u << lane) - 1u;
-        for (uint32_t j0 = 0; j0 < mch; j0 += 4) {
-            if ((j0 % KT) == 0 && tid == 0) sh.pass_off[j0 / KT] = ncell;
-            const uint32_t j = j0 + (tid >> 8), cl = tid & (CHUNK - 1);
-            uint32_t info = 0;
-            if (j < mch) {
-                const uint32_t c = sh.chunk[j] * CHUNK + cl;
-                if (c < C) info = cinfo[c];
-            }
-            const bool liq = info & 1u;
-            const uint32_t bal = __ballot_sync(0xffffffffu, liq);
-            if (lane == 0) sh.wcnt[warp] = (uint32_t)__popc(bal);
-            __syncthreads();
-            uint32_t before = 0, total = 0;
-            for (uint32_t w = 0; w < (uint32_t)CG_WARPS; w++) {
-                const uint32_t n = sh.wcnt[w];
-                if (w < warp) before += n;
-                total += n;
-            }
-            __syncthreads();
-            if (ncell + total > CELL_CAP) break;  // uniform: every thread sees the same totals
-            if (liq) sh.cell[ncell + before + __popc(bal & lt_mask)] = info | (cl << 10) | (j << 18);
-            ncell += total;
-            mc = j0 + 4 < mch ? j0 + 4 : mch;
-        }
-    }
-    const uint32_t npc = (mc + KT - 1) / KT;  // cached passes
-    if (tid == 0) sh.pass_off[npc] = ncell;
-    // One pass in all: non-liquid tree slots stay zero for the whole solve.
-    const bool multi = npc > 1 || mc < m;
-    __syncthreads();
-    // Resident operands: thread t owns listed cells t and t + CG_THREADS in
-    // both phases, so their {d, r, q, p} stay in shared memory for the whole
-    // solve.  Phase 2 then loads nothing from global memory, q is never
-    // written there, and p is written once at the end; d (phase 1) and r
-    // (phase 2) are still stored for the neighbours in other blocks.  At 128^3
-    // this took the update phase from 2300 to 1640 cycles per iteration.
-    const bool res = !quads && !multi && ncell <= 2u * CG_THREADS && A <= RES_MAX_A;
-    float4* const rv4 = reinterpret_cast<float4*>(sh.vals + VALS_HALF);
+    enum { SLOT_A, SLOT_B, SEG_A, SEG_B, WORD_A, WORD_B };
     if (tid == 0) {
-        sh.u_s0 = s0;
-        sh.u_m = m;
-        sh.u_mc = mc;
-        sh.u_npc = npc;
-        sh.u_ncell = ncell;
-        sh.u_res = res ? 1u : 0u;
-        sh.u_quad = quads ? 1u : 0u;
+        const size_t nslot = ((size_t)nchunks + 15) & ~(size_t)15, nseg = 16 * (size_t)G + CHUNK;
+        unsigned long long* a = b.cg_x + 16;
+        sh.area[SLOT_A] = a;                  // d.q chunk partials: split segments in plan order, or the tails'
+        sh.area[SLOT_B] = a += nslot;         // r.r chunk partials
+        sh.area[SEG_A] = a += nslot;          // segment sums
+        sh.area[SEG_B] = a += nseg;
+        sh.area[WORD_A] = a += nseg;          // extended forms: two words of block bb at 16*bb
+        sh.area[WORD_B] = a += 16 * (size_t)G;
+        sh.s0 = s0;
+        sh.m = m;
+        sh.nheads = start[G + 2];
+        sh.ah = hdr[CHUNK];  // plan entries of the heads
+        sh.one = 1.0f;
+        sh.limit = wait_limit_ns(b.prm);
     }
-    if (res)
-        for (uint32_t tu = tid; tu < ncell; tu += CG_THREADS) {
-            const uint32_t e = sh.cell[tu];
-            const uint32_t c = sh.chunk[e >> 18] * CHUNK + ((e >> 10) & 255u);
-            rv4[tu] = make_float4(b.dA[c], r[c], 0.0f, p[c]);
-        }
 
+    // ---- the block's chunks: active quads, stencil words, resident operands
+    // Stencil word of the quad at c: bits 0-3 liquid cells, 4-15 the cells'
+    // counts of non-solid neighbours.
+    auto load_info = [&](uint32_t c) -> uint32_t {
+        uint32_t w[4], e = 0;
+        if (VEC && c < C) {  // C is a multiple of 4
+            const uint2 v = *reinterpret_cast<const uint2*>(cinfo + c);
+            w[0] = v.x; w[1] = v.x >> 16; w[2] = v.y; w[3] = v.y >> 16;
+        } else {
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++) w[k] = c + CSTEP * k < C ? (uint32_t)cinfo[c + CSTEP * k] : 0u;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) e |= (w[k] & 1u) << k | ((w[k] >> 7) & 7u) << (4 + 3 * k);
+        return e;
+    };
+    const uint32_t mc = m < KCH ? m : KCH;
+    for (uint32_t j = warp; j < mc; j += CG_WARPS) {
+        const uint32_t id = plan[j], c = id * CHUNK + LSTEP * lane;
+        const uint32_t lo = __ballot_sync(0xffffffffu, (load_info(c) & 15u) != 0u);
+        const uint32_t hi = __ballot_sync(0xffffffffu, (load_info(c + CHUNK / 2) & 15u) != 0u);
+        if (lane == 0) sh.tab[j] = make_uint4(id, lo, hi, (lo != 0u) + (hi != 0u));
+    }
+    __syncthreads();
+    if (warp == 0) {
+        uint32_t run = 0;
+        for (uint32_t j0 = 0; j0 < mc; j0 += 32) {
+            const uint32_t n = j0 + lane < mc ? sh.tab[j0 + lane].w : 0u;
+            uint32_t x = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= (uint32_t)o) x += t;
+            }
+            if (j0 + lane < mc) sh.tab[j0 + lane].w = run + x - n;
+            run += __shfl_sync(0xffffffffu, x, 31);
+        }
+        if (lane == 0) sh.nh = run;
+    }
+    __syncthreads();
+    // Register form: one chunk per warp, whose d, r and q stay in registers.
+    const bool regs = m <= (uint32_t)CG_WARPS;
+    // Halves [0, HR) have their operands in the pool, [0, HL) their stencil words.
+    uint32_t HR, HL;
+    {
+        const uint32_t nh = sh.nh;
+        HR = regs ? 0u : nh * (HALF_BYTES + 128u) <= POOL_BYTES ? nh : (nh * 128u < POOL_BYTES ? (POOL_BYTES - nh * 128u) / HALF_BYTES : 0u);
+        HL = nh < (POOL_BYTES - HR * HALF_BYTES) / 128u ? nh : (POOL_BYTES - HR * HALF_BYTES) / 128u;
+    }
+    if (tid == 0) sh.HL = HL;
+    // The resident arrays: operand k (0 d, 1 r, 2 q, 3 p) of quad i; after them
+    // the stencil words of all halves.
+    auto op = [&](uint32_t k, uint32_t i) -> Quad& { return reinterpret_cast<Quad*>(sh.pool)[32u * k * HR + i]; };
+    auto lst = [&](uint32_t i) -> uint32_t& { return reinterpret_cast<uint32_t*>(sh.pool)[(HALF_BYTES / 4u) * HR + i]; };
+    __syncthreads();
+    // +1 and -1, which the assembler cannot see through (see addp2)
+    const Quad one = {pack2(vld(sh.one), vld(sh.one)), pack2(-vld(sh.one), -vld(sh.one))};
+    const uint32_t safe = (nxy + nx) & ~3u;
+    const Quad z4 = {0ull, 0ull};
+    // A quad of a vector: whole when VEC (cells that are not liquid hold
+    // zero), else its liquid cells (p may be a caller's array of any alignment).
+    auto ld_q = [&](const float* a, uint32_t c, uint32_t e) -> Quad {
+        if (VEC) return (e & 15u) ? ld_quad(a + c) : z4;
+        return quad((e & 1u) ? a[c] : 0.0f, (e & 2u) ? a[c + CSTEP] : 0.0f, (e & 4u) ? a[c + 2 * CSTEP] : 0.0f,
+                    (e & 8u) ? a[c + 3 * CSTEP] : 0.0f);
+    };
+    auto st_q = [&](float* a, uint32_t c, uint32_t e, Quad v) {
+        if (VEC) {
+            if (e & 15u) st_quad(a + c, v);
+        } else {
+            if (e & 1u) a[c] = lo2(v.a);
+            if (e & 2u) a[c + CSTEP] = hi2(v.a);
+            if (e & 4u) a[c + 2 * CSTEP] = lo2(v.b);
+            if (e & 8u) a[c + 3 * CSTEP] = hi2(v.b);
+        }
+    };
+    // The chunk's halves in the arrays: index of half h's quad of this lane.
+    auto slot_of = [&](uint4 t, int h) { return (t.w + (h && t.y ? 1u : 0u)) * 32u + lane; };
+    auto ends = [&](uint4 t) { return t.w + (t.y != 0u) + (t.z != 0u); };  // first half past the chunk's
+    for (uint32_t j = warp; j < mc && !regs; j += CG_WARPS) {
+        const uint4 t = sh.tab[j];
+        const uint32_t end = ends(t);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            if ((h ? t.z : t.y) == 0u) continue;
+            const uint32_t c = t.x * CHUNK + h * (CHUNK / 2) + LSTEP * lane, i = slot_of(t, h);
+            const uint32_t e = load_info(c);
+            if (end <= HL) lst(i) = e;
+            if (end <= HR) {
+                op(0, i) = ld_q(b.dA, c, e);
+                op(1, i) = ld_q(r, c, e);
+                op(2, i) = z4;
+                op(3, i) = ld_q(p, c, e);
+            }
+        }
+    }
+    {  // chunks [0, mres) have their operands here
+        uint32_t lo = 0, hi = mc;  // first chunk that ends past HR (ends grow with j)
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi) / 2;
+            if (ends(sh.tab[mid]) <= HR) lo = mid + 1;
+            else hi = mid;
+        }
+        if (tid == 0) sh.mres = lo;  // visible after the barrier before the loop
+    }
+
+    // The lane's two quads of chunk j: first cells (of some interior quad for an
+    // inactive one, whose results are masked), stencil words, indices of the
+    // resident operands, and whether the warp has an active quad in the half.
+    struct Quads {
+        uint32_t c[2], i[2], e[2];
+        bool any[2];
+    };
+    auto quads_of = [&](uint32_t j) -> Quads {
+        Quads k;
+        const bool in = j < KCH;
+        const uint4 t = in ? sh.tab[j] : make_uint4(b.cg_chunk[vld(sh.s0) + j], 1u, 1u, 0u);
+        const bool listed = in && ends(t) <= vld(sh.HL);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const uint32_t c = t.x * CHUNK + h * (CHUNK / 2) + LSTEP * lane;
+            uint32_t e = 0;
+            k.i[h] = slot_of(t, h);
+            if (h ? t.z : t.y) e = listed ? lst(k.i[h]) : load_info(c);
+            k.any[h] = __any_sync(0xffffffffu, (e & 15u) != 0u);
+            k.c[h] = (e & 15u) ? c : safe;
+            k.e[h] = e;
+        }
+        return k;
+    };
+    // Counts of non-solid neighbours as floats, and the quad with its cells that
+    // are not liquid cleared.
+    auto counts = [&](uint32_t e) -> Quad {
+        return quad((float)((e >> 4) & 7u), (float)((e >> 7) & 7u), (float)((e >> 10) & 7u), (float)((e >> 13) & 7u));
+    };
+    auto liquid = [&](Quad v, uint32_t e) -> Quad {
+        auto m2 = [&](float x, int k) { return (e >> k) & 1u ? x : 0.0f; };
+        return quad(m2(lo2(v.a), 0), m2(hi2(v.a), 1), m2(lo2(v.b), 2), m2(hi2(v.b), 3));
+    };
+
+    // ---- exchanges
     // The scalars that follow an exchange, from its sum v: post 1 alpha
     // (cg_alpha.wgsl:17-22, sc = rs_old / v), post 2 beta and the stopping test
     // (cg_beta.wgsl:16-30, sc = v / rs_old, dn).  Evaluated once, by lane 0 of
@@ -600,157 +732,161 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
         sh.scal[1] = sc;
         sh.scal[2] = dn ? 1.0f : 0.0f;
     };
-    // FL_CG_F32 scalar: the segment sums of cg_reduce_final.wgsl, then its
-    // 256-wide tree, evaluated by warp 0 (32 warps evaluating it redundantly
-    // competed for issue slots: 0.3 us per exchange at 128^3).  Every thread
-    // receives the sum (out) and the post scalars (sc, dn).  Returns false on
-    // abort.  Three ways to the segment sums:
-    //  * line layouts (all partials fit one window): every block stages every
-    //    block's slot line and sums all 256 segments itself (one hop);
-    //  * plan-order layout (more active chunks than one window: every block
-    //    reading every partial cost 6-9 us per exchange at 256^3): two hops.
-    //    Block bb owns segments bb, bb + G, ...; one warp per owned segment
-    //    polls its partials (plan entries off[li]..off[li+1]), sums them in
-    //    order in lane 0 and publishes the segment sum as a tagged word in
-    //    `segw` (release on the exchange after which vector writes are read:
-    //    the owners' acquires and releases carry every block's writes on);
-    //    then every block polls the 256 segment words;
-    //  * `x` == nullptr: the initial residual partials part_rr, indexed by
-    //    chunk, staged in windows.
-    auto reduce_f32 = [&](const unsigned long long* x, unsigned long long* segw, uint32_t tag, bool acq, int post,
-                          float& out, float& sc, bool& dn) -> bool {
-        float acc = 0.0f;
+    auto wait_word = [&](const unsigned long long* w, uint32_t tag, bool acq, bool& ok) -> float {
+        unsigned long long v = ld_tag(w, acq);
+        if ((uint32_t)(v >> 32) != tag && ok) {
+            v = wait_tag(w, tag, st, acq, &sh.limit);
+            ok = (uint32_t)(v >> 32) == tag;
+        }
+        return __uint_as_float((uint32_t)v);
+    };
+    // The end of a phase: chunk partials sh.part[0..n) of chunks j0.. are
+    // published (split segments).  A release fence comes first where the
+    // readers go on to load this block's vectors; the barrier before it orders
+    // the other warps' stores.
+    auto publish_parts = [&](uint32_t j0, uint32_t n, unsigned long long* slots, uint32_t tag, bool rel) {
+        __syncthreads();
+        if (warp * 32u < n) {
+            if (rel) asm volatile("fence.acq_rel.gpu;" ::: "memory");
+            for (uint32_t t = tid; t < n; t += CG_THREADS) publish(slots + vld(sh.s0) + j0 + t, tag, sh.part[t], false);
+        }
+    };
+    // FL_CG_F32: the segment sums of cg_reduce_final.wgsl, then its 256-wide
+    // tree and the post scalars by warp 0.  Returns false on abort.
+    auto reduce_f32 = [&](unsigned long long* slots, unsigned long long* segw, uint32_t tag, bool acq, int post,
+                          float& sc, bool& dn) -> bool {
         bool ok = true;
-        const uint32_t A = sh.off[CHUNK];
-        if (x && sh.layout == 0u) {
-            float* buf = sh.vals + warp * 256u;  // per-warp staging of 256 partials
-            for (uint32_t li = blockIdx.x + warp * G; li < (uint32_t)CHUNK; li += CG_WARPS * G) {
-                const uint32_t lo = sh.off[li], hi = sh.off[li + 1];
-                float s = 0.0f;
-                for (uint32_t e0 = lo; e0 < hi; e0 += 256u) {
-                    // all eight polls of a lane in flight, then the waits (the
-                    // wait after each load serialised them: one round trip per word)
-                    unsigned long long w[8];
-#pragma unroll
-                    for (int k2 = 0; k2 < 8; k2++) {
-                        const uint32_t e = e0 + lane + 32u * k2;
-                        w[k2] = e < hi ? ld_tag(x + e, acq) : 0ull;
-                    }
-#pragma unroll
-                    for (int k2 = 0; k2 < 8; k2++) {
-                        const uint32_t e = e0 + lane + 32u * k2;
-                        if (e < hi && (uint32_t)(w[k2] >> 32) != tag && ok) {
-                            w[k2] = wait_tag(x + e, tag, st, acq, b.prm);
-                            ok = (uint32_t)(w[k2] >> 32) == tag;
-                        }
-                        buf[lane + 32u * k2] = e < hi ? __uint_as_float((uint32_t)w[k2]) : 0.0f;
-                    }
-                    __syncwarp();
-                    if (lane == 0) {  // cg_reduce_final.wgsl:29-36: in plan order, from +0
-                        // entries past the segment's end were staged as +0,
-                        // which leaves s (never -0) unchanged
-                        const uint32_t n = hi - e0 < 256u ? hi - e0 : 256u;
-                        for (uint32_t j = 0; j < n; j += 16) {
-                            float t16[16];
-#pragma unroll
-                            for (int k2 = 0; k2 < 16; k2++) t16[k2] = buf[j + k2];
-#pragma unroll
-                            for (int k2 = 0; k2 < 16; k2++) s = __fadd_rn(s, t16[k2]);
-                        }
-                    }
-                    __syncwarp();
-                }
-                // a segment whose partials did not all arrive is not published
-                if (__all_sync(0xffffffffu, ok) && lane == 0) publish(segw + li, tag, s, acq);
-            }
+        if (whole) {
+            __syncthreads();  // sh.part is complete, the phase's stores are issued
+            const uint32_t ntail = vld(sh.toff[CHUNK]);
             if (tid < (uint32_t)CHUNK) {
-                unsigned long long w = ld_tag(segw + tid, acq);
-                if ((uint32_t)(w >> 32) != tag && ok) {
-                    w = wait_tag(segw + tid, tag, st, acq, b.prm);
-                    ok = (uint32_t)(w >> 32) == tag;
-                }
-                sh.seg[tid] = __uint_as_float((uint32_t)w);
-            }
-            if (__syncthreads_or(!ok)) return false;
-        } else {
-        for (uint32_t w0 = 0; w0 < A; w0 += VAL_CAP) {
-            const uint32_t wn = A - w0 < VAL_CAP ? A - w0 : VAL_CAP;
-            if (x && sh.layout != 0u) {  // one window (A <= VAL_CAP): walk the blocks' lines.  Written
-                                         // out rather than through stage_words: measured 0.5 ms/step faster.
-                const uint32_t nslot_used = sh.nslot;
-                const bool one_line = sh.layout == 2u;
-                for (uint32_t v0 = tid; v0 < nslot_used; v0 += LINE_BATCH * CG_THREADS) {
-                    unsigned long long w[LINE_BATCH];
-                    uint32_t dst[LINE_BATCH];
+                const uint32_t lo = sh.off[tid], hi = sh.off[tid + 1], s0 = vld(sh.s0);
+                const bool mine = segslot != 0xffffffffu && lo >= s0 && lo < s0 + vld(sh.m);
+                float s = 0.0f;
+                if (mine) {
+                    if (acq) asm volatile("fence.acq_rel.gpu;" ::: "memory");
+                    // 8 loads first (past the head's end: +0), then the sequential
+                    // adds.  s starts at +0 and a sum of floats is -0 only when both
+                    // terms are, so s is never -0 and adding +0 leaves it unchanged.
+                    for (uint32_t e = lo; e < hi; e += 8) {
+                        float v[8];
 #pragma unroll
-                    for (int k2 = 0; k2 < LINE_BATCH; k2++) {
-                        const uint32_t v = v0 + k2 * CG_THREADS;
-                        const uint32_t bb = v < nslot_used ? (one_line ? v >> 4 : (uint32_t)sh.lineblk[v >> 4]) : 0u;
-                        const uint32_t j = v - sh.spos[bb];
-                        const bool use = v < nslot_used && j < sh.bstart[bb + 1] - sh.bstart[bb];
-                        dst[k2] = use ? sh.bstart[bb] + j : 0xffffffffu;
-                        w[k2] = use ? ld_tag(x + v, acq) : 0ull;
+                        for (int k2 = 0; k2 < 8; k2++) v[k2] = e + k2 < hi ? sh.part[e - s0 + k2] : 0.0f;
+#pragma unroll
+                        for (int k2 = 0; k2 < 8; k2++) s = __fadd_rn(s, v[k2]);
                     }
+                    publish(segw + segslot, tag, s, false);
+                }
+                __syncwarp();  // every word of the warp is out before it waits
+                if (!mine && segslot != 0xffffffffu) s = wait_word(segw + segslot, tag, acq, ok);
+                sh.seg[tid] = s;
+            } else if (ntail) {
+                const uint32_t t = tid - CHUNK;
+                if (blockIdx.x >= vld(sh.nheads) && warp * 32u < (uint32_t)CHUNK + vld(sh.m)) {
+                    if (acq) asm volatile("fence.acq_rel.gpu;" ::: "memory");
+                    for (uint32_t j = t; j < vld(sh.m); j += CHUNK)
+                        publish(slots + (vld(sh.s0) - vld(sh.ah)) + j, tag, sh.part[j], false);
+                }
+                __syncwarp();
+                unsigned long long w[RAW_MAX / CHUNK];
 #pragma unroll
-                    for (int k2 = 0; k2 < LINE_BATCH; k2++) {
-                        if (dst[k2] != 0xffffffffu && ok) {
-                            if ((uint32_t)(w[k2] >> 32) != tag) {
-                                w[k2] = wait_tag(x + v0 + k2 * CG_THREADS, tag, st, acq, b.prm);
+                for (uint32_t k2 = 0; k2 < RAW_MAX / CHUNK; k2++)
+                    w[k2] = t + k2 * CHUNK < ntail ? ld_tag(slots + t + k2 * CHUNK, acq) : 0ull;
+#pragma unroll
+                for (uint32_t k2 = 0; k2 < RAW_MAX / CHUNK; k2++) {
+                    const uint32_t i = t + k2 * CHUNK;
+                    if (i >= ntail) continue;
+                    if ((uint32_t)(w[k2] >> 32) != tag && ok) {
+                        w[k2] = wait_tag(slots + i, tag, st, acq, &sh.limit);
+                        ok = (uint32_t)(w[k2] >> 32) == tag;
+                    }
+                    sh.raw[i] = __uint_as_float((uint32_t)w[k2]);
+                }
+            }
+            if (ntail) {  // the tails follow their heads, in order
+                __syncthreads();
+                if (tid < (uint32_t)CHUNK) {
+                    const uint32_t lo = sh.toff[tid], hi = sh.toff[tid + 1];
+                    if (lo != hi) {
+                        float s = sh.seg[tid];
+                        for (uint32_t e = lo; e < hi; e += 8) {
+                            float v[8];
+#pragma unroll
+                            for (int k2 = 0; k2 < 8; k2++) v[k2] = e + k2 < hi ? sh.raw[e + k2] : 0.0f;
+#pragma unroll
+                            for (int k2 = 0; k2 < 8; k2++) s = __fadd_rn(s, v[k2]);
+                        }
+                        sh.seg[tid] = s;
+                    }
+                }
+            }
+        } else {
+            if (warp < OWNER_WARPS) {
+                float* buf = sh.stage[warp];
+                for (uint32_t li = blockIdx.x + warp * nact; li < (uint32_t)CHUNK; li += OWNER_WARPS * nact) {
+                    const uint32_t lo = sh.off[li], hi = sh.off[li + 1];
+                    if (lo == hi) continue;
+                    float s = 0.0f;
+                    for (uint32_t e0 = lo; e0 < hi; e0 += 256u) {
+                        // all eight polls of a lane in flight, then the waits
+                        unsigned long long w[8];
+#pragma unroll
+                        for (int k2 = 0; k2 < 8; k2++) {
+                            const uint32_t e = e0 + lane + 32u * k2;
+                            w[k2] = e < hi ? ld_tag(slots + e, acq) : 0ull;
+                        }
+#pragma unroll
+                        for (int k2 = 0; k2 < 8; k2++) {
+                            const uint32_t e = e0 + lane + 32u * k2;
+                            if (e < hi && (uint32_t)(w[k2] >> 32) != tag && ok) {
+                                w[k2] = wait_tag(slots + e, tag, st, acq, &sh.limit);
                                 ok = (uint32_t)(w[k2] >> 32) == tag;
                             }
-                            sh.vals[vpos(dst[k2])] = __uint_as_float((uint32_t)w[k2]);
+                            buf[lane + 32u * k2] = e < hi ? __uint_as_float((uint32_t)w[k2]) : 0.0f;
                         }
+                        __syncwarp();
+                        if (lane == 0) {  // cg_reduce_final.wgsl:29-36: in plan order, from +0 (past the end: +0)
+                            const uint32_t n = hi - e0 < 256u ? hi - e0 : 256u;
+                            for (uint32_t j = 0; j < n; j += 8) {
+                                float t8[8];
+#pragma unroll
+                                for (int k2 = 0; k2 < 8; k2++) t8[k2] = buf[j + k2];
+#pragma unroll
+                                for (int k2 = 0; k2 < 8; k2++) s = __fadd_rn(s, t8[k2]);
+                            }
+                        }
+                        __syncwarp();
                     }
-                }
-            } else {
-                for (uint32_t i = tid; i < wn; i += CG_THREADS) sh.vals[vpos(i)] = b.part_rr[plan[w0 + i]];
-            }
-            if (__syncthreads_or(!ok)) return false;
-            if (tid < (uint32_t)CHUNK) {
-                // 16 loads first (past the segment's end: +0), then the
-                // sequential adds.  acc starts at +0 and a sum of floats is
-                // -0 only when both terms are, so acc is never -0 and adding
-                // +0 leaves it unchanged: the fold equals the loop over
-                // [lo, hi) exactly, with no per-lane tail loop.
-                const uint32_t lo = sh.off[tid] > w0 ? sh.off[tid] : w0;
-                const uint32_t hi = sh.off[tid + 1] < w0 + wn ? sh.off[tid + 1] : w0 + wn;
-                for (uint32_t e = lo; e < hi; e += 16) {
-                    float v[16];
-#pragma unroll
-                    for (int k2 = 0; k2 < 16; k2++) v[k2] = e + k2 < hi ? sh.vals[vpos(e - w0 + k2)] : 0.0f;
-#pragma unroll
-                    for (int k2 = 0; k2 < 16; k2++) acc = __fadd_rn(acc, v[k2]);
+                    // a segment whose partials did not all arrive is not published
+                    if (__all_sync(0xffffffffu, ok) && lane == 0) publish(segw + li, tag, s, acq);
                 }
             }
-            if (w0 + wn < A) __syncthreads();
+            if (tid < (uint32_t)CHUNK) sh.seg[tid] = segslot != 0xffffffffu ? wait_word(segw + tid, tag, acq, ok) : 0.0f;
         }
-        if (tid < (uint32_t)CHUNK) sh.seg[tid] = acc;
-        __syncthreads();
-        }
+        __syncwarp();
+        if (__syncthreads_or(!ok)) return false;
+        __syncwarp();
         if (warp == 0) {
-            const float v = chunk_tree(sh.seg, lane);
+            const float v = tree256(sh.seg, lane);
             if (lane == 0) post_f32(post, v);
         }
         __syncthreads();
-        out = sh.scal[0];
         sc = sh.scal[1];
         dn = sh.scal[2] != 0.0f;
         return true;
     };
-    // FL_CG_F64 scalar: the blocks' float-float partials (two words of block b
-    // at 16*b), summed by warp 0 in a fixed order (lanes stride over blocks,
-    // then a shuffle tree); lane 0 evaluates the post scalars (alpha, or beta
-    // and the stopping test, from rs_old) and broadcasts them with the sum.
+    // Extended forms: the blocks' partials (two words of block bb at 16*bb),
+    // summed by warp 0 in a fixed order (lanes stride over blocks, then a
+    // shuffle tree); lane 0 evaluates the post scalars.
     auto reduce_df = [&](const unsigned long long* words, uint32_t tag, bool acq, int post, float& sc,
                          bool& dn) -> bool {
-        const bool ok = stage_words(
-            2 * G, tag, acq, st, b.prm, sh.vals,
-            [&](uint32_t v) -> const unsigned long long* { return words + (v >> 1) * 16u + (v & 1u); },
-            [&](uint32_t v) -> uint32_t { return v; });
+        bool ok = true;
+        for (uint32_t v = tid; v < 2u * nact; v += CG_THREADS)
+            sh.words[v] = wait_word(words + (v >> 1) * 16u + (v & 1u), tag, acq, ok);
         if (__syncthreads_or(!ok)) return false;
         if (ieee && warp == 0) {  // the blocks' doubles, in the same fixed order
             double v = 0.0;
-            for (uint32_t bb = lane; bb < G; bb += 32) v += d_of(sh.vals[2 * bb], sh.vals[2 * bb + 1]);
+            for (uint32_t bb = lane; bb < nact; bb += 32) v += d_of(sh.words[2 * bb], sh.words[2 * bb + 1]);
             v = warp_sum_d(v);
             if (lane == 0) {
                 const double rs_old = sh.rs_d;
@@ -762,12 +898,12 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
                     d2 = stop_on && v <= sh.thr_d;
                     sh.rs_d = v;
                 }
-                sh.scal[2] = scv;
-                sh.scal[3] = d2 ? 1.0f : 0.0f;
+                sh.scal[1] = scv;
+                sh.scal[2] = d2 ? 1.0f : 0.0f;
             }
         } else if (warp == 0) {
             Df acc = {0.0f, 0.0f};
-            for (uint32_t bb = lane; bb < G; bb += 32) acc = df_add(acc, Df{sh.vals[2 * bb], sh.vals[2 * bb + 1]});
+            for (uint32_t bb = lane; bb < nact; bb += 32) acc = df_add(acc, Df{sh.words[2 * bb], sh.words[2 * bb + 1]});
             acc = warp_sum_df(acc);
             if (lane == 0) {
                 const Df rs_old = {sh.rs_hi, sh.rs_lo};
@@ -780,34 +916,29 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
                     sh.rs_hi = acc.hi;
                     sh.rs_lo = acc.lo;
                 }
-                sh.scal[0] = acc.hi;
-                sh.scal[1] = acc.lo;
-                sh.scal[2] = scv;
-                sh.scal[3] = d2 ? 1.0f : 0.0f;
+                sh.scal[1] = scv;
+                sh.scal[2] = d2 ? 1.0f : 0.0f;
             }
         }
         __syncthreads();
-        sc = sh.scal[2];
-        dn = sh.scal[3] != 0.0f;
+        sc = sh.scal[1];
+        dn = sh.scal[2] != 0.0f;
         return true;
     };
     // Block partial published as two tagged words on the block's line: the
-    // float-float {hi, lo}, or a double's low and high 32 bits.
+    // float-float {hi, lo}, or a double's low and high 32 bits (lanes 0 and 1
+    // store in one instruction, so a reader finds both).
     auto publish_df = [&](Acc acc, unsigned long long* words, uint32_t tag, bool rel) {
         if constexpr (ieee) {
             // The FP64 pipe (about 2 lane-operations per clock per SM) is the
-            // bound: warp 0 sums the 1024 thread partials (lane l: partials l,
+            // bound: warp 0 sums the thread partials (lane l: partials l,
             // l + 32, ... in sequence, then a 5-level tree) instead of a tree
-            // in every warp (36 double adds per block instead of 160).  The
-            // partials are staged in the chunk-tree buffer, which the
-            // extended-precision forms do not use (the exchange window is
-            // written by the other warps' polls while warp 0 reads).
-            double* part = reinterpret_cast<double*>(&sh.tree[0][0]);
-            part[tid] = acc;
+            // in every warp.
+            sh.dpart[tid] = acc;
             __syncthreads();
             if (warp == 0) {
                 double s = 0.0;
-                for (uint32_t t2 = lane; t2 < (uint32_t)CG_THREADS; t2 += 32) s += part[t2];
+                for (uint32_t t2 = lane; t2 < (uint32_t)CG_THREADS; t2 += 32) s += sh.dpart[t2];
                 const double v = warp_sum_d(s);
                 const float lo = __shfl_sync(0xffffffffu, d_lo(v), 0), hi = __shfl_sync(0xffffffffu, d_hi(v), 0);
                 if (lane < 2) publish(words + 16 * blockIdx.x + lane, tag, lane ? hi : lo, rel);
@@ -820,445 +951,407 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
             }
             __syncthreads();
             if (warp == 0) {
-                Df v = {sh.red[2 * lane], sh.red[2 * lane + 1]};
+                Df v = {0.0f, 0.0f};
+                if (lane < CG_WARPS) v = {sh.red[2 * lane], sh.red[2 * lane + 1]};
                 v = warp_sum_df(v);
-                // lanes 0 and 1 store {hi, lo} in one instruction (the FP64-reduction
-                // CG stage measured 1.96-1.98 vs 2.10-2.13 ms per substep at 128^3
-                // against two stores by lane 0: readers saw hi before lo)
                 const float lo = __shfl_sync(0xffffffffu, v.lo, 0);
                 if (lane < 2) publish(words + 16 * blockIdx.x + lane, tag, lane ? lo : v.hi, rel);
             }
         }
     };
-    // Warp w evaluates the trees of chunks j0 + w and j0 + w + 32 of the pass
-    // into shared memory (sh.red, KT floats); warp 0 then publishes them
-    // together, one store instruction per 32 words, so a polling block finds
-    // a block's slot line complete in one read instead of filling in word by
-    // word (the CG stage measured 2.06 vs 2.21-2.26 ms per substep at 128^3
-    // against one store per tree warp).
-    // With `rel`, warp 0 issues the release fence (after the barrier that
-    // orders the block's vector writes before it) while warps 1.. evaluate the
-    // trees, and then stores the words relaxed: fence + strong store in one
-    // thread is a release pattern, and the fence's wait for the block's
-    // stores overlaps the trees (1-2 % of the CG stage at 128^3 against a
-    // release store after the trees).
-    static_assert(2 * CG_WARPS == KT, "sh.red stages one pass of chunk trees");
-    // With `zero` (passes that share the tree rows), the tree warps clear
-    // the rows they read, so the next pass starts on zeroed rows without a
-    // clearing loop and barrier of its own; the next pass's first barrier
-    // orders this pass's publication before its trees rewrite sh.red.
-    auto publish_trees = [&](uint32_t j0, uint32_t nb, unsigned long long* slots, uint32_t tag, bool rel, bool zero) {
-        __syncthreads();
-        if (rel && warp == 0) {
-            asm volatile("fence.acq_rel.gpu;" ::: "memory");
-        } else {
-            const uint32_t w0 = rel ? warp - 1 : warp, nw = rel ? CG_WARPS - 1 : CG_WARPS;
-            for (uint32_t j = w0; j < nb; j += nw) {
-                const float v = chunk_tree(sh.tree[j], lane);
-                if (lane == 0) sh.red[j] = v;
-                if (zero) {
-                    __syncwarp();
-                    float4* row = reinterpret_cast<float4*>(sh.tree[j]);
-                    row[lane] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    row[lane + 32] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                }
-            }
-        }
-        __syncthreads();
-        if (warp == 0)
-            for (uint32_t j = lane; j < nb; j += 32) publish(slots + sh.spos[blockIdx.x] + j0 + j, tag, sh.red[j], false);
-    };
 
-    // Initial residual norm (cg_init.wgsl + cg_reduce of r.r).
+    // ---- initial residual norm (cg_init.wgsl + cg_reduce of r.r), from the
+    // per-chunk partials of all chunks (zero where a chunk holds no liquid)
     float rs_init_f = 0.0f;
     Df rs_init_d = {0.0f, 0.0f};
     if (ieee) {  // the chunks' float-float partials (exact in double), summed in double
         double acc = 0.0;
-        for (uint32_t e = tid; e < A; e += CG_THREADS) {
-            const float2 v = b.chunk_rr_df[plan[e]];
+        for (uint32_t c = tid; c < nchunks; c += CG_THREADS) {
+            const float2 v = b.chunk_rr_df[c];
             acc += (double)v.x + (double)v.y;
         }
-        acc = warp_allsum_d(acc);
-        if (lane == 0) {
-            sh.red[2 * warp] = d_lo(acc);
-            sh.red[2 * warp + 1] = d_hi(acc);
-        }
+        sh.dpart[tid] = acc;
         __syncthreads();
-        const double rs0 = warp_allsum_d(d_of(sh.red[2 * lane], sh.red[2 * lane + 1]));
-        if (tid == 0) {
-            sh.rs_d = rs0;
-            sh.thr_d = P.thr_abs ? P.thr_abs_d : tol_sq_d * rs0;
-            if (blockIdx.x == 0) st->rs_init = rs0;
+        if (warp == 0) {
+            double s = 0.0;
+            for (uint32_t t2 = lane; t2 < (uint32_t)CG_THREADS; t2 += 32) s += sh.dpart[t2];
+            s = warp_sum_d(s);
+            if (lane == 0) {
+                sh.rs_d = s;
+                sh.thr_d = P.thr_abs ? P.thr_abs_d : P.tol_sq_d * s;
+                if (blockIdx.x == 0) st->rs_init = s;
+            }
         }
-        __syncthreads();  // sh.red is reused
     } else if (f64) {
         Df acc = {0.0f, 0.0f};
-        for (uint32_t e = tid; e < A; e += CG_THREADS) {
-            const float2 v = b.chunk_rr_df[plan[e]];
+        for (uint32_t c = tid; c < nchunks; c += CG_THREADS) {
+            const float2 v = b.chunk_rr_df[c];
             acc = df_add(acc, Df{v.x, v.y});
         }
-        acc = warp_allsum_df(acc);
+        acc = warp_sum_df(acc);
         if (lane == 0) {
             sh.red[2 * warp] = acc.hi;
             sh.red[2 * warp + 1] = acc.lo;
         }
         __syncthreads();
-        rs_init_d = warp_allsum_df(Df{sh.red[2 * lane], sh.red[2 * lane + 1]});
-        // stopping threshold tol^2 * rs_init (or the absolute one), once per solve
-        if (tid == 0) {
-            sh.rs_hi = rs_init_d.hi;
-            sh.rs_lo = rs_init_d.lo;
-            const double thr = P.thr_abs ? P.thr_abs_d : tol_sq_d * df_to_double(rs_init_d);
-            sh.thr_dh = (float)thr;
-            sh.thr_dl = (float)(thr - (double)sh.thr_dh);
+        if (warp == 0) {
+            Df v = {0.0f, 0.0f};
+            if (lane < CG_WARPS) v = {sh.red[2 * lane], sh.red[2 * lane + 1]};
+            rs_init_d = warp_sum_df(v);
+            // stopping threshold tol^2 * rs_init (or the absolute one), once per solve
+            if (lane == 0) {
+                sh.rs_hi = rs_init_d.hi;
+                sh.rs_lo = rs_init_d.lo;
+                const double thr = P.thr_abs ? P.thr_abs_d : P.tol_sq_d * df_to_double(rs_init_d);
+                sh.thr_dh = (float)thr;
+                sh.thr_dl = (float)(thr - (double)sh.thr_dh);
+                if (blockIdx.x == 0) st->rs_init = df_to_double(rs_init_d);
+            }
         }
-        __syncthreads();  // sh.red is reused
     } else {
-        float sc0;
-        bool dn0;
-        reduce_f32(nullptr, nullptr, 0u, false, 0, rs_init_f, sc0, dn0);  // also sets sh.rs_hi
-    }
-    // Thresholds and rs_init are stored once here, not held in registers
-    // through the loop.  f32: tol^2 * rs_init (cg_beta.wgsl:25-30) or the
-    // absolute threshold.
-    if (tid == 0) {
-        if (!f64) sh.thr_f = P.thr_abs ? P.thr_abs_f : __fmul_rn(tol_sq, rs_init_f);
-        if (blockIdx.x == 0 && !ieee) st->rs_init = f64 ? df_to_double(rs_init_d) : (double)rs_init_f;
+        // thread li of cg_reduce_final.wgsl: partials li, li + 256, ... in order
+        if (tid < (uint32_t)CHUNK) {
+            float s = 0.0f;
+            for (uint32_t c = tid; c < nchunks; c += 16 * CHUNK) {
+                float v[16];
+#pragma unroll
+                for (int k2 = 0; k2 < 16; k2++) v[k2] = c + k2 * CHUNK < nchunks ? b.part_rr[c + k2 * CHUNK] : 0.0f;
+#pragma unroll
+                for (int k2 = 0; k2 < 16; k2++) s = __fadd_rn(s, v[k2]);
+            }
+            sh.seg[tid] = s;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            rs_init_f = tree256(sh.seg, lane);
+            // f32 threshold: tol^2 * rs_init (cg_beta.wgsl:25-30) or the absolute one
+            if (lane == 0) {
+                sh.rs_hi = rs_init_f;
+                sh.thr_f = P.thr_abs ? P.thr_abs_f : __fmul_rn(P.tol_sq, rs_init_f);
+                if (blockIdx.x == 0) st->rs_init = (double)rs_init_f;
+            }
+        }
     }
     __syncthreads();
 
-    float beta = 0.0f;
-    uint32_t k = 0, tag = tag_base;
-    for (uint32_t it = 0; it < iters; it++) {
-        float* __restrict__ d_cur = (it & 1u) ? b.dB : b.dA;
-        const float* __restrict__ d_prev = (it & 1u) ? b.dA : b.dB;
-        const bool first = it == 0;
-        const float* __restrict__ d_src = first ? d_cur : d_prev;
-        // ---------------- phase 1: direction + SpMV + d.q ----------------
-        Acc acc{};
-        tag++;
-        if (vld(sh.u_res)) {  // resident operands: own d, r from shared memory, neighbours' from global
-            uint32_t ent[2], cc[2];
-            float rv[2][7], dv[2][7];
-#pragma unroll
-            for (int u = 0; u < 2; u++) {
-                const uint32_t tu = tid + u * CG_THREADS;
-                const bool ok = tu < vld(sh.u_ncell);
-                ent[u] = ok ? sh.cell[tu] : 0u;
-                cc[u] = sh.chunk[ent[u] >> 18] * CHUNK + ((ent[u] >> 10) & 255u);
-                const uint32_t c = cc[u];
-                const float2 own = ok ? *reinterpret_cast<const float2*>(&rv4[tu]) : make_float2(0.0f, 0.0f);
-                dv[u][0] = own.x;
-                rv[u][0] = own.y;
-                const uint32_t nb6[6] = {c - 1, c + 1, c - nx, c + nx, c - nxy, c + nxy};
-#pragma unroll
-                for (int s = 1; s < 7; s++) {
-                    const bool need = ok && ((ent[u] >> s) & 1u);
-                    dv[u][s] = need ? d_src[nb6[s - 1]] : 0.0f;
-                    rv[u][s] = (need && !first) ? r[nb6[s - 1]] : 0.0f;
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < 2; u++) {
-                const uint32_t tu = tid + u * CG_THREADS;
-                if (tu >= vld(sh.u_ncell)) continue;
-                const uint32_t info = ent[u];
-                const float dc = first ? dv[u][0] : __fadd_rn(rv[u][0], __fmul_rn(beta, dv[u][0]));  // cg_dir.wgsl:30
-                float sum = 0.0f;
-#pragma unroll
-                for (int s = 1; s < 7; s++) {
-                    if ((info >> s) & 1u) {
-                        const float dn = first ? dv[u][s] : __fadd_rn(rv[u][s], __fmul_rn(beta, dv[u][s]));
-                        sum = __fadd_rn(sum, dn);
-                    }
-                }
-                const float qc = __fsub_rn(__fmul_rn((float)((info >> 7) & 7u), dc), sum);  // cg_spmv.wgsl:46-68
-                if (!first) d_cur[cc[u]] = dc;
-                rv4[tu].x = dc;
-                rv4[tu].z = qc;
-                if (f64) acc_add(acc, dc, qc);
-                else sh.tree[info >> 18][(info >> 10) & 255u] = __fmul_rn(dc, qc);
-            }
-            if (!f64) publish_trees(0, vld(sh.u_mc), slotA, tag, false, false);
-        } else {
-            uint32_t j0 = 0;
-            for (uint32_t ps = 0; ps < vld(sh.u_npc); ps++, j0 += KT) {
-                const uint32_t nb = vld(sh.u_mc) - j0 < KT ? vld(sh.u_mc) - j0 : KT;
-                const uint32_t beg = sh.pass_off[ps], end = sh.pass_off[ps + 1];
-                if (vld(sh.u_quad)) {
-                    for (uint32_t t = beg + tid; t < end; t += CG_THREADS) {
-                        // One quad: cells c0..c0+3 of one row.  Its own d, r and
-                        // its +-y, +-z rows as float4, the two x edges as scalars;
-                        // the -x/+x neighbours inside the quad are its own cells.
-                        const uint2 e = qlist[t];
-                        const uint32_t w[4] = {e.x & 1023u, (e.x >> 10) & 1023u, (e.x >> 20) & 1023u, e.y & 1023u};
-                        const uint32_t jq = e.y >> 16, qd = (e.y >> 10) & 63u;
-                        const uint32_t c0 = sh.chunk[jq] * CHUNK + 4u * qd;
-                        const uint32_t any = w[0] | w[1] | w[2] | w[3];
-                        const float4 z4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                        const float4 dc4 = ld_f4(d_src + c0);
-                        const float4 rc4 = first ? z4 : ld_f4(r + c0);
-                        const bool xm = (w[0] & 2u) != 0u, xp = (w[3] & 4u) != 0u;
-                        const float dxm = xm ? d_src[c0 - 1] : 0.0f, rxm = (xm && !first) ? r[c0 - 1] : 0.0f;
-                        const float dxp = xp ? d_src[c0 + 4] : 0.0f, rxp = (xp && !first) ? r[c0 + 4] : 0.0f;
-                        float4 dn4[4], rn4[4];  // -y, +y, -z, +z rows
-                        const uint32_t off4[4] = {c0 - nx, c0 + nx, c0 - nxy, c0 + nxy};
-#pragma unroll
-                        for (int s = 0; s < 4; s++) {
-                            const bool need = (any >> (3 + s)) & 1u;
-                            dn4[s] = need ? ld_f4(d_src + off4[s]) : z4;
-                            rn4[s] = (need && !first) ? ld_f4(r + off4[s]) : z4;
-                        }
-                        // cg_dir.wgsl:30 for the quad, the edges and the rows,
-                        // then cg_spmv.wgsl:46-68 per cell (order -x,+x,-y,+y,-z,+z)
-                        auto dir = [&](float dv, float rv) { return first ? dv : __fadd_rn(rv, __fmul_rn(beta, dv)); };
-                        const float dq[4] = {dir(dc4.x, rc4.x), dir(dc4.y, rc4.y), dir(dc4.z, rc4.z), dir(dc4.w, rc4.w)};
-                        const float dm = dir(dxm, rxm), dp = dir(dxp, rxp);
-                        float ov[4], oq[4], op[4];
-#pragma unroll
-                        for (int k = 0; k < 4; k++) {
-                            const uint32_t wk = w[k];
-                            float sum = 0.0f;
-                            if (wk & 2u) sum = __fadd_rn(sum, k == 0 ? dm : dq[k > 0 ? k - 1 : 0]);
-                            if (wk & 4u) sum = __fadd_rn(sum, k == 3 ? dp : dq[k < 3 ? k + 1 : 3]);
-#pragma unroll
-                            for (int s = 0; s < 4; s++)
-                                if ((wk >> (3 + s)) & 1u) sum = __fadd_rn(sum, dir(f4_at(dn4[s], k), f4_at(rn4[s], k)));
-                            const bool liq = (wk & 1u) != 0u;
-                            const float qc = __fsub_rn(__fmul_rn((float)((wk >> 7) & 7u), dq[k]), sum);
-                            ov[k] = liq ? dq[k] : 0.0f;
-                            oq[k] = liq ? qc : 0.0f;
-                            op[k] = liq ? __fmul_rn(dq[k], qc) : 0.0f;
-                            if (f64 && liq) acc_add(acc, dq[k], qc);
-                        }
-                        if (!first) st_f4(d_cur + c0, make_float4(ov[0], ov[1], ov[2], ov[3]));
-                        st_f4(q + c0, make_float4(oq[0], oq[1], oq[2], oq[3]));
-                        if (!f64) *reinterpret_cast<float4*>(&sh.tree[jq - j0][4u * qd]) = make_float4(op[0], op[1], op[2], op[3]);
-                    }
-                } else
-                for (uint32_t t = beg + tid; t < end; t += 2 * CG_THREADS) {
-                    // two cells in flight: all loads first
-                    uint32_t ent[2], cc[2];
-                    float rv[2][7], dv[2][7];
-#pragma unroll
-                    for (int u = 0; u < 2; u++) {
-                        const uint32_t tu = t + u * CG_THREADS;
-                        const bool ok = tu < end;
-                        ent[u] = ok ? sh.cell[tu] : 0u;
-                        cc[u] = sh.chunk[ent[u] >> 18] * CHUNK + ((ent[u] >> 10) & 255u);
-                        const uint32_t c = cc[u];
-                        const uint32_t nb7[7] = {c, c - 1, c + 1, c - nx, c + nx, c - nxy, c + nxy};
-#pragma unroll
-                        for (int s = 0; s < 7; s++) {
-                            const bool need = ok && (s == 0 || ((ent[u] >> s) & 1u));
-                            dv[u][s] = need ? d_src[nb7[s]] : 0.0f;
-                            rv[u][s] = (need && !first) ? r[nb7[s]] : 0.0f;
-                        }
-                    }
-#pragma unroll
-                    for (int u = 0; u < 2; u++) {
-                        if (t + u * CG_THREADS >= end) continue;
-                        const uint32_t info = ent[u];
-                        // cg_dir.wgsl:30 for the cell and its liquid neighbours,
-                        // then cg_spmv.wgsl:46-68 (order -x,+x,-y,+y,-z,+z)
-                        const float dc = first ? dv[u][0] : __fadd_rn(rv[u][0], __fmul_rn(beta, dv[u][0]));
-                        float sum = 0.0f;
-#pragma unroll
-                        for (int s = 1; s < 7; s++) {
-                            if ((info >> s) & 1u) {
-                                const float dn = first ? dv[u][s] : __fadd_rn(rv[u][s], __fmul_rn(beta, dv[u][s]));
-                                sum = __fadd_rn(sum, dn);
-                            }
-                        }
-                        const float cnt = (float)((info >> 7) & 7u);
-                        const float qc = __fsub_rn(__fmul_rn(cnt, dc), sum);
-                        const uint32_t c = cc[u];
-                        if (!first) d_cur[c] = dc;
-                        q[c] = qc;
-                        if (f64) acc_add(acc, dc, qc);
-                        else sh.tree[(info >> 18) - j0][(info >> 10) & 255u] = __fmul_rn(dc, qc);
-                    }
-                }
-                if (!f64) publish_trees(j0, nb, slotA, tag, false, multi);
-            }
-            for (j0 = vld(sh.u_mc); j0 < vld(sh.u_m); j0 += KT) {  // chunks beyond the list: one cell slot per thread
-                const uint32_t nb = vld(sh.u_m) - j0 < KT ? vld(sh.u_m) - j0 : KT;
-                for (uint32_t t = tid; t < nb * CHUNK; t += CG_THREADS) {
-                    const uint32_t j = j0 + t / CHUNK, cl = t & (CHUNK - 1);
-                    const uint32_t chunk = j < KCH ? sh.chunk[j] : plan[vld(sh.u_s0) + j];
-                    const uint32_t c = chunk * CHUNK + cl;
-                    const uint32_t info = c < C ? cinfo[c] : 0u;
-                    float prod = 0.0f;
-                    if (info & 1u) {
-                        const uint32_t nb7[7] = {c, c - 1, c + 1, c - nx, c + nx, c - nxy, c + nxy};
-                        float dc = 0.0f, sum = 0.0f;
-#pragma unroll
-                        for (int s = 0; s < 7; s++) {
-                            if (s == 0 || ((info >> s) & 1u)) {
-                                const float dn = first ? d_src[nb7[s]]
-                                                       : __fadd_rn(r[nb7[s]], __fmul_rn(beta, d_src[nb7[s]]));
-                                if (s == 0) dc = dn;
-                                else sum = __fadd_rn(sum, dn);
-                            }
-                        }
-                        const float qc = __fsub_rn(__fmul_rn((float)((info >> 7) & 7u), dc), sum);
-                        if (!first) d_cur[c] = dc;
-                        q[c] = qc;
-                        if (f64) acc_add(acc, dc, qc);
-                        prod = __fmul_rn(dc, qc);
-                    }
-                    if (!f64) sh.tree[t / CHUNK][cl] = prod;
-                }
-                if (!f64) {
-                    publish_trees(j0, nb, slotA, tag, false, true);  // clears its rows for the next phase's passes
-                    __syncthreads();
-                }
-            }
+    // Shared by both loops: the rows of a quad's neighbours, the sum over its x
+    // neighbours (within the quad, the lanes beside, left0 / right31 at the ends
+    // of the warp), and the products of a half in the extended forms.
+    auto row = [&](const float* a, uint32_t c, uint32_t e) -> Quad {
+        if (VEC) return ld_quad(a + c);
+        const float* const at = a + (int)c;  // below the array while a later component is inside
+        return quad((e & 1u) ? at[0] : 0.0f, (e & 2u) ? at[CSTEP] : 0.0f, (e & 4u) ? at[2 * CSTEP] : 0.0f,
+                    (e & 8u) ? at[3 * CSTEP] : 0.0f);
+    };
+    auto xsum = [&](Quad dq, float left0, float right31) -> Quad {
+        const float d0 = lo2(dq.a), d1 = hi2(dq.a), d2 = lo2(dq.b), d3 = hi2(dq.b);
+        if (VEC) {
+            const float ls = __shfl_up_sync(0xffffffffu, d3, 1), rs = __shfl_down_sync(0xffffffffu, d0, 1);
+            const float left = lane == 0 ? left0 : ls, right = lane == 31 ? right31 : rs;
+            return quad(__fadd_rn(__fadd_rn(0.0f, left), d1), __fadd_rn(__fadd_rn(0.0f, d0), d2),
+                        __fadd_rn(__fadd_rn(0.0f, d1), d3), __fadd_rn(__fadd_rn(0.0f, d2), right));
         }
-        float alpha;
-        {
-            bool dn_unused;
-            if (f64) {
-                publish_df(acc, wordA, tag, false);
-                if (!reduce_df(wordA, tag, false, 1, alpha, dn_unused)) return;
-            } else {
-                float dq;
-                if (!reduce_f32(slotA, segA, tag, false, 1, dq, alpha, dn_unused)) return;
-            }
+        const float v[4] = {d0, d1, d2, d3};
+        float u[4], d[4], s[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            u[k] = __shfl_sync(0xffffffffu, v[k], (lane + 31u) & 31u);
+            d[k] = __shfl_sync(0xffffffffu, v[k], (lane + 1u) & 31u);
         }
-        // ---------------- phase 2: update + r.r ----------------
-        acc = Acc{};
-        tag++;
-        if (vld(sh.u_res)) {  // every operand in shared memory; r also to global for the neighbours
 #pragma unroll
-            for (int u = 0; u < 2; u++) {
-                const uint32_t tu = tid + u * CG_THREADS;
-                if (tu >= vld(sh.u_ncell)) continue;
-                const uint32_t e = sh.cell[tu];
-                const float4 o = rv4[tu];
-                const float pn = __fadd_rn(o.w, __fmul_rn(alpha, o.x));  // cg_update.wgsl:33
-                const float rc = __fsub_rn(o.y, __fmul_rn(alpha, o.z));  // cg_update.wgsl:34
-                r[sh.chunk[e >> 18] * CHUNK + ((e >> 10) & 255u)] = rc;
-                rv4[tu].y = rc;
-                rv4[tu].w = pn;
-                if (f64) acc_add(acc, rc, rc);
-                else sh.tree[e >> 18][(e >> 10) & 255u] = __fmul_rn(rc, rc);
-            }
-            if (!f64) publish_trees(0, vld(sh.u_mc), slotB, tag, true, false);
-        } else {
-            uint32_t j0 = 0;
-            for (uint32_t ps = 0; ps < vld(sh.u_npc); ps++, j0 += KT) {
-                const uint32_t nb = vld(sh.u_mc) - j0 < KT ? vld(sh.u_mc) - j0 : KT;
-                const uint32_t beg = sh.pass_off[ps], end = sh.pass_off[ps + 1];
-                if (vld(sh.u_quad)) {
-                    for (uint32_t t = beg + tid; t < end; t += CG_THREADS) {
-                        // cg_update.wgsl:33-34 for the quad's liquid cells; the
-                        // others keep their p and r (written back unchanged)
-                        const uint2 e = qlist[t];
-                        const uint32_t w[4] = {e.x & 1u, (e.x >> 10) & 1u, (e.x >> 20) & 1u, e.y & 1u};
-                        const uint32_t jq = e.y >> 16, qd = (e.y >> 10) & 63u;
-                        const uint32_t c0 = sh.chunk[jq] * CHUNK + 4u * qd;
-                        float4 p4 = ld_f4(p + c0), r4 = ld_f4(r + c0);
-                        const float4 d4 = ld_f4(d_cur + c0), q4 = ld_f4(q + c0);
-                        float op[4];
-#pragma unroll
-                        for (int k = 0; k < 4; k++) {
-                            const float pn = __fadd_rn(f4_at(p4, k), __fmul_rn(alpha, f4_at(d4, k)));
-                            const float rc = __fsub_rn(f4_at(r4, k), __fmul_rn(alpha, f4_at(q4, k)));
-                            const bool liq = w[k] != 0u;
-                            if (liq) {
-                                f4_set(p4, k, pn);
-                                f4_set(r4, k, rc);
-                            }
-                            op[k] = liq ? __fmul_rn(rc, rc) : 0.0f;
-                            if (f64 && liq) acc_add(acc, rc, rc);
-                        }
-                        st_f4(p + c0, p4);
-                        st_f4(r + c0, r4);
-                        if (!f64) *reinterpret_cast<float4*>(&sh.tree[jq - j0][4u * qd]) = make_float4(op[0], op[1], op[2], op[3]);
-                    }
-                } else
-                for (uint32_t t = beg + tid; t < end; t += 2 * CG_THREADS) {
-                    uint32_t ent[2], cc[2];
-                    float pv[2], dv[2], rv[2], qv[2];
-#pragma unroll
-                    for (int u = 0; u < 2; u++) {
-                        const uint32_t tu = t + u * CG_THREADS;
-                        const bool ok = tu < end;
-                        ent[u] = ok ? sh.cell[tu] : 0u;
-                        cc[u] = sh.chunk[ent[u] >> 18] * CHUNK + ((ent[u] >> 10) & 255u);
-                        pv[u] = ok ? p[cc[u]] : 0.0f;
-                        dv[u] = ok ? d_cur[cc[u]] : 0.0f;
-                        rv[u] = ok ? r[cc[u]] : 0.0f;
-                        qv[u] = ok ? q[cc[u]] : 0.0f;
-                    }
-#pragma unroll
-                    for (int u = 0; u < 2; u++) {
-                        if (t + u * CG_THREADS >= end) continue;
-                        const uint32_t c = cc[u];
-                        p[c] = __fadd_rn(pv[u], __fmul_rn(alpha, dv[u]));       // cg_update.wgsl:33
-                        const float rc = __fsub_rn(rv[u], __fmul_rn(alpha, qv[u]));  // cg_update.wgsl:34
-                        r[c] = rc;
-                        if (f64) acc_add(acc, rc, rc);
-                        else sh.tree[(ent[u] >> 18) - j0][(ent[u] >> 10) & 255u] = __fmul_rn(rc, rc);
-                    }
-                }
-                if (!f64) publish_trees(j0, nb, slotB, tag, true, multi);
-            }
-            for (j0 = vld(sh.u_mc); j0 < vld(sh.u_m); j0 += KT) {
-                const uint32_t nb = vld(sh.u_m) - j0 < KT ? vld(sh.u_m) - j0 : KT;
-                for (uint32_t t = tid; t < nb * CHUNK; t += CG_THREADS) {
-                    const uint32_t j = j0 + t / CHUNK, cl = t & (CHUNK - 1);
-                    const uint32_t chunk = j < KCH ? sh.chunk[j] : plan[vld(sh.u_s0) + j];
-                    const uint32_t c = chunk * CHUNK + cl;
-                    const uint32_t info = c < C ? cinfo[c] : 0u;
-                    float prod = 0.0f;
-                    if (info & 1u) {
-                        p[c] = __fadd_rn(p[c], __fmul_rn(alpha, d_cur[c]));
-                        const float rc = __fsub_rn(r[c], __fmul_rn(alpha, q[c]));
-                        r[c] = rc;
-                        if (f64) acc_add(acc, rc, rc);
-                        prod = __fmul_rn(rc, rc);
-                    }
-                    if (!f64) sh.tree[t / CHUNK][cl] = prod;
-                }
-                if (!f64) {
-                    publish_trees(j0, nb, slotB, tag, true, true);  // clears its rows for the next phase's passes
-                    __syncthreads();
-                }
-            }
-        }
-        k = it + 1;
-        bool done;
+        for (int k = 0; k < 4; k++)
+            s[k] = __fadd_rn(__fadd_rn(0.0f, lane ? u[k] : k ? u[k ? k - 1 : 0] : left0),
+                             lane != 31 ? d[k] : k < 3 ? d[k < 3 ? k + 1 : 3] : right31);
+        return quad(s[0], s[1], s[2], s[3]);
+    };
+    // The cell before the chunk (lane 0) or after it (lane 31), if a liquid
+    // cell's neighbour.
+    auto edge = [&](uint32_t c0, uint32_t e0, uint32_t c1, uint32_t e1) -> uint32_t {
+        return lane == 0 && (e0 & 1u) ? c0 - 1u : lane == 31 && (e1 & 8u) ? c1 + 3u * CSTEP + 1u : 0u;
+    };
+    auto acc_quad = [&](Acc& a, Quad x, Quad y) {
+        acc_add(a, lo2(x.a), lo2(y.a));
+        acc_add(a, hi2(x.a), hi2(y.a));
+        acc_add(a, lo2(x.b), lo2(y.b));
+        acc_add(a, hi2(x.b), hi2(y.b));
+    };
+    // The exchange after a phase: post 1 alpha, post 2 beta and the stopping test.
+    auto exchange = [&](Acc (&acc)[2], uint32_t tag, int post, float& sc, bool& dn) -> bool {
         if (f64) {
-            publish_df(acc, wordB, tag, true);
-            if (!reduce_df(wordB, tag, true, 2, beta, done)) return;
-        } else {
-            float rs_new;
-            if (!reduce_f32(slotB, segB, tag, true, 2, rs_new, beta, done)) return;
+            if constexpr (ieee) acc[0] += acc[1];
+            else acc[0] = df_add(acc[0], acc[1]);
+            unsigned long long* const w = vld(sh.area[post == 1 ? WORD_A : WORD_B]);
+            publish_df(acc[0], w, tag, post == 2);
+            return reduce_df(w, tag, post == 2, post, sc, dn);
         }
-        if (done) break;
+        return reduce_f32(vld(sh.area[post == 1 ? SLOT_A : SLOT_B]), vld(sh.area[post == 1 ? SEG_A : SEG_B]), tag, post == 2,
+                          post, sc, dn);
+    };
+
+    float beta = 0.0f;  // the first direction is r + 0 * r
+    uint32_t k = 0, tag = tag_base;
+    if (regs) {
+        // One chunk per warp.  A lane keeps its two quads' d, r and stencil words
+        // in registers; p, q and the d of the y and z neighbours in shared
+        // memory (the latter are advanced here as their owners advance them, so
+        // only the neighbours' r is loaded, both halves' rows in flight).
+        const bool mine = warp < m;
+        uint32_t c[2], e[2];
+        Quad dq[2], r4[2];
+        Quad* const pool = reinterpret_cast<Quad*>(sh.pool) + (warp * 2u * 6u) * 32u + lane;  // [half][p, 4 rows, q][lane]
+        {
+            const uint32_t id = mine ? plan[warp] : 0u;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const uint32_t c0 = id * CHUNK + h * (CHUNK / 2) + LSTEP * lane;
+                e[h] = mine ? load_info(c0) : 0u;
+                c[h] = (e[h] & 15u) ? c0 : safe;
+                dq[h] = z4;  // beta is 0 in the first direction
+                r4[h] = ld_q(r, c[h], e[h]);
+                pool[(h * 6) * 32] = ld_q(p, c[h], e[h]);
+                for (int t = 1; t < 6; t++) pool[(h * 6 + t) * 32] = z4;
+            }
+        }
+        const bool any0 = __any_sync(0xffffffffu, (e[0] & 15u) != 0u), any1 = __any_sync(0xffffffffu, (e[1] & 15u) != 0u);
+        float de = 0.0f;  // lane 0: d of the cell before the chunk, lane 31: of the one after
+#pragma unroll 1
+        for (uint32_t it = 0; it < iters; it++) {
+            // ---------------- phase 1: direction + SpMV + d.q ----------------
+            // No branches per lane: d and r are zero in every cell that is not
+            // liquid, and a zero term leaves a sum that starts at +0 unchanged.
+            Acc acc[2] = {};
+            if (mine) {
+                Quad nr[2][4];  // -y, +y, -z, +z
+                auto load = [&](int h) {
+                    nr[h][0] = row(r, c[h] - nx, e[h]);
+                    nr[h][1] = row(r, c[h] + nx, e[h]);
+                    nr[h][2] = row(r, c[h] - nxy, e[h]);
+                    nr[h][3] = row(r, c[h] + nxy, e[h]);
+                };
+                if (any0) load(0);
+                if (any1) load(1);
+                const float re = r[edge(c[0], e[0], c[1], e[1])];
+                const Quad beta4 = qall(beta);
+                auto dir = [&](Quad dv, Quad rv) { return qaddp(qmul(beta4, dv), one, rv); };  // cg_dir.wgsl:30
+                dq[0] = dir(dq[0], r4[0]);
+                dq[1] = dir(dq[1], r4[1]);
+                float* const d_cur = (it & 1u) ? b.dB : b.dA;
+                st_q(d_cur, c[0], e[0], dq[0]);  // for blocks of the other form
+                st_q(d_cur, c[1], e[1], dq[1]);
+                const float b0 = __shfl_sync(0xffffffffu, hi2(dq[0].b), 31), b1 = __shfl_sync(0xffffffffu, lo2(dq[1].a), 0);
+                Quad prod[2] = {z4, z4};
+                de = __fadd_rn(re, __fmul_rn(beta, de));
+                auto stencil = [&](int h, float left0, float right31) {  // cg_spmv.wgsl:46-68, order -x,+x,-y,+y,-z,+z
+                    Quad sum = xsum(dq[h], left0, right31);
+#pragma unroll
+                    for (int t = 0; t < 4; t++) {
+                        Quad& d = pool[(h * 6 + 1 + t) * 32];
+                        d = dir(d, nr[h][t]);
+                        sum = qadd(sum, d);
+                    }
+                    const Quad q4 = liquid(qsubp(sum, one, qmul(counts(e[h]), dq[h])), e[h]);
+                    pool[(h * 6 + 5) * 32] = q4;
+                    if (f64) acc_quad(acc[h], dq[h], q4);
+                    else prod[h] = qmul(dq[h], q4);
+                };
+                if (any0) stencil(0, de, b1);
+                if (any1) stencil(1, b0, de);
+                if (!f64) {
+                    const float v = tree256_quads<VEC>(prod[0], prod[1], one, lane);
+                    if (lane == 0) sh.part[warp] = v;
+                }
+            }
+            tag++;
+            if (!f64 && !whole) publish_parts(0, vld(sh.m), vld(sh.area[SLOT_A]), tag, false);
+            float alpha;
+            bool dn;
+            if (!exchange(acc, tag, 1, alpha, dn)) return;
+            // ---------------- phase 2: update + r.r (cg_update.wgsl:33-34) ----------------
+            acc[0] = Acc{};
+            acc[1] = Acc{};
+            if (mine) {
+                const Quad na4 = qall(-alpha);
+                r4[0] = qaddp(qmul(na4, pool[5 * 32]), one, r4[0]);  // r - alpha q = r + (-alpha) q
+                r4[1] = qaddp(qmul(na4, pool[11 * 32]), one, r4[1]);
+                st_q(r, c[0], e[0], r4[0]);
+                st_q(r, c[1], e[1], r4[1]);
+                if (f64) {
+                    acc_quad(acc[0], r4[0], r4[0]);
+                    acc_quad(acc[1], r4[1], r4[1]);
+                } else {
+                    const float v = tree256_quads<VEC>(qmul(r4[0], r4[0]), qmul(r4[1], r4[1]), one, lane);
+                    if (lane == 0) sh.part[warp] = v;
+                }
+            }
+            tag++;
+            if (!f64 && !whole) publish_parts(0, vld(sh.m), vld(sh.area[SLOT_B]), tag, true);
+            k = it + 1;
+            if (mine) {
+                const Quad a4 = qall(alpha);
+                pool[0] = qaddp(qmul(a4, dq[0]), one, pool[0]);
+                pool[6 * 32] = qaddp(qmul(a4, dq[1]), one, pool[6 * 32]);
+            }
+            if (!exchange(acc, tag, 2, beta, dn)) return;
+            if (dn) break;
+        }
+        if (mine) {
+            st_q(p, c[0], e[0], pool[0]);
+            st_q(p, c[1], e[1], pool[6 * 32]);
+        }
+    } else {
+#pragma unroll 1
+        for (uint32_t it = 0; it < iters; it++) {
+            float* d_cur = (it & 1u) ? b.dB : b.dA;
+            const float* d_src = (it & 1u) || it == 0 ? b.dA : b.dB;
+            const Quad beta4 = qall(beta);
+            auto dir = [&](Quad dv, Quad rv) { return qaddp(qmul(beta4, dv), one, rv); };  // cg_dir.wgsl:30
+            // ---------------- phase 1: direction + SpMV + d.q ----------------
+            Acc acc[2] = {};
+            tag++;
+            auto phase1 = [&](uint32_t j) -> float {
+                const bool res = __any_sync(0xffffffffu, j < vld(sh.mres));
+                const Quads o = quads_of(j);
+                // One half's d and r rows in flight at a time (64 registers).
+                Quad nd[4], nr[4];
+                auto load = [&](int h) {
+                    const uint32_t c = o.c[h];
+                    const uint32_t off4[4] = {c - nx, c + nx, c - nxy, c + nxy};
+#pragma unroll
+                    for (int t = 0; t < 4; t++) {
+                        nd[t] = row(d_src, off4[t], o.e[h]);
+                        nr[t] = row(r, off4[t], o.e[h]);
+                    }
+                };
+                if (o.any[0]) load(0);
+                const uint32_t ce = edge(o.c[0], o.e[0], o.c[1], o.e[1]);
+                const float de = __fadd_rn(r[ce], __fmul_rn(beta, d_src[ce]));
+                Quad dq[2] = {z4, z4}, prod[2] = {z4, z4};
+                auto own = [&](int h) {
+                    if (res) dq[h] = dir(op(0, o.i[h]), op(1, o.i[h]));
+                    else dq[h] = dir(ld_q(d_src, o.c[h], o.e[h]), ld_q(r, o.c[h], o.e[h]));
+                };
+                if (o.any[0]) own(0);
+                if (o.any[1]) own(1);
+                const float b0 = __shfl_sync(0xffffffffu, hi2(dq[0].b), 31), b1 = __shfl_sync(0xffffffffu, lo2(dq[1].a), 0);
+                auto stencil = [&](int h, float left0, float right31) {
+                    Quad sum = xsum(dq[h], left0, right31);
+#pragma unroll
+                    for (int t = 0; t < 4; t++) sum = qadd(sum, dir(nd[t], nr[t]));
+                    const Quad q4 = liquid(qsubp(sum, one, qmul(counts(o.e[h]), dq[h])), o.e[h]);
+                    st_q(d_cur, o.c[h], o.e[h], dq[h]);  // the first iteration writes back what is there
+                    if (res) {
+                        op(0, o.i[h]) = dq[h];
+                        op(2, o.i[h]) = q4;
+                    } else {
+                        st_q(q, o.c[h], o.e[h], q4);
+                    }
+                    if (f64) acc_quad(acc[h], dq[h], q4);
+                    else prod[h] = qmul(dq[h], q4);
+                };
+                if (o.any[0]) stencil(0, de, b1);
+                if (o.any[1]) {
+                    load(1);
+                    stencil(1, b0, de);
+                }
+                return f64 ? 0.0f : tree256_quads<VEC>(prod[0], prod[1], one, lane);
+            };
+#pragma unroll 1
+            for (uint32_t jb = 0; jb < vld(sh.m); jb += KCH) {
+                const uint32_t je = vld(sh.m) - jb < KCH ? vld(sh.m) : jb + KCH;
+#pragma unroll 1
+                for (uint32_t j = jb + warp; j < je; j += CG_WARPS) {
+                    const float v = phase1(j);
+                    if (!f64 && lane == 0) sh.part[j - jb] = v;
+                }
+                if (!f64 && !whole) {
+                    publish_parts(jb, je - jb, vld(sh.area[SLOT_A]), tag, false);
+                    if (je < vld(sh.m)) __syncthreads();
+                }
+            }
+            float alpha;
+            bool dn;
+            if (!exchange(acc, tag, 1, alpha, dn)) return;
+            // ---------------- phase 2: update + r.r (cg_update.wgsl:33-34) ----------------
+            acc[0] = Acc{};
+            acc[1] = Acc{};
+            tag++;
+            const Quad a4 = qall(alpha), na4 = qall(-alpha);
+            auto phase2 = [&](uint32_t j) -> float {
+                const bool res = __any_sync(0xffffffffu, j < vld(sh.mres));
+                const Quads o = quads_of(j);
+                Quad prod[2] = {z4, z4};
+                auto update = [&](int h) {
+                    const uint32_t c = o.c[h], e = o.e[h], i = o.i[h];
+                    Quad d4, q4, r4, p4;
+                    if (res) {
+                        d4 = op(0, i); q4 = op(2, i); r4 = op(1, i); p4 = op(3, i);
+                    } else {
+                        d4 = ld_q(d_cur, c, e); q4 = ld_q(q, c, e); r4 = ld_q(r, c, e); p4 = ld_q(p, c, e);
+                    }
+                    p4 = qaddp(qmul(a4, d4), one, p4);
+                    r4 = qaddp(qmul(na4, q4), one, r4);  // r - alpha q = r + (-alpha) q
+                    st_q(r, c, e, r4);
+                    if (res) {
+                        op(1, i) = r4;
+                        op(3, i) = p4;
+                    } else {
+                        st_q(p, c, e, p4);
+                    }
+                    if (f64) acc_quad(acc[h], r4, r4);
+                    else prod[h] = qmul(r4, r4);
+                };
+                if (o.any[0]) update(0);
+                if (o.any[1]) update(1);
+                return f64 ? 0.0f : tree256_quads<VEC>(prod[0], prod[1], one, lane);
+            };
+#pragma unroll 1
+            for (uint32_t jb = 0; jb < vld(sh.m); jb += KCH) {
+                const uint32_t je = vld(sh.m) - jb < KCH ? vld(sh.m) : jb + KCH;
+#pragma unroll 1
+                for (uint32_t j = jb + warp; j < je; j += CG_WARPS) {
+                    const float v = phase2(j);
+                    if (!f64 && lane == 0) sh.part[j - jb] = v;
+                }
+                if (!f64 && !whole) {
+                    publish_parts(jb, je - jb, vld(sh.area[SLOT_B]), tag, true);
+                    if (je < vld(sh.m)) __syncthreads();
+                }
+            }
+            k = it + 1;
+            if (!exchange(acc, tag, 2, beta, dn)) return;
+            if (dn) break;
+        }
     }
-    if (res)  // the resident pressure, once
-        for (uint32_t tu = tid; tu < ncell; tu += CG_THREADS) {
-            const uint32_t e = sh.cell[tu];
-            p[sh.chunk[e >> 18] * CHUNK + ((e >> 10) & 255u)] = rv4[tu].w;
-        }
+    // the resident pressure, once
+    for (uint32_t j = warp; j < vld(sh.mres); j += CG_WARPS) {
+        const Quads o = quads_of(j);
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+            if (o.any[h]) st_q(p, o.c[h], o.e[h], op(3, o.i[h]));
+    }
     if (blockIdx.x == 0 && tid == 0) {
         st->cg_iters = k;
         st->rs_final = ieee ? sh.rs_d : (f64 ? df_to_double(Df{sh.rs_hi, sh.rs_lo}) : (double)sh.rs_hi);
     }
 }
 
+typedef void (*CgKernel)(DevBufs);
+static CgKernel cg_kernel(uint32_t precision, bool vec) {
+    switch (precision) {
+        case FL_CG_F64: return vec ? k_cg<FL_CG_F64, true> : k_cg<FL_CG_F64, false>;
+        case FL_CG_F64_IEEE: return vec ? k_cg<FL_CG_F64_IEEE, true> : k_cg<FL_CG_F64_IEEE, false>;
+        default: return vec ? k_cg<FL_CG_F32, true> : k_cg<FL_CG_F32, false>;
+    }
+}
+
 int cg_max_blocks_per_sm() {
-    const void* fs[3] = {(const void*)k_cg<FL_CG_F32>, (const void*)k_cg<FL_CG_F64>, (const void*)k_cg<FL_CG_F64_IEEE>};
     int lo = 1 << 30;
-    for (int i = 0; i < 3; i++) {
+    for (int i = 0; i < 6; i++) {
+        const void* f = (const void*)cg_kernel((uint32_t)i / 2, i & 1);
         int n = 0;
-        if (cudaFuncSetAttribute(fs[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CgShared)) !=
-            cudaSuccess)
+        if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CgShared)) != cudaSuccess)
             return 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fs[i], CG_THREADS, sizeof(CgShared)) != cudaSuccess) return 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, CG_THREADS, sizeof(CgShared)) != cudaSuccess) return 0;
         lo = n < lo ? n : lo;
     }
     return lo;
@@ -1266,14 +1359,14 @@ int cg_max_blocks_per_sm() {
 
 cudaError_t launch_cg_plan(const DevBufs& b, uint32_t G, cudaStream_t s) {
     if (G < 1 || G > MAX_CG_BLOCKS) return cudaErrorInvalidValue;
-    k_cg_plan<<<1, CHUNK, 0, s>>>(b, G);
+    k_cg_plan<<<1, CHUNK, 0, s>>>(b, G, PLAN_RANGES);
     return cudaGetLastError();
 }
 
-cudaError_t launch_cg(const DevBufs& b, const LaunchCfg& L, cudaStream_t s, uint32_t precision) {
+cudaError_t launch_cg(const DevBufs& b, const LaunchCfg& L, cudaStream_t s, uint32_t precision, uint32_t nx) {
     if (precision > FL_CG_F64_IEEE) return cudaErrorInvalidValue;
     if (L.cg_blocks < 1 || (uint32_t)L.cg_blocks > MAX_CG_BLOCKS) return cudaErrorInvalidValue;
-    k_cg_plan<<<1, CHUNK, 0, s>>>(b, (uint32_t)L.cg_blocks);
+    k_cg_plan<<<1, CHUNK, 0, s>>>(b, (uint32_t)L.cg_blocks, precision == FL_CG_F32 ? PLAN_F32 : PLAN_EXTENDED);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
@@ -1286,8 +1379,9 @@ cudaError_t launch_cg(const DevBufs& b, const LaunchCfg& L, cudaStream_t s, uint
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (precision == FL_CG_F64_IEEE) return cudaLaunchKernelEx(&cfg, k_cg<FL_CG_F64_IEEE>, b);
-    return precision == FL_CG_F64 ? cudaLaunchKernelEx(&cfg, k_cg<FL_CG_F64>, b) : cudaLaunchKernelEx(&cfg, k_cg<FL_CG_F32>, b);
+    const bool vec = (nx & 3u) == 0u && (((uintptr_t)b.p | (uintptr_t)b.r | (uintptr_t)b.q | (uintptr_t)b.dA |
+                                          (uintptr_t)b.dB) & 15u) == 0u;
+    return cudaLaunchKernelEx(&cfg, cg_kernel(precision, vec), b);
 }
 
 }  // namespace fl

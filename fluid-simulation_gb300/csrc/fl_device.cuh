@@ -15,8 +15,7 @@ namespace fl {
 
 constexpr uint8_t CELL_SOLID = 0, CELL_LIQUID = 1, CELL_AIR = 2;
 constexpr int CHUNK = 256;        // cells per reduction chunk (the 256-wide workgroup of cg_reduce.wgsl)
-constexpr int CG_GROUPS = 4;      // 256-thread chunk groups per CG block
-constexpr int CG_THREADS = CHUNK * CG_GROUPS;
+constexpr int CG_GROUPS = 4;      // the CG launches at most one block per CG_GROUPS chunks of the grid
 constexpr int SCAN_ITEMS = 4;     // counts per thread in the bin scan
 constexpr int SCAN_THREADS = 1024;
 constexpr int SCAN_TILE = SCAN_ITEMS * SCAN_THREADS;
@@ -98,11 +97,8 @@ struct DevBufs {
                            // liquid cells; null where no one reads it (the stand-alone solves)
     float* part_rr;        // per-chunk f32 tree partials of the initial residual
     float2* chunk_rr_df;   // per-chunk float-float partials {hi, lo} of the initial residual
-    uint32_t* cg_chunk;    // CG plan: active chunks grouped by (chunk mod 256), ascending
-    uint32_t* cg_off;      // CG plan header, cg_plan_words(max blocks) words: 257 segment
-                           // offsets into cg_chunk, the launch's tag base, the slot
-                           // layout, the first plan entry of every block and the
-                           // first exchange slot of every block (blocks + 1 each)
+    uint32_t* cg_chunk;    // CG plan: active chunks, by block
+    uint32_t* cg_off;      // CG plan header, cg_plan_words(max blocks) words (see k_cg_plan)
     unsigned long long* cg_x;  // CG exchange words, cg_x_words(nchunks, max blocks): [0] tag
                                // epoch (persists across solves), then tagged partials
 };
@@ -113,7 +109,7 @@ struct DevBufs {
 #else
 #define FL_HD
 #endif
-FL_HD constexpr size_t cg_plan_words(size_t max_blocks) { return (size_t)CHUNK + 3 + 2 * (max_blocks + 1); }
+FL_HD constexpr size_t cg_plan_words(size_t max_blocks) { return 3 * (size_t)CHUNK + 6 + (max_blocks + 1); }
 FL_HD constexpr size_t cg_x_words(size_t nchunks, size_t max_blocks) {
     return 16 + 2 * ((nchunks + 15) & ~(size_t)15) + 64 * max_blocks + 2 * 256;
 }
@@ -287,7 +283,7 @@ cudaError_t launch_p2g(const DevBufs& b, const LaunchCfg& L, uint32_t nx, uint32
                        cudaStream_t s, bool clear);
 cudaError_t launch_grid_prep(const DevBufs& b, uint32_t C, cudaStream_t s);
 // precision: FL_CG_F32, FL_CG_F64 or FL_CG_F64_IEEE (the kernel is specialised per precision).
-cudaError_t launch_cg(const DevBufs& b, const LaunchCfg& L, cudaStream_t s, uint32_t precision);
+cudaError_t launch_cg(const DevBufs& b, const LaunchCfg& L, cudaStream_t s, uint32_t precision, uint32_t nx);
 cudaError_t launch_project(const DevBufs& b, uint32_t C, cudaStream_t s);
 cudaError_t launch_g2p(const DevBufs& b, const LaunchCfg& L, cudaStream_t s);
 cudaError_t launch_iota(uint32_t* ids, uint32_t n, cudaStream_t s);

@@ -404,6 +404,7 @@ __global__ void __launch_bounds__(256) k_grid_prep(DevBufs b, uint32_t C) {
             b.p[c] = 0.0f;
             b.r[c] = 0.0f;
             b.dA[c] = 0.0f;
+            b.dB[c] = 0.0f;  // the CG reads neighbours of any type from both
             b.cinfo[c] = 0;
             if (b.div) b.div[c] = 0.0f;
         }
@@ -511,6 +512,7 @@ __global__ void __launch_bounds__(256) k_solve_init(DevBufs b, uint32_t C, const
             b.p[c] = 0.0f;
             b.r[c] = 0.0f;
             b.dA[c] = 0.0f;
+            b.dB[c] = 0.0f;  // the CG reads neighbours of any type from both
             b.cinfo[c] = 0;
         }
     }

@@ -276,7 +276,7 @@ cudaError_t enqueue_step(fl_handle* h, const DevBufs& b, cudaStream_t s, cudaEve
             return e;
     } else if (h->prm.pressure_solver == FL_SOLVER_MGPCG) {
         if ((e = fl::launch_mgpcg(b, h->mg, h->L, s)) != cudaSuccess) return e;
-    } else if ((e = fl::launch_cg(b, h->L, s, h->prm.cg_precision)) != cudaSuccess) {
+    } else if ((e = fl::launch_cg(b, h->L, s, h->prm.cg_precision, h->nx)) != cudaSuccess) {
         return e;
     }
     if ((e = mark(5)) != cudaSuccess) return e;
@@ -979,7 +979,7 @@ fl_status fl_solve_pressure(uint32_t nx, uint32_t ny, uint32_t nz, const uint8_t
         if ((e = cudaMemcpyAsync(ddiv, divergence, 4 * C, cudaMemcpyHostToDevice, st)) != cudaSuccess) break;
         if (warm_start && (e = cudaMemcpyAsync(b.p, pressure_in, 4 * C, cudaMemcpyHostToDevice, st)) != cudaSuccess) break;
         if ((e = fl::launch_solve_init(b, (uint32_t)C, ddiv, st)) != cudaSuccess) break;
-        if ((e = fl::launch_cg(b, L, st, cg_precision)) != cudaSuccess) break;
+        if ((e = fl::launch_cg(b, L, st, cg_precision, nx)) != cudaSuccess) break;
         if ((e = cudaMemcpyAsync(pressure_out, b.p, 4 * C, cudaMemcpyDeviceToHost, st)) != cudaSuccess) break;
         if ((e = cudaMemcpyAsync(&ds, b.st, sizeof(ds), cudaMemcpyDeviceToHost, st)) != cudaSuccess) break;
         e = cudaStreamSynchronize(st);
@@ -1411,7 +1411,7 @@ fl_status fl_step_adjoint(fl_handle* h, fl_tape* t, const void* dL_dout_dev, voi
         if (ms != FL_OK) return ms;
         FL_CUDA(h, fl::launch_mgpcg(cg, t->mg, h->L, st));
     } else {
-        FL_CUDA(h, fl::launch_cg(cg, h->L, st, h->prm.cg_precision));
+        FL_CUDA(h, fl::launch_cg(cg, h->L, st, h->prm.cg_precision, h->nx));
     }
     FL_CUDA(h, fl::launch_adj_faces(a, h->F3, st));
     FL_CUDA(h, fl::launch_adj_p2g(a, h->L, st));

@@ -54,8 +54,6 @@ constexpr int MG_PART = 1024;             // block partial slots per exchange pa
 constexpr int MG_CELLS = 20480;           // level-0 unknowns listed per block
 constexpr int MG_L1 = 4096;               // level-1 unknowns listed per block
 constexpr int MG_COARSE_SWEEPS = 2;       // symmetric Gauss-Seidel sweeps on the coarsest level
-constexpr int MG_BATCH = 1;               // level-0 cells per thread whose loads are issued together
-                                          // (2 measured slower: register pressure)
 
 // Level-0 cell metadata: bits 0-9 the CG's stencil mask (bit 0 liquid, bit
 // s+1 neighbour s of -x,+x,-y,+y,-z,+z liquid, bits 7-9 the non-solid count),
@@ -71,7 +69,7 @@ struct MgShared {
     uint32_t wc[MG_THREADS / 32];
     float2 res;
     int ok;
-    uint32_t ncell, nl1, list0, list1;
+    uint32_t nred, nblack, nl1, list0, list1;
     // solve scalars kept here rather than in registers through the loop
     float2 rs0, thr, rz;
 };
@@ -91,45 +89,91 @@ __device__ __forceinline__ float4 ld_st(const float4* st, uint32_t c) {
 }
 __device__ __forceinline__ uint32_t ld_ci(const uint16_t* ci, uint32_t c) { return __ldg(ci + c); }
 
-// Sum over the liquid neighbours of v(nb, side) (side 0..5 = -x,+x,-y,+y,-z,+z).
-template <class F>
-__device__ __forceinline__ float nbsum0(uint32_t meta, uint32_t c, uint32_t nx, uint32_t nxy, F v) {
+// The passes are chains of L2 loads, one cell or two per thread, so what a cell
+// costs is the number of loads that wait for one another.  Every load of a cell
+// is issued before the first value is used, and volatile: the compiler would
+// otherwise move each load behind the test that decides whether its value is
+// needed (each neighbour then waited for the one before: 105 us per iteration
+// on the 128^3 sphere-into-pool scene, against XXX).
+__device__ __forceinline__ float ld_if(const float* p, bool on) {  // 0 when off
+    float v;
+    asm volatile("{\n.reg .pred q;\nsetp.ne.u32 q, %2, 0;\nmov.f32 %0, 0f00000000;\n@q ld.global.f32 %0, [%1];\n}"
+                 : "=f"(v)
+                 : "l"(p), "r"((uint32_t)on));
+    return v;
+}
+__device__ __forceinline__ uint32_t ld_ci_if(const uint16_t* p, bool on) {
+    uint32_t v;
+    asm volatile("{\n.reg .pred q;\nsetp.ne.u32 q, %2, 0;\nmov.u32 %0, 0;\n@q ld.global.nc.u16 %0, [%1];\n}"
+                 : "=r"(v)
+                 : "l"(p), "r"((uint32_t)on));
+    return v;
+}
+__device__ __forceinline__ float ld_any(const float* p) {  // shared or global
+    float v;
+    asm volatile("ld.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+
+// The neighbours of level-0 cell c in side order (-x, +x, -y, +y, -z, +z), and
+// whether each is liquid.
+struct Nb0 {
+    uint32_t n[6];
+    bool on[6];
+    __device__ __forceinline__ Nb0(uint32_t mask, uint32_t c, uint32_t nx, uint32_t nxy) {
+        const uint32_t m[6] = {c - 1, c + 1, c - nx, c + nx, c - nxy, c + nxy};
+#pragma unroll
+        for (int s = 0; s < 6; s++) {
+            on[s] = (mask >> (s + 1)) & 1u;
+            n[s] = m[s];
+        }
+    }
+    __device__ __forceinline__ void load(const float* a, float (&v)[6]) const {
+#pragma unroll
+        for (int s = 0; s < 6; s++) v[s] = ld_if(a + n[s], on[s]);
+    }
+};
+// a[n] / D[n] of the liquid neighbours, summed in side order, from their values
+// and stencil words.
+__device__ __forceinline__ float quotient_sum(const Nb0& nb, const float (&v)[6], const uint32_t (&ci)[6]) {
     float s = 0.0f;
-    if (meta & (1u << 1)) s += v(c - 1, 0);
-    if (meta & (1u << 2)) s += v(c + 1, 1);
-    if (meta & (1u << 3)) s += v(c - nx, 2);
-    if (meta & (1u << 4)) s += v(c + nx, 3);
-    if (meta & (1u << 5)) s += v(c - nxy, 4);
-    if (meta & (1u << 6)) s += v(c + nxy, 5);
+#pragma unroll
+    for (int k = 0; k < 6; k++)
+        if (nb.on[k]) s += v[k] / (float)(ci[k] >> 7);
     return s;
 }
 
-// Coarse level: sum over the neighbours of w(nb) * v(nb, i, j, k of nb) (a
-// neighbour with a nonzero weight is an unknown).
-template <class F>
-__device__ __forceinline__ float nbsum(const float4* st, float4 sc, uint32_t c, uint32_t i, uint32_t j, uint32_t k,
-                                       const MgLevel& lv, F v) {
-    const uint32_t nxy = lv.nx * lv.ny;
-    float s = 0.0f;
-    if (sc.y != 0.0f) s += sc.y * v(c + 1, i + 1, j, k);
-    if (sc.z != 0.0f) s += sc.z * v(c + lv.nx, i, j + 1, k);
-    if (sc.w != 0.0f) s += sc.w * v(c + nxy, i, j, k + 1);
-    if (i > 0) {
-        const float w = ld_st(st, c - 1).y;
-        if (w != 0.0f) s += w * v(c - 1, i - 1, j, k);
+// A coarse cell's neighbours in the order +x, +y, +z, -x, -y, -z: indices (the
+// cell itself where the grid ends) and weights (0: not an unknown).
+struct NbC {
+    uint32_t n[6];
+    float w[6];
+    __device__ __forceinline__ NbC(const float4* st, float4 sc, uint32_t c, uint32_t i, uint32_t j, uint32_t k,
+                                   const MgLevel& lv) {
+        const uint32_t nx = lv.nx, nxy = lv.nx * lv.ny;
+        n[0] = sc.y != 0.0f ? c + 1 : c;
+        n[1] = sc.z != 0.0f ? c + nx : c;
+        n[2] = sc.w != 0.0f ? c + nxy : c;
+        n[3] = i ? c - 1 : c;
+        n[4] = j ? c - nx : c;
+        n[5] = k ? c - nxy : c;
+        const float wx = ld_st(st, n[3]).y, wy = ld_st(st, n[4]).z, wz = ld_st(st, n[5]).w;
+        w[0] = sc.y; w[1] = sc.z; w[2] = sc.w;
+        w[3] = i ? wx : 0.0f;
+        w[4] = j ? wy : 0.0f;
+        w[5] = k ? wz : 0.0f;
     }
-    if (j > 0) {
-        const float w = ld_st(st, c - lv.nx).z;
-        if (w != 0.0f) s += w * v(c - lv.nx, i, j - 1, k);
+    __device__ __forceinline__ void load(const float* a, float (&v)[6]) const {
+#pragma unroll
+        for (int s = 0; s < 6; s++) v[s] = ld_any(a + n[s]);
     }
-    if (k > 0) {
-        const float w = ld_st(st, c - nxy).w;
-        if (w != 0.0f) s += w * v(c - nxy, i, j, k - 1);
+    __device__ __forceinline__ float sum(const float (&v)[6]) const {
+        float t = 0.0f;
+#pragma unroll
+        for (int s = 0; s < 6; s++) t += w[s] != 0.0f ? w[s] * v[s] : 0.0f;
+        return t;
     }
-    return s;
-}
-// v(nb) = x[nb], the neighbour's coordinates unused
-#define MG_X_OF(lv) [&](uint32_t n, uint32_t, uint32_t, uint32_t) { return (lv).x[n]; }
+};
 
 // The coarse cell (aggregate) holding the cell at (i, j, k), or cell c.
 __device__ __forceinline__ uint32_t parent_at(uint32_t i, uint32_t j, uint32_t k, const MgLevel& up) {
@@ -244,7 +288,7 @@ __device__ void build_lists(Ctx& x) {
     MgShared& sh = x.sh;
     const DevParams& P = *x.b.prm;
     const uint32_t C = P.C, nx = P.nx, ny = P.ny, lo = threadIdx.x & (CHUNK - 1);
-    uint32_t n = 0;
+    uint32_t nr = 0, nb = 0;
     for (uint32_t base = 0; base < x.nown; base += MG_THREADS / CHUNK) {
         const uint32_t e = base + threadIdx.x / CHUNK;
         uint32_t c = 0, info = 0;
@@ -253,13 +297,17 @@ __device__ void build_lists(Ctx& x) {
             if (c < C) info = ld_ci(x.b.cinfo, c);
         }
         const bool u = info >= (1u << 7);
-        uint32_t tot;
-        const uint32_t pos = n + block_rank(sh, u, tot);
-        if (u && pos < (uint32_t)MG_CELLS) {
-            sh.cell[pos] = c;
-            sh.meta[pos] = (uint16_t)make_meta(info, c, nx, ny);
+        const uint32_t meta = u ? make_meta(info, c, nx, ny) : 0u;
+        const bool black = (meta & META_BLACK) != 0u;
+        uint32_t totr, totb;
+        const uint32_t pr = nr + block_rank(sh, u && !black, totr), pb = nb + block_rank(sh, u && black, totb);
+        nr += totr;
+        nb += totb;
+        if (u && nr + nb <= (uint32_t)MG_CELLS) {  // reds from the front, blacks from the back
+            const uint32_t at = black ? MG_CELLS - 1 - pb : pr;
+            sh.cell[at] = c;
+            sh.meta[at] = (uint16_t)meta;
         }
-        n += tot;
     }
     const MgLevel& l1 = x.m.lv[1];
     uint32_t n1 = 0, I0, I1;
@@ -273,20 +321,27 @@ __device__ void build_lists(Ctx& x) {
         n1 += tot;
     }
     if (threadIdx.x == 0) {
-        sh.ncell = n;
-        sh.list0 = n <= (uint32_t)MG_CELLS;
+        sh.nred = nr;
+        sh.nblack = nb;
+        sh.list0 = nr + nb <= (uint32_t)MG_CELLS;
         sh.nl1 = n1;
         sh.list1 = n1 <= (uint32_t)MG_L1;
     }
     __syncthreads();
 }
 
-// f(c, meta) for every level-0 unknown of this block.
+// f(c, meta) for every level-0 unknown of this block of a colour (0 red, 1
+// black).  The colours are listed apart: a pass that treats them differently
+// keeps all lanes at work.
 template <class F>
-__device__ __forceinline__ void for_own(const Ctx& x, F f) {
+__device__ __forceinline__ void for_own(const Ctx& x, uint32_t colour, F f) {
     const MgShared& sh = x.sh;
     if (sh.list0) {
-        for (uint32_t e = threadIdx.x; e < sh.ncell; e += MG_THREADS) f(sh.cell[e], (uint32_t)sh.meta[e]);
+        const uint32_t n = colour ? sh.nblack : sh.nred;
+        for (uint32_t e = threadIdx.x; e < n; e += MG_THREADS) {
+            const uint32_t at = colour ? MG_CELLS - 1 - e : e;
+            f(sh.cell[at], (uint32_t)sh.meta[at]);
+        }
         return;
     }
     const DevParams& P = *x.b.prm;
@@ -295,36 +350,9 @@ __device__ __forceinline__ void for_own(const Ctx& x, F f) {
         const uint32_t c = x.b.cg_chunk[x.e0 + e] * CHUNK + lo;
         if (c >= C) continue;
         const uint32_t info = ld_ci(x.b.cinfo, c);
-        if (info >= (1u << 7)) f(c, make_meta(info, c, P.nx, P.ny));
-    }
-}
-
-// The same cells with loads and stores in two phases: ld(c, meta) (loads
-// only) for MG_BATCH cells of the thread, then st(c, meta, value) for each,
-// so that the batch's loads are in flight together.
-template <int K = MG_BATCH, class Ld, class Stf>
-__device__ __forceinline__ void for_own_batched(const Ctx& x, Ld ld, Stf stf) {
-    const MgShared& sh = x.sh;
-    if (!sh.list0) {
-        for_own(x, [&](uint32_t c, uint32_t meta) { stf(c, meta, ld(c, meta)); });
-        return;
-    }
-    const uint32_t n = sh.ncell;
-    for (uint32_t e = threadIdx.x; e < n; e += K * MG_THREADS) {
-        decltype(ld(0u, 0u)) v[K];
-        uint32_t c[K], mt[K];
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            const uint32_t ek = e + k * MG_THREADS;
-            if (ek < n) {
-                c[k] = sh.cell[ek];
-                mt[k] = sh.meta[ek];
-                v[k] = ld(c[k], mt[k]);
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < K; k++)
-            if (e + k * MG_THREADS < n) stf(c[k], mt[k], v[k]);
+        if (info < (1u << 7)) continue;
+        const uint32_t meta = make_meta(info, c, P.nx, P.ny);
+        if (((meta & META_BLACK) != 0u) == (colour != 0u)) f(c, meta);
     }
 }
 
@@ -390,17 +418,19 @@ __device__ void pre0(const Ctx& x) {
     const DevParams& P = *x.b.prm;
     const uint32_t nx = P.nx, nxy = nx * P.ny;
     const float* r = x.r;
-    const uint16_t* __restrict__ ci = x.b.cinfo;
+    const uint16_t* ci = x.b.cinfo;
     float* z = x.m.lv[0].x;
-    for_own_batched(
-        x,
-        [&](uint32_t c, uint32_t meta) {
-            float v = r[c];
-            if (meta & META_BLACK)
-                v += nbsum0(meta, c, nx, nxy, [&](uint32_t n, int) { return r[n] / (float)(ld_ci(ci, n) >> 7); });
-            return v / diag0(meta);
-        },
-        [&](uint32_t c, uint32_t, float v) { z[c] = v; });
+    for_own(x, 1, [&](uint32_t c, uint32_t meta) {
+        const Nb0 nb(meta, c, nx, nxy);
+        float rn[6];
+        uint32_t cn[6];
+        nb.load(r, rn);
+#pragma unroll
+        for (int s = 0; s < 6; s++) cn[s] = ld_ci_if(ci + nb.n[s], nb.on[s]);
+        const float rc = ld_if(r + c, true);
+        z[c] = (rc + quotient_sum(nb, rn, cn)) / diag0(meta);
+    });
+    for_own(x, 0, [&](uint32_t c, uint32_t meta) { z[c] = r[c] / diag0(meta); });
 }
 
 // The CG update fused with pre0: p += alpha d, r_next = r - alpha q, and the
@@ -413,19 +443,33 @@ __device__ Df update_pre0(const Ctx& x, float alpha, const float* d, float* r_ne
     const float* r = x.r;
     const float* q = x.b.q;
     float* p = x.b.p;
-    const uint16_t* __restrict__ ci = x.b.cinfo;
+    const uint16_t* ci = x.b.cinfo;
     float* z = x.m.lv[0].x;
     Df acc = {0.0f, 0.0f};
-    for_own(x, [&](uint32_t c, uint32_t meta) {
-        const float rn = r[c] - alpha * q[c];
-        float v = rn;
-        if (meta & META_BLACK)
-            v += nbsum0(meta, c, nx, nxy,
-                        [&](uint32_t n, int) { return (r[n] - alpha * q[n]) / (float)(ld_ci(ci, n) >> 7); });
-        p[c] += alpha * d[c];
-        r_next[c] = rn;
-        z[c] = v / diag0(meta);
-        acc = df_add(acc, df_prod(rn, rn));
+    for_own(x, 1, [&](uint32_t c, uint32_t meta) {
+        const Nb0 nb(meta, c, nx, nxy);
+        float rn[6], qn[6];
+        uint32_t cn[6];
+        nb.load(r, rn);
+        nb.load(q, qn);
+#pragma unroll
+        for (int s = 0; s < 6; s++) cn[s] = ld_ci_if(ci + nb.n[s], nb.on[s]);
+        const float rc = ld_if(r + c, true), qc = ld_if(q + c, true), pc = ld_if(p + c, true), dc = ld_if(d + c, true);
+#pragma unroll
+        for (int s = 0; s < 6; s++) rn[s] -= alpha * qn[s];
+        const float rnew = rc - alpha * qc;
+        p[c] = pc + alpha * dc;
+        r_next[c] = rnew;
+        z[c] = (rnew + quotient_sum(nb, rn, cn)) / diag0(meta);
+        acc = df_add(acc, df_prod(rnew, rnew));
+    });
+    for_own(x, 0, [&](uint32_t c, uint32_t meta) {
+        const float rc = ld_if(r + c, true), qc = ld_if(q + c, true), pc = ld_if(p + c, true), dc = ld_if(d + c, true);
+        const float rnew = rc - alpha * qc;
+        p[c] = pc + alpha * dc;
+        r_next[c] = rnew;
+        z[c] = rnew / diag0(meta);
+        acc = df_add(acc, df_prod(rnew, rnew));
     });
     return acc;
 }
@@ -476,9 +520,9 @@ __device__ __forceinline__ void for_level8(const Ctx& x, uint32_t l, const MgLev
 // b1 = P^T (r - A z)
 __device__ void restrict0(const Ctx& x) {
     const DevParams& P = *x.b.prm;
-    const uint32_t nx = P.nx, ny = P.ny, nz = P.nz, nxy = nx * ny;
+    const uint32_t nx = P.nx, ny = P.ny, nz = P.nz, nxy = nx * ny, last = P.C - 1;
     const float* r = x.r;
-    const uint16_t* __restrict__ ci = x.b.cinfo;
+    const uint16_t* ci = x.b.cinfo;
     const float* z = x.m.lv[0].x;
     const MgLevel& up = x.m.lv[1];
     for_level8(
@@ -487,9 +531,19 @@ __device__ void restrict0(const Ctx& x) {
             const uint32_t i = 2 * ii + (d & 1), j = 2 * jj + ((d >> 1) & 1), k = 2 * kk + (d >> 2);
             if (i >= nx || j >= ny || k >= nz) return 0.0f;
             const uint32_t c = i + nx * (j + ny * k);
-            const uint32_t info = ld_ci(ci, c);
+            // the neighbours' z with the cell's own stencil word (some cell
+            // where the grid ends), kept where the word names them
+            const uint32_t info = ld_ci_if(ci + c, true);
+            const uint32_t n[6] = {c - 1, c + 1, c - nx, c + nx, c - nxy, c + nxy};
+            float zn[6];
+#pragma unroll
+            for (int s = 0; s < 6; s++) zn[s] = ld_if(z + (n[s] < last ? n[s] : last), true);
+            const float rc = ld_if(r + c, true), zc = ld_if(z + c, true);
             if (info < (1u << 7)) return 0.0f;
-            return r[c] - (diag0(info) * z[c] - nbsum0(info, c, nx, nxy, [&](uint32_t n, int) { return z[n]; }));
+            float sum = 0.0f;
+#pragma unroll
+            for (int s = 0; s < 6; s++) sum += (info >> (s + 1)) & 1u ? zn[s] : 0.0f;
+            return rc - (diag0(info) * zc - sum);
         },
         [&](uint32_t I, float s) { up.b[I] = s; });
 }
@@ -503,29 +557,25 @@ __device__ void post0_black(const Ctx& x) {
     const MgLevel& up = x.m.lv[1];
     const float* e = up.x;
     const uint32_t unx = up.nx, unxy = up.nx * up.ny;
-    for_own_batched(
-        x,
-        [&](uint32_t c, uint32_t meta) {
-            if (!(meta & META_BLACK)) return 0.0f;
-            const uint32_t pc = parent_of(c, nx, ny, up);
-            // parent of the neighbour on side s: the own parent, or the next
-            // one when the step leaves the 2x2x2 aggregate
-            auto pn = [&](int side) {
-                switch (side) {
-                    case 0: return (meta & META_IODD) ? pc : pc - 1;
-                    case 1: return (meta & META_IODD) ? pc + 1 : pc;
-                    case 2: return (meta & META_JODD) ? pc : pc - unx;
-                    case 3: return (meta & META_JODD) ? pc + unx : pc;
-                    case 4: return (meta & META_KODD) ? pc : pc - unxy;
-                    default: return (meta & META_KODD) ? pc + unxy : pc;
-                }
-            };
-            const float s = nbsum0(meta, c, nx, nxy, [&](uint32_t n, int side) { return z[n] + e[pn(side)]; });
-            return (r[c] + s) / diag0(meta);
-        },
-        [&](uint32_t c, uint32_t meta, float v) {
-            if (meta & META_BLACK) z[c] = v;
-        });
+    for_own(x, 1, [&](uint32_t c, uint32_t meta) {
+        const Nb0 nb(meta, c, nx, nxy);
+        const uint32_t pc = parent_of(c, nx, ny, up);
+        const bool io = meta & META_IODD, jo = meta & META_JODD, ko = meta & META_KODD;
+        // parents of the neighbours: the own parent, or the next one when the
+        // step leaves the 2x2x2 aggregate
+        const uint32_t pn[6] = {io ? pc : pc - 1, io ? pc + 1 : pc, jo ? pc : pc - unx, jo ? pc + unx : pc,
+                                ko ? pc : pc - unxy, ko ? pc + unxy : pc};
+        float zn[6], en[6];
+        nb.load(z, zn);
+#pragma unroll
+        for (int s = 0; s < 6; s++) en[s] = ld_if(e + pn[s], nb.on[s]);
+        const float rc = ld_if(r + c, true);
+        float sum = 0.0f;
+#pragma unroll
+        for (int s = 0; s < 6; s++)
+            if (nb.on[s]) sum += zn[s] + en[s];
+        z[c] = (rc + sum) / diag0(meta);
+    });
 }
 
 // red sweep; returns this thread's share of r.z
@@ -535,19 +585,22 @@ __device__ Df post0_red(const Ctx& x) {
     const float* r = x.r;
     float* z = x.m.lv[0].x;
     Df acc = {0.0f, 0.0f};
-    for_own_batched(
-        x,
-        [&](uint32_t c, uint32_t meta) {
-            const float rc = r[c];
-            const float zc = (meta & META_BLACK)
-                                 ? z[c]
-                                 : (rc + nbsum0(meta, c, nx, nxy, [&](uint32_t n, int) { return z[n]; })) / diag0(meta);
-            return make_float2(rc, zc);
-        },
-        [&](uint32_t c, uint32_t meta, float2 v) {
-            if (!(meta & META_BLACK)) z[c] = v.y;
-            acc = df_add(acc, df_prod(v.x, v.y));
-        });
+    for_own(x, 0, [&](uint32_t c, uint32_t meta) {
+        const Nb0 nb(meta, c, nx, nxy);
+        float zn[6];
+        nb.load(z, zn);
+        const float rc = ld_if(r + c, true);
+        float sum = 0.0f;
+#pragma unroll
+        for (int s = 0; s < 6; s++) sum += zn[s];  // 0 where there is none
+        const float zc = (rc + sum) / diag0(meta);
+        z[c] = zc;
+        acc = df_add(acc, df_prod(rc, zc));
+    });
+    for_own(x, 1, [&](uint32_t c, uint32_t) {
+        const float rc = ld_if(r + c, true), zc = ld_if(z + c, true);
+        acc = df_add(acc, df_prod(rc, zc));
+    });
     return acc;
 }
 
@@ -556,10 +609,19 @@ __device__ Df post0_red(const Ctx& x) {
 __device__ void pre_l(const Ctx& x, uint32_t l, const MgLevel& lv, bool local) {
     const float4* st = lv.st;
     for_level(x, l, lv, local, [&](uint32_t c, uint32_t i, uint32_t j, uint32_t k, float4 sc) {
-        float v = lv.b[c];
-        if (((i + j + k) & 1u) != 0u)
-            v += nbsum(st, sc, c, i, j, k, lv,
-                       [&](uint32_t n, uint32_t, uint32_t, uint32_t) { return lv.b[n] / ld_st(st, n).x; });
+        float v = ld_any(lv.b + c);
+        if (((i + j + k) & 1u) != 0u) {
+            const NbC nb(st, sc, c, i, j, k, lv);
+            float bn[6], dn[6];
+            nb.load(lv.b, bn);
+#pragma unroll
+            for (int s = 0; s < 6; s++) dn[s] = ld_st(st, nb.n[s]).x;
+            float sum = 0.0f;
+#pragma unroll
+            for (int s = 0; s < 6; s++)
+                if (nb.w[s] != 0.0f) sum += nb.w[s] * (bn[s] / dn[s]);
+            v += sum;
+        }
         lv.x[c] = v / sc.x;
     });
 }
@@ -573,8 +635,12 @@ __device__ void restrict_l(const Ctx& x, uint32_t l, const MgLevel& lv, const Mg
             if (i >= lv.nx || j >= lv.ny || k >= lv.nz) return 0.0f;
             const uint32_t c = i + lv.nx * (j + lv.ny * k);
             const float4 sc = ld_st(st, c);
+            const float bc = ld_any(lv.b + c), xc = ld_any(lv.x + c);
             if (!(sc.x > 0.0f)) return 0.0f;
-            return lv.b[c] - (sc.x * lv.x[c] - nbsum(st, sc, c, i, j, k, lv, MG_X_OF(lv)));
+            const NbC nb(st, sc, c, i, j, k, lv);
+            float xn[6];
+            nb.load(lv.x, xn);
+            return bc - (sc.x * xc - nb.sum(xn));
         },
         [&](uint32_t I, float s) { up.b[I] = s; });
 }
@@ -583,10 +649,20 @@ __device__ void post_black_l(const Ctx& x, uint32_t l, const MgLevel& lv, const 
     const float4* st = lv.st;
     for_level(x, l, lv, local, [&](uint32_t c, uint32_t i, uint32_t j, uint32_t k, float4 sc) {
         if (((i + j + k) & 1u) == 0u) return;
-        const float s = nbsum(st, sc, c, i, j, k, lv, [&](uint32_t n, uint32_t ni, uint32_t nj, uint32_t nk) {
-            return lv.x[n] + up.x[parent_at(ni, nj, nk, up)];
-        });
-        lv.x[c] = (lv.b[c] + s) / sc.x;
+        const NbC nb(st, sc, c, i, j, k, lv);
+        const uint32_t pc = parent_at(i, j, k, up), unx = up.nx, unxy = up.nx * up.ny;
+        // the neighbours' parents (the own one where there is no neighbour)
+        const uint32_t pn[6] = {nb.n[0] != c && (i & 1u) ? pc + 1 : pc,       nb.n[1] != c && (j & 1u) ? pc + unx : pc,
+                                nb.n[2] != c && (k & 1u) ? pc + unxy : pc,    nb.n[3] != c && !(i & 1u) ? pc - 1 : pc,
+                                nb.n[4] != c && !(j & 1u) ? pc - unx : pc,    nb.n[5] != c && !(k & 1u) ? pc - unxy : pc};
+        float xn[6], en[6];
+        nb.load(lv.x, xn);
+#pragma unroll
+        for (int s = 0; s < 6; s++) en[s] = ld_any(up.x + pn[s]);
+        const float bc = ld_any(lv.b + c);
+#pragma unroll
+        for (int s = 0; s < 6; s++) xn[s] += en[s];
+        lv.x[c] = (bc + nb.sum(xn)) / sc.x;
     });
 }
 
@@ -594,7 +670,11 @@ __device__ void post_red_l(const Ctx& x, uint32_t l, const MgLevel& lv, bool loc
     const float4* st = lv.st;
     for_level(x, l, lv, local, [&](uint32_t c, uint32_t i, uint32_t j, uint32_t k, float4 sc) {
         if (((i + j + k) & 1u) != 0u) return;
-        lv.x[c] = (lv.b[c] + nbsum(st, sc, c, i, j, k, lv, MG_X_OF(lv))) / sc.x;
+        const NbC nb(st, sc, c, i, j, k, lv);
+        float xn[6];
+        nb.load(lv.x, xn);
+        const float bc = ld_any(lv.b + c);
+        lv.x[c] = (bc + nb.sum(xn)) / sc.x;
     });
 }
 
@@ -638,12 +718,18 @@ __device__ void local_cycle(const Ctx& x) {
             sc = ld_st(lv.st, t);
             lv.x[t] = 0.0f;
         }
+        const uint32_t at = t < lv.C ? t : 0u;
+        const NbC nb(lv.st, sc, at, i, j, k, lv);
+        const float bt = lv.b[at];
         __syncthreads();
         for (int h = 0; h < 4 * MG_COARSE_SWEEPS; h++) {
             // forward sweeps red, black; backward sweeps black, red
             const uint32_t want = h < 2 * MG_COARSE_SWEEPS ? (uint32_t)(h & 1) : (uint32_t)((h & 1) ^ 1);
-            if (t < lv.C && sc.x > 0.0f && col == want)
-                lv.x[t] = (lv.b[t] + nbsum(lv.st, sc, t, i, j, k, lv, MG_X_OF(lv))) / sc.x;
+            if (t < lv.C && sc.x > 0.0f && col == want) {
+                float xn[6];
+                nb.load(lv.x, xn);
+                lv.x[t] = (bt + nb.sum(xn)) / sc.x;
+            }
             __syncthreads();
         }
     }
@@ -731,9 +817,11 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_mgpcg(DevBufs b, MgBufs m) {
 
     // r0.r0 (grid_prep left r = rhs - A p0)
     Df acc = {0.0f, 0.0f};
-    for_own_batched(
-        x, [&](uint32_t c, uint32_t) { return x.r[c]; },
-        [&](uint32_t, uint32_t, float rc) { acc = df_add(acc, df_prod(rc, rc)); });
+    for (uint32_t colour = 0; colour < 2; colour++)
+        for_own(x, colour, [&](uint32_t c, uint32_t) {
+            const float rc = x.r[c];
+            acc = df_add(acc, df_prod(rc, rc));
+        });
     Df rs;
     if (!mg_allreduce(x, acc, rs)) return;
     if (tid == 0) {
@@ -755,17 +843,22 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_mgpcg(DevBufs b, MgBufs m) {
         const bool first = it == 0;
         // direction d = z + beta d_prev and q = A d (neighbours' d on the fly)
         acc = Df{0.0f, 0.0f};
-        for_own_batched(
-            x,
-            [&](uint32_t c, uint32_t meta) {
-                auto dv = [&](uint32_t n, int) { return first ? z[n] : z[n] + beta * d_prev[n]; };
-                const float dc = dv(c, 0);
-                return make_float2(dc, diag0(meta) * dc - nbsum0(meta, c, nx, nxy, dv));
-            },
-            [&](uint32_t c, uint32_t, float2 v) {
-                d_cur[c] = v.x;
-                q[c] = v.y;
-                acc = df_add(acc, df_prod(v.x, v.y));
+        for (uint32_t colour = 0; colour < 2; colour++)
+            for_own(x, colour, [&](uint32_t c, uint32_t meta) {
+                const Nb0 nb(meta, c, nx, nxy);
+                float zn[6], dn[6];
+                nb.load(z, zn);
+#pragma unroll
+                for (int s = 0; s < 6; s++) dn[s] = ld_if(d_prev + nb.n[s], nb.on[s] && !first);
+                const float zc = ld_if(z + c, true), dp = ld_if(d_prev + c, !first);
+                auto dir = [&](float zv, float dv) { return first ? zv : zv + beta * dv; };
+                float sum = 0.0f;
+#pragma unroll
+                for (int s = 0; s < 6; s++) sum += dir(zn[s], dn[s]);  // 0 where there is none
+                const float dc = dir(zc, dp), qc = diag0(meta) * dc - sum;
+                d_cur[c] = dc;
+                q[c] = qc;
+                acc = df_add(acc, df_prod(dc, qc));
             });
         Df dq;
         if (!mg_allreduce(x, acc, dq)) return;

@@ -65,11 +65,13 @@ struct MgShared {
     uint16_t meta[MG_CELLS];
     uint32_t l1[MG_L1];
     float lb[MG_LOCAL_TOTAL], lx[MG_LOCAL_TOTAL];  // b and x of the levels block 0 runs alone
+    uint16_t loc[MG_LOCAL_TOTAL];                  // and their unknowns, by colour
+    uint32_t nloc[MG_MAX_LEVELS][2];
     float2 red[MG_THREADS / 32];
     uint32_t wc[MG_THREADS / 32];
     float2 res;
     int ok;
-    uint32_t nred, nblack, nl1, list0, list1;
+    uint32_t n0[2], n1[2], list0, list1;  // unknowns listed per colour: level 0, level 1
     // solve scalars kept here rather than in registers through the loop
     float2 rs0, thr, rz;
 };
@@ -277,11 +279,16 @@ __device__ __forceinline__ uint32_t block_rank(MgShared& sh, bool flag, uint32_t
     return off + __popc(ball & ((1u << lane) - 1u));
 }
 
-// Level-l cell range of this block (levels >= 1 outside block 0's share).
-__device__ __forceinline__ void block_range(uint32_t C, uint32_t& lo, uint32_t& hi) {
-    lo = (uint32_t)(((uint64_t)C * blockIdx.x) / gridDim.x);
-    hi = (uint32_t)(((uint64_t)C * (blockIdx.x + 1)) / gridDim.x);
+// This block's share of a coarse grid level: groups of 32 cells dealt out in
+// turn, so that blocks get equal numbers of unknowns wherever the liquid is
+// (contiguous ranges gave the slowest block twice the median's work in a pool).
+// share_size counts them (the last group may reach past the level's end),
+// share_cell gives the e-th.
+__device__ __forceinline__ uint32_t share_size(uint32_t C) {
+    const uint32_t groups = (C + 31) / 32;
+    return blockIdx.x < groups ? ((groups - blockIdx.x + gridDim.x - 1) / gridDim.x) * 32u : 0u;
 }
+__device__ __forceinline__ uint32_t share_cell(uint32_t e) { return ((e >> 5) * gridDim.x + blockIdx.x) * 32u + (e & 31u); }
 
 // Lists this block's level-0 unknowns (plan order) and level-1 unknowns.
 __device__ void build_lists(Ctx& x) {
@@ -310,22 +317,25 @@ __device__ void build_lists(Ctx& x) {
         }
     }
     const MgLevel& l1 = x.m.lv[1];
-    uint32_t n1 = 0, I0, I1;
-    block_range(l1.C, I0, I1);
-    for (uint32_t base = I0; base < I1; base += MG_THREADS) {
-        const uint32_t I = base + threadIdx.x;
-        const bool u = I < I1 && ld_st(l1.st, I).x > 0.0f;
-        uint32_t tot;
-        const uint32_t pos = n1 + block_rank(sh, u, tot);
-        if (u && pos < (uint32_t)MG_L1) sh.l1[pos] = I;
-        n1 += tot;
+    uint32_t n1r = 0, n1b = 0;
+    const uint32_t n1 = share_size(l1.C);
+    for (uint32_t base = 0; base < n1; base += MG_THREADS) {
+        const uint32_t e = base + threadIdx.x, I = share_cell(e);
+        const bool u = e < n1 && I < l1.C && ld_st(l1.st, I).x > 0.0f;
+        const bool black = u && ((I % l1.nx + (I / l1.nx) % l1.ny + I / (l1.nx * l1.ny)) & 1u) != 0u;
+        uint32_t totr, totb;
+        const uint32_t pr = n1r + block_rank(sh, u && !black, totr), pb = n1b + block_rank(sh, u && black, totb);
+        n1r += totr;
+        n1b += totb;
+        if (u && n1r + n1b <= (uint32_t)MG_L1) sh.l1[black ? MG_L1 - 1 - pb : pr] = I;
     }
     if (threadIdx.x == 0) {
-        sh.nred = nr;
-        sh.nblack = nb;
+        sh.n0[0] = nr;
+        sh.n0[1] = nb;
         sh.list0 = nr + nb <= (uint32_t)MG_CELLS;
-        sh.nl1 = n1;
-        sh.list1 = n1 <= (uint32_t)MG_L1;
+        sh.n1[0] = n1r;
+        sh.n1[1] = n1b;
+        sh.list1 = n1r + n1b <= (uint32_t)MG_L1;
     }
     __syncthreads();
 }
@@ -337,7 +347,7 @@ template <class F>
 __device__ __forceinline__ void for_own(const Ctx& x, uint32_t colour, F f) {
     const MgShared& sh = x.sh;
     if (sh.list0) {
-        const uint32_t n = colour ? sh.nblack : sh.nred;
+        const uint32_t n = sh.n0[colour];
         for (uint32_t e = threadIdx.x; e < n; e += MG_THREADS) {
             const uint32_t at = colour ? MG_CELLS - 1 - e : e;
             f(sh.cell[at], (uint32_t)sh.meta[at]);
@@ -356,9 +366,9 @@ __device__ __forceinline__ void for_own(const Ctx& x, uint32_t colour, F f) {
     }
 }
 
-// f(c, i, j, k, st) for every unknown of coarse level l: level 1 from this
-// block's list, other grid levels over this block's range, local levels
-// (block 0 alone, shared memory) over all cells.
+// f(c, i, j, k, st) for every unknown of coarse level l of a colour: level 1 and
+// the local levels (block 0 alone, shared memory) from lists, other grid levels
+// over this block's share.
 // (i, j, k) of cell c of a level of at most MG_BLOCK0_CELLS cells by
 // multiply-high with rounded-up reciprocals ceil(2^32 / d): exact because
 // c * d stays below 2^32 (integer division by a runtime divisor is a long
@@ -378,36 +388,50 @@ struct SmallDiv {
 };
 static_assert((uint64_t)MG_BLOCK0_CELLS * MG_BLOCK0_CELLS < (1ull << 32), "SmallDiv needs c * divisor < 2^32");
 
+// Block 0's unknowns of local level l: position of the e-th of a colour in its lists.
+__device__ __forceinline__ uint32_t local_at(const Ctx& x, uint32_t l, uint32_t colour, uint32_t e) {
+    uint32_t off = 0;
+    for (uint32_t k = x.Lg; k < l; k++) off += x.m.lv[k].C;
+    return colour ? off + x.m.lv[l].C - 1 - e : off + e;
+}
+
+// colour: 0 red, 1 black.
 template <class F>
-__device__ __forceinline__ void for_level(const Ctx& x, uint32_t l, const MgLevel& lv, bool local, F f) {
-    auto visit = [&](uint32_t c, float4 sc) {
-        const uint32_t i = c % lv.nx, j = (c / lv.nx) % lv.ny, k = c / (lv.nx * lv.ny);
-        f(c, i, j, k, sc);
-    };
+__device__ __forceinline__ void for_level(const Ctx& x, uint32_t l, const MgLevel& lv, bool local, uint32_t colour, F f) {
     if (local) {
         const SmallDiv dv(lv);
-        for (uint32_t c = threadIdx.x; c < lv.C; c += MG_THREADS) {
-            const float4 sc = ld_st(lv.st, c);
-            if (sc.x > 0.0f) {
-                uint32_t i, j, k;
-                dv.ijk(c, i, j, k);
-                f(c, i, j, k, sc);
-            }
+        const uint32_t n = x.sh.nloc[l][colour], at0 = local_at(x, l, colour, 0);
+        for (uint32_t e = threadIdx.x; e < n; e += MG_THREADS) {
+            const uint32_t c = x.sh.loc[colour ? at0 - e : at0 + e];
+            uint32_t i, j, k;
+            dv.ijk(c, i, j, k);
+            f(c, i, j, k, ld_st(lv.st, c));
         }
         return;
     }
+    auto ijk = [&](uint32_t c, uint32_t& i, uint32_t& j, uint32_t& k) {
+        i = c % lv.nx;
+        j = (c / lv.nx) % lv.ny;
+        k = c / (lv.nx * lv.ny);
+    };
     if (l == 1 && x.sh.list1) {
-        for (uint32_t e = threadIdx.x; e < x.sh.nl1; e += MG_THREADS) {
-            const uint32_t c = x.sh.l1[e];
-            visit(c, ld_st(lv.st, c));
+        const uint32_t n = x.sh.n1[colour];
+        for (uint32_t e = threadIdx.x; e < n; e += MG_THREADS) {
+            const uint32_t c = x.sh.l1[colour ? MG_L1 - 1 - e : e];
+            uint32_t i, j, k;
+            ijk(c, i, j, k);
+            f(c, i, j, k, ld_st(lv.st, c));
         }
         return;
     }
-    uint32_t lo, hi;
-    block_range(lv.C, lo, hi);
-    for (uint32_t c = lo + threadIdx.x; c < hi; c += MG_THREADS) {
+    const uint32_t n = share_size(lv.C);
+    for (uint32_t e = threadIdx.x; e < n; e += MG_THREADS) {
+        const uint32_t c = share_cell(e);
+        if (c >= lv.C) continue;
         const float4 sc = ld_st(lv.st, c);
-        if (sc.x > 0.0f) visit(c, sc);
+        uint32_t i, j, k;
+        ijk(c, i, j, k);
+        if (sc.x > 0.0f && ((i + j + k) & 1u) == colour) f(c, i, j, k, sc);
     }
 }
 
@@ -501,19 +525,20 @@ __device__ __forceinline__ void for_level8(const Ctx& x, uint32_t l, const MgLev
         t += __shfl_xor_sync(0xffffffffu, t, 4);
         if (valid && d == 0) g(I, t);
     };
-    if (!local && l == 1 && x.sh.list1) {
-        const uint32_t n = x.sh.nl1;
+    if (local || (l == 1 && x.sh.list1)) {  // the lists: reds, then blacks
+        const uint32_t nr = local ? x.sh.nloc[l][0] : x.sh.n1[0], n = nr + (local ? x.sh.nloc[l][1] : x.sh.n1[1]);
+        const uint32_t r0 = local ? local_at(x, l, 0, 0) : 0u, b0 = local ? local_at(x, l, 1, 0) : MG_L1 - 1u;
         for (uint32_t e0 = 0; e0 < n; e0 += per) {
-            const uint32_t e = e0 + slot;
-            one(e < n, e < n ? x.sh.l1[e] : 0u);
+            const uint32_t e = e0 + slot, at = e < nr ? r0 + e : b0 - (e - nr);
+            one(e < n, e < n ? (local ? (uint32_t)x.sh.loc[at] : x.sh.l1[at]) : 0u);
         }
         return;
     }
-    uint32_t lo = 0, hi = lv.C;
-    if (!local) block_range(lv.C, lo, hi);
-    for (uint32_t c0 = lo; c0 < hi; c0 += per) {
-        const uint32_t I = c0 + slot;
-        one(I < hi && ld_st(lv.st, I < hi ? I : lo).x > 0.0f, I);
+    const uint32_t n = share_size(lv.C);
+    for (uint32_t e0 = 0; e0 < n; e0 += per) {
+        const uint32_t e = e0 + slot, I = share_cell(e);
+        const bool in = e < n && I < lv.C;
+        one(in && ld_st(lv.st, in ? I : 0u).x > 0.0f, I);
     }
 }
 
@@ -606,24 +631,29 @@ __device__ Df post0_red(const Ctx& x) {
 
 // ---- coarse level passes (grid levels, or block 0's local levels) ----
 
+// Pre-smoothing from zero: red x = b/D, black x = (b + sum w b_nb/D_nb)/D.  Block
+// 0 alone puts a block barrier between the colours and reads the reds' quotients.
 __device__ void pre_l(const Ctx& x, uint32_t l, const MgLevel& lv, bool local) {
     const float4* st = lv.st;
-    for_level(x, l, lv, local, [&](uint32_t c, uint32_t i, uint32_t j, uint32_t k, float4 sc) {
-        float v = ld_any(lv.b + c);
-        if (((i + j + k) & 1u) != 0u) {
-            const NbC nb(st, sc, c, i, j, k, lv);
-            float bn[6], dn[6];
-            nb.load(lv.b, bn);
+    auto red = [&](uint32_t c, uint32_t, uint32_t, uint32_t, float4 sc) { lv.x[c] = lv.b[c] / sc.x; };
+    if (local) {
+        for_level(x, l, lv, local, 0, red);
+        __syncthreads();
+    }
+    for_level(x, l, lv, local, 1, [&](uint32_t c, uint32_t i, uint32_t j, uint32_t k, float4 sc) {
+        const NbC nb(st, sc, c, i, j, k, lv);
+        float bn[6], dn[6];
+        nb.load(local ? lv.x : lv.b, bn);
 #pragma unroll
-            for (int s = 0; s < 6; s++) dn[s] = ld_st(st, nb.n[s]).x;
-            float sum = 0.0f;
+        for (int s = 0; s < 6; s++) dn[s] = local ? 1.0f : ld_st(st, nb.n[s]).x;
+        const float bc = ld_any(lv.b + c);
+        float sum = 0.0f;
 #pragma unroll
-            for (int s = 0; s < 6; s++)
-                if (nb.w[s] != 0.0f) sum += nb.w[s] * (bn[s] / dn[s]);
-            v += sum;
-        }
-        lv.x[c] = v / sc.x;
+        for (int s = 0; s < 6; s++)
+            if (nb.w[s] != 0.0f) sum += nb.w[s] * (local ? bn[s] : bn[s] / dn[s]);
+        lv.x[c] = (bc + sum) / sc.x;
     });
+    if (!local) for_level(x, l, lv, local, 0, red);
 }
 
 __device__ void restrict_l(const Ctx& x, uint32_t l, const MgLevel& lv, const MgLevel& up, bool local) {
@@ -647,8 +677,7 @@ __device__ void restrict_l(const Ctx& x, uint32_t l, const MgLevel& lv, const Mg
 
 __device__ void post_black_l(const Ctx& x, uint32_t l, const MgLevel& lv, const MgLevel& up, bool local) {
     const float4* st = lv.st;
-    for_level(x, l, lv, local, [&](uint32_t c, uint32_t i, uint32_t j, uint32_t k, float4 sc) {
-        if (((i + j + k) & 1u) == 0u) return;
+    for_level(x, l, lv, local, 1, [&](uint32_t c, uint32_t i, uint32_t j, uint32_t k, float4 sc) {
         const NbC nb(st, sc, c, i, j, k, lv);
         const uint32_t pc = parent_at(i, j, k, up), unx = up.nx, unxy = up.nx * up.ny;
         // the neighbours' parents (the own one where there is no neighbour)
@@ -668,8 +697,7 @@ __device__ void post_black_l(const Ctx& x, uint32_t l, const MgLevel& lv, const 
 
 __device__ void post_red_l(const Ctx& x, uint32_t l, const MgLevel& lv, bool local) {
     const float4* st = lv.st;
-    for_level(x, l, lv, local, [&](uint32_t c, uint32_t i, uint32_t j, uint32_t k, float4 sc) {
-        if (((i + j + k) & 1u) != 0u) return;
+    for_level(x, l, lv, local, 0, [&](uint32_t c, uint32_t i, uint32_t j, uint32_t k, float4 sc) {
         const NbC nb(st, sc, c, i, j, k, lv);
         float xn[6];
         nb.load(lv.x, xn);
@@ -797,6 +825,29 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_mgpcg(DevBufs b, MgBufs m) {
     }
     Ctx x{sh, b, m, e0, nown, Lg, b.r, 0u, 0u, nullptr};
     build_lists(x);
+    if (blockIdx.x == 0) {  // the unknowns of the levels it runs alone
+        uint32_t off = 0;
+        for (uint32_t l = Lg; l < m.L; l++) {
+            const MgLevel& lv = m.lv[l];
+            uint32_t nr = 0, nb = 0;
+            for (uint32_t base = 0; base < lv.C; base += MG_THREADS) {
+                const uint32_t c = base + tid;
+                const bool u = c < lv.C && ld_st(lv.st, c).x > 0.0f;
+                const bool black = u && ((c % lv.nx + (c / lv.nx) % lv.ny + c / (lv.nx * lv.ny)) & 1u) != 0u;
+                uint32_t totr, totb;
+                const uint32_t pr = nr + block_rank(sh, u && !black, totr), pb = nb + block_rank(sh, u && black, totb);
+                if (u) sh.loc[black ? off + lv.C - 1 - pb : off + pr] = (uint16_t)c;
+                nr += totr;
+                nb += totb;
+            }
+            if (tid == 0) {
+                sh.nloc[l][0] = nr;
+                sh.nloc[l][1] = nb;
+            }
+            off += lv.C;
+        }
+        __syncthreads();
+    }
     if (b0_local && blockIdx.x == 0) {
         static_assert(sizeof(sh.cell) >= MG_LOCAL_TOTAL * sizeof(float4), "local stencils exceed the cell list");
         float4* lst = reinterpret_cast<float4*>(sh.cell);

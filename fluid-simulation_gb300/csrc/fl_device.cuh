@@ -314,6 +314,7 @@ cudaError_t launch_seed(const SeedArgs& a, float4* part, cudaStream_t s);
 constexpr int MG_MAX_LEVELS = 12;
 constexpr uint32_t MG_COARSE_CELLS = 64;  // the coarsest level holds at most this many cells
 constexpr uint32_t MG_BLOCK0_CELLS = 4096;  // levels this small run inside one block (block barriers)
+constexpr uint32_t MG_COUNTERS = 8;         // barrier counters
 constexpr uint32_t MG_LOCAL_TOTAL = 4800;   // cells of all those levels together (b, x in shared memory)
 struct MgLevel {
     uint32_t nx, ny, nz, C;
@@ -326,7 +327,7 @@ struct MgBufs {
     MgLevel lv[MG_MAX_LEVELS];
     float* r2;          // second residual buffer (level-0 size)
     float2* part;       // 2 x MAX_CG_BLOCKS float-float block partials
-    uint32_t* bar;      // barrier counter, zeroed before each solve
+    uint32_t* bar;      // MG_COUNTERS barrier counters, 128 bytes apart, zeroed before each solve
 };
 // Level sizes of an nx x ny x nz grid; returns L.
 FL_HD inline uint32_t mg_levels(uint32_t nx, uint32_t ny, uint32_t nz, uint32_t dims[MG_MAX_LEVELS][3]) {

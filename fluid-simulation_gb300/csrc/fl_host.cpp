@@ -196,7 +196,7 @@ fl_status mg_alloc(fl_handle* h, uint32_t nx, uint32_t ny, uint32_t nz, float* r
         o_x[l] = pl.take<float>(C);
     }
     const size_t o_r2 = pl.take<float>((size_t)nx * ny * nz);
-    const size_t o_part = pl.take<float2>(2 * 1024), o_bar = pl.take<uint32_t>(1);
+    const size_t o_part = pl.take<float2>(2 * 1024), o_bar = pl.take<uint32_t>(32 * fl::MG_COUNTERS);
     void* base = nullptr;
     cudaError_t e = cudaMalloc(&base, pl.off);
     if (e != cudaSuccess) {

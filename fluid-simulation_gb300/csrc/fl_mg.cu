@@ -60,17 +60,26 @@ constexpr int MG_COARSE_SWEEPS = 2;       // symmetric Gauss-Seidel sweeps on th
 // bits 10-12 the parities of i, j, k, bit 13 the colour (i+j+k)&1 (0 = red).
 constexpr uint32_t META_IODD = 1u << 10, META_JODD = 1u << 11, META_KODD = 1u << 12, META_BLACK = 1u << 13;
 
+// A level that block 0 runs alone, as its passes need it (set up once per
+// solve: deriving it in every pass cost more than the cells).
+struct LocalLevel {
+    MgLevel lv;               // vectors (and stencils) in shared memory
+    uint32_t mx, mxy;         // SmallDiv's reciprocals
+    uint32_t n[2], first[2];  // unknowns per colour, their places in MgShared::loc (blacks go down)
+};
+
 struct MgShared {
     uint32_t cell[MG_CELLS];
     uint16_t meta[MG_CELLS];
     uint32_t l1[MG_L1];
     float lb[MG_LOCAL_TOTAL], lx[MG_LOCAL_TOTAL];  // b and x of the levels block 0 runs alone
     uint16_t loc[MG_LOCAL_TOTAL];                  // and their unknowns, by colour
-    uint32_t nloc[MG_MAX_LEVELS][2];
+    LocalLevel local[MG_MAX_LEVELS];
     float2 red[MG_THREADS / 32];
     uint32_t wc[MG_THREADS / 32];
     float2 res;
     int ok;
+    uint64_t limit;  // of a wait, in ns
     uint32_t n0[2], n1[2], list0, list1;  // unknowns listed per colour: level 0, level 1
     // solve scalars kept here rather than in registers through the loop
     float2 rs0, thr, rz;
@@ -84,19 +93,15 @@ __device__ __forceinline__ uint32_t make_meta(uint32_t info, uint32_t c, uint32_
 
 __device__ __forceinline__ float diag0(uint32_t meta) { return (float)((meta >> 7) & 7u); }
 
-// Stencils and masks do not change during the solve: read-only cache; the
-// levels block 0 runs alone read their stencils from its shared-memory copy.
-__device__ __forceinline__ float4 ld_st(const float4* st, uint32_t c) {
-    return __isShared(st) ? st[c] : __ldg(st + c);
-}
+// Stencils and masks do not change during the solve: read-only cache.
 __device__ __forceinline__ uint32_t ld_ci(const uint16_t* ci, uint32_t c) { return __ldg(ci + c); }
 
 // The passes are chains of L2 loads, one cell or two per thread, so what a cell
 // costs is the number of loads that wait for one another.  Every load of a cell
 // is issued before the first value is used, and volatile: the compiler would
 // otherwise move each load behind the test that decides whether its value is
-// needed (each neighbour then waited for the one before: 105 us per iteration
-// on the 128^3 sphere-into-pool scene, against XXX).
+// needed (each neighbour then waited for the one before: 107 us per iteration
+// on the 128^3 sphere-into-pool scene, against 91; 69 with the lists below).
 __device__ __forceinline__ float ld_if(const float* p, bool on) {  // 0 when off
     float v;
     asm volatile("{\n.reg .pred q;\nsetp.ne.u32 q, %2, 0;\nmov.f32 %0, 0f00000000;\n@q ld.global.f32 %0, [%1];\n}"
@@ -111,9 +116,24 @@ __device__ __forceinline__ uint32_t ld_ci_if(const uint16_t* p, bool on) {
                  : "l"(p), "r"((uint32_t)on));
     return v;
 }
-__device__ __forceinline__ float ld_any(const float* p) {  // shared or global
+// Where a coarse level's vectors and stencils are: global memory, block 0's
+// shared memory, or (a grid of one block) vectors in shared memory and
+// stencils in global.
+enum Mem { GRID, LOCAL, LOCAL_ONE };
+template <Mem M>
+__device__ __forceinline__ float ld_x(const float* p) {
     float v;
-    asm volatile("ld.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    if (M == GRID) asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    else asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"((uint32_t)__cvta_generic_to_shared(p)));
+    return v;
+}
+template <Mem M>
+__device__ __forceinline__ float4 ld_st(const float4* p) {  // fixed during the solve: read-only cache
+    if (M != LOCAL) return __ldg(p);
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)));
     return v;
 }
 
@@ -147,6 +167,7 @@ __device__ __forceinline__ float quotient_sum(const Nb0& nb, const float (&v)[6]
 
 // A coarse cell's neighbours in the order +x, +y, +z, -x, -y, -z: indices (the
 // cell itself where the grid ends) and weights (0: not an unknown).
+template <Mem M>
 struct NbC {
     uint32_t n[6];
     float w[6];
@@ -159,7 +180,7 @@ struct NbC {
         n[3] = i ? c - 1 : c;
         n[4] = j ? c - nx : c;
         n[5] = k ? c - nxy : c;
-        const float wx = ld_st(st, n[3]).y, wy = ld_st(st, n[4]).z, wz = ld_st(st, n[5]).w;
+        const float wx = ld_st<M>(st + n[3]).y, wy = ld_st<M>(st + n[4]).z, wz = ld_st<M>(st + n[5]).w;
         w[0] = sc.y; w[1] = sc.z; w[2] = sc.w;
         w[3] = i ? wx : 0.0f;
         w[4] = j ? wy : 0.0f;
@@ -167,7 +188,7 @@ struct NbC {
     }
     __device__ __forceinline__ void load(const float* a, float (&v)[6]) const {
 #pragma unroll
-        for (int s = 0; s < 6; s++) v[s] = ld_any(a + n[s]);
+        for (int s = 0; s < 6; s++) v[s] = ld_x<M>(a + n[s]);
     }
     __device__ __forceinline__ float sum(const float (&v)[6]) const {
         float t = 0.0f;
@@ -192,36 +213,46 @@ struct Ctx {
     uint32_t e0, nown;  // this block's level-0 plan entries
     uint32_t Lg;        // first level run inside block 0 alone (>= 1)
     const float* r;     // the current residual (level 0's b)
-    uint32_t epoch;     // barrier target
+    uint32_t epoch;     // barriers so far
     uint32_t parity;    // exchange slot parity
     float4* lst;        // block 0: shared-memory copy of the stencils of levels Lg.. (nullptr: global)
 };
 
+// Block bb arrives at counter bb mod MG_COUNTERS (each on its own line: 152
+// arrivals at one address follow one another); lane k of warp 0 waits for
+// counter k.
 __device__ bool mg_barrier(Ctx& x) {
     __syncthreads();
-    x.epoch += gridDim.x;
-    if (threadIdx.x == 0) {
+    x.epoch++;
+    if (threadIdx.x < 32) {
+        const uint32_t k = threadIdx.x;
         // the release add orders the block's writes (before the barrier
         // above) ahead of the arrival; a separate fence only added its wait
-        red_release_add(x.m.bar, 1u);
+        if (k == 0) red_release_add(x.m.bar + (blockIdx.x % MG_COUNTERS) * 32u, 1u);
+        __syncwarp();
         bool ok = true;
-        const uint64_t t0 = global_ns(), limit = wait_limit_ns(x.b.prm);
-        uint32_t spins = 0;
-        while (ld_acquire(x.m.bar) < x.epoch) {
-            // clock on the first re-poll and every 64 polls, status every 64
-            ++spins;
-            const bool slow = (spins & 63u) == 0u;
-            if (slow && *(volatile uint32_t*)&x.b.st->status != 0u) {
-                ok = false;
-                break;
-            }
-            if ((slow || spins == 1u) && global_ns() - t0 > limit) {
-                atomicCAS(&x.b.st->status, 0u, 5u /* FL_TIMEOUT */);
-                ok = false;
-                break;
+        if (k < MG_COUNTERS) {
+            const uint32_t* const bar = x.m.bar + k * 32u;
+            const uint32_t target = x.epoch * ((gridDim.x + MG_COUNTERS - 1 - k) / MG_COUNTERS);
+            const uint64_t t0 = global_ns();
+            uint32_t spins = 0;
+            while (ld_acquire(bar) < target) {
+                // clock on the first re-poll and every 64 polls, status every 64
+                ++spins;
+                const bool slow = (spins & 63u) == 0u;
+                if (slow && *(volatile uint32_t*)&x.b.st->status != 0u) {
+                    ok = false;
+                    break;
+                }
+                if ((slow || spins == 1u) && global_ns() - t0 > x.sh.limit) {
+                    atomicCAS(&x.b.st->status, 0u, 5u /* FL_TIMEOUT */);
+                    ok = false;
+                    break;
+                }
             }
         }
-        x.sh.ok = ok;
+        ok = __all_sync(0xffffffffu, ok);
+        if (k == 0) x.sh.ok = ok;
     }
     __syncthreads();
     return x.sh.ok != 0;
@@ -321,7 +352,7 @@ __device__ void build_lists(Ctx& x) {
     const uint32_t n1 = share_size(l1.C);
     for (uint32_t base = 0; base < n1; base += MG_THREADS) {
         const uint32_t e = base + threadIdx.x, I = share_cell(e);
-        const bool u = e < n1 && I < l1.C && ld_st(l1.st, I).x > 0.0f;
+        const bool u = e < n1 && I < l1.C && ld_st<GRID>(l1.st + I).x > 0.0f;
         const bool black = u && ((I % l1.nx + (I / l1.nx) % l1.ny + I / (l1.nx * l1.ny)) & 1u) != 0u;
         uint32_t totr, totb;
         const uint32_t pr = n1r + block_rank(sh, u && !black, totr), pb = n1b + block_rank(sh, u && black, totb);
@@ -377,8 +408,8 @@ __device__ __forceinline__ void for_own(const Ctx& x, uint32_t colour, F f) {
 struct SmallDiv {
     uint32_t nx, nxy, mx, mxy;
     __device__ __forceinline__ static uint32_t recip(uint32_t d) { return d > 1u ? 0xffffffffu / d + 1u : 0u; }
-    __device__ __forceinline__ explicit SmallDiv(const MgLevel& lv)
-        : nx(lv.nx), nxy(lv.nx * lv.ny), mx(recip(lv.nx)), mxy(recip(lv.nx * lv.ny)) {}
+    __device__ __forceinline__ explicit SmallDiv(const LocalLevel& l)
+        : nx(l.lv.nx), nxy(l.lv.nx * l.lv.ny), mx(l.mx), mxy(l.mxy) {}
     __device__ __forceinline__ void ijk(uint32_t c, uint32_t& i, uint32_t& j, uint32_t& k) const {
         k = mxy ? __umulhi(c, mxy) : c;
         const uint32_t rem = c - k * nxy;
@@ -388,24 +419,18 @@ struct SmallDiv {
 };
 static_assert((uint64_t)MG_BLOCK0_CELLS * MG_BLOCK0_CELLS < (1ull << 32), "SmallDiv needs c * divisor < 2^32");
 
-// Block 0's unknowns of local level l: position of the e-th of a colour in its lists.
-__device__ __forceinline__ uint32_t local_at(const Ctx& x, uint32_t l, uint32_t colour, uint32_t e) {
-    uint32_t off = 0;
-    for (uint32_t k = x.Lg; k < l; k++) off += x.m.lv[k].C;
-    return colour ? off + x.m.lv[l].C - 1 - e : off + e;
-}
-
 // colour: 0 red, 1 black.
-template <class F>
-__device__ __forceinline__ void for_level(const Ctx& x, uint32_t l, const MgLevel& lv, bool local, uint32_t colour, F f) {
-    if (local) {
-        const SmallDiv dv(lv);
-        const uint32_t n = x.sh.nloc[l][colour], at0 = local_at(x, l, colour, 0);
+template <Mem M, class F>
+__device__ __forceinline__ void for_level(const Ctx& x, uint32_t l, const MgLevel& lv, uint32_t colour, F f) {
+    if (M != GRID) {
+        const LocalLevel& ll = x.sh.local[l];
+        const SmallDiv dv(ll);
+        const uint32_t n = ll.n[colour], at0 = ll.first[colour];
         for (uint32_t e = threadIdx.x; e < n; e += MG_THREADS) {
             const uint32_t c = x.sh.loc[colour ? at0 - e : at0 + e];
             uint32_t i, j, k;
             dv.ijk(c, i, j, k);
-            f(c, i, j, k, ld_st(lv.st, c));
+            f(c, i, j, k, ld_st<M>(lv.st + c));
         }
         return;
     }
@@ -420,7 +445,7 @@ __device__ __forceinline__ void for_level(const Ctx& x, uint32_t l, const MgLeve
             const uint32_t c = x.sh.l1[colour ? MG_L1 - 1 - e : e];
             uint32_t i, j, k;
             ijk(c, i, j, k);
-            f(c, i, j, k, ld_st(lv.st, c));
+            f(c, i, j, k, ld_st<M>(lv.st + c));
         }
         return;
     }
@@ -428,7 +453,7 @@ __device__ __forceinline__ void for_level(const Ctx& x, uint32_t l, const MgLeve
     for (uint32_t e = threadIdx.x; e < n; e += MG_THREADS) {
         const uint32_t c = share_cell(e);
         if (c >= lv.C) continue;
-        const float4 sc = ld_st(lv.st, c);
+        const float4 sc = ld_st<GRID>(lv.st + c);
         uint32_t i, j, k;
         ijk(c, i, j, k);
         if (sc.x > 0.0f && ((i + j + k) & 1u) == colour) f(c, i, j, k, sc);
@@ -502,11 +527,13 @@ __device__ Df update_pre0(const Ctx& x, float alpha, const float* d, float* r_ne
 // consecutive lanes per cell: f(I, ii, jj, kk, child d = lane & 7) returns the
 // child's term, the eight terms are summed in a fixed shuffle order and
 // g(I, sum) runs on the first lane.  A cell's children are visited together.
-template <class F, class G>
-__device__ __forceinline__ void for_level8(const Ctx& x, uint32_t l, const MgLevel& lv, bool local, F f, G g) {
+template <Mem M, class F, class G>
+__device__ __forceinline__ void for_level8(const Ctx& x, uint32_t l, const MgLevel& lv, F f, G g) {
+    constexpr bool local = M != GRID;
     const uint32_t d = threadIdx.x & 7u, slot = threadIdx.x >> 3;
     constexpr uint32_t per = MG_THREADS / 8;
-    const SmallDiv dv(lv);  // used for local levels only (at most MG_BLOCK0_CELLS cells)
+    const LocalLevel& ll = x.sh.local[l];
+    const SmallDiv dv(ll);  // used for local levels only (at most MG_BLOCK0_CELLS cells)
     auto one = [&](bool valid, uint32_t I) {
         float t = 0.0f;
         if (valid) {
@@ -526,8 +553,8 @@ __device__ __forceinline__ void for_level8(const Ctx& x, uint32_t l, const MgLev
         if (valid && d == 0) g(I, t);
     };
     if (local || (l == 1 && x.sh.list1)) {  // the lists: reds, then blacks
-        const uint32_t nr = local ? x.sh.nloc[l][0] : x.sh.n1[0], n = nr + (local ? x.sh.nloc[l][1] : x.sh.n1[1]);
-        const uint32_t r0 = local ? local_at(x, l, 0, 0) : 0u, b0 = local ? local_at(x, l, 1, 0) : MG_L1 - 1u;
+        const uint32_t nr = local ? ll.n[0] : x.sh.n1[0], n = nr + (local ? ll.n[1] : x.sh.n1[1]);
+        const uint32_t r0 = local ? ll.first[0] : 0u, b0 = local ? ll.first[1] : MG_L1 - 1u;
         for (uint32_t e0 = 0; e0 < n; e0 += per) {
             const uint32_t e = e0 + slot, at = e < nr ? r0 + e : b0 - (e - nr);
             one(e < n, e < n ? (local ? (uint32_t)x.sh.loc[at] : x.sh.l1[at]) : 0u);
@@ -538,7 +565,7 @@ __device__ __forceinline__ void for_level8(const Ctx& x, uint32_t l, const MgLev
     for (uint32_t e0 = 0; e0 < n; e0 += per) {
         const uint32_t e = e0 + slot, I = share_cell(e);
         const bool in = e < n && I < lv.C;
-        one(in && ld_st(lv.st, in ? I : 0u).x > 0.0f, I);
+        one(in && ld_st<GRID>(lv.st + (in ? I : 0u)).x > 0.0f, I);
     }
 }
 
@@ -550,8 +577,8 @@ __device__ void restrict0(const Ctx& x) {
     const uint16_t* ci = x.b.cinfo;
     const float* z = x.m.lv[0].x;
     const MgLevel& up = x.m.lv[1];
-    for_level8(
-        x, 1, up, false,
+    for_level8<GRID>(
+        x, 1, up,
         [&](uint32_t, uint32_t ii, uint32_t jj, uint32_t kk, uint32_t d) {
             const uint32_t i = 2 * ii + (d & 1), j = 2 * jj + ((d >> 1) & 1), k = 2 * kk + (d >> 2);
             if (i >= nx || j >= ny || k >= nz) return 0.0f;
@@ -633,41 +660,44 @@ __device__ Df post0_red(const Ctx& x) {
 
 // Pre-smoothing from zero: red x = b/D, black x = (b + sum w b_nb/D_nb)/D.  Block
 // 0 alone puts a block barrier between the colours and reads the reds' quotients.
-__device__ void pre_l(const Ctx& x, uint32_t l, const MgLevel& lv, bool local) {
+template <Mem M>
+__device__ void pre_l(const Ctx& x, uint32_t l, const MgLevel& lv) {
     const float4* st = lv.st;
     auto red = [&](uint32_t c, uint32_t, uint32_t, uint32_t, float4 sc) { lv.x[c] = lv.b[c] / sc.x; };
+    constexpr bool local = M != GRID;
     if (local) {
-        for_level(x, l, lv, local, 0, red);
+        for_level<M>(x, l, lv, 0, red);
         __syncthreads();
     }
-    for_level(x, l, lv, local, 1, [&](uint32_t c, uint32_t i, uint32_t j, uint32_t k, float4 sc) {
-        const NbC nb(st, sc, c, i, j, k, lv);
+    for_level<M>(x, l, lv, 1, [&](uint32_t c, uint32_t i, uint32_t j, uint32_t k, float4 sc) {
+        const NbC<M> nb(st, sc, c, i, j, k, lv);
         float bn[6], dn[6];
         nb.load(local ? lv.x : lv.b, bn);
 #pragma unroll
-        for (int s = 0; s < 6; s++) dn[s] = local ? 1.0f : ld_st(st, nb.n[s]).x;
-        const float bc = ld_any(lv.b + c);
+        for (int s = 0; s < 6; s++) dn[s] = local ? 1.0f : ld_st<M>(st + nb.n[s]).x;
+        const float bc = ld_x<M>(lv.b + c);
         float sum = 0.0f;
 #pragma unroll
         for (int s = 0; s < 6; s++)
             if (nb.w[s] != 0.0f) sum += nb.w[s] * (local ? bn[s] : bn[s] / dn[s]);
         lv.x[c] = (bc + sum) / sc.x;
     });
-    if (!local) for_level(x, l, lv, local, 0, red);
+    if (!local) for_level<M>(x, l, lv, 0, red);
 }
 
-__device__ void restrict_l(const Ctx& x, uint32_t l, const MgLevel& lv, const MgLevel& up, bool local) {
+template <Mem M>
+__device__ void restrict_l(const Ctx& x, uint32_t l, const MgLevel& lv, const MgLevel& up) {
     const float4* st = lv.st;
-    for_level8(
-        x, l + 1, up, local,
+    for_level8<M>(
+        x, l + 1, up,
         [&](uint32_t, uint32_t ii, uint32_t jj, uint32_t kk, uint32_t d) {
             const uint32_t i = 2 * ii + (d & 1), j = 2 * jj + ((d >> 1) & 1), k = 2 * kk + (d >> 2);
             if (i >= lv.nx || j >= lv.ny || k >= lv.nz) return 0.0f;
             const uint32_t c = i + lv.nx * (j + lv.ny * k);
-            const float4 sc = ld_st(st, c);
-            const float bc = ld_any(lv.b + c), xc = ld_any(lv.x + c);
+            const float4 sc = ld_st<M>(st + c);
+            const float bc = ld_x<M>(lv.b + c), xc = ld_x<M>(lv.x + c);
             if (!(sc.x > 0.0f)) return 0.0f;
-            const NbC nb(st, sc, c, i, j, k, lv);
+            const NbC<M> nb(st, sc, c, i, j, k, lv);
             float xn[6];
             nb.load(lv.x, xn);
             return bc - (sc.x * xc - nb.sum(xn));
@@ -675,10 +705,11 @@ __device__ void restrict_l(const Ctx& x, uint32_t l, const MgLevel& lv, const Mg
         [&](uint32_t I, float s) { up.b[I] = s; });
 }
 
-__device__ void post_black_l(const Ctx& x, uint32_t l, const MgLevel& lv, const MgLevel& up, bool local) {
+template <Mem M>
+__device__ void post_black_l(const Ctx& x, uint32_t l, const MgLevel& lv, const MgLevel& up) {
     const float4* st = lv.st;
-    for_level(x, l, lv, local, 1, [&](uint32_t c, uint32_t i, uint32_t j, uint32_t k, float4 sc) {
-        const NbC nb(st, sc, c, i, j, k, lv);
+    for_level<M>(x, l, lv, 1, [&](uint32_t c, uint32_t i, uint32_t j, uint32_t k, float4 sc) {
+        const NbC<M> nb(st, sc, c, i, j, k, lv);
         const uint32_t pc = parent_at(i, j, k, up), unx = up.nx, unxy = up.nx * up.ny;
         // the neighbours' parents (the own one where there is no neighbour)
         const uint32_t pn[6] = {nb.n[0] != c && (i & 1u) ? pc + 1 : pc,       nb.n[1] != c && (j & 1u) ? pc + unx : pc,
@@ -687,67 +718,57 @@ __device__ void post_black_l(const Ctx& x, uint32_t l, const MgLevel& lv, const 
         float xn[6], en[6];
         nb.load(lv.x, xn);
 #pragma unroll
-        for (int s = 0; s < 6; s++) en[s] = ld_any(up.x + pn[s]);
-        const float bc = ld_any(lv.b + c);
+        for (int s = 0; s < 6; s++) en[s] = ld_x<M>(up.x + pn[s]);
+        const float bc = ld_x<M>(lv.b + c);
 #pragma unroll
         for (int s = 0; s < 6; s++) xn[s] += en[s];
         lv.x[c] = (bc + nb.sum(xn)) / sc.x;
     });
 }
 
-__device__ void post_red_l(const Ctx& x, uint32_t l, const MgLevel& lv, bool local) {
+template <Mem M>
+__device__ void post_red_l(const Ctx& x, uint32_t l, const MgLevel& lv) {
     const float4* st = lv.st;
-    for_level(x, l, lv, local, 0, [&](uint32_t c, uint32_t i, uint32_t j, uint32_t k, float4 sc) {
-        const NbC nb(st, sc, c, i, j, k, lv);
+    for_level<M>(x, l, lv, 0, [&](uint32_t c, uint32_t i, uint32_t j, uint32_t k, float4 sc) {
+        const NbC<M> nb(st, sc, c, i, j, k, lv);
         float xn[6];
         nb.load(lv.x, xn);
-        const float bc = ld_any(lv.b + c);
+        const float bc = ld_x<M>(lv.b + c);
         lv.x[c] = (bc + nb.sum(xn)) / sc.x;
     });
-}
-
-// Block 0's view of level l >= Lg: b, x and (with more than one block) the
-// stencil in shared memory.
-__device__ __forceinline__ MgLevel local_level(const Ctx& x, uint32_t l) {
-    MgLevel v = x.m.lv[l];
-    uint32_t off = 0;
-    for (uint32_t k = x.Lg; k < l; k++) off += x.m.lv[k].C;
-    v.b = x.sh.lb + off;
-    v.x = x.sh.lx + off;
-    if (x.lst) v.st = x.lst + off;
-    return v;
 }
 
 // Levels Lg .. L-1 by block 0 alone (block barriers instead of grid
 // barriers): V-cycle with symmetric Gauss-Seidel sweeps from zero on the
 // coarsest level.
+template <Mem M>
 __device__ void local_cycle(const Ctx& x) {
     const uint32_t L = x.m.L, Lg = x.Lg;
     {
-        const MgLevel g = x.m.lv[Lg], s = local_level(x, Lg);
+        const MgLevel g = x.m.lv[Lg], s = x.sh.local[Lg].lv;
         for (uint32_t c = threadIdx.x; c < g.C; c += MG_THREADS) s.b[c] = g.b[c];
         __syncthreads();
     }
     for (uint32_t l = Lg; l + 1 < L; l++) {
-        const MgLevel lv = local_level(x, l), up = local_level(x, l + 1);
-        pre_l(x, l, lv, true);
+        const MgLevel lv = x.sh.local[l].lv, up = x.sh.local[l + 1].lv;
+        pre_l<M>(x, l, lv);
         __syncthreads();
-        restrict_l(x, l, lv, up, true);
+        restrict_l<M>(x, l, lv, up);
         __syncthreads();
     }
     {
-        const MgLevel lv = local_level(x, L - 1);
+        const MgLevel lv = x.sh.local[L - 1].lv;
         const uint32_t t = threadIdx.x, nx = lv.nx, ny = lv.ny, nxy = nx * ny;
         uint32_t i = 0, j = 0, k = 0, col = 0;
         float4 sc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (t < lv.C) {
             i = t % nx; j = (t / nx) % ny; k = t / nxy;
             col = (i + j + k) & 1u;
-            sc = ld_st(lv.st, t);
+            sc = ld_st<M>(lv.st + t);
             lv.x[t] = 0.0f;
         }
         const uint32_t at = t < lv.C ? t : 0u;
-        const NbC nb(lv.st, sc, at, i, j, k, lv);
+        const NbC<M> nb(lv.st, sc, at, i, j, k, lv);
         const float bt = lv.b[at];
         __syncthreads();
         for (int h = 0; h < 4 * MG_COARSE_SWEEPS; h++) {
@@ -762,14 +783,14 @@ __device__ void local_cycle(const Ctx& x) {
         }
     }
     for (uint32_t l = L - 1; l-- > Lg;) {
-        const MgLevel lv = local_level(x, l), up = local_level(x, l + 1);
-        post_black_l(x, l, lv, up, true);
+        const MgLevel lv = x.sh.local[l].lv, up = x.sh.local[l + 1].lv;
+        post_black_l<M>(x, l, lv, up);
         __syncthreads();
-        post_red_l(x, l, lv, true);
+        post_red_l<M>(x, l, lv);
         __syncthreads();
     }
     {
-        const MgLevel g = x.m.lv[Lg], s = local_level(x, Lg);
+        const MgLevel g = x.m.lv[Lg], s = x.sh.local[Lg].lv;
         for (uint32_t c = threadIdx.x; c < g.C; c += MG_THREADS) g.x[c] = s.x[c];
     }
 }
@@ -786,17 +807,20 @@ __device__ bool vcycle(Ctx& x, Df& rz, bool presmoothed) {
     restrict0(x);
     if (!mg_barrier(x)) return false;
     for (uint32_t l = 1; l < Lg; l++) {
-        pre_l(x, l, m.lv[l], false);
+        pre_l<GRID>(x, l, m.lv[l]);
         if (!mg_barrier(x)) return false;
-        restrict_l(x, l, m.lv[l], m.lv[l + 1], false);
+        restrict_l<GRID>(x, l, m.lv[l], m.lv[l + 1]);
         if (!mg_barrier(x)) return false;
     }
-    if (blockIdx.x == 0) local_cycle(x);
+    if (blockIdx.x == 0) {
+        if (x.lst) local_cycle<LOCAL>(x);
+        else local_cycle<LOCAL_ONE>(x);
+    }
     if (!mg_barrier(x)) return false;
     for (uint32_t l = Lg; l-- > 1;) {
-        post_black_l(x, l, m.lv[l], m.lv[l + 1], false);
+        post_black_l<GRID>(x, l, m.lv[l], m.lv[l + 1]);
         if (!mg_barrier(x)) return false;
-        post_red_l(x, l, m.lv[l], false);
+        post_red_l<GRID>(x, l, m.lv[l]);
         if (!mg_barrier(x)) return false;
     }
     post0_black(x);
@@ -824,6 +848,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_mgpcg(DevBufs b, MgBufs m) {
         nown = start[pb + 1] - start[pb];
     }
     Ctx x{sh, b, m, e0, nown, Lg, b.r, 0u, 0u, nullptr};
+    if (tid == 0) sh.limit = wait_limit_ns(&P);
     build_lists(x);
     if (blockIdx.x == 0) {  // the unknowns of the levels it runs alone
         uint32_t off = 0;
@@ -832,7 +857,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_mgpcg(DevBufs b, MgBufs m) {
             uint32_t nr = 0, nb = 0;
             for (uint32_t base = 0; base < lv.C; base += MG_THREADS) {
                 const uint32_t c = base + tid;
-                const bool u = c < lv.C && ld_st(lv.st, c).x > 0.0f;
+                const bool u = c < lv.C && ld_st<GRID>(lv.st + c).x > 0.0f;
                 const bool black = u && ((c % lv.nx + (c / lv.nx) % lv.ny + c / (lv.nx * lv.ny)) & 1u) != 0u;
                 uint32_t totr, totb;
                 const uint32_t pr = nr + block_rank(sh, u && !black, totr), pb = nb + block_rank(sh, u && black, totb);
@@ -841,8 +866,17 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_mgpcg(DevBufs b, MgBufs m) {
                 nb += totb;
             }
             if (tid == 0) {
-                sh.nloc[l][0] = nr;
-                sh.nloc[l][1] = nb;
+                LocalLevel& ll = sh.local[l];
+                ll.lv = lv;
+                ll.lv.b = sh.lb + off;
+                ll.lv.x = sh.lx + off;
+                if (b0_local) ll.lv.st = reinterpret_cast<float4*>(sh.cell) + off;
+                ll.mx = SmallDiv::recip(lv.nx);
+                ll.mxy = SmallDiv::recip(lv.nx * lv.ny);
+                ll.n[0] = nr;
+                ll.n[1] = nb;
+                ll.first[0] = off;
+                ll.first[1] = off + lv.C - 1;
             }
             off += lv.C;
         }
@@ -853,7 +887,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_mgpcg(DevBufs b, MgBufs m) {
         float4* lst = reinterpret_cast<float4*>(sh.cell);
         uint32_t off = 0;
         for (uint32_t l = Lg; l < m.L; l++) {
-            for (uint32_t c = tid; c < m.lv[l].C; c += MG_THREADS) lst[off + c] = ld_st(m.lv[l].st, c);
+            for (uint32_t c = tid; c < m.lv[l].C; c += MG_THREADS) lst[off + c] = ld_st<GRID>(m.lv[l].st + c);
             off += m.lv[l].C;
         }
         x.lst = lst;
@@ -1002,7 +1036,7 @@ cudaError_t launch_mgpcg(const DevBufs& b, const MgBufs& m, const LaunchCfg& L, 
     // level-0 cells go to blocks 1..G-1 (block 0 runs the coarse levels)
     cudaError_t e = launch_cg_plan(b, L.cg_blocks > 1 ? (uint32_t)L.cg_blocks - 1 : 1u, s);
     if (e != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(m.bar, 0, sizeof(uint32_t), s)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(m.bar, 0, MG_COUNTERS * 128, s)) != cudaSuccess) return e;
     const int gb = L.num_sms * 8;
     k_mg_agg0<<<gb, 256, 0, s>>>(b, m);
     for (uint32_t l = 1; l + 1 < m.L; l++) k_mg_agg<<<gb, 256, 0, s>>>(m, l);

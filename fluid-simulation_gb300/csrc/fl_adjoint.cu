@@ -405,12 +405,19 @@ __global__ void __launch_bounds__(1024) k_adj_thr(const float2* __restrict__ par
 }
 
 // Face stage: projection (divergence transposed), boundaries, forces, save_vel.
-__global__ void __launch_bounds__(256) k_adj_faces(AdjBufs a, int axis) {
+// One launch for the three axes (blockIdx.y).  A warp without a face that
+// gravity acts on skips the double sums: the FP64 pipe does about two lane
+// operations per clock and SM, and summing zeros there was four fifths of the
+// 39 us that each axis took at 128^3.
+__global__ void __launch_bounds__(256) k_adj_faces(AdjBufs a) {
     __shared__ double s_red[8];
     const DevParams& P = *a.prm;
+    const int axis = (int)blockIdx.y;
     const uint32_t nf = P.F3[axis];
+    if (blockIdx.x * blockDim.x >= nf) return;
     const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
-    double gg = 0.0;
+    float gpre = 0.0f;
+    bool wet_face = false;
     if (f < nf) {
         const uint32_t dx = face_dim(P, axis, 0), dy = face_dim(P, axis, 1);
         const uint32_t i = f % dx, j = (f / dx) % dy, k = f / (dx * dy);
@@ -421,7 +428,6 @@ __global__ void __launch_bounds__(256) k_adj_faces(AdjBufs a, int axis) {
         const uint8_t tl = comp > 0 ? a.ct[hi_c - step] : CELL_SOLID;
         const uint8_t th = comp < nax ? a.ct[hi_c] : CELL_SOLID;
         const bool solid = comp == 0 || comp == nax || tl == CELL_SOLID || th == CELL_SOLID;
-        float gpre = 0.0f;
         if (!solid) {
             // vel_final = vel_pre - coeff*(p_hi - p_lo) on gradient faces; p = A^-1(-scale*div(vel_pre))
             const float2 gfs = a.g_fs[axis][f];
@@ -431,20 +437,25 @@ __global__ void __launch_bounds__(256) k_adj_faces(AdjBufs a, int axis) {
             if (th == CELL_LIQUID) dl -= a.lam[hi_c];
             g += -P.scale_rhs * P.inv_h * dl;
             gpre = g;
-            const bool wet = tl == CELL_LIQUID || th == CELL_LIQUID;
-            if (wet) gg = (double)gpre * (double)P.dt;
+            wet_face = tl == CELL_LIQUID || th == CELL_LIQUID;
         }
         a.g_norm[axis][f] = gpre + a.g_fs[axis][f].y;
     }
     // dL/dg_axis: the block's partial in a fixed order (k_adj_grav sums the
     // blocks' partials in order)
+    const bool some = __any_sync(0xffffffffu, wet_face);
+    if (some) {
+        double gg = wet_face ? (double)gpre * (double)P.dt : 0.0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) gg += __shfl_down_sync(0xffffffffu, gg, o);
-    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = gg;
-    __syncthreads();
+        for (int o = 16; o > 0; o >>= 1) gg += __shfl_down_sync(0xffffffffu, gg, o);
+        if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = gg;
+    } else if ((threadIdx.x & 31) == 0) {
+        s_red[threadIdx.x >> 5] = 0.0;
+    }
+    const bool block_some = __syncthreads_or(some);
     if (threadIdx.x == 0) {
         double s = 0.0;
-        for (int w = 0; w < 8; w++) s += s_red[w];
+        for (int w = 0; block_some && w < 8; w++) s += s_red[w];
         a.grav_part[axis][blockIdx.x] = s;
     }
 }
@@ -516,38 +527,31 @@ __global__ void __launch_bounds__(256) k_adj_mid(AdjBufs a) {
 //   g_fs = {sum w gpic/W, sum w gsaved/W}  (0 on faces touching the static
 //          walls, which the wall-aware gathers skip) + the midpoint stencil's sum,
 //   wsum = {sum w, sum w v_axis}  (every in-range tap, like scatter.wgsl).
-// Candidates read the compact record {q, v_x} (16 B); the rest of a
-// particle's record only when it has a tap among the faces.
-__global__ void __launch_bounds__(256) k_adj_gather(AdjBufs a, int midpoint) {
-    const DevParams& P = *a.prm;
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= P.C) return;
+//
+// Without strays a particle's cell is its bin, so its offset from the thread's
+// cell is the loop's, and each weight is one expression of the fraction
+// (gather_bins).  Deriving the stencil of every candidate instead took 717 us
+// of the 128^3 adjoint step (2.0 M particles, issue-bound: 120 instructions a
+// candidate, 27 cells of them per thread).  Steps with strays and the cells of
+// the grid's high sides keep that general form (gather_any).
+
+struct FaceSums {
+    float gf[6], gs[6], W[6], WV[6];  // low faces of axis 0..2, high-side faces of axis 0..2
+};
+
+__device__ __noinline__ void gather_any(const AdjBufs& a, const DevParams& P, int i, int j, int k, int rad, FaceSums& o) {
     const int nx = (int)P.nx, ny = (int)P.ny, nz = (int)P.nz;
-    const int i = (int)(c % (uint32_t)nx), j = (int)((c / (uint32_t)nx) % (uint32_t)ny), k = (int)(c / ((uint32_t)nx * ny));
     const int cc[3] = {i, j, k}, n3[3] = {nx, ny, nz};
-    // faces: 0..2 the low faces of axis 0..2, 3..5 the high-side faces of axis 0..2
-    bool has[6];
-    int fc[6][3];
-    bool wall[6];
-#pragma unroll
-    for (int e = 0; e < 6; e++) {
-        const int ax = e % 3;
-#pragma unroll
-        for (int b = 0; b < 3; b++) fc[e][b] = cc[b] + (e >= 3 && b == ax ? 1 : 0);
-        has[e] = e < 3 || cc[ax] == n3[ax] - 1;
-        wall[e] = touches_static_a(ax, fc[e][0], fc[e][1], fc[e][2], nx, ny, nz);
-    }
-    const int rad = a.flags[0] ? 2 : 1;
     int lo[3], hi[3];
+    bool has[6];
+#pragma unroll
+    for (int e = 0; e < 6; e++) has[e] = e < 3 || cc[e % 3] == n3[e % 3] - 1;
 #pragma unroll
     for (int b = 0; b < 3; b++) {
         lo[b] = max(cc[b] - rad, 0);
         hi[b] = min(cc[b] + rad, n3[b] - 1);
     }
     const uint32_t n = P.n, C = P.C;
-    float gf[6], gs[6], W[6], WV[6];
-#pragma unroll
-    for (int e = 0; e < 6; e++) gf[e] = gs[e] = W[e] = WV[e] = 0.0f;
     for (int ck = lo[2]; ck <= hi[2]; ck++) {
         for (int cj = lo[1]; cj <= hi[1]; cj++) {
             const uint32_t row = (uint32_t)nx * ((uint32_t)cj + (uint32_t)ny * (uint32_t)ck);
@@ -589,27 +593,106 @@ __global__ void __launch_bounds__(256) k_adj_gather(AdjBufs a, int midpoint) {
                 for (int e = 0; e < 6; e++) {
                     const int ax = e % 3;
                     if (w[e] == 0.0f) continue;  // not a tap (a tap of weight 0 adds nothing either)
-                    W[e] += w[e];
-                    WV[e] += w[e] * v[ax];
-                    if (!wall[e]) {
-                        gf[e] += w[e] * cf[ax];
-                        gs[e] += w[e] * cs[ax];
+                    o.W[e] += w[e];
+                    o.WV[e] += w[e] * v[ax];
+                    o.gf[e] += w[e] * cf[ax];
+                    o.gs[e] += w[e] * cs[ax];
+                }
+            }
+        }
+    }
+}
+
+// Weight of the tap at face coordinate cc for a particle at fraction f of cell
+// cc + o: along the face's axis, and across it.
+__device__ __forceinline__ float tap_along(int o, float f) { return o == 0 ? 1.0f - f : (o < 0 ? f : 0.0f); }
+__device__ __forceinline__ float tap_across(int o, float f) {
+    return o == 0 ? 1.0f - fabsf(f - 0.5f) : fmaxf(o < 0 ? f - 0.5f : 0.5f - f, 0.0f);
+}
+
+__device__ __forceinline__ FaceSums gather_bins(const AdjBufs& a, const DevParams& P, int i, int j, int k) {
+    FaceSums o = {};
+    const int nx = (int)P.nx, ny = (int)P.ny, nz = (int)P.nz;
+    const uint32_t n = P.n, C = P.C;
+    for (int oz = -1; oz <= 1; oz++) {
+        const int ck = k + oz;
+        if (ck < 0 || ck >= nz) continue;
+        for (int oy = -1; oy <= 1; oy++) {
+            const int cj = j + oy;
+            if (cj < 0 || cj >= ny) continue;
+            const uint32_t c = (uint32_t)nx * ((uint32_t)cj + (uint32_t)ny * (uint32_t)ck) + (uint32_t)i;
+            // first particle of the row's cells i - 1, i, i + 1, and the end
+            uint32_t at[4];
+            at[1] = a.cell_first[c];
+            at[0] = i > 0 ? a.cell_first[c - 1] : at[1];
+            at[2] = c + 1 < C ? a.cell_first[c + 1] : n;
+            at[3] = i + 1 < nx ? (c + 2 < C ? a.cell_first[c + 2] : n) : at[2];
+            const float fj = (float)cj, fk = (float)ck;
+#pragma unroll
+            for (int ox = -1; ox <= 1; ox++) {
+                const float fi = (float)(i + ox);
+                for (uint32_t d = at[ox + 1]; d < at[ox + 2]; d++) {
+                    const float4 r0 = a.coef[3 * (size_t)d], r1 = a.coef[3 * (size_t)d + 1], r2 = a.coef[3 * (size_t)d + 2];
+                    const float fx = r0.x - fi, fy = r0.y - fj, fz = r0.z - fk;
+                    const float cx = tap_across(ox, fx), cy = tap_across(oy, fy), cz = tap_across(oz, fz);
+                    if (ox <= 0) {
+                        const float w = tap_along(ox, fx) * cy * cz;
+                        o.W[0] += w;
+                        o.WV[0] = fmaf(w, r0.w, o.WV[0]);
+                        o.gf[0] = fmaf(w, r1.z, o.gf[0]);
+                        o.gs[0] = fmaf(w, r2.y, o.gs[0]);
+                    }
+                    if (oy <= 0) {
+                        const float w = cx * tap_along(oy, fy) * cz;
+                        o.W[1] += w;
+                        o.WV[1] = fmaf(w, r1.x, o.WV[1]);
+                        o.gf[1] = fmaf(w, r1.w, o.gf[1]);
+                        o.gs[1] = fmaf(w, r2.z, o.gs[1]);
+                    }
+                    if (oz <= 0) {
+                        const float w = cx * cy * tap_along(oz, fz);
+                        o.W[2] += w;
+                        o.WV[2] = fmaf(w, r1.y, o.WV[2]);
+                        o.gf[2] = fmaf(w, r2.x, o.gf[2]);
+                        o.gs[2] = fmaf(w, r2.w, o.gs[2]);
                     }
                 }
             }
         }
     }
+    return o;
+}
+
+__global__ void __launch_bounds__(256) k_adj_gather(AdjBufs a, int midpoint) {
+    const DevParams& P = *a.prm;
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= P.C) return;
+    const int nx = (int)P.nx, ny = (int)P.ny, nz = (int)P.nz;
+    const int i = (int)(c % (uint32_t)nx), j = (int)((c / (uint32_t)nx) % (uint32_t)ny), k = (int)(c / ((uint32_t)nx * ny));
+    const int cc[3] = {i, j, k}, n3[3] = {nx, ny, nz};
+    FaceSums o;
+    if (a.flags[0] || i == nx - 1 || j == ny - 1 || k == nz - 1) {
+        FaceSums t = {};
+        gather_any(a, P, i, j, k, a.flags[0] ? 2 : 1, t);
+        o = t;
+    } else {
+        o = gather_bins(a, P, i, j, k);
+    }
     const double mscale = midpoint && a.flags[1] != 0u ? ldexp(1.0, -mid_exponent(a)) : 0.0;
 #pragma unroll
     for (int e = 0; e < 6; e++) {
-        if (!has[e]) continue;
         const int ax = e % 3;
+        if (e >= 3 && cc[ax] != n3[ax] - 1) continue;
+        int fc[3];  // the face's coordinates
+#pragma unroll
+        for (int b = 0; b < 3; b++) fc[b] = cc[b] + (e >= 3 && b == ax ? 1 : 0);
+        const bool wall = touches_static_a(ax, fc[0], fc[1], fc[2], nx, ny, nz);
         const uint32_t dxa = (uint32_t)nx + (ax == 0), dya = (uint32_t)ny + (ax == 1);
-        const size_t f = (size_t)fc[e][0] + dxa * ((size_t)fc[e][1] + (size_t)dya * fc[e][2]);
-        float g = gf[e];
-        if (mscale != 0.0 && !wall[e]) g += (float)((double)(long long)a.gmid[ax][f] * mscale);
-        a.g_fs[ax][f] = make_float2(g, gs[e]);
-        a.wsum[ax][f] = make_float2(W[e], WV[e]);
+        const size_t f = (size_t)fc[0] + dxa * ((size_t)fc[1] + (size_t)dya * fc[2]);
+        float g = wall ? 0.0f : o.gf[e];
+        if (mscale != 0.0 && !wall) g += (float)((double)(long long)a.gmid[ax][f] * mscale);
+        a.g_fs[ax][f] = make_float2(g, wall ? 0.0f : o.gs[e]);
+        a.wsum[ax][f] = make_float2(o.W[e], o.WV[e]);
     }
 }
 
@@ -667,7 +750,8 @@ cudaError_t launch_adj_thr(const AdjBufs& a, uint32_t nchunks, double tol_sq, De
     return cudaGetLastError();
 }
 cudaError_t launch_adj_faces(const AdjBufs& a, const uint32_t F3[3], cudaStream_t s) {
-    for (int ax = 0; ax < 3; ax++) k_adj_faces<<<(F3[ax] + 255) / 256, 256, 0, s>>>(a, ax);
+    const uint32_t most = F3[0] > F3[1] ? (F3[0] > F3[2] ? F3[0] : F3[2]) : (F3[1] > F3[2] ? F3[1] : F3[2]);
+    k_adj_faces<<<dim3((most + 255) / 256, 3), 256, 0, s>>>(a);
     k_adj_grav<<<3, 1024, 0, s>>>(a, (F3[0] + 255) / 256, (F3[1] + 255) / 256, (F3[2] + 255) / 256);
     return cudaGetLastError();
 }

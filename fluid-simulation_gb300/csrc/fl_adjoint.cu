@@ -32,8 +32,8 @@
 //                   the normalised P2G face velocity; dL/dgravity as block
 //                   partials, summed in order by k_adj_grav
 //   k_adj_p2g       scatter.wgsl transposed: a gather from faces to particles
-//                   (velocity and position gradients)
-//   k_adj_unsort    sort_scatter.wgsl transposed: back to the step's input order
+//                   (velocity and position gradients), and sort_scatter.wgsl
+//                   transposed: back to the step's input order
 #include "fl_device.cuh"
 
 namespace fl {
@@ -112,17 +112,74 @@ __device__ __forceinline__ void stencil(const DevParams& P, int axis, const floa
 // ---------------------------------------------------------------------------
 // G2P + advection adjoint.
 
+// Value and gradient (per unit cell coordinate) of the trilinear interpolant of
+// eight values f[z][y][x] at fractions t.
+__device__ __forceinline__ float lerp_fma(float a, float b, float t) { return fmaf(t, b - a, a); }
+__device__ __forceinline__ void trilinear(const float (&f)[2][2][2], const float t[3], float& val, float grad[3]) {
+    float x[2][2], dx[2][2];
+#pragma unroll
+    for (int z = 0; z < 2; z++)
+#pragma unroll
+        for (int y = 0; y < 2; y++) {
+            dx[z][y] = f[z][y][1] - f[z][y][0];
+            x[z][y] = fmaf(t[0], dx[z][y], f[z][y][0]);
+        }
+    const float y0 = lerp_fma(x[0][0], x[0][1], t[1]), y1 = lerp_fma(x[1][0], x[1][1], t[1]);
+    val = lerp_fma(y0, y1, t[2]);
+    grad[0] = lerp_fma(lerp_fma(dx[0][0], dx[0][1], t[1]), lerp_fma(dx[1][0], dx[1][1], t[1]), t[2]);
+    grad[1] = lerp_fma(x[0][1] - x[0][0], x[1][1] - x[1][0], t[2]);
+    grad[2] = y1 - y0;
+}
+
 // Wall-aware renormalised gather of the final (and saved) face velocities at
 // cell-space point q (g2p.wgsl:56-129), with the position derivatives of the
-// quotients per unit world coordinate.  W = sum of weights (0: no tap).
+// quotients per unit world coordinate.  W = sum of weights (0: no tap).  Where
+// all eight taps count (away from the walls) the weights sum to one and the
+// quotient is the trilinear interpolant: nested interpolation, a quarter of the
+// operations of summing every tap's weight and its three derivatives (the
+// kernel is issue-bound: 200 us of the 128^3 adjoint step in that form).
 template <bool WITH_SAVED>
 __device__ __forceinline__ void gather_d(const AdjBufs& a, const DevParams& P, const float q[3], float val[3],
                                          float dval[3][3], float sav[3], float dsav[3][3], float W[3]) {
+    const int n3[3] = {(int)P.nx, (int)P.ny, (int)P.nz};
     #pragma unroll
     for (int ax = 0; ax < 3; ax++) {
-        float fsum = 0.0f, ssum = 0.0f, wsum = 0.0f, dws[3] = {0, 0, 0}, dfs[3] = {0, 0, 0}, dss[3] = {0, 0, 0};
         const float* fv = a.fin[ax];
         const float* svv = a.sav[ax];
+        int base[3];
+        float t[3];
+        bool all_in = true;
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+            const float g = q[b] + (b == ax ? 0.0f : -0.5f);
+            base[b] = __float2int_rz(floorf(g));
+            t[b] = g - (float)base[b];
+            all_in = all_in && base[b] >= (ax == b ? 2 : 1) && base[b] + 1 <= n3[b] - 2;
+        }
+        if (all_in) {
+            const size_t dx = (size_t)n3[0] + (ax == 0), dxy = dx * ((size_t)n3[1] + (ax == 1));
+            const size_t at = (size_t)base[0] + dx * (size_t)base[1] + dxy * (size_t)base[2];
+            float f[2][2][2], s[2][2][2];
+#pragma unroll
+            for (int z = 0; z < 2; z++)
+#pragma unroll
+                for (int y = 0; y < 2; y++)
+#pragma unroll
+                    for (int x = 0; x < 2; x++) {
+                        f[z][y][x] = fv[at + z * dxy + y * dx + x];
+                        if (WITH_SAVED) s[z][y][x] = svv[at + z * dxy + y * dx + x];
+                    }
+            W[ax] = 1.0f;
+            trilinear(f, t, val[ax], dval[ax]);
+            if (WITH_SAVED) trilinear(s, t, sav[ax], dsav[ax]);
+#pragma unroll
+            for (int b = 0; b < 3; b++) {
+                dval[ax][b] *= P.inv_h;
+                if (WITH_SAVED) dsav[ax][b] *= P.inv_h;
+            }
+            continue;
+        }
+        float fsum = 0.0f, ssum = 0.0f, wsum = 0.0f, dws[3] = {0, 0, 0}, dfs[3] = {0, 0, 0}, dss[3] = {0, 0, 0};
         stencil(P, ax, q, true, [&](size_t idx, float w, const float* dw) {
             const float f = fv[idx];
             fsum += w * f;
@@ -439,7 +496,11 @@ __global__ void __launch_bounds__(256) k_adj_faces(AdjBufs a) {
             gpre = g;
             wet_face = tl == CELL_LIQUID || th == CELL_LIQUID;
         }
-        a.g_norm[axis][f] = gpre + a.g_fs[axis][f].y;
+        // the P2G transpose's factors, divided once per face: {dL/d(normalised
+        // velocity) / sum w, sum w v / sum w}, in place of the sums
+        const float2 s = a.wsum[axis][f];
+        const float gn = gpre + a.g_fs[axis][f].y;
+        a.wsum[axis][f] = s.x > 0.0f ? make_float2(gn / s.x, s.y / s.x) : make_float2(0.0f, 0.0f);
     }
     // dL/dg_axis: the block's partial in a fixed order (k_adj_grav sums the
     // blocks' partials in order)
@@ -610,12 +671,14 @@ __device__ __forceinline__ float tap_across(int o, float f) {
     return o == 0 ? 1.0f - fabsf(f - 0.5f) : fmaxf(o < 0 ? f - 0.5f : 0.5f - f, 0.0f);
 }
 
-__device__ __forceinline__ FaceSums gather_bins(const AdjBufs& a, const DevParams& P, int i, int j, int k) {
-    FaceSums o = {};
+// The low faces of the NZ cells (i, j, k .. k + NZ - 1).
+template <int NZ>
+__device__ __forceinline__ void gather_bins(const AdjBufs& a, const DevParams& P, int i, int j, int k, FaceSums (&o)[NZ]) {
     const int nx = (int)P.nx, ny = (int)P.ny, nz = (int)P.nz;
     const uint32_t n = P.n, C = P.C;
-    for (int oz = -1; oz <= 1; oz++) {
-        const int ck = k + oz;
+#pragma unroll
+    for (int sz = -1; sz <= NZ; sz++) {
+        const int ck = k + sz;
         if (ck < 0 || ck >= nz) continue;
         for (int oy = -1; oy <= 1; oy++) {
             const int cj = j + oy;
@@ -634,106 +697,110 @@ __device__ __forceinline__ FaceSums gather_bins(const AdjBufs& a, const DevParam
                 for (uint32_t d = at[ox + 1]; d < at[ox + 2]; d++) {
                     const float4 r0 = a.coef[3 * (size_t)d], r1 = a.coef[3 * (size_t)d + 1], r2 = a.coef[3 * (size_t)d + 2];
                     const float fx = r0.x - fi, fy = r0.y - fj, fz = r0.z - fk;
-                    const float cx = tap_across(ox, fx), cy = tap_across(oy, fy), cz = tap_across(oz, fz);
-                    if (ox <= 0) {
-                        const float w = tap_along(ox, fx) * cy * cz;
-                        o.W[0] += w;
-                        o.WV[0] = fmaf(w, r0.w, o.WV[0]);
-                        o.gf[0] = fmaf(w, r1.z, o.gf[0]);
-                        o.gs[0] = fmaf(w, r2.y, o.gs[0]);
-                    }
-                    if (oy <= 0) {
-                        const float w = cx * tap_along(oy, fy) * cz;
-                        o.W[1] += w;
-                        o.WV[1] = fmaf(w, r1.x, o.WV[1]);
-                        o.gf[1] = fmaf(w, r1.w, o.gf[1]);
-                        o.gs[1] = fmaf(w, r2.z, o.gs[1]);
-                    }
-                    if (oz <= 0) {
-                        const float w = cx * cy * tap_along(oz, fz);
-                        o.W[2] += w;
-                        o.WV[2] = fmaf(w, r1.y, o.WV[2]);
-                        o.gf[2] = fmaf(w, r2.x, o.gf[2]);
-                        o.gs[2] = fmaf(w, r2.w, o.gs[2]);
+                    const float cx = tap_across(ox, fx), cy = tap_across(oy, fy);
+                    const float u = tap_along(ox, fx) * cy, v = cx * tap_along(oy, fy), x = cx * cy;
+#pragma unroll
+                    for (int z = 0; z < NZ; z++) {
+                        const int oz = sz - z;  // of the particle's cell from this one
+                        if (oz < -1 || oz > 1) continue;
+                        const float cz = tap_across(oz, fz);
+                        if (ox <= 0) {
+                            const float w = u * cz;
+                            o[z].W[0] += w;
+                            o[z].WV[0] = fmaf(w, r0.w, o[z].WV[0]);
+                            o[z].gf[0] = fmaf(w, r1.z, o[z].gf[0]);
+                            o[z].gs[0] = fmaf(w, r2.y, o[z].gs[0]);
+                        }
+                        if (oy <= 0) {
+                            const float w = v * cz;
+                            o[z].W[1] += w;
+                            o[z].WV[1] = fmaf(w, r1.x, o[z].WV[1]);
+                            o[z].gf[1] = fmaf(w, r1.w, o[z].gf[1]);
+                            o[z].gs[1] = fmaf(w, r2.z, o[z].gs[1]);
+                        }
+                        if (oz <= 0) {
+                            const float w = x * tap_along(oz, fz);
+                            o[z].W[2] += w;
+                            o[z].WV[2] = fmaf(w, r1.y, o[z].WV[2]);
+                            o[z].gf[2] = fmaf(w, r2.x, o[z].gf[2]);
+                            o[z].gs[2] = fmaf(w, r2.w, o[z].gs[2]);
+                        }
                     }
                 }
             }
         }
     }
-    return o;
 }
 
+template <int NZ>
 __global__ void __launch_bounds__(256) k_adj_gather(AdjBufs a, int midpoint) {
     const DevParams& P = *a.prm;
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= P.C) return;
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const int nx = (int)P.nx, ny = (int)P.ny, nz = (int)P.nz;
-    const int i = (int)(c % (uint32_t)nx), j = (int)((c / (uint32_t)nx) % (uint32_t)ny), k = (int)(c / ((uint32_t)nx * ny));
+    const int i = (int)(t % (uint32_t)nx), j = (int)((t / (uint32_t)nx) % (uint32_t)ny), k = (int)(t / ((uint32_t)nx * ny)) * NZ;
+    if (k >= nz) return;
     const int cc[3] = {i, j, k}, n3[3] = {nx, ny, nz};
-    FaceSums o;
-    if (a.flags[0] || i == nx - 1 || j == ny - 1 || k == nz - 1) {
-        FaceSums t = {};
-        gather_any(a, P, i, j, k, a.flags[0] ? 2 : 1, t);
-        o = t;
-    } else {
-        o = gather_bins(a, P, i, j, k);
-    }
+    FaceSums o[NZ];
+#pragma unroll
+    for (int z = 0; z < NZ; z++) o[z] = FaceSums{};
+    const bool any = a.flags[0] || i == nx - 1 || j == ny - 1;
+    if (!any) gather_bins<NZ>(a, P, i, j, k, o);
     const double mscale = midpoint && a.flags[1] != 0u ? ldexp(1.0, -mid_exponent(a)) : 0.0;
 #pragma unroll
-    for (int e = 0; e < 6; e++) {
-        const int ax = e % 3;
-        if (e >= 3 && cc[ax] != n3[ax] - 1) continue;
-        int fc[3];  // the face's coordinates
+    for (int z = 0; z < NZ; z++) {
+        const int kz = k + z;
+        if (kz >= nz) continue;
+        FaceSums s = o[z];
+        if (any || kz == nz - 1) {
+            FaceSums g = {};
+            gather_any(a, P, i, j, kz, a.flags[0] ? 2 : 1, g);
+            s = g;
+        }
 #pragma unroll
-        for (int b = 0; b < 3; b++) fc[b] = cc[b] + (e >= 3 && b == ax ? 1 : 0);
-        const bool wall = touches_static_a(ax, fc[0], fc[1], fc[2], nx, ny, nz);
-        const uint32_t dxa = (uint32_t)nx + (ax == 0), dya = (uint32_t)ny + (ax == 1);
-        const size_t f = (size_t)fc[0] + dxa * ((size_t)fc[1] + (size_t)dya * fc[2]);
-        float g = wall ? 0.0f : o.gf[e];
-        if (mscale != 0.0 && !wall) g += (float)((double)(long long)a.gmid[ax][f] * mscale);
-        a.g_fs[ax][f] = make_float2(g, wall ? 0.0f : o.gs[e]);
-        a.wsum[ax][f] = make_float2(o.W[e], o.WV[e]);
+        for (int e = 0; e < 6; e++) {
+            const int ax = e % 3;
+            if (e >= 3 && (ax == 2 ? kz : cc[ax]) != n3[ax] - 1) continue;
+            const int fc[3] = {i + (e == 3), j + (e == 4), kz + (e == 5)};  // the face's coordinates
+            const bool wall = touches_static_a(ax, fc[0], fc[1], fc[2], nx, ny, nz);
+            const uint32_t dxa = (uint32_t)nx + (ax == 0), dya = (uint32_t)ny + (ax == 1);
+            const size_t f = (size_t)fc[0] + dxa * ((size_t)fc[1] + (size_t)dya * fc[2]);
+            float g = wall ? 0.0f : s.gf[e];
+            if (mscale != 0.0 && !wall) g += (float)((double)(long long)a.gmid[ax][f] * mscale);
+            a.g_fs[ax][f] = make_float2(g, wall ? 0.0f : s.gs[e]);
+            a.wsum[ax][f] = make_float2(s.W[e], s.WV[e]);
+        }
     }
 }
 
-// P2G transposed: vel_f = sum_p w v / sum_p w  ->  gather per particle, with
-// the normalisation linearised at the unquantised sums k_adj_gather wrote.
+// P2G transposed: vel_f = sum_p w v / sum_p w  ->  gather per particle of the
+// factors that k_adj_faces left, with the normalisation linearised at the
+// unquantised sums; then back to the step's input order (sort_scatter.wgsl
+// transposed).
 __global__ void __launch_bounds__(256) k_adj_p2g(AdjBufs a) {
     const DevParams& P = *a.prm;
     const uint32_t n = P.n;
     const float inv_h = P.inv_h;
     for (uint32_t d = blockIdx.x * blockDim.x + threadIdx.x; d < n; d += gridDim.x * blockDim.x) {
         const float4 pos = a.part[2 * (size_t)d], pvel = a.part[2 * (size_t)d + 1];
+        float4 s0 = a.g_sorted[2 * (size_t)d], s1 = a.g_sorted[2 * (size_t)d + 1];
+        const uint32_t src = a.perm[d];
         const float q[3] = {(pos.x - P.origin[0]) * inv_h, (pos.y - P.origin[1]) * inv_h, (pos.z - P.origin[2]) * inv_h};
         const float pv[3] = {pvel.x, pvel.y, pvel.z};
         float gX[3] = {0, 0, 0}, gv[3] = {0, 0, 0};
+#pragma unroll
         for (int ax = 0; ax < 3; ax++) {
-            const float2* ws = a.wsum[ax];
-            const float* gn = a.g_norm[ax];
+            const float2* fs = a.wsum[ax];
             stencil(P, ax, q, false, [&](size_t idx, float w, const float* dw) {
-                const float2 s = ws[idx];
-                const float W = s.x;
-                if (!(W > 0.0f)) return;
-                const float g = gn[idx] / W;
-                gv[ax] += w * g;
-                const float diff = (pv[ax] - s.y / W) * g * inv_h;
-                for (int b = 0; b < 3; b++) gX[b] += dw[b] * diff;
+                const float2 s = fs[idx];
+                gv[ax] = fmaf(w, s.x, gv[ax]);
+                const float diff = (pv[ax] - s.y) * s.x;
+                for (int b = 0; b < 3; b++) gX[b] = fmaf(dw[b], diff, gX[b]);
             });
         }
-        float4 s0 = a.g_sorted[2 * (size_t)d], s1 = a.g_sorted[2 * (size_t)d + 1];
-        s0.x += gX[0]; s0.y += gX[1]; s0.z += gX[2];
+        s0.x += gX[0] * inv_h; s0.y += gX[1] * inv_h; s0.z += gX[2] * inv_h;
         s1.x += gv[0]; s1.y += gv[1]; s1.z += gv[2];
-        a.g_sorted[2 * (size_t)d] = s0;
-        a.g_sorted[2 * (size_t)d + 1] = s1;
-    }
-}
-
-__global__ void __launch_bounds__(256) k_adj_unsort(AdjBufs a) {
-    const uint32_t n = a.prm->n;
-    for (uint32_t d = blockIdx.x * blockDim.x + threadIdx.x; d < n; d += gridDim.x * blockDim.x) {
-        const uint32_t src = a.perm[d];
-        a.g_in[2 * (size_t)src] = a.g_sorted[2 * (size_t)d];
-        a.g_in[2 * (size_t)src + 1] = a.g_sorted[2 * (size_t)d + 1];
+        a.g_in[2 * (size_t)src] = s0;
+        a.g_in[2 * (size_t)src + 1] = s1;
     }
 }
 
@@ -759,17 +826,14 @@ cudaError_t launch_adj_mid(const AdjBufs& a, const LaunchCfg& L, cudaStream_t s)
     k_adj_mid<<<L.particle_blocks, 256, 0, s>>>(a);
     return cudaGetLastError();
 }
-cudaError_t launch_adj_gather(const AdjBufs& a, uint32_t C, bool midpoint, cudaStream_t s) {
-    k_adj_gather<<<(C + 255) / 256, 256, 0, s>>>(a, midpoint ? 1 : 0);
+cudaError_t launch_adj_gather(const AdjBufs& a, uint32_t nx, uint32_t ny, uint32_t nz, bool midpoint, cudaStream_t s) {
+    constexpr int NZ = 2;
+    const uint32_t threads = nx * ny * ((nz + NZ - 1) / NZ);
+    k_adj_gather<NZ><<<(threads + 255) / 256, 256, 0, s>>>(a, midpoint ? 1 : 0);
     return cudaGetLastError();
 }
 cudaError_t launch_adj_p2g(const AdjBufs& a, const LaunchCfg& L, cudaStream_t s) {
     k_adj_p2g<<<L.particle_blocks, 256, 0, s>>>(a);
     return cudaGetLastError();
 }
-cudaError_t launch_adj_unsort(const AdjBufs& a, const LaunchCfg& L, cudaStream_t s) {
-    k_adj_unsort<<<L.particle_blocks, 256, 0, s>>>(a);
-    return cudaGetLastError();
-}
-
 }  // namespace fl

@@ -128,8 +128,8 @@ struct AdjBufs {
     float4* g_sorted;        // dL/d(input particle in bin order), 2 float4 each
     float4* g_in;            // dL/d(input particle), input order
     float2* g_fs[3];         // {dL/d final face velocity, dL/d saved face velocity} per face
-    float* g_norm[3];
-    // Unquantised P2G sums {sum w, sum w v} of the recorded step.
+    // Unquantised P2G sums {sum w, sum w v} of the recorded step; the face stage
+    // replaces them by {dL/d(normalised velocity) / sum w, sum w v / sum w}.
     float2* wsum[3];
     float* lam;              // adjoint pressure (the solve's x)
     float* rhs;              // dL/dp
@@ -359,9 +359,8 @@ cudaError_t launch_adj_faces(const AdjBufs& a, const uint32_t F3[3], cudaStream_
 // the midpoint step's face gradients into gmid (zeroed by the caller)
 cudaError_t launch_adj_mid(const AdjBufs& a, const LaunchCfg& L, cudaStream_t s);
 // g_fs and wsum of every face, gathered per cell in a fixed order
-cudaError_t launch_adj_gather(const AdjBufs& a, uint32_t C, bool midpoint, cudaStream_t s);
+cudaError_t launch_adj_gather(const AdjBufs& a, uint32_t nx, uint32_t ny, uint32_t nz, bool midpoint, cudaStream_t s);
 cudaError_t launch_adj_p2g(const AdjBufs& a, const LaunchCfg& L, cudaStream_t s);
-cudaError_t launch_adj_unsort(const AdjBufs& a, const LaunchCfg& L, cudaStream_t s);
 // Stand-alone CG on prepared cell arrays (used by fl_solve_pressure).
 cudaError_t launch_solve_init(const DevBufs& b, uint32_t C, const float* div, cudaStream_t s);
 }  // namespace fl

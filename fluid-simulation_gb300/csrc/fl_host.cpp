@@ -1138,7 +1138,6 @@ struct fl_tape {
     size_t slot_bytes = 0, o_part = 0, o_perm = 0, o_ct = 0, o_off = 0, o_sav[3] = {}, o_fin[3] = {};
     float4* g_sorted = nullptr;
     float2* g_fs[3] = {};
-    float* g_norm[3] = {};
     float2* wsum[3] = {};
     unsigned long long* gmid[3] = {};
     double* grav_part[3] = {};
@@ -1179,10 +1178,9 @@ fl_status fl_tape_create(fl_handle* h, uint32_t max_steps, fl_tape** out) {
     t->slot_bytes = (slot.off + 255) & ~size_t(255);
     PoolPlan pl;
     pl.off = t->slot_bytes * max_steps;
-    size_t o_gs = pl.take<float4>(2 * cap), o_gf[3], o_gn[3], o_ws[3], o_gm[3], o_gp[3];
+    size_t o_gs = pl.take<float4>(2 * cap), o_gf[3], o_ws[3], o_gm[3], o_gp[3];
     for (int a = 0; a < 3; a++) {
         o_gf[a] = pl.take<float2>(h->F3[a]);
-        o_gn[a] = pl.take<float>(h->F3[a]);
         o_ws[a] = pl.take<float2>(h->F3[a]);
         o_gm[a] = pl.take<unsigned long long>(h->F3[a]);
         o_gp[a] = pl.take<double>((h->F3[a] + 255) / 256);
@@ -1206,7 +1204,6 @@ fl_status fl_tape_create(fl_handle* h, uint32_t max_steps, fl_tape** out) {
     t->g_sorted = (float4*)(base + o_gs);
     for (int a = 0; a < 3; a++) {
         t->g_fs[a] = (float2*)(base + o_gf[a]);
-        t->g_norm[a] = (float*)(base + o_gn[a]);
         t->wsum[a] = (float2*)(base + o_ws[a]);
         t->gmid[a] = (unsigned long long*)(base + o_gm[a]);
         t->grav_part[a] = (double*)(base + o_gp[a]);
@@ -1361,7 +1358,6 @@ fl_status fl_step_adjoint(fl_handle* h, fl_tape* t, const void* dL_dout_dev, voi
         a.sav[ax] = (const float*)(slot + t->o_sav[ax]);
         a.fin[ax] = (const float*)(slot + t->o_fin[ax]);
         a.g_fs[ax] = t->g_fs[ax];
-        a.g_norm[ax] = t->g_norm[ax];
         a.wsum[ax] = t->wsum[ax];
         a.gmid[ax] = t->gmid[ax];
         a.grav_part[ax] = t->grav_part[ax];
@@ -1380,7 +1376,7 @@ fl_status fl_step_adjoint(fl_handle* h, fl_tape* t, const void* dL_dout_dev, voi
     a.g_grav = t->g_grav;
     FL_CUDA(h, fl::launch_adj_g2p(a, h->L, st));
     if (midpoint) FL_CUDA(h, fl::launch_adj_mid(a, h->L, st));
-    FL_CUDA(h, fl::launch_adj_gather(a, h->C, midpoint, st));
+    FL_CUDA(h, fl::launch_adj_gather(a, h->nx, h->ny, h->nz, midpoint, st));
     FL_CUDA(h, fl::launch_adj_prhs(a, h->C, st));
     // adjoint pressure solve: A lambda = dL/dp (k_solve_init's rhs is
     // -scale*div, so scale = -1 passes dL/dp through unchanged).  Cold start:
@@ -1415,7 +1411,6 @@ fl_status fl_step_adjoint(fl_handle* h, fl_tape* t, const void* dL_dout_dev, voi
     }
     FL_CUDA(h, fl::launch_adj_faces(a, h->F3, st));
     FL_CUDA(h, fl::launch_adj_p2g(a, h->L, st));
-    FL_CUDA(h, fl::launch_adj_unsort(a, h->L, st));
     double gg[3];
     DevStats ds;
     FL_CUDA(h, cudaMemcpyAsync(gg, t->g_grav, sizeof(gg), cudaMemcpyDeviceToHost, st));

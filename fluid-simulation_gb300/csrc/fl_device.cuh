@@ -21,6 +21,8 @@ constexpr int SCAN_THREADS = 1024;
 constexpr int SCAN_TILE = SCAN_ITEMS * SCAN_THREADS;
 constexpr int BIG_BUCKET_SMEM = 4096;  // larger buckets use the global-memory rank pass
 constexpr int TILE = 8;           // P2G tile edge (cells)
+constexpr uint32_t BAR_COUNTERS = 8;  // of a grid barrier, 128 bytes apart
+constexpr size_t BAR_BYTES = BAR_COUNTERS * 128;
 
 // Device copy of the step settings.  Derived scalars are computed once on the
 // host with the same f32 operations the shaders use (see fl_host.cpp).
@@ -243,10 +245,6 @@ __device__ __forceinline__ int32_t fixed_round(float x) { return __float2int_rn(
 // dk (outer), dj, di (inner) of scatter.wgsl:55-67.
 __device__ __forceinline__ float tent(float t, int d) { return d == 1 ? t : __fsub_rn(1.0f, t); }
 
-// Grid barrier over all blocks of a cooperative launch.  Arrival is a
-// release-add on a counter that only grows within one launch; waiting is an
-// acquire-load spin bounded by %globaltimer (about 2 s).  On expiry, or when
-// another block has recorded an error, it records FL_TIMEOUT and returns false.
 __device__ __forceinline__ uint64_t global_ns() {
     uint64_t t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -263,6 +261,60 @@ __device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
 }
 __device__ __forceinline__ void red_release_add(uint32_t* p, uint32_t v) {
     asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// Grid barrier over all blocks of a cooperative launch; every thread calls it.
+// Block bb arrives at counter bb mod BAR_COUNTERS (each on its own 128-byte
+// line: 152 arrivals at one address follow one another); lane k of warp 0 waits
+// for counter k, at most `limit` ns.  On expiry, or when another block has
+// recorded an error in *status, it records FL_TIMEOUT and returns false in
+// every thread.  `epoch` counts the launch's barriers from 1; the counters start
+// at zero; s_ok is shared memory.
+__device__ __forceinline__ bool grid_barrier(uint32_t* bars, uint32_t epoch, uint64_t limit, uint32_t* status,
+                                             volatile int* s_ok) {
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const uint32_t k = threadIdx.x;
+        // the release add orders the block's writes (before the barrier
+        // above) ahead of the arrival; a separate fence only added its wait
+        if (k == 0) red_release_add(bars + (blockIdx.x % BAR_COUNTERS) * 32u, 1u);
+        __syncwarp();
+        bool ok = true;
+        if (k < BAR_COUNTERS) {
+            const uint32_t* const bar = bars + k * 32u;
+            const uint32_t target = epoch * ((gridDim.x + BAR_COUNTERS - 1 - k) / BAR_COUNTERS);
+            const uint64_t t0 = global_ns();
+            uint32_t spins = 0;
+            while (ld_acquire(bar) < target) {
+                // clock on the first re-poll and every 64 polls, status every 64
+                ++spins;
+                const bool slow = (spins & 63u) == 0u;
+                if (slow && *(volatile uint32_t*)status != 0u) {
+                    ok = false;
+                    break;
+                }
+                if ((slow || spins == 1u) && global_ns() - t0 > limit) {
+                    atomicCAS(status, 0u, 5u /* FL_TIMEOUT */);
+                    ok = false;
+                    break;
+                }
+            }
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        if (k == 0) *s_ok = ok;
+    }
+    __syncthreads();
+    return *s_ok != 0;
+}
+
+// A load that the compiler may not move behind the test that decides whether
+// its value is needed (chains of such loads wait for one another); 0 when off.
+__device__ __forceinline__ float ld_if(const float* p, bool on) {
+    float v;
+    asm volatile("{\n.reg .pred q;\nsetp.ne.u32 q, %2, 0;\nmov.f32 %0, 0f00000000;\n@q ld.global.f32 %0, [%1];\n}"
+                 : "=f"(v)
+                 : "l"(p), "r"((uint32_t)on));
+    return v;
 }
 
 #endif  // __CUDACC__
@@ -314,7 +366,6 @@ cudaError_t launch_seed(const SeedArgs& a, float4* part, cudaStream_t s);
 constexpr int MG_MAX_LEVELS = 12;
 constexpr uint32_t MG_COARSE_CELLS = 64;  // the coarsest level holds at most this many cells
 constexpr uint32_t MG_BLOCK0_CELLS = 4096;  // levels this small run inside one block (block barriers)
-constexpr uint32_t MG_COUNTERS = 8;         // barrier counters
 constexpr uint32_t MG_LOCAL_TOTAL = 4800;   // cells of all those levels together (b, x in shared memory)
 struct MgLevel {
     uint32_t nx, ny, nz, C;
@@ -327,7 +378,7 @@ struct MgBufs {
     MgLevel lv[MG_MAX_LEVELS];
     float* r2;          // second residual buffer (level-0 size)
     float2* part;       // 2 x MAX_CG_BLOCKS float-float block partials
-    uint32_t* bar;      // MG_COUNTERS barrier counters, 128 bytes apart, zeroed before each solve
+    uint32_t* bar;      // barrier counters (grid_barrier), zeroed before each solve
 };
 // Level sizes of an nx x ny x nz grid; returns L.
 FL_HD inline uint32_t mg_levels(uint32_t nx, uint32_t ny, uint32_t nz, uint32_t dims[MG_MAX_LEVELS][3]) {
@@ -341,10 +392,12 @@ FL_HD inline uint32_t mg_levels(uint32_t nx, uint32_t ny, uint32_t nz, uint32_t 
     return L;
 }
 // Relaxation solves from zero (fl_relax.cu): method 0 Jacobi (ping-pong
-// between pa and pb), 1 red-black Gauss-Seidel (in place in pa); *result is
-// the buffer that holds the answer.
-cudaError_t launch_relax(const uint8_t* ct, const float* div, float scale, float* pa, float* pb, uint32_t nx,
-                         uint32_t ny, uint32_t nz, uint32_t method, uint32_t iters, cudaStream_t s, float** result);
+// between pa and pb, both zeroed), 1 red-black Gauss-Seidel (in place in pa);
+// bars: BAR_BYTES of zeroed counters, then the status word; *result is the
+// buffer that holds the answer.
+cudaError_t launch_relax(const uint8_t* ct, const float* div, float scale, float* pa, float* pb, uint32_t* bars,
+                         uint32_t nx, uint32_t ny, uint32_t nz, uint32_t method, uint32_t iters, int num_sms,
+                         cudaStream_t s, float** result);
 // The CG's plan of active chunks split over G blocks (fl_cg.cu).
 cudaError_t launch_cg_plan(const DevBufs& b, uint32_t G, cudaStream_t s);
 cudaError_t launch_mgpcg(const DevBufs& b, const MgBufs& m, const LaunchCfg& L, cudaStream_t s);

@@ -196,7 +196,7 @@ fl_status mg_alloc(fl_handle* h, uint32_t nx, uint32_t ny, uint32_t nz, float* r
         o_x[l] = pl.take<float>(C);
     }
     const size_t o_r2 = pl.take<float>((size_t)nx * ny * nz);
-    const size_t o_part = pl.take<float2>(2 * 1024), o_bar = pl.take<uint32_t>(32 * fl::MG_COUNTERS);
+    const size_t o_part = pl.take<float2>(2 * 1024), o_bar = pl.take<uint32_t>(fl::BAR_BYTES / 4);
     void* base = nullptr;
     cudaError_t e = cudaMalloc(&base, pl.off);
     if (e != cudaSuccess) {
@@ -1011,7 +1011,7 @@ fl_status fl_relax_pressure(uint32_t nx, uint32_t ny, uint32_t nz, const uint8_t
     const float scale = rho * h * h / dt;  // ProjectionParams::rhs_scale (sim/pressure.rs:31-33)
     PoolPlan pl;
     const size_t o_ct = pl.take<uint8_t>(C), o_div = pl.take<float>(C), o_a = pl.take<float>(C),
-                 o_b = pl.take<float>(C);
+                 o_b = pl.take<float>(C), o_bar = pl.take<uint32_t>(fl::BAR_BYTES / 4 + 1);
     void* pool = nullptr;
     cudaError_t e = cudaMalloc(&pool, pl.off);
     if (e != cudaSuccess) {
@@ -1023,21 +1023,25 @@ fl_status fl_relax_pressure(uint32_t nx, uint32_t ny, uint32_t nz, const uint8_t
     float* ddiv = (float*)(base + o_div);
     float* pa = (float*)(base + o_a);
     float* pb = (float*)(base + o_b);
+    uint32_t* bars = (uint32_t*)(base + o_bar);
     float* res = pa;
+    uint32_t status = 0;
     cudaStream_t st = nullptr;
     do {
         if ((e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking)) != cudaSuccess) break;
         if ((e = cudaMemsetAsync(pool, 0, pl.off, st)) != cudaSuccess) break;
         if ((e = cudaMemcpyAsync(dct, cell_type, C, cudaMemcpyHostToDevice, st)) != cudaSuccess) break;
         if ((e = cudaMemcpyAsync(ddiv, divergence, 4 * C, cudaMemcpyHostToDevice, st)) != cudaSuccess) break;
-        if ((e = fl::launch_relax(dct, ddiv, scale, pa, pb, nx, ny, nz, method, iters, st, &res)) != cudaSuccess)
+        if ((e = fl::launch_relax(dct, ddiv, scale, pa, pb, bars, nx, ny, nz, method, iters, g_num_sms, st, &res)) != cudaSuccess)
             break;
         if ((e = cudaMemcpyAsync(pressure_out, res, 4 * C, cudaMemcpyDeviceToHost, st)) != cudaSuccess) break;
+        if ((e = cudaMemcpyAsync(&status, bars + fl::BAR_BYTES / 4, 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess) break;
         e = cudaStreamSynchronize(st);
     } while (0);
     fl_status rs = e != cudaSuccess ? cuda_err(nullptr, e, "fl_relax_pressure") : FL_OK;
     if (st) cudaStreamDestroy(st);
     cudaFree(pool);
+    if (rs == FL_OK && status) return set_err(nullptr, (fl_status)status, "a device-side wait expired");
     return rs;
 }
 

@@ -98,17 +98,10 @@ __device__ __forceinline__ uint32_t ld_ci(const uint16_t* ci, uint32_t c) { retu
 
 // The passes are chains of L2 loads, one cell or two per thread, so what a cell
 // costs is the number of loads that wait for one another.  Every load of a cell
-// is issued before the first value is used, and volatile: the compiler would
-// otherwise move each load behind the test that decides whether its value is
+// is issued before the first value is used, and volatile (ld_if): the compiler
+// would otherwise move each load behind the test that decides whether its value is
 // needed (each neighbour then waited for the one before: 107 us per iteration
 // on the 128^3 sphere-into-pool scene, against 91; 69 with the lists below).
-__device__ __forceinline__ float ld_if(const float* p, bool on) {  // 0 when off
-    float v;
-    asm volatile("{\n.reg .pred q;\nsetp.ne.u32 q, %2, 0;\nmov.f32 %0, 0f00000000;\n@q ld.global.f32 %0, [%1];\n}"
-                 : "=f"(v)
-                 : "l"(p), "r"((uint32_t)on));
-    return v;
-}
 __device__ __forceinline__ uint32_t ld_ci_if(const uint16_t* p, bool on) {
     uint32_t v;
     asm volatile("{\n.reg .pred q;\nsetp.ne.u32 q, %2, 0;\nmov.u32 %0, 0;\n@q ld.global.nc.u16 %0, [%1];\n}"
@@ -218,44 +211,8 @@ struct Ctx {
     float4* lst;        // block 0: shared-memory copy of the stencils of levels Lg.. (nullptr: global)
 };
 
-// Block bb arrives at counter bb mod MG_COUNTERS (each on its own line: 152
-// arrivals at one address follow one another); lane k of warp 0 waits for
-// counter k.
 __device__ bool mg_barrier(Ctx& x) {
-    __syncthreads();
-    x.epoch++;
-    if (threadIdx.x < 32) {
-        const uint32_t k = threadIdx.x;
-        // the release add orders the block's writes (before the barrier
-        // above) ahead of the arrival; a separate fence only added its wait
-        if (k == 0) red_release_add(x.m.bar + (blockIdx.x % MG_COUNTERS) * 32u, 1u);
-        __syncwarp();
-        bool ok = true;
-        if (k < MG_COUNTERS) {
-            const uint32_t* const bar = x.m.bar + k * 32u;
-            const uint32_t target = x.epoch * ((gridDim.x + MG_COUNTERS - 1 - k) / MG_COUNTERS);
-            const uint64_t t0 = global_ns();
-            uint32_t spins = 0;
-            while (ld_acquire(bar) < target) {
-                // clock on the first re-poll and every 64 polls, status every 64
-                ++spins;
-                const bool slow = (spins & 63u) == 0u;
-                if (slow && *(volatile uint32_t*)&x.b.st->status != 0u) {
-                    ok = false;
-                    break;
-                }
-                if ((slow || spins == 1u) && global_ns() - t0 > x.sh.limit) {
-                    atomicCAS(&x.b.st->status, 0u, 5u /* FL_TIMEOUT */);
-                    ok = false;
-                    break;
-                }
-            }
-        }
-        ok = __all_sync(0xffffffffu, ok);
-        if (k == 0) x.sh.ok = ok;
-    }
-    __syncthreads();
-    return x.sh.ok != 0;
+    return grid_barrier(x.m.bar, ++x.epoch, x.sh.limit, &x.b.st->status, &x.sh.ok);
 }
 
 // Sum of v over all threads of all blocks, in a fixed order; false on abort.
@@ -1036,7 +993,7 @@ cudaError_t launch_mgpcg(const DevBufs& b, const MgBufs& m, const LaunchCfg& L, 
     // level-0 cells go to blocks 1..G-1 (block 0 runs the coarse levels)
     cudaError_t e = launch_cg_plan(b, L.cg_blocks > 1 ? (uint32_t)L.cg_blocks - 1 : 1u, s);
     if (e != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(m.bar, 0, MG_COUNTERS * 128, s)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(m.bar, 0, BAR_BYTES, s)) != cudaSuccess) return e;
     const int gb = L.num_sms * 8;
     k_mg_agg0<<<gb, 256, 0, s>>>(b, m);
     for (uint32_t l = 1; l + 1 < m.L; l++) k_mg_agg<<<gb, 256, 0, s>>>(m, l);

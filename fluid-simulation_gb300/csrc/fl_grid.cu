@@ -47,22 +47,26 @@ __global__ void __launch_bounds__(256) k_classify(DevBufs b, uint32_t C) {
 
 constexpr int P2G_BATCH = 4;  // particles in flight per thread
 
-// k_p2g_own: one 256-thread block per 8^3 tile of cells, visiting only the
+// k_p2g_own: one 256-thread block per tile of 8 x 8 x TZ cells, visiting only the
 // particles binned in the tile (each particle once; a tile that also read its
 // one-cell halo, to own its faces outright, visited about 1.95 per particle
 // at 128^3).  A particle of cell c
 // reaches faces c..c+1 along the face axis and c-1..c+1 along the other two
 // (scatter.wgsl:55-67), so the block accumulates its fixed-point terms over a
-// box of (TILE+1) x (TILE+2) x (TILE+2) faces per axis -- the tile's faces
-// and a one-face rim -- in shared memory, then adds every nonzero sum to the
-// face arrays (cleared before the launch) with integer reductions.  Integer
-// sums are order-free, so num/den equal the reference's atomic scatter
-// exactly, whatever order the blocks add in.
-constexpr int PB_A = TILE + 1;                  // box faces along the face axis
-constexpr int PB_O = TILE + 2;                  // box faces along the other axes
-constexpr int PB_N = PB_A * PB_O * PB_O;        // box faces per axis
-constexpr int P2G_OWN_ROWS = TILE * TILE;       // (y, z) rows of a tile
+// box of faces per axis -- the tile's faces and a one-face rim -- in shared
+// memory, then adds every nonzero sum to the face arrays (cleared before the
+// launch) with integer reductions.  Integer sums are order-free, so num/den
+// equal the reference's atomic scatter exactly, whatever order the blocks add in.
+// What bounds it is the shared-memory pipe: 48 atomics per particle, several
+// cycles each where lanes meet in a bank.  The pitches 12 and 128 and the order
+// of rows (k_p2g_own) put lanes eight particles apart, one cell of every second
+// row and plane each, in different banks: 1.0 passes per atomic for particles on
+// a lattice and 3.0 for random ones, against 2.0 and 3.4 with dense pitches
+// (counted on the CPU).  128^3, 2.0 M particles: 91 us -> 77 us.
+constexpr int PB_Y = 12;   // box pitch of y, words
+constexpr int PB_Z = 128;  // of z
 
+template <int TZ>
 __device__ __forceinline__ void p2g_box(const DevParams& P, DevStats* st, const int o[3], int axis, const float q[3],
                                         float vcomp, int32_t* s_num, int32_t* s_den) {
     float t[3];
@@ -74,16 +78,18 @@ __device__ __forceinline__ void p2g_box(const DevParams& P, DevStats* st, const 
         t[bb] = __fsub_rn(g, floorf(g));
     }
     // A particle that is not a stray has floor(q) == its bin cell, so the taps
-    // lie in the box (first tap 0..TILE-1 along the face axis, 0..TILE along
+    // lie in the box (first tap 0..edge-1 along the face axis, 0..edge along
     // the others); anything else is recorded and skipped, never written.
     const uint32_t lim[3] = {axis == 0 ? (uint32_t)TILE - 1u : (uint32_t)TILE, axis == 1 ? (uint32_t)TILE - 1u : (uint32_t)TILE,
-                             axis == 2 ? (uint32_t)TILE - 1u : (uint32_t)TILE};
+                             axis == 2 ? (uint32_t)TZ - 1u : (uint32_t)TZ};
     if ((uint32_t)base[0] > lim[0] || (uint32_t)base[1] > lim[1] || (uint32_t)base[2] > lim[2]) {
         atomicCAS(&st->status, 0u, 7u /* FL_INTERNAL */);
         return;
     }
-    const int sx = axis == 0 ? PB_A : PB_O, sy = axis == 1 ? PB_A : PB_O;
     const float scale = P.fixed_scale;
+    int32_t* const num = s_num + base[0] + PB_Y * base[1] + PB_Z * base[2];
+    int32_t* const den = s_den + (num - s_num);
+    // scatter.wgsl:62 skips a weight that is not above zero; its terms are zero
 #pragma unroll
     for (int dk = 0; dk < 2; dk++) {
         const float wz = tent(t[2], dk);
@@ -92,32 +98,35 @@ __device__ __forceinline__ void p2g_box(const DevParams& P, DevStats* st, const 
             const float wy = tent(t[1], dj);
 #pragma unroll
             for (int di = 0; di < 2; di++) {
-                const float wx = tent(t[0], di);
-                const float w = __fmul_rn(__fmul_rn(wx, wy), wz);
-                if (w <= 0.0f) continue;
-                const int li = (base[0] + di) + sx * ((base[1] + dj) + sy * (base[2] + dk));
-                atomicAdd(&s_num[li], fixed_round(__fmul_rn(__fmul_rn(w, vcomp), scale)));
-                atomicAdd(&s_den[li], fixed_round(__fmul_rn(w, scale)));
+                const float w = __fmul_rn(__fmul_rn(tent(t[0], di), wy), wz);
+                atomicAdd(num + di + PB_Y * dj + PB_Z * dk, fixed_round(__fmul_rn(__fmul_rn(w, vcomp), scale)));
+                atomicAdd(den + di + PB_Y * dj + PB_Z * dk, fixed_round(__fmul_rn(w, scale)));
             }
         }
     }
 }
 
+template <int TZ>
 __global__ void __launch_bounds__(256) k_p2g_own(DevBufs b, int tiles_x, int tiles_y) {
-    __shared__ int32_t s_num[3][PB_N];
-    __shared__ int32_t s_den[3][PB_N];
-    __shared__ uint32_t s_row_beg[P2G_OWN_ROWS];      // first sorted particle of each row of the tile
-    __shared__ uint32_t s_row_off[P2G_OWN_ROWS + 1];  // prefix of the row lengths
+    constexpr int PB_N = PB_Z * (TZ + 2);  // words of a box
+    __shared__ __align__(16) int32_t s_num[3][PB_N];
+    __shared__ __align__(16) int32_t s_den[3][PB_N];
+    __shared__ uint32_t s_row_beg[TILE * TZ];      // first sorted particle of each row of the tile
+    __shared__ uint32_t s_row_off[TILE * TZ + 1];  // prefix of the row lengths
     __shared__ uint32_t s_wsum[2];
     const DevParams& P = *b.prm;
     const int nx = (int)P.nx, ny = (int)P.ny, nz = (int)P.nz;
     const int tile = blockIdx.x;
-    const int x0 = (tile % tiles_x) * TILE, y0 = ((tile / tiles_x) % tiles_y) * TILE, z0 = (tile / (tiles_x * tiles_y)) * TILE;
-    const int xe = min(x0 + TILE, nx), ye = min(y0 + TILE, ny), ze = min(z0 + TILE, nz);
-    const int rows_y = ye - y0, rows = rows_y * (ze - z0);
+    const int x0 = (tile % tiles_x) * TILE, y0 = ((tile / tiles_x) % tiles_y) * TILE, z0 = (tile / (tiles_x * tiles_y)) * TZ;
+    const int xe = min(x0 + TILE, nx), ye = min(y0 + TILE, ny), ze = min(z0 + TZ, nz);
+    const int rows_y = ye - y0, rows_z = ze - z0, rows = rows_y * rows_z;
     uint32_t len = 0;
     if ((int)threadIdx.x < rows) {
-        const uint32_t cy = (uint32_t)(y0 + (int)threadIdx.x % rows_y), cz = (uint32_t)(z0 + (int)threadIdx.x / rows_y);
+        // even planes before odd ones, even rows before odd ones: see swz
+        const int ry = (int)threadIdx.x % rows_y, rz = (int)threadIdx.x / rows_y;
+        const int ey = (rows_y + 1) / 2, ez = (rows_z + 1) / 2;
+        const uint32_t cy = (uint32_t)(y0 + (ry < ey ? 2 * ry : 2 * (ry - ey) + 1));
+        const uint32_t cz = (uint32_t)(z0 + (rz < ez ? 2 * rz : 2 * (rz - ez) + 1));
         const uint32_t c0 = (uint32_t)x0 + P.nx * (cy + P.ny * cz), c1 = c0 + (uint32_t)(xe - x0 - 1);
         const uint32_t pbeg = b.offsets[c0];
         len = b.offsets[c1] + b.counts[c1] - pbeg;
@@ -139,9 +148,9 @@ __global__ void __launch_bounds__(256) k_p2g_own(DevBufs b, int tiles_x, int til
     }
     const uint32_t total = s_wsum[0] + s_wsum[1];
     if (total == 0) return;  // no particle binned in the tile: nothing to add (the face arrays are cleared)
-    for (int i = threadIdx.x; i < 3 * PB_N; i += blockDim.x) {
-        (&s_num[0][0])[i] = 0;
-        (&s_den[0][0])[i] = 0;
+    for (int i = threadIdx.x; i < 3 * PB_N / 4; i += blockDim.x) {
+        reinterpret_cast<int4*>(s_num)[i] = make_int4(0, 0, 0, 0);
+        reinterpret_cast<int4*>(s_den)[i] = make_int4(0, 0, 0, 0);
     }
     __syncthreads();
     const float inv_h = P.inv_h;
@@ -149,7 +158,7 @@ __global__ void __launch_bounds__(256) k_p2g_own(DevBufs b, int tiles_x, int til
     const int orig[3] = {x0, y0, z0};
     // Within each group of 256 particle indices thread t takes (t % 32) * 8
     // + t / 32, so the lanes of a warp hold particles of different cells (8
-    // per cell when dense) and their shared-memory atomics rarely meet.
+    // per cell when dense), two rows apart, and their atomics rarely meet.
     const uint32_t swz = (threadIdx.x & 31u) * 8u + (threadIdx.x >> 5);
     for (uint32_t g0 = 0; g0 < total; g0 += 256u * P2G_BATCH) {
         float4 pos[P2G_BATCH], vel[P2G_BATCH];
@@ -176,23 +185,24 @@ __global__ void __launch_bounds__(256) k_p2g_own(DevBufs b, int tiles_x, int til
             if (!use[k] || pos[k].w != 0.0f) continue;  // stray: handled by k_p2g_strays
             const float q[3] = {__fmul_rn(__fsub_rn(pos[k].x, o0), inv_h), __fmul_rn(__fsub_rn(pos[k].y, o1), inv_h),
                                 __fmul_rn(__fsub_rn(pos[k].z, o2), inv_h)};
-            p2g_box(P, b.st, orig, 0, q, vel[k].x, s_num[0], s_den[0]);
-            p2g_box(P, b.st, orig, 1, q, vel[k].y, s_num[1], s_den[1]);
-            p2g_box(P, b.st, orig, 2, q, vel[k].z, s_num[2], s_den[2]);
+            p2g_box<TZ>(P, b.st, orig, 0, q, vel[k].x, s_num[0], s_den[0]);
+            p2g_box<TZ>(P, b.st, orig, 1, q, vel[k].y, s_num[1], s_den[1]);
+            p2g_box<TZ>(P, b.st, orig, 2, q, vel[k].z, s_num[2], s_den[2]);
         }
     }
     __syncthreads();
 
     // Add the box to the face arrays: every nonzero sum of a face inside the grid.
+    // Warps take (y, z) rows of the box, half a warp a row.
     for (int axis = 0; axis < 3; axis++) {
-        const int sx = axis == 0 ? PB_A : PB_O, sy = axis == 1 ? PB_A : PB_O;
         const int fx0 = x0 - (axis != 0), fy0 = y0 - (axis != 1), fz0 = z0 - (axis != 2);
         const int dx = (int)face_dim(P, axis, 0), dy = (int)face_dim(P, axis, 1), dz = (int)face_dim(P, axis, 2);
-        for (int li = threadIdx.x; li < PB_N; li += blockDim.x) {
+        const int x = threadIdx.x & 15;
+        for (int row = threadIdx.x >> 4; row < (TILE + 2) * (TZ + 2); row += 16) {
+            const int fi = fx0 + x, fj = fy0 + row % (TILE + 2), fk = fz0 + row / (TILE + 2);
+            if (x >= TILE + 2 || fi < 0 || fj < 0 || fk < 0 || fi >= dx || fj >= dy || fk >= dz) continue;
+            const int li = x + PB_Y * (row % (TILE + 2)) + PB_Z * (row / (TILE + 2));
             const int32_t vn = s_num[axis][li], vd = s_den[axis][li];
-            if ((vn | vd) == 0) continue;
-            const int fi = fx0 + li % sx, fj = fy0 + (li / sx) % sy, fk = fz0 + li / (sx * sy);
-            if (fi < 0 || fj < 0 || fk < 0 || fi >= dx || fj >= dy || fk >= dz) continue;
             const size_t gidx = (size_t)fi + (size_t)dx * ((size_t)fj + (size_t)dy * fk);
             if (vn) atomicAdd(&b.num[axis][gidx], vn);
             if (vd) atomicAdd(&b.den[axis][gidx], vd);
@@ -543,7 +553,6 @@ cudaError_t launch_classify(const DevBufs& b, uint32_t C, cudaStream_t s) {
 
 cudaError_t launch_p2g(const DevBufs& b, const LaunchCfg& L, uint32_t nx, uint32_t ny, uint32_t nz, cudaStream_t s,
                        bool clear) {
-    const int tx = (int)((nx + TILE - 1) / TILE), ty = (int)((ny + TILE - 1) / TILE), tz = (int)((nz + TILE - 1) / TILE);
     // scatter.wgsl's accumulators start at zero (the reference's clear pass)
     for (int a = 0; clear && a < 3; a++) {
         const size_t faces = (size_t)(nx + (a == 0)) * (ny + (a == 1)) * (nz + (a == 2));
@@ -551,7 +560,16 @@ cudaError_t launch_p2g(const DevBufs& b, const LaunchCfg& L, uint32_t nx, uint32
         if (e == cudaSuccess) e = cudaMemsetAsync(b.den[a], 0, 4 * faces, s);
         if (e != cudaSuccess) return e;
     }
-    k_p2g_own<<<tx * ty * tz, 256, 0, s>>>(b, tx, ty);
+    const uint32_t tx = (nx + TILE - 1) / TILE, ty = (ny + TILE - 1) / TILE;
+    // A grid of few tiles takes flat ones: with 8^3 tiles a 64^3 half-tank has some
+    // 100 blocks with particles, and the kernel took as long as one block (38 us at
+    // 32^3, 46 us at 64^3; tiles of 8 x 8 x 2: 17 and 29 us, of 8 x 8 x 4: 19 and 37).
+    // A larger one fills the chip either way, and flat tiles add more rim sums to
+    // the face arrays (128^3: 77 us with 8^3, 95 us with 8 x 8 x 2; 256^3: 530 and 735).
+    if (tx * ty * ((nz + 7) / 8) < 8u * (uint32_t)L.num_sms)
+        k_p2g_own<2><<<tx * ty * ((nz + 1) / 2), 256, 0, s>>>(b, (int)tx, (int)ty);
+    else
+        k_p2g_own<8><<<tx * ty * ((nz + 7) / 8), 256, 0, s>>>(b, (int)tx, (int)ty);
     k_p2g_strays<<<L.num_sms, 256, 0, s>>>(b);
     return cudaGetLastError();
 }

@@ -35,7 +35,7 @@
 // load, then instruction issue (about 300 instructions per warp and phase 1);
 // beyond, L2 throughput and the same latencies per round of chunks.  Solves of
 // 40 / 179 / 200 / 200 iterations on 32^3 / 64^3 / 128^3 (2.0 M particles) /
-// 256^3 (18.3 M): 179 / 867 / 1,315 / 6,580 us against 224 / 1,123 / 1,558 /
+// 256^3 (18.3 M): 177 / 842 / 1,268 / 5,280 us against 224 / 1,123 / 1,558 /
 // 7,197 for the earlier kernel (1,024 threads over listed cells or quads, chunk
 // trees from shared memory, every block reading every chunk partial).
 //
@@ -66,8 +66,8 @@
 //                    go to other blocks and are published one by one.  Every
 //                    block adds the tails to the heads itself: one hop.
 //   split segments   (more chunks than that is good for) ranges of equal weight;
-//                    all chunk partials are published, one warp per segment adds
-//                    them and publishes the segment sum: two hops.
+//                    all chunk partials are published, a block adds those of its
+//                    segments and publishes the sums: two hops.
 //
 // Every block then evaluates the 256-wide tree of cg_reduce_final.wgsl over the
 // segment sums, so in FL_CG_F32 the scalars are the reference's f32 arithmetic
@@ -82,20 +82,21 @@ namespace fl {
 constexpr int CG_THREADS = 512;
 constexpr int CG_WARPS = CG_THREADS / 32;
 constexpr uint32_t KCH = 512;            // chunks a block keeps a table of
-constexpr uint32_t OWNER_WARPS = 4;      // warps of a block that add split segments
 constexpr uint32_t RAW_MAX = 1024;       // tail partials read by every block
 constexpr uint32_t TAG_SPAN_MAX = 1u << 30;
 constexpr uint32_t MAX_CG_BLOCKS = 256;
 // Per-chunk cost in liquid-cell units for ranges of equal weight: a warp takes a
 // chunk at once, so a sparsely filled one costs it nearly as much as a full one
-// (with 32, the slowest block's phase 1 at 256^3 took 38,000 cycles against
-// 26,000; with 256, 29,500); solvers that list cells use 32.
-constexpr uint32_t CHUNK_WEIGHT = 256, CELL_CHUNK_WEIGHT = 32;
+// (with 256, the slowest block at 256^3 got 170 chunks where the others had 150);
+// solvers that list cells use 32.
+constexpr uint32_t CHUNK_WEIGHT = 1024, CELL_CHUNK_WEIGHT = 32;
 // What the pool leaves of the 228 KB serves as L1 for the neighbours' rows: 140 KB
 // against 200 KB and 100 KB on the full-depth 128^3 dam (FL_CG_F64): 2,073, 2,094
 // and 2,206 us per solve; 256^3 within 1 %.
 constexpr uint32_t POOL_BYTES = 140 * 1024;
 constexpr uint32_t HALF_BYTES = 32 * 4 * 16;  // a resident half chunk: float4 d, r, q, p of 32 quads
+
+enum { SLOT_A, SLOT_B, SEG_A, SEG_B, WORD_A, WORD_B };  // exchange areas
 
 struct CgShared {
     // Per half chunk (32 quads, one per lane).  Register form: float4 p and the
@@ -103,7 +104,7 @@ struct CgShared {
     // stencil words of all (4 B per quad).
     alignas(16) unsigned char pool[POOL_BYTES];
     union {
-        float stage[OWNER_WARPS][CHUNK];   // partials of a split segment
+        alignas(16) float stage[2 * CHUNK];  // partials of two split segments
         float raw[RAW_MAX];                // tail partials
         struct {
             double dpart[CG_THREADS];      // FL_CG_F64_IEEE: thread partials
@@ -114,6 +115,7 @@ struct CgShared {
     float part[KCH];           // chunk partials of one phase
     uint32_t off[CHUNK + 1];   // plan entries of the segments' heads
     uint32_t toff[CHUNK + 1];  // and of their tails
+    uint32_t segslot[CHUNK];   // exchange words of the segments, ~0 for an empty one
     float seg[CHUNK];          // segment sums (cg_reduce_final.wgsl thread accumulators)
     float red[2 * CG_THREADS / 32];   // extended forms: warp partials
     float scal[4];             // scalars of an exchange, broadcast by warp 0
@@ -121,7 +123,7 @@ struct CgShared {
     // Block-uniform values read where they are used: the cell loops are at the
     // 128-register limit of a 512-thread block, and a spilled register costs an
     // L2 round trip after every exchange (the acquire empties the L1).
-    uint32_t nh, s0, m, mres, HL, nheads, ah;
+    uint32_t iters, nh, s0, m, mres, HL, HR, nheads, ah, nact, segline;
     uint64_t limit;            // of every wait, in ns
     float one;                 // 1.0f (see addp2)
     float thr_f;               // f32 stopping threshold on r.r
@@ -324,6 +326,11 @@ __device__ __forceinline__ double d_of(float lo, float hi) { return __hiloint2do
 enum { PLAN_F32, PLAN_EXTENDED, PLAN_RANGES };
 constexpr uint32_t H_TAG = CHUNK + 1, H_FORM = CHUNK + 2, H_START = CHUNK + 3;
 
+// Words of one owner block among the segment sums of the split form: whole
+// 128-byte lines (with the sums of sixteen blocks in a line, the exchange took
+// 1,000-2,000 cycles more), at most 16 G + 256 words in all.
+__device__ __forceinline__ uint32_t seg_line(uint32_t nact) { return ((CHUNK + nact - 1) / nact + 15u) & ~15u; }
+
 // One block of 256 threads.  Lists the active chunks, gives each block a
 // contiguous range of the list, and reserves this solve's tag range.  When the
 // 32-bit epoch would wrap, the exchange words are cleared first, so no stale
@@ -457,7 +464,8 @@ __global__ void __launch_bounds__(CHUNK) k_cg_plan(DevBufs b, uint32_t G, int fo
             for (; bbW <= XG; bb_next++, bbW += W) start[bb_next] = hoff + k;
         }
     }
-    uint32_t slot = li;
+    // split segments: block li % nact adds segment li
+    uint32_t slot = seg_line(nact) * (li % nact) + li / nact;
     if (T && A) {  // each block's words start on a 128-byte line
         const uint32_t blk = s_blk[li][s_sel];
         if (cnt && (li == 0 || s_blk[li - 1][s_sel] != blk)) {
@@ -551,11 +559,10 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
             sh.toff[i] = toffs[i];
         }
     }
-    const uint32_t segslot = tid < (uint32_t)CHUNK && hdr[tid] != hdr[tid + 1] ? start[G + 3 + tid] : 0xffffffffu;
+    if (tid < (uint32_t)CHUNK) sh.segslot[tid] = hdr[tid] != hdr[tid + 1] ? start[G + 3 + tid] : 0xffffffffu;
     // Every exchange area starts on a 128-byte line (the pool is 256-byte
     // aligned): a block's line must not share a physical line with a
     // neighbour's (measured 8-11 % of the solve at 128^3 when it did).
-    enum { SLOT_A, SLOT_B, SEG_A, SEG_B, WORD_A, WORD_B };
     if (tid == 0) {
         const size_t nslot = ((size_t)nchunks + 15) & ~(size_t)15, nseg = 16 * (size_t)G + CHUNK;
         unsigned long long* a = b.cg_x + 16;
@@ -565,10 +572,13 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
         sh.area[SEG_B] = a += nseg;
         sh.area[WORD_A] = a += nseg;          // extended forms: two words of block bb at 16*bb
         sh.area[WORD_B] = a += 16 * (size_t)G;
+        sh.iters = iters;
         sh.s0 = s0;
         sh.m = m;
         sh.nheads = start[G + 2];
         sh.ah = hdr[CHUNK];  // plan entries of the heads
+        sh.nact = nact;
+        sh.segline = seg_line(nact);
         sh.one = 1.0f;
         sh.limit = wait_limit_ns(b.prm);
     }
@@ -622,7 +632,10 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
         HR = regs ? 0u : nh * (HALF_BYTES + 128u) <= POOL_BYTES ? nh : (nh * 128u < POOL_BYTES ? (POOL_BYTES - nh * 128u) / HALF_BYTES : 0u);
         HL = nh < (POOL_BYTES - HR * HALF_BYTES) / 128u ? nh : (POOL_BYTES - HR * HALF_BYTES) / 128u;
     }
-    if (tid == 0) sh.HL = HL;
+    if (tid == 0) {
+        sh.HL = HL;
+        sh.HR = HR;
+    }
     // The resident arrays: operand k (0 d, 1 r, 2 q, 3 p) of quad i; after them
     // the stencil words of all halves.
     auto op = [&](uint32_t k, uint32_t i) -> Quad& { return reinterpret_cast<Quad*>(sh.pool)[32u * k * HR + i]; };
@@ -726,7 +739,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
         if (post != 1) sh.rs_hi = v;  // the initial r.r, or rs_new
         if (post == 2) {
             sc = rs_old > 1e-30f ? __fdiv_rn(v, rs_old) : 0.0f;
-            dn = stop_on && v <= sh.thr_f;
+            dn = v <= sh.thr_f;
         }
         sh.scal[0] = v;
         sh.scal[1] = sc;
@@ -760,6 +773,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
             __syncthreads();  // sh.part is complete, the phase's stores are issued
             const uint32_t ntail = vld(sh.toff[CHUNK]);
             if (tid < (uint32_t)CHUNK) {
+                const uint32_t segslot = sh.segslot[tid];
                 const uint32_t lo = sh.off[tid], hi = sh.off[tid + 1], s0 = vld(sh.s0);
                 const bool mine = segslot != 0xffffffffu && lo >= s0 && lo < s0 + vld(sh.m);
                 float s = 0.0f;
@@ -821,47 +835,44 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
                 }
             }
         } else {
-            if (warp < OWNER_WARPS) {
-                float* buf = sh.stage[warp];
-                for (uint32_t li = blockIdx.x + warp * nact; li < (uint32_t)CHUNK; li += OWNER_WARPS * nact) {
-                    const uint32_t lo = sh.off[li], hi = sh.off[li + 1];
-                    if (lo == hi) continue;
-                    float s = 0.0f;
-                    for (uint32_t e0 = lo; e0 < hi; e0 += 256u) {
-                        // all eight polls of a lane in flight, then the waits
-                        unsigned long long w[8];
-#pragma unroll
-                        for (int k2 = 0; k2 < 8; k2++) {
-                            const uint32_t e = e0 + lane + 32u * k2;
-                            w[k2] = e < hi ? ld_tag(slots + e, acq) : 0ull;
+            // Block bb adds segments bb, bb + nact, ...: two at a time, a half of the
+            // block each, so that a thread waits for one word.  (One warp per segment
+            // with eight words per lane waited for up to eight round trips, one after
+            // the other: 12,000 cycles per exchange at 256^3 instead of 6,300.)
+            const uint32_t half = tid / CHUNK;
+            for (uint32_t l0 = blockIdx.x; l0 < (uint32_t)CHUNK; l0 += 2u * vld(sh.nact)) {
+                const uint32_t l1 = l0 + vld(sh.nact), li = half ? l1 : l0;
+                const uint32_t lo = li < (uint32_t)CHUNK ? sh.off[li] : 0u, hi = li < (uint32_t)CHUNK ? sh.off[li + 1] : 0u;
+                const uint32_t n0 = sh.off[l0 + 1] - sh.off[l0], n1 = l1 < (uint32_t)CHUNK ? sh.off[l1 + 1] - sh.off[l1] : 0u;
+                float s = 0.0f;
+                for (uint32_t e0 = 0; e0 < (n0 > n1 ? n0 : n1); e0 += CHUNK) {
+                    const uint32_t e = lo + e0 + (tid & (CHUNK - 1u));
+                    sh.stage[tid] = e < hi ? wait_word(slots + e, tag, acq, ok) : 0.0f;
+                    __syncthreads();
+                    if ((tid & (CHUNK - 1u)) == 0u && lo + e0 < hi) {
+                        // cg_reduce_final.wgsl:29-36: in plan order, from +0 (past the end: +0);
+                        // the next eight are loaded ahead: the chain is the adds alone
+                        const float4* const b4 = reinterpret_cast<const float4*>(sh.stage + tid);
+                        const uint32_t n = hi - lo - e0 < (uint32_t)CHUNK ? hi - lo - e0 : CHUNK;
+                        float4 u = b4[0], v = b4[1];
+                        for (uint32_t j = 0; j < n; j += 8) {
+                            const uint32_t jn = j + 8 < (uint32_t)CHUNK ? j / 4 + 2 : 0u;
+                            const float4 un = b4[jn], vn = b4[jn + 1];
+                            s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, u.x), u.y), u.z), u.w);
+                            s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, v.x), v.y), v.z), v.w);
+                            u = un;
+                            v = vn;
                         }
-#pragma unroll
-                        for (int k2 = 0; k2 < 8; k2++) {
-                            const uint32_t e = e0 + lane + 32u * k2;
-                            if (e < hi && (uint32_t)(w[k2] >> 32) != tag && ok) {
-                                w[k2] = wait_tag(slots + e, tag, st, acq, &sh.limit);
-                                ok = (uint32_t)(w[k2] >> 32) == tag;
-                            }
-                            buf[lane + 32u * k2] = e < hi ? __uint_as_float((uint32_t)w[k2]) : 0.0f;
-                        }
-                        __syncwarp();
-                        if (lane == 0) {  // cg_reduce_final.wgsl:29-36: in plan order, from +0 (past the end: +0)
-                            const uint32_t n = hi - e0 < 256u ? hi - e0 : 256u;
-                            for (uint32_t j = 0; j < n; j += 8) {
-                                float t8[8];
-#pragma unroll
-                                for (int k2 = 0; k2 < 8; k2++) t8[k2] = buf[j + k2];
-#pragma unroll
-                                for (int k2 = 0; k2 < 8; k2++) s = __fadd_rn(s, t8[k2]);
-                            }
-                        }
-                        __syncwarp();
                     }
                     // a segment whose partials did not all arrive is not published
-                    if (__all_sync(0xffffffffu, ok) && lane == 0) publish(segw + li, tag, s, acq);
+                    if (__syncthreads_or(!ok)) return false;
                 }
+                if ((tid & (CHUNK - 1u)) == 0u && lo != hi)
+                    publish(segw + vld(sh.segline) * blockIdx.x + li / vld(sh.nact), tag, s, acq);
             }
-            if (tid < (uint32_t)CHUNK) sh.seg[tid] = segslot != 0xffffffffu ? wait_word(segw + tid, tag, acq, ok) : 0.0f;
+            __syncwarp();
+            const uint32_t segslot = sh.segslot[tid & (CHUNK - 1u)];
+            if (tid < (uint32_t)CHUNK) sh.seg[tid] = segslot != 0xffffffffu ? wait_word(segw + segslot, tag, acq, ok) : 0.0f;
         }
         __syncwarp();
         if (__syncthreads_or(!ok)) return false;
@@ -895,7 +906,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
                 if (post == 1) scv = fabs(v) > 1e-30 ? (float)(rs_old / v) : 0.0f;
                 if (post == 2) {
                     scv = rs_old > 1e-30 ? (float)(v / rs_old) : 0.0f;
-                    d2 = stop_on && v <= sh.thr_d;
+                    d2 = v <= sh.thr_d;
                     sh.rs_d = v;
                 }
                 sh.scal[1] = scv;
@@ -912,7 +923,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
                 if (post == 1) scv = fabsf(acc.hi) > 1e-30f ? df_div(rs_old, acc) : 0.0f;
                 if (post == 2) {
                     scv = rs_old.hi > 1e-30f ? df_div(acc, rs_old) : 0.0f;
-                    d2 = stop_on && df_le(acc, Df{sh.thr_dh, sh.thr_dl});
+                    d2 = df_le(acc, Df{sh.thr_dh, sh.thr_dl});
                     sh.rs_hi = acc.hi;
                     sh.rs_lo = acc.lo;
                 }
@@ -978,7 +989,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
             s = warp_sum_d(s);
             if (lane == 0) {
                 sh.rs_d = s;
-                sh.thr_d = P.thr_abs ? P.thr_abs_d : P.tol_sq_d * s;
+                sh.thr_d = !stop_on ? -1.0 : P.thr_abs ? P.thr_abs_d : P.tol_sq_d * s;  // r.r is never below 0
                 if (blockIdx.x == 0) st->rs_init = s;
             }
         }
@@ -1002,7 +1013,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
             if (lane == 0) {
                 sh.rs_hi = rs_init_d.hi;
                 sh.rs_lo = rs_init_d.lo;
-                const double thr = P.thr_abs ? P.thr_abs_d : P.tol_sq_d * df_to_double(rs_init_d);
+                const double thr = !stop_on ? -1.0 : P.thr_abs ? P.thr_abs_d : P.tol_sq_d * df_to_double(rs_init_d);
                 sh.thr_dh = (float)thr;
                 sh.thr_dl = (float)(thr - (double)sh.thr_dh);
                 if (blockIdx.x == 0) st->rs_init = df_to_double(rs_init_d);
@@ -1027,7 +1038,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
             // f32 threshold: tol^2 * rs_init (cg_beta.wgsl:25-30) or the absolute one
             if (lane == 0) {
                 sh.rs_hi = rs_init_f;
-                sh.thr_f = P.thr_abs ? P.thr_abs_f : __fmul_rn(P.tol_sq, rs_init_f);
+                sh.thr_f = !stop_on ? -1.0f : P.thr_abs ? P.thr_abs_f : __fmul_rn(P.tol_sq, rs_init_f);
                 if (blockIdx.x == 0) st->rs_init = (double)rs_init_f;
             }
         }
@@ -1089,7 +1100,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
     };
 
     float beta = 0.0f;  // the first direction is r + 0 * r
-    uint32_t k = 0, tag = tag_base;
+    uint32_t it = 0, tag = tag_base;
     if (regs) {
         // One chunk per warp.  A lane keeps its two quads' d, r and stencil words
         // in registers; p, q and the d of the y and z neighbours in shared
@@ -1115,7 +1126,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
         const bool any0 = __any_sync(0xffffffffu, (e[0] & 15u) != 0u), any1 = __any_sync(0xffffffffu, (e[1] & 15u) != 0u);
         float de = 0.0f;  // lane 0: d of the cell before the chunk, lane 31: of the one after
 #pragma unroll 1
-        for (uint32_t it = 0; it < iters; it++) {
+        for (; it < vld(sh.iters); it++) {
             // ---------------- phase 1: direction + SpMV + d.q ----------------
             // No branches per lane: d and r are zero in every cell that is not
             // liquid, and a zero term leaves a sum that starts at +0 unchanged.
@@ -1185,22 +1196,25 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
             }
             tag++;
             if (!f64 && !whole) publish_parts(0, vld(sh.m), vld(sh.area[SLOT_B]), tag, true);
-            k = it + 1;
             if (mine) {
                 const Quad a4 = qall(alpha);
                 pool[0] = qaddp(qmul(a4, dq[0]), one, pool[0]);
                 pool[6 * 32] = qaddp(qmul(a4, dq[1]), one, pool[6 * 32]);
             }
             if (!exchange(acc, tag, 2, beta, dn)) return;
-            if (dn) break;
+            if (dn) {
+                it++;
+                break;
+            }
         }
         if (mine) {
             st_q(p, c[0], e[0], pool[0]);
             st_q(p, c[1], e[1], pool[6 * 32]);
         }
     } else {
+        HR = vld(sh.HR);  // not live in the loop above
 #pragma unroll 1
-        for (uint32_t it = 0; it < iters; it++) {
+        for (; it < vld(sh.iters); it++) {
             float* d_cur = (it & 1u) ? b.dB : b.dA;
             const float* d_src = (it & 1u) || it == 0 ? b.dA : b.dB;
             const Quad beta4 = qall(beta);
@@ -1317,12 +1331,15 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
                     if (je < vld(sh.m)) __syncthreads();
                 }
             }
-            k = it + 1;
             if (!exchange(acc, tag, 2, beta, dn)) return;
-            if (dn) break;
+            if (dn) {
+                it++;
+                break;
+            }
         }
     }
     // the resident pressure, once
+    HR = vld(sh.HR);
     for (uint32_t j = warp; j < vld(sh.mres); j += CG_WARPS) {
         const Quads o = quads_of(j);
 #pragma unroll
@@ -1330,7 +1347,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
             if (o.any[h]) st_q(p, o.c[h], o.e[h], op(3, o.i[h]));
     }
     if (blockIdx.x == 0 && tid == 0) {
-        st->cg_iters = k;
+        st->cg_iters = it;
         st->rs_final = ieee ? sh.rs_d : (f64 ? df_to_double(Df{sh.rs_hi, sh.rs_lo}) : (double)sh.rs_hi);
     }
 }

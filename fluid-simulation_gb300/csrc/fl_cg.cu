@@ -1087,17 +1087,22 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
         acc_add(a, hi2(x.b), hi2(y.b));
     };
     // The exchange after a phase: post 1 alpha, post 2 beta and the stopping test.
-    auto exchange = [&](Acc (&acc)[2], uint32_t tag, int post, float& sc, bool& dn) -> bool {
-        if (f64) {
+    // `meanwhile` (extended forms) is done while the words travel.
+    auto exchange = [&](Acc (&acc)[2], uint32_t tag, int post, float& sc, bool& dn, auto&& meanwhile) -> bool {
+        if constexpr (f64) {
             if constexpr (ieee) acc[0] += acc[1];
             else acc[0] = df_add(acc[0], acc[1]);
             unsigned long long* const w = vld(sh.area[post == 1 ? WORD_A : WORD_B]);
             publish_df(acc[0], w, tag, post == 2);
+            __syncwarp();
+            meanwhile();
             return reduce_df(w, tag, post == 2, post, sc, dn);
+        } else {
+            return reduce_f32(vld(sh.area[post == 1 ? SLOT_A : SLOT_B]), vld(sh.area[post == 1 ? SEG_A : SEG_B]), tag,
+                              post == 2, post, sc, dn);
         }
-        return reduce_f32(vld(sh.area[post == 1 ? SLOT_A : SLOT_B]), vld(sh.area[post == 1 ? SEG_A : SEG_B]), tag, post == 2,
-                          post, sc, dn);
     };
+    const auto nothing = [] {};
 
     float beta = 0.0f;  // the first direction is r + 0 * r
     uint32_t it = 0, tag = tag_base;
@@ -1176,7 +1181,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
             if (!f64 && !whole) publish_parts(0, vld(sh.m), vld(sh.area[SLOT_A]), tag, false);
             float alpha;
             bool dn;
-            if (!exchange(acc, tag, 1, alpha, dn)) return;
+            if (!exchange(acc, tag, 1, alpha, dn, nothing)) return;
             // ---------------- phase 2: update + r.r (cg_update.wgsl:33-34) ----------------
             acc[0] = Acc{};
             acc[1] = Acc{};
@@ -1201,7 +1206,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
                 pool[0] = qaddp(qmul(a4, dq[0]), one, pool[0]);
                 pool[6 * 32] = qaddp(qmul(a4, dq[1]), one, pool[6 * 32]);
             }
-            if (!exchange(acc, tag, 2, beta, dn)) return;
+            if (!exchange(acc, tag, 2, beta, dn, nothing)) return;
             if (dn) {
                 it++;
                 break;
@@ -1284,7 +1289,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
             }
             float alpha;
             bool dn;
-            if (!exchange(acc, tag, 1, alpha, dn)) return;
+            if (!exchange(acc, tag, 1, alpha, dn, nothing)) return;
             // ---------------- phase 2: update + r.r (cg_update.wgsl:33-34) ----------------
             acc[0] = Acc{};
             acc[1] = Acc{};
@@ -1296,20 +1301,21 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
                 Quad prod[2] = {z4, z4};
                 auto update = [&](int h) {
                     const uint32_t c = o.c[h], e = o.e[h], i = o.i[h];
-                    Quad d4, q4, r4, p4;
+                    Quad q4, r4, d4 = z4, p4 = z4;
                     if (res) {
-                        d4 = op(0, i); q4 = op(2, i); r4 = op(1, i); p4 = op(3, i);
+                        q4 = op(2, i); r4 = op(1, i);
+                        if (!f64) { d4 = op(0, i); p4 = op(3, i); }
                     } else {
-                        d4 = ld_q(d_cur, c, e); q4 = ld_q(q, c, e); r4 = ld_q(r, c, e); p4 = ld_q(p, c, e);
+                        q4 = ld_q(q, c, e); r4 = ld_q(r, c, e);
+                        d4 = ld_q(d_cur, c, e); p4 = ld_q(p, c, e);
                     }
-                    p4 = qaddp(qmul(a4, d4), one, p4);
                     r4 = qaddp(qmul(na4, q4), one, r4);  // r - alpha q = r + (-alpha) q
                     st_q(r, c, e, r4);
-                    if (res) {
-                        op(1, i) = r4;
-                        op(3, i) = p4;
-                    } else {
-                        st_q(p, c, e, p4);
+                    if (res) op(1, i) = r4;
+                    if (!f64 || !res) {
+                        p4 = qaddp(qmul(a4, d4), one, p4);
+                        if (res) op(3, i) = p4;
+                        else st_q(p, c, e, p4);
                     }
                     if (f64) acc_quad(acc[h], r4, r4);
                     else prod[h] = qmul(r4, r4);
@@ -1331,7 +1337,23 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
                     if (je < vld(sh.m)) __syncthreads();
                 }
             }
-            if (!exchange(acc, tag, 2, beta, dn)) return;
+            // Extended forms: nothing waits for p, so the resident chunks' is advanced
+            // while the words travel (full-depth 128^3 dam: 2,058 -> 1,980 us; the others'
+            // loads are in the polls' way: with them 256^3 took 4,432 us, without 4,140, before 4,270).  FL_CG_F32's
+            // exchange is busy with the segments (256^3, 5,205 -> 5,317 us).
+            auto resident_p = [&] {
+#pragma unroll 1
+                for (uint32_t j = warp; j < vld(sh.mres); j += CG_WARPS) {
+                    const uint4 t = sh.tab[j];
+#pragma unroll
+                    for (int h = 0; h < 2; h++)
+                        if (h ? t.z : t.y) {
+                            const uint32_t i = slot_of(t, h);
+                            op(3, i) = qaddp(qmul(a4, op(0, i)), one, op(3, i));
+                        }
+                }
+            };
+            if (!exchange(acc, tag, 2, beta, dn, resident_p)) return;
             if (dn) {
                 it++;
                 break;

@@ -324,6 +324,7 @@ __device__ __forceinline__ double d_of(float lo, float hi) { return __hiloint2do
 // blocks that own heads, exchange word of every segment [CHUNK], offsets of the
 // tails [CHUNK + 1].
 enum { PLAN_F32, PLAN_EXTENDED, PLAN_RANGES };
+constexpr uint32_t TILE_Y = 4, TILE_Z = 4;  // chunks of a tile of the list (k_cg_plan)
 constexpr uint32_t H_TAG = CHUNK + 1, H_FORM = CHUNK + 2, H_START = CHUNK + 3;
 
 // Words of one owner block among the segment sums of the split form: whole
@@ -348,9 +349,16 @@ __device__ __forceinline__ uint32_t seg_line(uint32_t nact) { return ((CHUNK + n
 // ranges of equal weight (liquid cells + CHUNK_WEIGHT per chunk) of the list in
 // segment order; with at least 9 chunks per block on average no range is empty.
 //
-// form: PLAN_EXTENDED (no segment sums) takes heads and tails only where each
-// warp gets one chunk; PLAN_RANGES the G ranges of equal weight, for solvers
-// that use just those.
+// PLAN_EXTENDED (no segment sums) and PLAN_RANGES (solvers that use just the
+// ranges, of equal weight) are free to give a block any chunks: they list them in
+// tiles of TILE_Y neighbours along y by TILE_Z planes, so that the chunks that a
+// block's warps work on at a time share their neighbours' rows in the L1 (reads of
+// the L2 are what bounds phase 1).  Against the segment order, whose neighbours
+// are 256 chunks apart: FL_CG_F64 1,976 -> 1,890 us on the full-depth 128^3 dam,
+// 4,126 -> 3,990 at 256^3, multigrid 1,584 -> 1,555; tiles of 2 x 8 and 8 x 2 give
+// the same within 1 %.  Blocks of one chunk per warp (or half of that) where there
+// are enough blocks.  For split segments the order did not pay: a block's partials
+// then belong to many segments (256^3: 5,183 -> 5,238 us).
 __global__ void __launch_bounds__(CHUNK) k_cg_plan(DevBufs b, uint32_t G, int form) {
     const bool ranges_only = form == PLAN_RANGES;
     const uint32_t per_chunk = ranges_only ? CELL_CHUNK_WEIGHT : CHUNK_WEIGHT;
@@ -402,7 +410,7 @@ __global__ void __launch_bounds__(CHUNK) k_cg_plan(DevBufs b, uint32_t G, int fo
         A += s_wc[w];
         W += s_ww[w];
     }
-    if (!ranges_only && warp == 0) {
+    if (form == PLAN_F32 && warp == 0) {
         const uint32_t T = lane ? CG_WARPS * lane : CG_WARPS / 2;
         uint32_t blk = 0xffffffffu, cur = T, tails = 0;
 #pragma unroll 16
@@ -426,13 +434,17 @@ __global__ void __launch_bounds__(CHUNK) k_cg_plan(DevBufs b, uint32_t G, int fo
         }
     }
     __syncthreads();
-    uint32_t Gs = G, T = 0;
-    if (!ranges_only) {
-        Gs = A / 9u < 1u ? 1u : (A / 9u < G ? A / 9u : G);
-        const uint32_t per = (A + Gs - 1) / Gs;
+    // chunks per block: T of heads and tails, Tq of ranges that give each warp one
+    uint32_t Gs = G, T = 0, Tq = 0;
+    if (form == PLAN_EXTENDED) {
+        Tq = A <= G * (CG_WARPS / 2) ? CG_WARPS / 2 : A <= G * CG_WARPS ? CG_WARPS : 0u;
+    } else if (form == PLAN_F32) {
+        const uint32_t per = (A + G - 1) / G;
         const uint32_t rounds = (s_T + CG_WARPS - 1) / CG_WARPS;
-        if (s_T && (form == PLAN_F32 || rounds == 1) && rounds <= (per + CG_WARPS - 1) / CG_WARPS + 1) T = s_T;
+        if (s_T && rounds <= (per + CG_WARPS - 1) / CG_WARPS + 1) T = s_T;
     }
+    if (form != PLAN_RANGES) Gs = A / 9u < 1u ? 1u : (A / 9u < G ? A / 9u : G);
+    if (Tq) Gs = A ? (A + Tq - 1) / Tq : 1u;
     // head and tail of segment li, their places in the list
     const uint32_t nh = T && cnt > T ? T : cnt;
     const uint32_t xh = scan(nh);
@@ -448,21 +460,79 @@ __global__ void __launch_bounds__(CHUNK) k_cg_plan(DevBufs b, uint32_t G, int fo
     if (li == CHUNK - 1) hdr[CHUNK] = hoff + nh;
     const uint32_t nheads = T ? s_nblk : Gs, ntails = T ? (A - Ah + T - 1) / T : 0u;
     const uint32_t nact = A == 0 ? 1u : nheads + ntails;
-    uint64_t XG = (uint64_t)(wbase + y - wsum) * Gs;  // Gs x the weight of all entries before this segment
     // Blocks bb with X*Gs < bb*W <= X1*Gs start after the entry spanning
-    // weights [X, X1).  X only grows along this thread's entries, so the
-    // next such block is tracked incrementally from one division.
-    uint64_t bb_next = W ? XG / W + 1 : 0, bbW = bb_next * W;
-    uint32_t k = 0;
-    for (uint32_t c = li; c < nchunks; c += CHUNK) {
-        const uint32_t f = b.chunk_flag[c];
-        if (!f) continue;
-        b.cg_chunk[k < nh ? hoff + k : Ah + toff + (k - nh)] = c;
-        k++;
-        if (!T) {
-            XG += (uint64_t)(f + per_chunk) * Gs;
-            for (; bbW <= XG; bb_next++, bbW += W) start[bb_next] = hoff + k;
+    // weights [X, X1).  X only grows along a thread's entries, so the next such
+    // block is tracked incrementally from one division.
+    if (form == PLAN_F32) {  // in segment order
+        uint64_t XG = (uint64_t)(wbase + y - wsum) * Gs;  // Gs x the weight of all entries before this segment
+        uint64_t bb_next = W ? XG / W + 1 : 0, bbW = bb_next * W;
+        uint32_t k = 0;
+        for (uint32_t c = li; c < nchunks; c += CHUNK) {
+            const uint32_t f = b.chunk_flag[c];
+            if (!f) continue;
+            b.cg_chunk[k < nh ? hoff + k : Ah + toff + (k - nh)] = c;
+            k++;
+            if (!T) {
+                XG += (uint64_t)(f + per_chunk) * Gs;
+                for (; bbW <= XG; bb_next++, bbW += W) start[bb_next] = hoff + k;
+            }
         }
+    } else {  // in tile order
+        // Z chunks per plane (whole ones: the tiles shear a little where a plane is no
+        // multiple of 256 cells); every chunk is in one tile whatever Z is
+        const uint32_t Z = P.nx * P.ny / CHUNK ? P.nx * P.ny / CHUNK : 1u, planes = (nchunks + Z - 1) / Z;
+        const uint32_t ty = (Z + TILE_Y - 1) / TILE_Y, ntile = ty * ((planes + TILE_Z - 1) / TILE_Z);
+        const uint32_t per = (ntile + CHUNK - 1) / CHUNK;  // of a thread
+        const uint32_t t0 = li * per < ntile ? li * per : ntile, t1 = t0 + per < ntile ? t0 + per : ntile;
+        auto flags = [&](uint32_t t, uint8_t (&f)[16]) {  // returns the tile's first chunk
+            const uint32_t y0 = TILE_Y * (t % ty), c0 = TILE_Z * (t / ty) * Z + y0;
+#pragma unroll
+            for (uint32_t i = 0; i < 16; i++) {
+                const uint32_t c = c0 + (i / TILE_Y) * Z + i % TILE_Y;
+                f[i] = y0 + i % TILE_Y < Z && c < nchunks ? b.chunk_flag[c] : (uint8_t)0;
+            }
+            return c0;
+        };
+        uint32_t n = 0, w = 0;
+        for (uint32_t t = t0; t < t1; t++) {
+            uint8_t f[16];
+            flags(t, f);
+#pragma unroll
+            for (int i = 0; i < 16; i++)
+                if (f[i]) {
+                    n++;
+                    w += f[i] + per_chunk;
+                }
+        }
+        const uint32_t xn = scan(n), xw = scan(w);
+        __syncthreads();
+        if (lane == 31) {
+            s_wc[warp] = xn;
+            s_ww[warp] = xw;
+        }
+        __syncthreads();
+        uint32_t e = xn - n, wb = xw - w;
+        for (uint32_t v = 0; v < warp; v++) {
+            e += s_wc[v];
+            wb += s_ww[v];
+        }
+        uint64_t XG = (uint64_t)wb * Gs;  // Gs x the weight of all entries before
+        uint64_t bb_next = W ? XG / W + 1 : 0, bbW = bb_next * W;
+        for (uint32_t t = t0; t < t1; t++) {
+            uint8_t f[16];
+            const uint32_t c0 = flags(t, f);
+#pragma unroll
+            for (uint32_t i = 0; i < 16; i++) {
+                if (!f[i]) continue;
+                b.cg_chunk[e++] = c0 + (i / TILE_Y) * Z + i % TILE_Y;
+                if (!Tq) {
+                    XG += (uint64_t)(f[i] + per_chunk) * Gs;
+                    for (; bbW <= XG; bb_next++, bbW += W) start[bb_next] = e;
+                }
+            }
+        }
+        if (Tq)
+            for (uint32_t bb = li; bb <= Gs; bb += CHUNK) start[bb] = bb * Tq < A ? bb * Tq : A;
     }
     // split segments: block li % nact adds segment li
     uint32_t slot = seg_line(nact) * (li % nact) + li / nact;

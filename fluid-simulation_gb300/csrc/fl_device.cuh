@@ -49,6 +49,8 @@ struct DevParams {
     // in ns; 0 = the default of 2 s.  On expiry the kernel records FL_TIMEOUT
     // and every block returns.
     uint64_t wait_ns;
+    // Division of a cell index (below 2^31) by nx and ny: see cell_coords.
+    uint32_t nx_mul, nx_shift, ny_mul, ny_shift;
 };
 
 // Per-step device counters and results.
@@ -234,6 +236,18 @@ __device__ __forceinline__ bool is_stray(const DevParams& P, float4 pos, const u
     float q1 = __fmul_rn(__fsub_rn(pos.y, P.origin[1]), P.inv_h);
     float q2 = __fmul_rn(__fsub_rn(pos.z, P.origin[2]), P.inv_h);
     return floorf(q0) != (float)kc[0] || floorf(q1) != (float)kc[1] || floorf(q2) != (float)kc[2];
+}
+
+// (i, j, k) of cell c.  n / d = umulhi(n, mul) >> shift with mul =
+// ceil(2^(31 + L) / d), shift = L - 1, L = ceil(log2 d): mul exceeds 2^(31+L) / d by
+// less than 1 <= 2^L / d, so the product is above n / d by less than 1 / d for n < 2^31
+// and the quotient is exact (Granlund and Montgomery 1994).  Three divisions took
+// the cell kernels some 60 instructions a cell.
+__device__ __forceinline__ void cell_coords(const DevParams& P, uint32_t c, uint32_t& i, uint32_t& j, uint32_t& k) {
+    const uint32_t row = __umulhi(c, P.nx_mul) >> P.nx_shift;
+    k = __umulhi(row, P.ny_mul) >> P.ny_shift;
+    i = c - row * P.nx;
+    j = row - k * P.ny;
 }
 
 __device__ __forceinline__ int32_t floor_to_i32(float x) { return __float2int_rz(floorf(x)); }

@@ -17,29 +17,44 @@
 
 namespace fl {
 
+// Four cells per thread and one atomic per 1,024 cells: with a cell per thread and
+// an atomic per warp, the additions to the one counter and the divisions took 70 us
+// at 256^3, where the counts read and the types written are 12 us of traffic; now 33.
+constexpr int CLASSIFY_CELLS = 4;
+
 __global__ void __launch_bounds__(256) k_classify(DevBufs b, uint32_t C) {
+    __shared__ uint32_t s_n;
     const DevParams& P = *b.prm;
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    bool liquid = false;
-    if (c < C) {
-        const uint32_t nx = P.nx, ny = P.ny, nz = P.nz;
-        const uint32_t i = c % nx, j = (c / nx) % ny, k = c / (nx * ny);
-        const bool boundary = i == 0 || j == 0 || k == 0 || i == nx - 1 || j == ny - 1 || k == nz - 1;
-        uint8_t t = CELL_SOLID;
-        if (!boundary) {
-            const uint32_t th = P.thresh;
-            const uint32_t* occ = b.counts;
-            liquid = occ[c] >= th;
-            if (!liquid && P.dilation) {
-                liquid = occ[c - 1] >= th || occ[c + 1] >= th || occ[c - nx] >= th || occ[c + nx] >= th ||
-                         occ[c - nx * ny] >= th || occ[c + nx * ny] >= th;
+    if (threadIdx.x == 0) s_n = 0;
+    const uint32_t c0 = blockIdx.x * 256u * CLASSIFY_CELLS + threadIdx.x;
+    const uint32_t nx = P.nx, ny = P.ny, nz = P.nz, th = P.thresh;
+    const uint32_t* __restrict__ occ = b.counts;
+    uint32_t n[CLASSIFY_CELLS], liquids = 0;
+#pragma unroll
+    for (int q = 0; q < CLASSIFY_CELLS; q++) n[q] = c0 + 256u * q < C ? occ[c0 + 256u * q] : 0u;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < CLASSIFY_CELLS; q++) {
+        const uint32_t c = c0 + 256u * q;
+        bool liquid = false;
+        if (c < C) {
+            uint32_t i, j, k;
+            cell_coords(P, c, i, j, k);
+            uint8_t t = CELL_SOLID;
+            if (i - 1u < nx - 2u && j - 1u < ny - 2u && k - 1u < nz - 2u) {  // inside the boundary layer
+                liquid = n[q] >= th;
+                if (!liquid && P.dilation)
+                    liquid = occ[c - 1] >= th || occ[c + 1] >= th || occ[c - nx] >= th || occ[c + nx] >= th ||
+                             occ[c - nx * ny] >= th || occ[c + nx * ny] >= th;
+                t = liquid ? CELL_LIQUID : CELL_AIR;
             }
-            t = liquid ? CELL_LIQUID : CELL_AIR;
+            b.ct[c] = t;
         }
-        b.ct[c] = t;
+        liquids += (uint32_t)__popc(__ballot_sync(0xffffffffu, liquid));
     }
-    const uint32_t m = __ballot_sync(0xffffffffu, liquid);
-    if ((threadIdx.x & 31u) == 0 && m) atomicAdd(&b.st->liquid, (uint32_t)__popc(m));
+    if ((threadIdx.x & 31u) == 0 && liquids) atomicAdd(&s_n, liquids);
+    __syncthreads();
+    if (threadIdx.x == 0 && s_n) atomicAdd(&b.st->liquid, s_n);
 }
 
 // ---------------------------------------------------------------------------
@@ -277,24 +292,42 @@ __device__ __forceinline__ float face_value(const DevParams& P, int axis, int32_
     return v;
 }
 
-// cg_reduce.wgsl:38-49 tree over a 256-thread block (s has 256 floats).
-// Steps 128/64/32 go through shared memory, 16..1 through shuffles of warp 0;
-// the pairing (i with i+off) is the same at every level.
-__device__ __forceinline__ float block_tree256(float prod, float* s) {
+// The partial sums of r.r of a 256-cell chunk, one cell per thread of a 256-thread
+// block (s: 256 floats, s2: 8): the tree of cg_reduce.wgsl:38-49, whose steps 128,
+// 64 and 32 are formed by warp 0 from shared memory (with the same pairs: i with
+// i + 128, then + 64, then + 32) and whose other steps are shuffles; the
+// float-float sum in a fixed order (warp shuffles, then the warps in order); the
+// number of liquid cells.  A chunk without liquid is done without either.
+__device__ __forceinline__ void chunk_partials(const DevBufs& b, uint32_t chunk, bool liquid, float prod, Df pdf, float* s,
+                                               float2* s2) {
     const int t = threadIdx.x;
     s[t] = prod;
+    const int nliq = __syncthreads_count(liquid);
+    if (nliq == 0) {
+        if (t == 0) {
+            b.part_rr[chunk] = 0.0f;
+            b.chunk_rr_df[chunk] = make_float2(0.0f, 0.0f);
+            b.chunk_flag[chunk] = 0;
+        }
+        return;
+    }
+    pdf = warp_sum_df(pdf);
+    if ((t & 31) == 0) s2[t >> 5] = make_float2(pdf.hi, pdf.lo);
     __syncthreads();
-    if (t < 128) s[t] = __fadd_rn(s[t], s[t + 128]);
-    __syncthreads();
-    if (t < 64) s[t] = __fadd_rn(s[t], s[t + 64]);
-    __syncthreads();
-    float v = 0.0f;
     if (t < 32) {
-        v = __fadd_rn(s[t], s[t + 32]);
+        const float a = __fadd_rn(__fadd_rn(s[t], s[t + 128]), __fadd_rn(s[t + 64], s[t + 192]));
+        const float c = __fadd_rn(__fadd_rn(s[t + 32], s[t + 160]), __fadd_rn(s[t + 96], s[t + 224]));
+        float v = __fadd_rn(a, c);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v = __fadd_rn(v, __shfl_down_sync(0xffffffffu, v, o));
+        if (t == 0) {
+            Df d = {0.0f, 0.0f};
+            for (int w = 0; w < 8; w++) d = df_add(d, Df{s2[w].x, s2[w].y});
+            b.part_rr[chunk] = v;
+            b.chunk_rr_df[chunk] = make_float2(d.hi, d.lo);
+            b.chunk_flag[chunk] = (uint8_t)(nliq < 255 ? nliq : 255);
+        }
     }
-    return v;
 }
 
 // (A x)_c of cg_spmv.wgsl:46-68 / cg_init.wgsl:24-48, neighbour order -x,+x,-y,+y,-z,+z.
@@ -335,26 +368,31 @@ __global__ void __launch_bounds__(256) k_grid_prep(DevBufs b, uint32_t C) {
     float prod = 0.0f;
     Df pdf = {0.0f, 0.0f};
     if (c < C) {
-        // Every load a cell needs is issued before its results are used: the
+        // What bounds it is latency and branches, with 64 registers and half the warps:
+        // no branch around a load of the first round (128^3: 47 -> 37 us, 256^3:
+        // 365 -> 268; 48 or 40 registers, or blocks that stay for several chunks, are
+        // slower).  Every load a cell needs is issued before its results are used: the
         // lower faces' sums and cell types first, then (liquid cells) the
         // upper faces', the neighbours' types and pressures; all stores come
         // after.  The arithmetic is face_value's and apply_A's, in their order.
         const uint32_t nx = P.nx, ny = P.ny, nz = P.nz;
-        const uint32_t i = c % nx, j = (c / nx) % ny, k = c / (nx * ny);
-        const size_t nxy = (size_t)nx * ny;
-        const size_t i0 = (size_t)i + (size_t)(nx + 1) * ((size_t)j + (size_t)ny * k);  // u face (i, j, k)
-        const size_t i1 = (size_t)i + (size_t)nx * ((size_t)j + (size_t)(ny + 1) * k);  // v face (i, j, k)
-        const size_t i2 = c;                                                            // w face (i, j, k)
+        uint32_t i, j, k;
+        cell_coords(P, c, i, j, k);
+        // face indices: below 2^31 for grids of up to 2^30 cells
+        const uint32_t nxy = nx * ny;
+        const uint32_t i0 = c + j + ny * k;  // u face (i, j, k) of (nx + 1) per row
+        const uint32_t i1 = c + nx * k;      // v face (i, j, k) of ny + 1 rows per plane
+        const uint32_t i2 = c;                                                            // w face (i, j, k)
         const int32_t d0 = b.den[0][i0], n0 = b.num[0][i0], d1 = b.den[1][i1], n1 = b.num[1][i1];
         const int32_t d2 = b.den[2][i2], n2 = b.num[2][i2];
         const uint8_t tc = b.ct[c];
-        const uint8_t tmx = i > 0 ? b.ct[c - 1] : CELL_SOLID, tmy = j > 0 ? b.ct[c - nx] : CELL_SOLID,
-                      tmz = k > 0 ? b.ct[c - nxy] : CELL_SOLID;
+        // (a cell without a neighbour below reads its own type instead)
+        uint8_t tmx = b.ct[i > 0 ? c - 1 : c], tmy = b.ct[j > 0 ? c - nx : c], tmz = b.ct[k > 0 ? c - nxy : c];
+        if (i == 0) tmx = CELL_SOLID;
+        if (j == 0) tmy = CELL_SOLID;
+        if (k == 0) tmz = CELL_SOLID;
         // the grid's far faces, written by the last cell of each line
         const bool eu = i == nx - 1, ev = j == ny - 1, ew = k == nz - 1;
-        const int32_t ed0 = eu ? b.den[0][i0 + 1] : 0, en0 = eu ? b.num[0][i0 + 1] : 0;
-        const int32_t ed1 = ev ? b.den[1][i1 + nx] : 0, en1 = ev ? b.num[1][i1 + nx] : 0;
-        const int32_t ed2 = ew ? b.den[2][i2 + nxy] : 0, en2 = ew ? b.num[2][i2 + nxy] : 0;
         float su, sv, sw;
         const float ul = face_value(P, 0, d0, n0, i, nx, tmx, tc, &su);
         const float vl = face_value(P, 1, d1, n1, j, ny, tmy, tc, &sv);
@@ -368,7 +406,7 @@ __global__ void __launch_bounds__(256) k_grid_prep(DevBufs b, uint32_t C) {
             const bool drift_on = P.stiff > 0.0f && P.rest > 0.0f;
             const uint32_t occ = drift_on ? b.counts[c] : 0u;
             const bool warm = P.warm != 0u;
-            const size_t nb6[6] = {c - 1, c + 1, c - nx, c + nx, c - nxy, c + nxy};
+            const uint32_t nb6[6] = {c - 1, c + 1, c - nx, c + nx, c - nxy, c + nxy};
             float pn[6];
 #pragma unroll
             for (int s2 = 0; s2 < 6; s2++) pn[s2] = warm ? b.p[nb6[s2]] : 0.0f;
@@ -426,53 +464,42 @@ __global__ void __launch_bounds__(256) k_grid_prep(DevBufs b, uint32_t C) {
         b.sav[2][i2] = sw;
         float se;
         if (eu) {
-            b.vel[0][i0 + 1] = face_value(P, 0, ed0, en0, nx, nx, tc, CELL_SOLID, &se);
+            b.vel[0][i0 + 1] = face_value(P, 0, b.den[0][i0 + 1], b.num[0][i0 + 1], nx, nx, tc, CELL_SOLID, &se);
             b.sav[0][i0 + 1] = se;
         }
         if (ev) {
-            b.vel[1][i1 + nx] = face_value(P, 1, ed1, en1, ny, ny, tc, CELL_SOLID, &se);
+            b.vel[1][i1 + nx] = face_value(P, 1, b.den[1][i1 + nx], b.num[1][i1 + nx], ny, ny, tc, CELL_SOLID, &se);
             b.sav[1][i1 + nx] = se;
         }
         if (ew) {
-            b.vel[2][i2 + nxy] = face_value(P, 2, ed2, en2, nz, nz, tc, CELL_SOLID, &se);
+            b.vel[2][i2 + nxy] = face_value(P, 2, b.den[2][i2 + nxy], b.num[2][i2 + nxy], nz, nz, tc, CELL_SOLID, &se);
             b.sav[2][i2 + nxy] = se;
         }
     }
-    const int nliq = __syncthreads_count(liquid);
-    const float v = block_tree256(prod, s_tree);
-    // float-float partial of this chunk (fixed order: warp shuffles, then warps in order)
-    pdf = warp_sum_df(pdf);
-    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = make_float2(pdf.hi, pdf.lo);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        Df a = {0.0f, 0.0f};
-        for (int w = 0; w < 8; w++) a = df_add(a, Df{s_red[w].x, s_red[w].y});
-        b.part_rr[chunk] = v;
-        b.chunk_rr_df[chunk] = make_float2(a.hi, a.lo);
-        b.chunk_flag[chunk] = (uint8_t)(nliq < 255 ? nliq : 255);
-    }
+    chunk_partials(b, chunk, liquid, prod, pdf, s_tree, s_red);
 }
 
 // gradient.wgsl:23-67 on the cell's three lower faces: an interior face
 // with no solid side and a liquid side gets vel -= coeff * (p_hi - p_lo).
 // The cell types, pressures and face values are loaded before any face is
 // written (the kernel is latency-bound, and a face's store would otherwise
-// hold back the next face's loads).
+// hold back the next face's loads).  256^3: 65 us (78 with divisions for the
+// coordinates); four cells per thread take 75.
 __global__ void __launch_bounds__(256) k_project(DevBufs b, uint32_t C) {
     const DevParams& P = *b.prm;
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
     const uint32_t nx = P.nx, ny = P.ny;
-    const uint32_t i = c % nx, j = (c / nx) % ny, k = c / (nx * ny);
-    const size_t nxy = (size_t)nx * ny;
-    const size_t lo[3] = {c - 1, c - nx, c - nxy};
-    const size_t idx[3] = {(size_t)i + (size_t)(nx + 1) * ((size_t)j + (size_t)ny * k),
-                           (size_t)i + (size_t)nx * ((size_t)j + (size_t)(ny + 1) * k), (size_t)c};
+    uint32_t i, j, k;
+    cell_coords(P, c, i, j, k);
     const bool inner[3] = {i > 0, j > 0, k > 0};  // comp == nax never holds for a lower face (comp < n)
+    // the cell below (its own where there is none: no branch around a load)
+    const uint32_t lo[3] = {inner[0] ? c - 1 : c, inner[1] ? c - nx : c, inner[2] ? c - nx * ny : c};
+    const uint32_t idx[3] = {c + j + ny * k, c + nx * k, c};
     const uint8_t ht = b.ct[c];
     uint8_t lt[3];
 #pragma unroll
-    for (int a = 0; a < 3; a++) lt[a] = inner[a] ? b.ct[lo[a]] : CELL_SOLID;
+    for (int a = 0; a < 3; a++) lt[a] = b.ct[lo[a]];
     bool on[3];
 #pragma unroll
     for (int a = 0; a < 3; a++)  // gradient.wgsl:45-60
@@ -526,19 +553,7 @@ __global__ void __launch_bounds__(256) k_solve_init(DevBufs b, uint32_t C, const
             b.cinfo[c] = 0;
         }
     }
-    const int nliq = __syncthreads_count(liquid);
-    const float v = block_tree256(prod, s_tree);
-    // float-float partial of this chunk (fixed order: warp shuffles, then warps in order)
-    pdf = warp_sum_df(pdf);
-    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = make_float2(pdf.hi, pdf.lo);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        Df a = {0.0f, 0.0f};
-        for (int w = 0; w < 8; w++) a = df_add(a, Df{s_red[w].x, s_red[w].y});
-        b.part_rr[chunk] = v;
-        b.chunk_rr_df[chunk] = make_float2(a.hi, a.lo);
-        b.chunk_flag[chunk] = (uint8_t)(nliq < 255 ? nliq : 255);
-    }
+    chunk_partials(b, chunk, liquid, prod, pdf, s_tree, s_red);
 }
 
 cudaError_t launch_solve_init(const DevBufs& b, uint32_t C, const float* div, cudaStream_t s) {
@@ -547,7 +562,7 @@ cudaError_t launch_solve_init(const DevBufs& b, uint32_t C, const float* div, cu
 }
 
 cudaError_t launch_classify(const DevBufs& b, uint32_t C, cudaStream_t s) {
-    k_classify<<<(C + 255) / 256, 256, 0, s>>>(b, C);
+    k_classify<<<(C + 256 * CLASSIFY_CELLS - 1) / (256 * CLASSIFY_CELLS), 256, 0, s>>>(b, C);
     return cudaGetLastError();
 }
 

@@ -113,6 +113,14 @@ fl_status validate(const fl_params* p, std::string* why) {
     return FL_OK;
 }
 
+// Multiplier and shift of a division by d >= 2 (see cell_coords).
+void division_by(uint32_t d, uint32_t& mul, uint32_t& shift) {
+    uint32_t L = 1;
+    while ((1ull << L) < d) L++;
+    mul = (uint32_t)(((1ull << (31 + L)) + d - 1) / d);
+    shift = L - 1;
+}
+
 // Derived settings, in the shaders' f32 operation order.
 void derive(const fl_params& p, uint32_t n, DevParams& d) {
     d = DevParams{};
@@ -148,6 +156,8 @@ void derive(const fl_params& p, uint32_t n, DevParams& d) {
     d.advect_order = p.advect_order == 2u ? 2u : 1u;
     d.nchunks = (d.C + fl::CHUNK - 1) / fl::CHUNK;
     d.solver = p.pressure_solver;
+    division_by(d.nx, d.nx_mul, d.nx_shift);
+    division_by(d.ny, d.ny_mul, d.ny_shift);
 }
 
 struct PoolPlan {

@@ -251,6 +251,7 @@ __device__ __forceinline__ void clamp_bwd(const Clamp& c, const float v[3], cons
 // the band's min and which axis of the band's max are taken, which components
 // are pinned to the walls.
 __global__ void __launch_bounds__(256) k_adj_g2p(AdjBufs a) {
+    after_previous();
     const DevParams& P = *a.prm;
     const uint32_t n = P.n;
     const float alpha = P.flip, dt = P.dt, maxs = P.maxs, inv_h = P.inv_h, friction = P.friction;
@@ -401,6 +402,7 @@ __device__ __forceinline__ bool grad_face(uint8_t lt, uint8_t ht) {
 // One block per 256-cell chunk; with rhs_part set it also writes the chunk's
 // float-float sum of rhs^2 (fixed order: warp shuffles, then warps in order).
 __global__ void __launch_bounds__(256) k_adj_prhs(AdjBufs a) {
+    after_previous();
     __shared__ float2 s_red[8];
     const DevParams& P = *a.prm;
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -442,8 +444,9 @@ __global__ void __launch_bounds__(256) k_adj_prhs(AdjBufs a) {
 // the squared norm of its right-hand side, the value the cold-start test
 // tol^2 * (r0.r0) uses (r0 = rhs when the solve starts from zero).  One block;
 // the chunk partials are summed in a fixed order.
-__global__ void __launch_bounds__(1024) k_adj_thr(const float2* __restrict__ part, uint32_t nchunks, double tol_sq,
-                                                  DevParams* __restrict__ cg_prm) {
+__global__ void __launch_bounds__(1024) k_adj_thr(const float2* part, uint32_t nchunks, double tol_sq,
+                                                  DevParams* cg_prm) {
+    after_previous();
     __shared__ float2 s_red[32];
     Df t = {0.0f, 0.0f};
     for (uint32_t i = threadIdx.x; i < nchunks; i += blockDim.x) t = df_add(t, Df{part[i].x, part[i].y});
@@ -467,6 +470,7 @@ __global__ void __launch_bounds__(1024) k_adj_thr(const float2* __restrict__ par
 // operations per clock and SM, and summing zeros there was four fifths of the
 // 39 us that each axis took at 128^3.
 __global__ void __launch_bounds__(256) k_adj_faces(AdjBufs a) {
+    after_previous();
     __shared__ double s_red[8];
     const DevParams& P = *a.prm;
     const int axis = (int)blockIdx.y;
@@ -524,6 +528,7 @@ __global__ void __launch_bounds__(256) k_adj_faces(AdjBufs a) {
 // dL/dgravity: per axis (one block each) the k_adj_faces partials, thread t
 // summing partials t, t + 1024, ... in sequence, then a fixed tree.
 __global__ void __launch_bounds__(1024) k_adj_grav(AdjBufs a, uint32_t nb0, uint32_t nb1, uint32_t nb2) {
+    after_previous();
     __shared__ double s_red[32];
     const uint32_t axis = blockIdx.x, nb = axis == 0 ? nb0 : (axis == 1 ? nb1 : nb2);
     const double* part = a.grav_part[axis];
@@ -558,6 +563,7 @@ __device__ __forceinline__ int mid_exponent(const AdjBufs& a) {
 // its midpoint Xm, w * (gfin/W at Xm), added as 64-bit fixed-point integers
 // (integer sums do not depend on the order of the atomics).
 __global__ void __launch_bounds__(256) k_adj_mid(AdjBufs a) {
+    after_previous();
     const DevParams& P = *a.prm;
     const uint32_t n = P.n;
     if (a.flags[1] == 0u) return;
@@ -734,6 +740,7 @@ __device__ __forceinline__ void gather_bins(const AdjBufs& a, const DevParams& P
 
 template <int NZ>
 __global__ void __launch_bounds__(256) k_adj_gather(AdjBufs a, int midpoint) {
+    after_previous();
     const DevParams& P = *a.prm;
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const int nx = (int)P.nx, ny = (int)P.ny, nz = (int)P.nz;
@@ -777,6 +784,7 @@ __global__ void __launch_bounds__(256) k_adj_gather(AdjBufs a, int midpoint) {
 // unquantised sums; then back to the step's input order (sort_scatter.wgsl
 // transposed).
 __global__ void __launch_bounds__(256) k_adj_p2g(AdjBufs a) {
+    after_previous();
     const DevParams& P = *a.prm;
     const uint32_t n = P.n;
     const float inv_h = P.inv_h;
@@ -805,35 +813,35 @@ __global__ void __launch_bounds__(256) k_adj_p2g(AdjBufs a) {
 }
 
 cudaError_t launch_adj_g2p(const AdjBufs& a, const LaunchCfg& L, cudaStream_t s) {
-    k_adj_g2p<<<L.particle_blocks, 256, 0, s>>>(a);
+    launch_after(k_adj_g2p, dim3(L.particle_blocks), 256, s, a);
     return cudaGetLastError();
 }
 cudaError_t launch_adj_prhs(const AdjBufs& a, uint32_t C, cudaStream_t s) {
-    k_adj_prhs<<<(C + 255) / 256, 256, 0, s>>>(a);
+    launch_after(k_adj_prhs, dim3((C + 255) / 256), 256, s, a);
     return cudaGetLastError();
 }
 cudaError_t launch_adj_thr(const AdjBufs& a, uint32_t nchunks, double tol_sq, DevParams* cg_prm, cudaStream_t s) {
-    k_adj_thr<<<1, 1024, 0, s>>>(a.rhs_part, nchunks, tol_sq, cg_prm);
+    launch_after(k_adj_thr, dim3(1), 1024, s, a.rhs_part, nchunks, tol_sq, cg_prm);
     return cudaGetLastError();
 }
 cudaError_t launch_adj_faces(const AdjBufs& a, const uint32_t F3[3], cudaStream_t s) {
     const uint32_t most = F3[0] > F3[1] ? (F3[0] > F3[2] ? F3[0] : F3[2]) : (F3[1] > F3[2] ? F3[1] : F3[2]);
-    k_adj_faces<<<dim3((most + 255) / 256, 3), 256, 0, s>>>(a);
-    k_adj_grav<<<3, 1024, 0, s>>>(a, (F3[0] + 255) / 256, (F3[1] + 255) / 256, (F3[2] + 255) / 256);
+    launch_after(k_adj_faces, dim3((most + 255) / 256, 3), 256, s, a);
+    launch_after(k_adj_grav, dim3(3), 1024, s, a, (F3[0] + 255) / 256, (F3[1] + 255) / 256, (F3[2] + 255) / 256);
     return cudaGetLastError();
 }
 cudaError_t launch_adj_mid(const AdjBufs& a, const LaunchCfg& L, cudaStream_t s) {
-    k_adj_mid<<<L.particle_blocks, 256, 0, s>>>(a);
+    launch_after(k_adj_mid, dim3(L.particle_blocks), 256, s, a);
     return cudaGetLastError();
 }
 cudaError_t launch_adj_gather(const AdjBufs& a, uint32_t nx, uint32_t ny, uint32_t nz, bool midpoint, cudaStream_t s) {
     constexpr int NZ = 2;
     const uint32_t threads = nx * ny * ((nz + NZ - 1) / NZ);
-    k_adj_gather<NZ><<<(threads + 255) / 256, 256, 0, s>>>(a, midpoint ? 1 : 0);
+    launch_after(k_adj_gather<NZ>, dim3((threads + 255) / 256), 256, s, a, midpoint ? 1 : 0);
     return cudaGetLastError();
 }
 cudaError_t launch_adj_p2g(const AdjBufs& a, const LaunchCfg& L, cudaStream_t s) {
-    k_adj_p2g<<<L.particle_blocks, 256, 0, s>>>(a);
+    launch_after(k_adj_p2g, dim3(L.particle_blocks), 256, s, a);
     return cudaGetLastError();
 }
 }  // namespace fl

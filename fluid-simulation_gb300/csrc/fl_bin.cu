@@ -19,6 +19,7 @@ namespace fl {
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
 
 __global__ void __launch_bounds__(256) k_bin_count(DevBufs b) {
+    after_previous();
     const DevParams P = *b.prm;
     const uint32_t n = P.n;
     const uint32_t lane = lane_id();
@@ -79,8 +80,8 @@ __device__ __forceinline__ uint4 scan_counts(const uint32_t* counts, uint64_t ba
     return make_uint4(base < C ? counts[base] : 0u, base + 1 < C ? counts[base + 1] : 0u, base + 2 < C ? counts[base + 2] : 0u, 0u);
 }
 
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_reduce(const uint32_t* __restrict__ counts, uint32_t C,
-                                                             uint32_t* __restrict__ spine) {
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_reduce(const uint32_t* counts, uint32_t C, uint32_t* spine) {
+    after_previous();
     __shared__ uint32_t s_warp[32];
     const uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE + (uint64_t)threadIdx.x * SCAN_ITEMS;
     const uint4 n = scan_counts(counts, base, C);
@@ -98,7 +99,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_reduce(const uint32_t* __
 }
 
 // One block scans the spine of per-tile totals in place (exclusive).
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_spine(uint32_t* __restrict__ spine, uint32_t nb) {
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_spine(uint32_t* spine, uint32_t nb) {
+    after_previous();
     __shared__ uint32_t s_warp[32];
     __shared__ uint32_t s_total;
     uint32_t carry = 0;
@@ -113,10 +115,9 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_spine(uint32_t* __restric
     }
 }
 
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_down(const uint32_t* __restrict__ counts, uint32_t C,
-                                                           const uint32_t* __restrict__ spine,
-                                                           uint32_t* __restrict__ offsets,
-                                                           uint32_t* __restrict__ cursor) {
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_down(const uint32_t* counts, uint32_t C, const uint32_t* spine,
+                                                           uint32_t* offsets, uint32_t* cursor) {
+    after_previous();
     __shared__ uint32_t s_warp[32];
     __shared__ uint32_t s_total;
     const uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE + (uint64_t)threadIdx.x * SCAN_ITEMS;
@@ -138,6 +139,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_down(const uint32_t* __re
 }
 
 __global__ void __launch_bounds__(256) k_bin_scatter(DevBufs b) {
+    after_previous();
     const uint32_t n = b.prm->n;
     const uint32_t lane = lane_id();
     const uint32_t stride = gridDim.x * blockDim.x;
@@ -186,6 +188,7 @@ __device__ __forceinline__ void sort16(uint32_t (&a)[16]) {
 // Sort small buckets (the networks above up to 16 keys, an insertion sort up
 // to 32); queue large ones for k_bin_fix_big.
 __global__ void __launch_bounds__(256) k_bin_fix(DevBufs b, uint32_t C) {
+    after_previous();
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
     const uint32_t n = b.counts[c];
@@ -225,6 +228,7 @@ __global__ void __launch_bounds__(256) k_bin_fix(DevBufs b, uint32_t C) {
 // BIG_BUCKET_SMEM entries, else a rank pass through global memory (a bucket that
 // large is > 500x the rest density; correct, quadratic in the bucket size).
 __global__ void __launch_bounds__(1024) k_bin_fix_big(DevBufs b) {
+    after_previous();
     __shared__ uint32_t s[BIG_BUCKET_SMEM];
     const uint32_t nbig = b.st->big_buckets;
     for (uint32_t bi = blockIdx.x; bi < nbig; bi += gridDim.x) {
@@ -269,6 +273,7 @@ __global__ void __launch_bounds__(1024) k_bin_fix_big(DevBufs b) {
 }
 
 __global__ void __launch_bounds__(256) k_bin_gather(DevBufs b) {
+    after_previous();
     const DevParams P = *b.prm;
     const uint32_t n = P.n;
     const uint32_t stride = gridDim.x * blockDim.x;
@@ -293,14 +298,14 @@ __global__ void __launch_bounds__(256) k_bin_gather(DevBufs b) {
 cudaError_t launch_bin(const DevBufs& b, const LaunchCfg& L, uint32_t C, uint32_t cap, cudaStream_t s) {
     (void)cap;
     const uint32_t nb = (C + SCAN_TILE - 1) / SCAN_TILE;
-    k_bin_count<<<L.particle_blocks, 256, 0, s>>>(b);
-    k_scan_reduce<<<nb, SCAN_THREADS, 0, s>>>(b.counts, C, b.spine);
-    k_scan_spine<<<1, SCAN_THREADS, 0, s>>>(b.spine, nb);
-    k_scan_down<<<nb, SCAN_THREADS, 0, s>>>(b.counts, C, b.spine, b.offsets, b.cursor);
-    k_bin_scatter<<<L.particle_blocks, 256, 0, s>>>(b);
-    k_bin_fix<<<(C + 255) / 256, 256, 0, s>>>(b, C);
-    k_bin_fix_big<<<L.num_sms, 1024, 0, s>>>(b);
-    k_bin_gather<<<L.particle_blocks, 256, 0, s>>>(b);
+    launch_after(k_bin_count, dim3(L.particle_blocks), 256, s, b);
+    launch_after(k_scan_reduce, dim3(nb), SCAN_THREADS, s, b.counts, C, b.spine);
+    launch_after(k_scan_spine, dim3(1), SCAN_THREADS, s, b.spine, nb);
+    launch_after(k_scan_down, dim3(nb), SCAN_THREADS, s, b.counts, C, b.spine, b.offsets, b.cursor);
+    launch_after(k_bin_scatter, dim3(L.particle_blocks), 256, s, b);
+    launch_after(k_bin_fix, dim3((C + 255) / 256), 256, s, b, C);
+    launch_after(k_bin_fix_big, dim3(L.num_sms), 1024, s, b);
+    launch_after(k_bin_gather, dim3(L.particle_blocks), 256, s, b);
     return cudaGetLastError();
 }
 

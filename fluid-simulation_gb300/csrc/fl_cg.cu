@@ -360,6 +360,7 @@ __device__ __forceinline__ uint32_t seg_line(uint32_t nact) { return ((CHUNK + n
 // are enough blocks.  For split segments the order did not pay: a block's partials
 // then belong to many segments (256^3: 5,183 -> 5,238 us).
 __global__ void __launch_bounds__(CHUNK) k_cg_plan(DevBufs b, uint32_t G, int form) {
+    after_previous();
     const bool ranges_only = form == PLAN_RANGES;
     const uint32_t per_chunk = ranges_only ? CELL_CHUNK_WEIGHT : CHUNK_WEIGHT;
     __shared__ uint32_t s_wc[CHUNK / 32], s_ww[CHUNK / 32], s_wa[CHUNK / 32], s_wh[CHUNK / 32];
@@ -1468,14 +1469,14 @@ int cg_max_blocks_per_sm() {
 
 cudaError_t launch_cg_plan(const DevBufs& b, uint32_t G, cudaStream_t s) {
     if (G < 1 || G > MAX_CG_BLOCKS) return cudaErrorInvalidValue;
-    k_cg_plan<<<1, CHUNK, 0, s>>>(b, G, PLAN_RANGES);
+    launch_after(k_cg_plan, dim3(1), CHUNK, s, b, G, PLAN_RANGES);
     return cudaGetLastError();
 }
 
 cudaError_t launch_cg(const DevBufs& b, const LaunchCfg& L, cudaStream_t s, uint32_t precision, uint32_t nx) {
     if (precision > FL_CG_F64_IEEE) return cudaErrorInvalidValue;
     if (L.cg_blocks < 1 || (uint32_t)L.cg_blocks > MAX_CG_BLOCKS) return cudaErrorInvalidValue;
-    k_cg_plan<<<1, CHUNK, 0, s>>>(b, (uint32_t)L.cg_blocks, precision == FL_CG_F32 ? PLAN_F32 : PLAN_EXTENDED);
+    launch_after(k_cg_plan, dim3(1), CHUNK, s, b, (uint32_t)L.cg_blocks, precision == FL_CG_F32 ? PLAN_F32 : PLAN_EXTENDED);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};

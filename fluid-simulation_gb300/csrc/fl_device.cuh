@@ -331,6 +331,32 @@ __device__ __forceinline__ float ld_if(const float* p, bool on) {
     return v;
 }
 
+// Programmatic dependent launch.  A kernel launched with launch_after may be set up
+// while the kernel before it in the stream still runs; every thread of it calls
+// after_previous() before it touches memory, which waits until that kernel has
+// finished and its writes are visible.  A substep is some sixteen kernels of a few
+// microseconds on a small grid; this takes the launch latency between them (four 32^3
+// substeps with their frame output: 1,000 -> 945 us; a 39 x 43 x 45 step in place,
+// 30 iterations: 277 -> 251 us).  Nothing may be read before the call: no const
+// __restrict__ arguments in such kernels (loads through them may move above it).
+__device__ __forceinline__ void after_previous() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+cudaError_t launch_after(void (*kernel)(P...), dim3 grid, uint32_t threads, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 #endif  // __CUDACC__
 }  // namespace fl
 

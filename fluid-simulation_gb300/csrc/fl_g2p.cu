@@ -109,6 +109,7 @@ __device__ __forceinline__ void speed_clamp(float& x, float& y, float& z, float 
 // registers let more loads be in flight than 40 or 80 (256^3, 18.3 M particles:
 // 605 us -> 539 us -> 529 us; 84 registers 674, 40 registers 580).
 __global__ void __launch_bounds__(256, 4) k_g2p(DevBufs b) {
+    after_previous();
     const DevParams& P = *b.prm;
     const uint32_t n = P.n;
     const float alpha = P.flip, dt = P.dt, maxs = P.maxs, friction = P.friction;
@@ -197,7 +198,7 @@ cudaError_t launch_iota(uint32_t* ids, uint32_t n, cudaStream_t s) {
 }
 
 cudaError_t launch_g2p(const DevBufs& b, const LaunchCfg& L, cudaStream_t s) {
-    k_g2p<<<L.particle_blocks, 256, 0, s>>>(b);
+    launch_after(k_g2p, dim3(L.particle_blocks), 256, s, b);
     return cudaGetLastError();
 }
 

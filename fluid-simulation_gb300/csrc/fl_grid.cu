@@ -23,12 +23,13 @@ namespace fl {
 constexpr int CLASSIFY_CELLS = 4;
 
 __global__ void __launch_bounds__(256) k_classify(DevBufs b, uint32_t C) {
+    after_previous();
     __shared__ uint32_t s_n;
     const DevParams& P = *b.prm;
     if (threadIdx.x == 0) s_n = 0;
     const uint32_t c0 = blockIdx.x * 256u * CLASSIFY_CELLS + threadIdx.x;
     const uint32_t nx = P.nx, ny = P.ny, nz = P.nz, th = P.thresh;
-    const uint32_t* __restrict__ occ = b.counts;
+    const uint32_t* occ = b.counts;
     uint32_t n[CLASSIFY_CELLS], liquids = 0;
 #pragma unroll
     for (int q = 0; q < CLASSIFY_CELLS; q++) n[q] = c0 + 256u * q < C ? occ[c0 + 256u * q] : 0u;
@@ -123,6 +124,7 @@ __device__ __forceinline__ void p2g_box(const DevParams& P, DevStats* st, const 
 
 template <int TZ>
 __global__ void __launch_bounds__(256) k_p2g_own(DevBufs b, int tiles_x, int tiles_y) {
+    after_previous();
     constexpr int PB_N = PB_Z * (TZ + 2);  // words of a box
     __shared__ __align__(16) int32_t s_num[3][PB_N];
     __shared__ __align__(16) int32_t s_den[3][PB_N];
@@ -226,6 +228,7 @@ __global__ void __launch_bounds__(256) k_p2g_own(DevBufs b, int tiles_x, int til
 }
 
 __global__ void __launch_bounds__(256) k_p2g_strays(DevBufs b) {
+    after_previous();
     const DevParams& P = *b.prm;
     const uint32_t ns = b.st->strays;
     const int n3[3] = {(int)P.nx, (int)P.ny, (int)P.nz};
@@ -359,6 +362,7 @@ __device__ __forceinline__ uint16_t stencil_info(const uint8_t* ct, size_t c, si
 }
 
 __global__ void __launch_bounds__(256) k_grid_prep(DevBufs b, uint32_t C) {
+    after_previous();
     __shared__ float s_tree[256];
     __shared__ float2 s_red[8];
     const DevParams& P = *b.prm;
@@ -486,6 +490,7 @@ __global__ void __launch_bounds__(256) k_grid_prep(DevBufs b, uint32_t C) {
 // hold back the next face's loads).  256^3: 65 us (78 with divisions for the
 // coordinates); four cells per thread take 75.
 __global__ void __launch_bounds__(256) k_project(DevBufs b, uint32_t C) {
+    after_previous();
     const DevParams& P = *b.prm;
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
@@ -519,7 +524,8 @@ __global__ void __launch_bounds__(256) k_project(DevBufs b, uint32_t C) {
 
 // Stand-alone solve: cg_init.wgsl:50-87 from a given divergence field (the
 // tail of k_grid_prep without the face passes).
-__global__ void __launch_bounds__(256) k_solve_init(DevBufs b, uint32_t C, const float* __restrict__ div) {
+__global__ void __launch_bounds__(256) k_solve_init(DevBufs b, uint32_t C, const float* div) {
+    after_previous();
     __shared__ float s_tree[256];
     __shared__ float2 s_red[8];
     const DevParams& P = *b.prm;
@@ -557,12 +563,12 @@ __global__ void __launch_bounds__(256) k_solve_init(DevBufs b, uint32_t C, const
 }
 
 cudaError_t launch_solve_init(const DevBufs& b, uint32_t C, const float* div, cudaStream_t s) {
-    k_solve_init<<<(C + 255) / 256, 256, 0, s>>>(b, C, div);
+    launch_after(k_solve_init, dim3((C + 255) / 256), 256, s, b, C, div);
     return cudaGetLastError();
 }
 
 cudaError_t launch_classify(const DevBufs& b, uint32_t C, cudaStream_t s) {
-    k_classify<<<(C + 256 * CLASSIFY_CELLS - 1) / (256 * CLASSIFY_CELLS), 256, 0, s>>>(b, C);
+    launch_after(k_classify, dim3((C + 256 * CLASSIFY_CELLS - 1) / (256 * CLASSIFY_CELLS)), 256, s, b, C);
     return cudaGetLastError();
 }
 
@@ -582,20 +588,20 @@ cudaError_t launch_p2g(const DevBufs& b, const LaunchCfg& L, uint32_t nx, uint32
     // A larger one fills the chip either way, and flat tiles add more rim sums to
     // the face arrays (128^3: 77 us with 8^3, 95 us with 8 x 8 x 2; 256^3: 530 and 735).
     if (tx * ty * ((nz + 7) / 8) < 8u * (uint32_t)L.num_sms)
-        k_p2g_own<2><<<tx * ty * ((nz + 1) / 2), 256, 0, s>>>(b, (int)tx, (int)ty);
+        launch_after(k_p2g_own<2>, dim3(tx * ty * ((nz + 1) / 2)), 256, s, b, (int)tx, (int)ty);
     else
-        k_p2g_own<8><<<tx * ty * ((nz + 7) / 8), 256, 0, s>>>(b, (int)tx, (int)ty);
-    k_p2g_strays<<<L.num_sms, 256, 0, s>>>(b);
+        launch_after(k_p2g_own<8>, dim3(tx * ty * ((nz + 7) / 8)), 256, s, b, (int)tx, (int)ty);
+    launch_after(k_p2g_strays, dim3(L.num_sms), 256, s, b);
     return cudaGetLastError();
 }
 
 cudaError_t launch_grid_prep(const DevBufs& b, uint32_t C, cudaStream_t s) {
-    k_grid_prep<<<(C + 255) / 256, 256, 0, s>>>(b, C);
+    launch_after(k_grid_prep, dim3((C + 255) / 256), 256, s, b, C);
     return cudaGetLastError();
 }
 
 cudaError_t launch_project(const DevBufs& b, uint32_t C, cudaStream_t s) {
-    k_project<<<(C + 255) / 256, 256, 0, s>>>(b, C);
+    launch_after(k_project, dim3((C + 255) / 256), 256, s, b, C);
     return cudaGetLastError();
 }
 

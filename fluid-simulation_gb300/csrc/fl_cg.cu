@@ -364,8 +364,8 @@ __global__ void __launch_bounds__(CHUNK) k_cg_plan(DevBufs b, uint32_t G, int fo
     const bool ranges_only = form == PLAN_RANGES;
     const uint32_t per_chunk = ranges_only ? CELL_CHUNK_WEIGHT : CHUNK_WEIGHT;
     __shared__ uint32_t s_wc[CHUNK / 32], s_ww[CHUNK / 32], s_wa[CHUNK / 32], s_wh[CHUNK / 32];
-    __shared__ uint32_t s_cnt[CHUNK];
-    __shared__ uint16_t s_blk[CHUNK][32];  // block of segment i's head under lane l's T
+    __shared__ __align__(16) uint32_t s_cnt[CHUNK];
+    __shared__ uint32_t s_blk[CHUNK / 2][32];  // blocks of the heads of segments 2i and 2i + 1 under lane l's T
     __shared__ uint16_t s_first[MAX_CG_BLOCKS];
     __shared__ uint32_t s_sel, s_T, s_nblk;
     __shared__ int s_wrap;
@@ -376,14 +376,24 @@ __global__ void __launch_bounds__(CHUNK) k_cg_plan(DevBufs b, uint32_t G, int fo
     uint32_t* start = hdr + H_START;
     uint32_t* segslot = start + G + 3;
     uint32_t* toffs = segslot + CHUNK;
-    uint32_t cnt = 0, wsum = 0;
-    for (uint32_t c = li; c < nchunks; c += CHUNK) {
-        const uint32_t f = b.chunk_flag[c];
-        if (f) {
-            cnt++;
-            wsum += f + per_chunk;
+    const uint32_t epoch = (uint32_t)b.cg_x[0], max_iters = P.iters;  // for the tags, below
+    // fn(chunk, liquid cells) for the active chunks of segment li, in order; sixteen
+    // loads at a time (one after the other: 19 us more per plan at 256^3).
+    auto segment = [&](auto&& fn) {
+        for (uint32_t c0 = li; c0 < nchunks; c0 += 16 * CHUNK) {
+            uint8_t f[16];
+#pragma unroll
+            for (uint32_t i = 0; i < 16; i++) f[i] = c0 + i * CHUNK < nchunks ? b.chunk_flag[c0 + i * CHUNK] : (uint8_t)0;
+#pragma unroll
+            for (uint32_t i = 0; i < 16; i++)
+                if (f[i]) fn(c0 + i * CHUNK, (uint32_t)f[i]);
         }
-    }
+    };
+    uint32_t cnt = 0, wsum = 0;
+    segment([&](uint32_t, uint32_t f) {
+        cnt++;
+        wsum += f + per_chunk;
+    });
     const uint32_t has = __ballot_sync(0xffffffffu, cnt != 0u);
     auto scan = [&](uint32_t v) {  // inclusive, within the warp
 #pragma unroll
@@ -413,17 +423,29 @@ __global__ void __launch_bounds__(CHUNK) k_cg_plan(DevBufs b, uint32_t G, int fo
     }
     if (form == PLAN_F32 && warp == 0) {
         const uint32_t T = lane ? CG_WARPS * lane : CG_WARPS / 2;
+        // A chain of an add, a compare and a select per segment: the counts are loaded
+        // sixteen at a time and the blocks stored in pairs (with a load, a branch and
+        // a store in every step it took 9 us, at any size).
         uint32_t blk = 0xffffffffu, cur = T, tails = 0;
-#pragma unroll 16
-        for (uint32_t i = 0; i < (uint32_t)CHUNK; i++) {
-            const uint32_t c = s_cnt[i], h = c < T ? c : T;
-            tails += c - h;
-            if (h && cur + h > T) {
-                blk++;
-                cur = 0;
+#pragma unroll 1
+        for (uint32_t i0 = 0; i0 < (uint32_t)CHUNK; i0 += 16) {
+            uint32_t c[16];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const uint4 v = reinterpret_cast<const uint4*>(s_cnt + i0)[i];
+                c[4 * i] = v.x; c[4 * i + 1] = v.y; c[4 * i + 2] = v.z; c[4 * i + 3] = v.w;
             }
-            cur += h;
-            s_blk[i][lane] = (uint16_t)blk;
+            uint32_t pair = 0;
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                const uint32_t h = c[i] < T ? c[i] : T, sum = cur + h;
+                const bool next = h != 0u && sum > T;
+                tails += c[i] - h;
+                cur = next ? h : sum;
+                blk += next ? 1u : 0u;
+                if (i & 1) s_blk[(i0 + i) / 2][lane] = pair | blk << 16;
+                else pair = blk & 0xffffu;
+            }
         }
         const uint32_t nb = blk + 1u + (tails + T - 1) / T;
         const uint32_t fits = __ballot_sync(0xffffffffu, nb <= G && tails <= (lane ? RAW_MAX : 0u) && T <= KCH);
@@ -465,18 +487,21 @@ __global__ void __launch_bounds__(CHUNK) k_cg_plan(DevBufs b, uint32_t G, int fo
     // weights [X, X1).  X only grows along a thread's entries, so the next such
     // block is tracked incrementally from one division.
     if (form == PLAN_F32) {  // in segment order
-        uint64_t XG = (uint64_t)(wbase + y - wsum) * Gs;  // Gs x the weight of all entries before this segment
-        uint64_t bb_next = W ? XG / W + 1 : 0, bbW = bb_next * W;
         uint32_t k = 0;
-        for (uint32_t c = li; c < nchunks; c += CHUNK) {
-            const uint32_t f = b.chunk_flag[c];
-            if (!f) continue;
-            b.cg_chunk[k < nh ? hoff + k : Ah + toff + (k - nh)] = c;
-            k++;
-            if (!T) {
+        if (T) {
+            segment([&](uint32_t c, uint32_t) {
+                b.cg_chunk[k < nh ? hoff + k : Ah + toff + (k - nh)] = c;
+                k++;
+            });
+        } else {
+            uint64_t XG = (uint64_t)(wbase + y - wsum) * Gs;  // Gs x the weight of all entries before this segment
+            uint64_t bb_next = W ? XG / W + 1 : 0, bbW = bb_next * W;
+            segment([&](uint32_t c, uint32_t f) {
+                b.cg_chunk[hoff + k] = c;
+                k++;
                 XG += (uint64_t)(f + per_chunk) * Gs;
                 for (; bbW <= XG; bb_next++, bbW += W) start[bb_next] = hoff + k;
-            }
+            });
         }
     } else {  // in tile order
         // Z chunks per plane (whole ones: the tiles shear a little where a plane is no
@@ -538,8 +563,9 @@ __global__ void __launch_bounds__(CHUNK) k_cg_plan(DevBufs b, uint32_t G, int fo
     // split segments: block li % nact adds segment li
     uint32_t slot = seg_line(nact) * (li % nact) + li / nact;
     if (T && A) {  // each block's words start on a 128-byte line
-        const uint32_t blk = s_blk[li][s_sel];
-        if (cnt && (li == 0 || s_blk[li - 1][s_sel] != blk)) {
+        auto block_of = [&](uint32_t i) { return s_blk[i / 2][s_sel] >> (16u * (i & 1u)) & 0xffffu; };
+        const uint32_t blk = block_of(li);
+        if (cnt && (li == 0 || block_of(li - 1) != blk)) {
             s_first[blk] = (uint16_t)act;
             start[blk] = hoff;
         }
@@ -564,8 +590,8 @@ __global__ void __launch_bounds__(CHUNK) k_cg_plan(DevBufs b, uint32_t G, int fo
             start[G + 1] = nact;
             start[G + 2] = nheads;
         }
-        const uint32_t span = 2u * (P.iters < TAG_SPAN_MAX ? P.iters : TAG_SPAN_MAX) + 4u;
-        uint32_t e0 = (uint32_t)b.cg_x[0];
+        const uint32_t span = 2u * (max_iters < TAG_SPAN_MAX ? max_iters : TAG_SPAN_MAX) + 4u;
+        uint32_t e0 = epoch;
         int wrap = 0;
         if (e0 > 0xffffffffu - span) {
             wrap = 1;

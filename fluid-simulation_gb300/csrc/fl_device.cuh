@@ -336,7 +336,7 @@ __device__ __forceinline__ float ld_if(const float* p, bool on) {
 // after_previous() before it touches memory, which waits until that kernel has
 // finished and its writes are visible.  A substep is some sixteen kernels of a few
 // microseconds on a small grid; this takes the launch latency between them (four 32^3
-// substeps with their frame output: 1,000 -> 945 us; a 39 x 43 x 45 step in place,
+// substeps with their frame output: 1,000 -> 945 us; a 97 x 61 x 83 step in place,
 // 30 iterations: 277 -> 251 us).  Nothing may be read before the call: no const
 // __restrict__ arguments in such kernels (loads through them may move above it).
 __device__ __forceinline__ void after_previous() {

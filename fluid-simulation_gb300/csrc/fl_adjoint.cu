@@ -713,23 +713,23 @@ __device__ __forceinline__ void gather_bins(const AdjBufs& a, const DevParams& P
                         if (ox <= 0) {
                             const float w = u * cz;
                             o[z].W[0] += w;
-                            o[z].WV[0] = fmaf(w, r0.w, o[z].WV[0]);
-                            o[z].gf[0] = fmaf(w, r1.z, o[z].gf[0]);
-                            o[z].gs[0] = fmaf(w, r2.y, o[z].gs[0]);
+                            o[z].WV[0] += w * r0.w;
+                            o[z].gf[0] += w * r1.z;
+                            o[z].gs[0] += w * r2.y;
                         }
                         if (oy <= 0) {
                             const float w = v * cz;
                             o[z].W[1] += w;
-                            o[z].WV[1] = fmaf(w, r1.x, o[z].WV[1]);
-                            o[z].gf[1] = fmaf(w, r1.w, o[z].gf[1]);
-                            o[z].gs[1] = fmaf(w, r2.z, o[z].gs[1]);
+                            o[z].WV[1] += w * r1.x;
+                            o[z].gf[1] += w * r1.w;
+                            o[z].gs[1] += w * r2.z;
                         }
                         if (oz <= 0) {
                             const float w = x * tap_along(oz, fz);
                             o[z].W[2] += w;
-                            o[z].WV[2] = fmaf(w, r1.y, o[z].WV[2]);
-                            o[z].gf[2] = fmaf(w, r2.x, o[z].gf[2]);
-                            o[z].gs[2] = fmaf(w, r2.w, o[z].gs[2]);
+                            o[z].WV[2] += w * r1.y;
+                            o[z].gf[2] += w * r2.x;
+                            o[z].gs[2] += w * r2.w;
                         }
                     }
                 }

@@ -299,7 +299,7 @@ __device__ __forceinline__ float face_value(const DevParams& P, int axis, int32_
 // block (s: 256 floats, s2: 8): the tree of cg_reduce.wgsl:38-49, whose steps 128,
 // 64 and 32 are formed by warp 0 from shared memory (with the same pairs: i with
 // i + 128, then + 64, then + 32) and whose other steps are shuffles; the
-// float-float sum in a fixed order (warp shuffles, then the warps in order); the
+// float-float sum in a fixed order (warp shuffles, then the warps likewise); the
 // number of liquid cells.  A chunk without liquid is done without either.
 __device__ __forceinline__ void chunk_partials(const DevBufs& b, uint32_t chunk, bool liquid, float prod, Df pdf, float* s,
                                                float2* s2) {
@@ -323,9 +323,9 @@ __device__ __forceinline__ void chunk_partials(const DevBufs& b, uint32_t chunk,
         float v = __fadd_rn(a, c);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v = __fadd_rn(v, __shfl_down_sync(0xffffffffu, v, o));
+        Df d = t < 8 ? Df{s2[t].x, s2[t].y} : Df{0.0f, 0.0f};
+        d = warp_sum_df<8>(d);
         if (t == 0) {
-            Df d = {0.0f, 0.0f};
-            for (int w = 0; w < 8; w++) d = df_add(d, Df{s2[w].x, s2[w].y});
             b.part_rr[chunk] = v;
             b.chunk_rr_df[chunk] = make_float2(d.hi, d.lo);
             b.chunk_flag[chunk] = (uint8_t)(nliq < 255 ? nliq : 255);

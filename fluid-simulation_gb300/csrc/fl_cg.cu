@@ -286,6 +286,37 @@ __device__ __forceinline__ float tree256_quads(Quad a, Quad b, Quad one, uint32_
     return __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 8));
 }
 
+// Two chunks' trees in one, from their level-128 sums (the products' halves added):
+// once a lane holds one component (VEC) or one slot, partner lanes swap, so that half of
+// the lanes carry each chunk through the remaining shuffles: 11 instead of 16 (6 instead
+// of 10), and one latency for both.  Lane 0 ends with the first chunk's sum, lane
+// PAIR_LANE with the second's; the pairs that are added are those of the tree above.
+template <bool VEC>
+constexpr uint32_t PAIR_LANE = VEC ? 4u : 16u;
+template <bool VEC>
+__device__ __forceinline__ float tree256_pair(Quad s, Quad t, uint32_t lane) {
+    const bool h4 = (lane & 16u) != 0u, h3 = (lane & 8u) != 0u, h2 = (lane & 4u) != 0u;
+    auto first = [&](Quad q) {
+        const float x = lo2(q.a), y = hi2(q.a), z = lo2(q.b), w = hi2(q.b);
+        if (!VEC) return __fadd_rn(__fadd_rn(x, z), __fadd_rn(y, w));
+        const float u0 = __fadd_rn(h4 ? z : x, __shfl_xor_sync(0xffffffffu, h4 ? x : z, 16));
+        const float u1 = __fadd_rn(h4 ? w : y, __shfl_xor_sync(0xffffffffu, h4 ? y : w, 16));
+        return __fadd_rn(h3 ? u1 : u0, __shfl_xor_sync(0xffffffffu, h3 ? u0 : u1, 8));
+    };
+    const float a = first(s), b = first(t);
+    if (!VEC) {
+        float v = __fadd_rn(h4 ? b : a, __shfl_xor_sync(0xffffffffu, h4 ? a : b, 16));
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, o));
+        return v;
+    }
+    float v = __fadd_rn(h2 ? b : a, __shfl_xor_sync(0xffffffffu, h2 ? a : b, 4));
+    v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 2));
+    v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 1));
+    v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 16));
+    return __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 8));
+}
+
 // Per-thread inner-product accumulator of the extended-precision forms:
 // float-float (FL_CG_F64: exact products by two-product, sums by two-sum on
 // the FP32 pipe) or IEEE double (FL_CG_F64_IEEE: f32 x f32 products are
@@ -1335,10 +1366,34 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
             const float* d_src = (it & 1u) || it == 0 ? b.dA : b.dB;
             const Quad beta4 = qall(beta);
             auto dir = [&](Quad dv, Quad rv) { return qaddp(qmul(beta4, dv), one, rv); };  // cg_dir.wgsl:30
+            // The warp's chunks of [jb, je), two at a time for their trees (256^3: 5,148 ->
+            // 5,066 us; the extended forms have none, and the loop in the loop cost them
+            // 1.5 %).
+            auto chunks = [&](uint32_t jb, uint32_t je, auto&& phase) {
+                if constexpr (f64) {
+#pragma unroll 1
+                    for (uint32_t j = jb + warp; j < je; j += CG_WARPS) phase(j);
+                } else {
+#pragma unroll 1
+                    for (uint32_t j = jb + warp; j < je; j += 2u * CG_WARPS) {
+                        Quad s0 = z4, s1 = z4;
+#pragma unroll 1
+                        for (uint32_t k = j; k < je && k <= j + CG_WARPS; k += CG_WARPS) {
+                            s0 = s1;
+                            s1 = phase(k);
+                        }
+                        const bool two = j + CG_WARPS < je;
+                        if (!two) s0 = s1;
+                        const float v = tree256_pair<VEC>(s0, s1, lane);
+                        if (lane == 0u) sh.part[j - jb] = v;
+                        if (two && lane == PAIR_LANE<VEC>) sh.part[j + CG_WARPS - jb] = v;
+                    }
+                }
+            };
             // ---------------- phase 1: direction + SpMV + d.q ----------------
             Acc acc[2] = {};
             tag++;
-            auto phase1 = [&](uint32_t j) -> float {
+            auto phase1 = [&](uint32_t j) -> Quad {
                 const bool res = __any_sync(0xffffffffu, j < vld(sh.mres));
                 const Quads o = quads_of(j);
                 // One half's d and r rows in flight at a time (64 registers).
@@ -1383,16 +1438,12 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
                     load(1);
                     stencil(1, b0, de);
                 }
-                return f64 ? 0.0f : tree256_quads<VEC>(prod[0], prod[1], one, lane);
+                return f64 ? z4 : qaddp(prod[0], one, prod[1]);  // level 128 of the chunk's tree
             };
 #pragma unroll 1
             for (uint32_t jb = 0; jb < vld(sh.m); jb += KCH) {
                 const uint32_t je = vld(sh.m) - jb < KCH ? vld(sh.m) : jb + KCH;
-#pragma unroll 1
-                for (uint32_t j = jb + warp; j < je; j += CG_WARPS) {
-                    const float v = phase1(j);
-                    if (!f64 && lane == 0) sh.part[j - jb] = v;
-                }
+                chunks(jb, je, phase1);
                 if (!f64 && !whole) {
                     publish_parts(jb, je - jb, vld(sh.area[SLOT_A]), tag, false);
                     if (je < vld(sh.m)) __syncthreads();
@@ -1406,7 +1457,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
             acc[1] = Acc{};
             tag++;
             const Quad a4 = qall(alpha), na4 = qall(-alpha);
-            auto phase2 = [&](uint32_t j) -> float {
+            auto phase2 = [&](uint32_t j) -> Quad {
                 const bool res = __any_sync(0xffffffffu, j < vld(sh.mres));
                 const Quads o = quads_of(j);
                 Quad prod[2] = {z4, z4};
@@ -1433,16 +1484,12 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
                 };
                 if (o.any[0]) update(0);
                 if (o.any[1]) update(1);
-                return f64 ? 0.0f : tree256_quads<VEC>(prod[0], prod[1], one, lane);
+                return f64 ? z4 : qaddp(prod[0], one, prod[1]);  // level 128 of the chunk's tree
             };
 #pragma unroll 1
             for (uint32_t jb = 0; jb < vld(sh.m); jb += KCH) {
                 const uint32_t je = vld(sh.m) - jb < KCH ? vld(sh.m) : jb + KCH;
-#pragma unroll 1
-                for (uint32_t j = jb + warp; j < je; j += CG_WARPS) {
-                    const float v = phase2(j);
-                    if (!f64 && lane == 0) sh.part[j - jb] = v;
-                }
+                chunks(jb, je, phase2);
                 if (!f64 && !whole) {
                     publish_parts(jb, je - jb, vld(sh.area[SLOT_B]), tag, true);
                     if (je < vld(sh.m)) __syncthreads();

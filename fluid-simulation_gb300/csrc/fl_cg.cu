@@ -31,11 +31,11 @@
 //                   pool holds in shared memory, the rest in global memory.
 //
 // What bounds it: up to one chunk per warp, the latency of the two exchanges
-// (2,000-4,000 cycles each: publication, L2 round trip, trees) and of one L2
+// (4,000-6,000 cycles each: publication, L2 round trip, skew, trees) and of one L2
 // load, then instruction issue (about 300 instructions per warp and phase 1);
-// beyond, L2 throughput and the same latencies per round of chunks.  Solves of
+// beyond, reads of the L2 (about 20 B per clock and SM) and the same latencies.  Solves of
 // 40 / 179 / 200 / 200 iterations on 32^3 / 64^3 / 128^3 (2.0 M particles) /
-// 256^3 (18.3 M): 177 / 842 / 1,268 / 5,280 us against 224 / 1,123 / 1,558 /
+// 256^3 (18.3 M): 161 / 830 / 1,255 / 5,000 us (ncu, one launch) against 224 / 1,123 / 1,558 /
 // 7,197 for the earlier kernel (1,024 threads over listed cells or quads, chunk
 // trees from shared memory, every block reading every chunk partial).
 //

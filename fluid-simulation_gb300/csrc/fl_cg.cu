@@ -132,6 +132,7 @@ struct CgShared {
     float rs_hi, rs_lo;        // r.r of the last exchange (rs_old); FL_CG_F32 uses rs_hi
 };
 static_assert(CG_WARPS * 2 * 6 * 32 * 16 <= POOL_BYTES, "register form: six quads per lane and half in the pool");
+static_assert(CG_THREADS == 2 * CHUNK, "split segments: half a block per segment");
 static_assert(sizeof(CgShared) <= 227 * 1024, "CG shared memory exceeds the 227 KB per-block limit");
 
 // ---------------------------------------------------------------------------

@@ -84,12 +84,6 @@ constexpr int CG_WARPS = CG_THREADS / 32;
 constexpr uint32_t KCH = 512;            // chunks a block keeps a table of
 constexpr uint32_t RAW_MAX = 1024;       // tail partials read by every block
 constexpr uint32_t TAG_SPAN_MAX = 1u << 30;
-constexpr uint32_t MAX_CG_BLOCKS = 256;
-// Per-chunk cost in liquid-cell units for ranges of equal weight: a warp takes a
-// chunk at once, so a sparsely filled one costs it nearly as much as a full one
-// (with 256, the slowest block at 256^3 got 170 chunks where the others had 150);
-// solvers that list cells use 32.
-constexpr uint32_t CHUNK_WEIGHT = 1024, CELL_CHUNK_WEIGHT = 32;
 // What the pool leaves of the 228 KB serves as L1 for the neighbours' rows: 140 KB
 // against 200 KB and 100 KB on the full-depth 128^3 dam (FL_CG_F64): 2,073, 2,094
 // and 2,206 us per solve; 256^3 within 1 %.
@@ -357,7 +351,6 @@ __device__ __forceinline__ double d_of(float lo, float hi) { return __hiloint2do
 // blocks that own heads, exchange word of every segment [CHUNK], offsets of the
 // tails [CHUNK + 1].
 enum { PLAN_F32, PLAN_EXTENDED, PLAN_RANGES };
-constexpr uint32_t TILE_Y = 4, TILE_Z = 4;  // chunks of a tile of the list (k_cg_plan)
 constexpr uint32_t H_TAG = CHUNK + 1, H_FORM = CHUNK + 2, H_START = CHUNK + 3;
 
 // Words of one owner block among the segment sums of the split form: whole
@@ -444,16 +437,16 @@ __global__ void __launch_bounds__(CHUNK) k_cg_plan(DevBufs b, uint32_t G, int fo
         s_wa[warp] = (uint32_t)__popc(has);
     }
     __syncthreads();
-    uint32_t base = 0, wbase = 0, A = 0, W = 0, act = (uint32_t)__popc(has & ((1u << lane) - 1u));
+    uint32_t base = 0, A = 0, act = (uint32_t)__popc(has & ((1u << lane) - 1u));
     for (uint32_t w = 0; w < CHUNK / 32; w++) {
         if (w < warp) {
             base += s_wc[w];
-            wbase += s_ww[w];
             act += s_wa[w];
         }
         A += s_wc[w];
-        W += s_ww[w];
     }
+    uint64_t wbase, W;
+    weights_of_warps(s_ww, CHUNK / 32, warp, wbase, W);
     if (form == PLAN_F32 && warp == 0) {
         const uint32_t T = lane ? CG_WARPS * lane : CG_WARPS / 2;
         // A chain of an add, a compare and a select per segment: the counts are loaded
@@ -516,9 +509,6 @@ __global__ void __launch_bounds__(CHUNK) k_cg_plan(DevBufs b, uint32_t G, int fo
     if (li == CHUNK - 1) hdr[CHUNK] = hoff + nh;
     const uint32_t nheads = T ? s_nblk : Gs, ntails = T ? (A - Ah + T - 1) / T : 0u;
     const uint32_t nact = A == 0 ? 1u : nheads + ntails;
-    // Blocks bb with X*Gs < bb*W <= X1*Gs start after the entry spanning
-    // weights [X, X1).  X only grows along a thread's entries, so the next such
-    // block is tracked incrementally from one division.
     if (form == PLAN_F32) {  // in segment order
         uint32_t k = 0;
         if (T) {
@@ -527,30 +517,23 @@ __global__ void __launch_bounds__(CHUNK) k_cg_plan(DevBufs b, uint32_t G, int fo
                 k++;
             });
         } else {
-            uint64_t XG = (uint64_t)(wbase + y - wsum) * Gs;  // Gs x the weight of all entries before this segment
-            uint64_t bb_next = W ? XG / W + 1 : 0, bbW = bb_next * W;
+            RangeSplit split(wbase + (y - wsum), W, Gs);
             segment([&](uint32_t c, uint32_t f) {
                 b.cg_chunk[hoff + k] = c;
                 k++;
-                XG += (uint64_t)(f + per_chunk) * Gs;
-                for (; bbW <= XG; bb_next++, bbW += W) start[bb_next] = hoff + k;
+                split.add(f + per_chunk, hoff + k, start);
             });
         }
     } else {  // in tile order
-        // Z chunks per plane (whole ones: the tiles shear a little where a plane is no
-        // multiple of 256 cells); every chunk is in one tile whatever Z is
-        const uint32_t Z = P.nx * P.ny / CHUNK ? P.nx * P.ny / CHUNK : 1u, planes = (nchunks + Z - 1) / Z;
-        const uint32_t ty = (Z + TILE_Y - 1) / TILE_Y, ntile = ty * ((planes + TILE_Z - 1) / TILE_Z);
-        const uint32_t per = (ntile + CHUNK - 1) / CHUNK;  // of a thread
-        const uint32_t t0 = li * per < ntile ? li * per : ntile, t1 = t0 + per < ntile ? t0 + per : ntile;
-        auto flags = [&](uint32_t t, uint8_t (&f)[16]) {  // returns the tile's first chunk
-            const uint32_t y0 = TILE_Y * (t % ty), c0 = TILE_Z * (t / ty) * Z + y0;
+        const ChunkTiles tiles(P.nx, P.ny, nchunks);
+        const uint32_t per = (tiles.count + CHUNK - 1) / CHUNK;  // of a thread
+        const uint32_t t0 = li * per < tiles.count ? li * per : tiles.count, t1 = t0 + per < tiles.count ? t0 + per : tiles.count;
+        auto flags = [&](uint32_t t, uint8_t (&f)[16]) {
 #pragma unroll
             for (uint32_t i = 0; i < 16; i++) {
-                const uint32_t c = c0 + (i / TILE_Y) * Z + i % TILE_Y;
-                f[i] = y0 + i % TILE_Y < Z && c < nchunks ? b.chunk_flag[c] : (uint8_t)0;
+                const uint32_t c = tiles.chunk(t, i);
+                f[i] = c < nchunks ? b.chunk_flag[c] : (uint8_t)0;
             }
-            return c0;
         };
         uint32_t n = 0, w = 0;
         for (uint32_t t = t0; t < t1; t++) {
@@ -570,24 +553,19 @@ __global__ void __launch_bounds__(CHUNK) k_cg_plan(DevBufs b, uint32_t G, int fo
             s_ww[warp] = xw;
         }
         __syncthreads();
-        uint32_t e = xn - n, wb = xw - w;
-        for (uint32_t v = 0; v < warp; v++) {
-            e += s_wc[v];
-            wb += s_ww[v];
-        }
-        uint64_t XG = (uint64_t)wb * Gs;  // Gs x the weight of all entries before
-        uint64_t bb_next = W ? XG / W + 1 : 0, bbW = bb_next * W;
+        uint32_t e = xn - n;
+        for (uint32_t v = 0; v < warp; v++) e += s_wc[v];
+        uint64_t wb, all;
+        weights_of_warps(s_ww, CHUNK / 32, warp, wb, all);
+        RangeSplit split(wb + (xw - w), all, Gs);
         for (uint32_t t = t0; t < t1; t++) {
             uint8_t f[16];
-            const uint32_t c0 = flags(t, f);
+            flags(t, f);
 #pragma unroll
             for (uint32_t i = 0; i < 16; i++) {
                 if (!f[i]) continue;
-                b.cg_chunk[e++] = c0 + (i / TILE_Y) * Z + i % TILE_Y;
-                if (!Tq) {
-                    XG += (uint64_t)(f[i] + per_chunk) * Gs;
-                    for (; bbW <= XG; bb_next++, bbW += W) start[bb_next] = e;
-                }
+                b.cg_chunk[e++] = tiles.chunk(t, i);
+                if (!Tq) split.add(f[i] + per_chunk, e, start);
             }
         }
         if (Tq)

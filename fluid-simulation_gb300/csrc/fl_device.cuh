@@ -10,11 +10,11 @@
 #include <stdint.h>
 
 #include "../../include/fluidgb.h"
+#include "fl_index.cuh"
 
 namespace fl {
 
 constexpr uint8_t CELL_SOLID = 0, CELL_LIQUID = 1, CELL_AIR = 2;
-constexpr int CHUNK = 256;        // cells per reduction chunk (the 256-wide workgroup of cg_reduce.wgsl)
 constexpr int CG_GROUPS = 4;      // the CG launches at most one block per CG_GROUPS chunks of the grid
 constexpr int SCAN_ITEMS = 4;     // counts per thread in the bin scan
 constexpr int SCAN_THREADS = 1024;
@@ -108,11 +108,6 @@ struct DevBufs {
 };
 
 // Sizes of the CG plan header and exchange area (fl_cg.cu).
-#if defined(__CUDACC__)
-#define FL_HD __host__ __device__
-#else
-#define FL_HD
-#endif
 FL_HD constexpr size_t cg_plan_words(size_t max_blocks) { return 3 * (size_t)CHUNK + 6 + (max_blocks + 1); }
 FL_HD constexpr size_t cg_x_words(size_t nchunks, size_t max_blocks) {
     return 16 + 2 * ((nchunks + 15) & ~(size_t)15) + 64 * max_blocks + 2 * 256;
@@ -255,14 +250,11 @@ __device__ __forceinline__ bool is_stray(const DevParams& P, float4 pos, const u
     return floorf(q0) != (float)kc[0] || floorf(q1) != (float)kc[1] || floorf(q2) != (float)kc[2];
 }
 
-// (i, j, k) of cell c.  n / d = umulhi(n, mul) >> shift with mul =
-// ceil(2^(31 + L) / d), shift = L - 1, L = ceil(log2 d): mul exceeds 2^(31+L) / d by
-// less than 1 <= 2^L / d, so the product is above n / d by less than 1 / d for n < 2^31
-// and the quotient is exact (Granlund and Montgomery 1994).  Three divisions took
-// the cell kernels some 60 instructions a cell.
+// (i, j, k) of cell c (see division_by).  Three divisions took the cell kernels some 60
+// instructions a cell.
 __device__ __forceinline__ void cell_coords(const DevParams& P, uint32_t c, uint32_t& i, uint32_t& j, uint32_t& k) {
-    const uint32_t row = __umulhi(c, P.nx_mul) >> P.nx_shift;
-    k = __umulhi(row, P.ny_mul) >> P.ny_shift;
+    const uint32_t row = quotient(c, P.nx_mul, P.nx_shift);
+    k = quotient(row, P.ny_mul, P.ny_shift);
     i = c - row * P.nx;
     j = row - k * P.ny;
 }

@@ -98,7 +98,7 @@ fl_status validate(const fl_params* p, std::string* why) {
     if (!p) { *why = "params is NULL"; return FL_INVALID_ARG; }
     if (p->gdim[0] < 3 || p->gdim[1] < 3 || p->gdim[2] < 3) { *why = "each grid dimension must be >= 3"; return FL_INVALID_ARG; }
     if (p->gdim[0] > 2048 || p->gdim[1] > 2048 || p->gdim[2] > 2048) { *why = "grid dimension > 2048"; return FL_INVALID_ARG; }
-    if ((uint64_t)p->gdim[0] * p->gdim[1] * p->gdim[2] > (1ull << 30)) { *why = "more than 2^30 cells"; return FL_INVALID_ARG; }
+    if ((uint64_t)p->gdim[0] * p->gdim[1] * p->gdim[2] > fl::MAX_CELLS) { *why = "more than 2^30 cells"; return FL_INVALID_ARG; }
     if (!(p->geom[0] > 0.0f) || !(p->geom[1] > 0.0f)) { *why = "h and inv_h must be > 0"; return FL_INVALID_ARG; }
     if (!(p->geom[2] > 0.0f)) { *why = "dt must be > 0"; return FL_INVALID_ARG; }
     if (!(p->phys[1] > 0.0f)) { *why = "rho must be > 0"; return FL_INVALID_ARG; }
@@ -111,14 +111,6 @@ fl_status validate(const fl_params* p, std::string* why) {
     for (int i = 0; i < 3; i++)
         if (p->reserved[i]) { *why = "reserved fields must be zero"; return FL_INVALID_ARG; }
     return FL_OK;
-}
-
-// Multiplier and shift of a division by d >= 2 (see cell_coords).
-void division_by(uint32_t d, uint32_t& mul, uint32_t& shift) {
-    uint32_t L = 1;
-    while ((1ull << L) < d) L++;
-    mul = (uint32_t)(((1ull << (31 + L)) + d - 1) / d);
-    shift = L - 1;
 }
 
 // Derived settings, in the shaders' f32 operation order.
@@ -156,8 +148,8 @@ void derive(const fl_params& p, uint32_t n, DevParams& d) {
     d.advect_order = p.advect_order == 2u ? 2u : 1u;
     d.nchunks = (d.C + fl::CHUNK - 1) / fl::CHUNK;
     d.solver = p.pressure_solver;
-    division_by(d.nx, d.nx_mul, d.nx_shift);
-    division_by(d.ny, d.ny_mul, d.ny_shift);
+    fl::division_by(d.nx, d.nx_mul, d.nx_shift);
+    fl::division_by(d.ny, d.ny_mul, d.ny_shift);
 }
 
 struct PoolPlan {
@@ -925,7 +917,7 @@ fl_status fl_solve_pressure(uint32_t nx, uint32_t ny, uint32_t nz, const uint8_t
                             fl_stats* stats_out) {
     if (!cell_type || !divergence || !pressure_out) return set_err(nullptr, FL_INVALID_ARG, "NULL argument");
     if (warm_start && !pressure_in) return set_err(nullptr, FL_INVALID_ARG, "warm start needs pressure_in");
-    if (nx < 3 || ny < 3 || nz < 3 || (uint64_t)nx * ny * nz > (1ull << 30))
+    if (nx < 3 || ny < 3 || nz < 3 || (uint64_t)nx * ny * nz > fl::MAX_CELLS)
         return set_err(nullptr, FL_INVALID_ARG, "bad grid size");
     if (!(h > 0.0f) || !(rho > 0.0f) || !(dt > 0.0f)) return set_err(nullptr, FL_INVALID_ARG, "h, rho, dt must be > 0");
     if (cg_precision > FL_CG_F64_IEEE) return set_err(nullptr, FL_INVALID_ARG, "bad cg_precision");
@@ -1011,7 +1003,7 @@ fl_status fl_solve_pressure(uint32_t nx, uint32_t ny, uint32_t nz, const uint8_t
 fl_status fl_relax_pressure(uint32_t nx, uint32_t ny, uint32_t nz, const uint8_t* cell_type, const float* divergence,
                             float h, float rho, float dt, uint32_t method, uint32_t iters, float* pressure_out) {
     if (!cell_type || !divergence || !pressure_out) return set_err(nullptr, FL_INVALID_ARG, "NULL argument");
-    if (nx < 3 || ny < 3 || nz < 3 || (uint64_t)nx * ny * nz > (1ull << 30))
+    if (nx < 3 || ny < 3 || nz < 3 || (uint64_t)nx * ny * nz > fl::MAX_CELLS)
         return set_err(nullptr, FL_INVALID_ARG, "bad grid size");
     if (!(h > 0.0f) || !(rho > 0.0f) || !(dt > 0.0f)) return set_err(nullptr, FL_INVALID_ARG, "h, rho, dt must be > 0");
     if (method > 1u) return set_err(nullptr, FL_INVALID_ARG, "method must be FL_RELAX_JACOBI or FL_RELAX_RBGS");

@@ -346,8 +346,10 @@ __device__ __forceinline__ float ld_if(const float* p, bool on) {
 // finished and its writes are visible.  A substep is some sixteen kernels of a few
 // microseconds on a small grid; this takes the launch latency between them (four 32^3
 // substeps with their frame output: 1,000 -> 945 us; a 97 x 61 x 83 step in place,
-// 30 iterations: 277 -> 251 us).  Nothing may be read before the call: no const
-// __restrict__ arguments in such kernels (loads through them may move above it).
+// 30 iterations: 277 -> 251 us).  Nothing may be read before the call, and
+// nothing that the kernel before may have written may be read through the read-only
+// path (__ldg, ld.global.nc, const __restrict__ pointers): it wants memory that nobody
+// writes while the kernel lives, and the two lives overlap.
 __device__ __forceinline__ void after_previous() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");

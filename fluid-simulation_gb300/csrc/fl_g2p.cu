@@ -17,6 +17,18 @@ __device__ __forceinline__ bool touches_static(int axis, int ii, int jj, int kk,
     return ii <= 0 || ii >= nx - 1 || jj <= 0 || jj >= ny - 1 || kk <= 1 || kk >= nz - 1;
 }
 
+// A load of a face value.  An ordinary one: k_project may still be writing them when
+// this kernel starts, so the read-only path is closed (after_previous).  Nothing in the
+// kernel writes them, so the statement is not volatile and the compiler orders it as it
+// likes; it cannot come before the wait, because its address hangs on a particle's
+// position that is loaded after it.  256^3, 18.3 M particles / 64^3: 548 / 21.1 us; as
+// plain C++ loads 546 / 22.2, through the read-only path 536 / 20.7.
+__device__ __forceinline__ float ld_face(const float* p) {
+    float v;
+    asm("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+
 // g2p.wgsl:56-129 sample_u / sample_v / sample_w.  with_saved=false skips the
 // saved gather (midpoint sample).
 template <bool WITH_SAVED>
@@ -29,8 +41,8 @@ __device__ __forceinline__ void sample(const DevBufs& b, const DevParams& P, int
     const float g2 = __fadd_rn(__fmul_rn(__fsub_rn(pz, P.origin[2]), P.inv_h), axis == 2 ? 0.0f : -0.5f);
     const int b0 = floor_to_i32(g0), b1 = floor_to_i32(g1), b2 = floor_to_i32(g2);
     const float t0 = __fsub_rn(g0, (float)b0), t1 = __fsub_rn(g1, (float)b1), t2 = __fsub_rn(g2, (float)b2);
-    const float* __restrict__ fv = b.vel[axis];
-    const float* __restrict__ sv = b.sav[axis];
+    const float* const fv = b.vel[axis];
+    const float* const sv = b.sav[axis];
     float fin = 0.0f, sav = 0.0f, wsum = 0.0f;
     // All eight taps in range and off the static walls (the common case away
     // from the walls): the same sums in the same order, without the per-tap
@@ -50,8 +62,8 @@ __device__ __forceinline__ void sample(const DevBufs& b, const DevParams& P, int
 #pragma unroll
                 for (int di = 0; di < 2; di++) {
                     const float w = __fmul_rn(__fmul_rn(tent(t0, di), wy), wz);
-                    fin = __fadd_rn(fin, __fmul_rn(w, __ldg(pf + row + di)));
-                    if (WITH_SAVED) sav = __fadd_rn(sav, __fmul_rn(w, __ldg(ps + row + di)));
+                    fin = __fadd_rn(fin, __fmul_rn(w, ld_face(pf + row + di)));
+                    if (WITH_SAVED) sav = __fadd_rn(sav, __fmul_rn(w, ld_face(ps + row + di)));
                     wsum = __fadd_rn(wsum, w);
                 }
             }
@@ -78,8 +90,8 @@ __device__ __forceinline__ void sample(const DevBufs& b, const DevParams& P, int
                 const float wx = tent(t0, di);
                 const float w = __fmul_rn(__fmul_rn(wx, wy), wz);
                 const size_t idx = (size_t)ii + (size_t)dim0 * ((size_t)jj + (size_t)dim1 * kk);
-                fin = __fadd_rn(fin, __fmul_rn(w, __ldg(fv + idx)));
-                if (WITH_SAVED) sav = __fadd_rn(sav, __fmul_rn(w, __ldg(sv + idx)));
+                fin = __fadd_rn(fin, __fmul_rn(w, ld_face(fv + idx)));
+                if (WITH_SAVED) sav = __fadd_rn(sav, __fmul_rn(w, ld_face(sv + idx)));
                 wsum = __fadd_rn(wsum, w);
             }
         }
@@ -107,7 +119,7 @@ __device__ __forceinline__ void speed_clamp(float& x, float& y, float& z, float 
 // What bounds it is instruction issue and the latency of 48 loads per particle; the
 // face indices are 32-bit (64-bit products took a tenth of the instructions) and 64
 // registers let more loads be in flight than 40 or 80 (256^3, 18.3 M particles:
-// 605 us -> 539 us -> 529 us; 84 registers 674, 40 registers 580).
+// 605 us -> 539 us -> 529 us; 84 registers 674, 40 registers 580; 545 with ld_face).
 __global__ void __launch_bounds__(256, 4) k_g2p(DevBufs b) {
     after_previous();
     const DevParams& P = *b.prm;

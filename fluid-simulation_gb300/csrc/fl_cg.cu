@@ -324,8 +324,7 @@ template <>
 struct AccT<FL_CG_F64_IEEE> {
     using type = double;
 };
-// (df_norm follows every fourth: see acc_quad)
-__device__ __forceinline__ void acc_add(Df& a, float x, float y) { a = df_add_raw(a, df_prod(x, y)); }
+__device__ __forceinline__ void acc_add(Df& a, float x, float y) { a = df_acc(a, x, y); }
 // f32 x f32 is exact in double, so one fma = the exact product added with one rounding
 __device__ __forceinline__ void acc_add(double& a, float x, float y) { a = __fma_rn((double)x, (double)y, a); }
 __device__ __forceinline__ double warp_sum_d(double v) {  // result in lane 0
@@ -1030,12 +1029,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
                 const uint32_t bb = lane + 32u * i;
                 v[i] = bb < nact ? Df{sh.words[2 * bb], sh.words[2 * bb + 1]} : Df{0.0f, 0.0f};
             }
-#pragma unroll
-            for (uint32_t w = MAX_CG_BLOCKS / 64; w > 0; w >>= 1)
-#pragma unroll
-                for (uint32_t i = 0; i < w; i++) v[i] = df_add_raw(v[i], v[i + w]);
-            Df acc = v[0];
-            acc = warp_sum_df(acc);
+            const Df acc = warp_sum_df(df_tree(v));
             if (lane == 0) {
                 const Df rs_old = {sh.rs_hi, sh.rs_lo};
                 float scv = 0.0f;
@@ -1205,7 +1199,6 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
         acc_add(a, hi2(x.a), hi2(y.a));
         acc_add(a, lo2(x.b), lo2(y.b));
         acc_add(a, hi2(x.b), hi2(y.b));
-        if constexpr (f64 && !ieee) a = df_norm(a);  // four terms at a time: the low part stays an ulp of the high one
     };
     // The exchange after a phase: post 1 alpha, post 2 beta and the stopping test.
     // `meanwhile` (extended forms) is done while the words travel.

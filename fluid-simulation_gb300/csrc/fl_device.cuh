@@ -11,6 +11,9 @@
 
 #include "../../include/fluidgb.h"
 #include "fl_index.cuh"
+#if defined(__CUDACC__)
+#include "fl_df.cuh"
+#endif
 
 namespace fl {
 
@@ -148,44 +151,6 @@ struct AdjBufs {
 // helpers (device code only; fl_host.cpp sees the layout above)
 #if defined(__CUDACC__)
 
-// Float-float ("double-single") arithmetic: a value is hi + lo with two f32,
-// |lo| <= ulp(hi)/2, about 48 significand bits.  GB300's FP64 pipe has a
-// dependent-op latency of ~64 cycles for one warp and ~600 with a full SM
-// issuing (DDIV ~640 for one warp), so the FL_CG_F64 inner products, residual
-// norms and stopping test are carried in float-float on the FP32 pipe
-// (df_add: ~32 cycles dependent latency) and converted to double only for the
-// statistics.  Products use the exact two-product (fmaf), sums the two-sum.
-struct Df {
-    float hi, lo;
-};
-__device__ __forceinline__ Df df_add(Df a, Df b) {
-    const float s = __fadd_rn(a.hi, b.hi);
-    const float bb = __fsub_rn(s, a.hi);
-    float e = __fadd_rn(__fsub_rn(a.hi, __fsub_rn(s, bb)), __fsub_rn(b.hi, bb));
-    e = __fadd_rn(e, __fadd_rn(a.lo, b.lo));
-    const float hi = __fadd_rn(s, e);
-    return {hi, __fsub_rn(e, __fsub_rn(hi, s))};
-}
-__device__ __forceinline__ Df df_prod(float x, float y) {
-    const float p = __fmul_rn(x, y);
-    return {p, __fmaf_rn(x, y, -p)};
-}
-// A sum whose parts are left unnormalised: the rounded sum of the high parts, and the
-// low parts with the (exact) error of that rounding.  In a chain or a tree of these the
-// high parts follow one another at one add each, and the rest trails behind, where
-// df_add's result waits for all eleven; df_norm at the end.  (FL_CG_F64, full-depth
-// 128^3 dam: 1,877 us per solve with df_add, 1,748 with these, four terms or a tree
-// at a time.)
-__device__ __forceinline__ Df df_add_raw(Df a, Df b) {
-    const float s = __fadd_rn(a.hi, b.hi);
-    const float bb = __fsub_rn(s, a.hi);
-    const float e = __fadd_rn(__fsub_rn(a.hi, __fsub_rn(s, bb)), __fsub_rn(b.hi, bb));
-    return {s, __fadd_rn(__fadd_rn(a.lo, b.lo), e)};
-}
-__device__ __forceinline__ Df df_norm(Df a) {
-    const float hi = __fadd_rn(a.hi, a.lo);
-    return {hi, __fsub_rn(a.lo, __fsub_rn(hi, a.hi))};
-}
 template <int LANES = 32>
 __device__ __forceinline__ Df warp_sum_df(Df v) {  // of the first LANES lanes, result in lane 0
 #pragma unroll
@@ -193,9 +158,9 @@ __device__ __forceinline__ Df warp_sum_df(Df v) {  // of the first LANES lanes, 
         Df w;
         w.hi = __shfl_down_sync(0xffffffffu, v.hi, o);
         w.lo = __shfl_down_sync(0xffffffffu, v.lo, o);
-        v = df_add_raw(v, w);
+        v = df_add(v, w);
     }
-    return df_norm(v);
+    return v;
 }
 __device__ __forceinline__ Df warp_allsum_df(Df v) {  // result in every lane
 #pragma unroll
@@ -203,9 +168,9 @@ __device__ __forceinline__ Df warp_allsum_df(Df v) {  // result in every lane
         Df w;
         w.hi = __shfl_xor_sync(0xffffffffu, v.hi, o);
         w.lo = __shfl_xor_sync(0xffffffffu, v.lo, o);
-        v = df_add_raw(v, w);
+        v = df_add(v, w);
     }
-    return df_norm(v);
+    return v;
 }
 
 // a/b to f32 precision from float-float operands (one Newton correction).

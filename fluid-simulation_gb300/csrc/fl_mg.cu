@@ -232,15 +232,14 @@ __device__ bool mg_allreduce(Ctx& x, Df v, Df& out) {
     if (warp == 0) {
         Df s = {0.0f, 0.0f};
         for (uint32_t g0 = 0; g0 < gridDim.x; g0 += 8 * 32) {
-            float2 p[8];
+            Df p[8];
 #pragma unroll
             for (int k = 0; k < 8; k++) {
                 const uint32_t g = g0 + lane + 32u * k;
-                p[k] = g < gridDim.x ? part[g] : make_float2(0.0f, 0.0f);
+                const float2 v2 = g < gridDim.x ? part[g] : make_float2(0.0f, 0.0f);
+                p[k] = {v2.x, v2.y};
             }
-#pragma unroll
-            for (int k = 0; k < 8; k++) s = df_add_raw(s, Df{p[k].x, p[k].y});
-            s = df_norm(s);
+            s = df_add(s, df_tree(p));
         }
         s = warp_allsum_df(s);
         if (lane == 0) x.sh.res = make_float2(s.hi, s.lo);

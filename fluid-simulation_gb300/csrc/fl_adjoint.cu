@@ -387,6 +387,11 @@ __global__ void __launch_bounds__(256) k_adj_g2p(AdjBufs a) {
         a.coef[3 * (size_t)d] = make_float4(q[0], q[1], q[2], pv[0]);
         a.coef[3 * (size_t)d + 1] = make_float4(pv[1], pv[2], cf[0], cf[1]);
         a.coef[3 * (size_t)d + 2] = make_float4(cf[2], cs[0], cs[1], cs[2]);
+        // 0 unless one of them is infinite or NaN (see k_adj_gather)
+        float zero = 0.0f;
+#pragma unroll
+        for (int ax = 0; ax < 3; ax++) zero += 0.0f * pv[ax] + 0.0f * cf[ax] + 0.0f * cs[ax];
+        if (zero != 0.0f) a.flags[2] = 1u;
         if (pos.w != 0.0f) a.flags[0] = 1u;  // a stray particle (its P2G cell is not its bin)
         a.g_sorted[2 * (size_t)d] = make_float4(gX[0], gX[1], gX[2], 0.0f);
         a.g_sorted[2 * (size_t)d + 1] = make_float4(gpv[0], gpv[1], gpv[2], 0.0f);
@@ -599,8 +604,11 @@ __global__ void __launch_bounds__(256) k_adj_mid(AdjBufs a) {
 // cell is the loop's, and each weight is one expression of the fraction
 // (gather_bins).  Deriving the stencil of every candidate instead took 717 us
 // of the 128^3 adjoint step (2.0 M particles, issue-bound: 120 instructions a
-// candidate, 27 cells of them per thread).  Steps with strays and the cells of
-// the grid's high sides keep that general form (gather_any).
+// candidate, 27 cells of them per thread).  gather_bins multiplies every candidate's
+// coefficients by its weights, also where they are 0, so a particle whose gradient or
+// velocity is not finite would make NaN of faces that it has no part in.  Steps with
+// strays or such a particle and the cells of the grid's high sides keep the general
+// form (gather_any), which leaves out a weight of 0.
 
 struct FaceSums {
     float gf[6], gs[6], W[6], WV[6];  // low faces of axis 0..2, high-side faces of axis 0..2
@@ -750,7 +758,7 @@ __global__ void __launch_bounds__(256) k_adj_gather(AdjBufs a, int midpoint) {
     FaceSums o[NZ];
 #pragma unroll
     for (int z = 0; z < NZ; z++) o[z] = FaceSums{};
-    const bool any = a.flags[0] || i == nx - 1 || j == ny - 1;
+    const bool any = a.flags[0] || a.flags[2] || i == nx - 1 || j == ny - 1;
     if (!any) gather_bins<NZ>(a, P, i, j, k, o);
     const double mscale = midpoint && a.flags[1] != 0u ? ldexp(1.0, -mid_exponent(a)) : 0.0;
 #pragma unroll

@@ -142,7 +142,8 @@ struct AdjBufs {
     float4* coef;            // per particle (bin order), 3 float4: {q, v_x}, {v_y, v_z, gpic_x/W, gpic_y/W},
                              // {gpic_z/W, gsaved/W per axis}
     const uint32_t* cell_first;  // first bin-ordered particle of every cell (the step's bin offsets)
-    uint32_t* flags;         // [0] the step has stray particles, [1] max |midpoint coefficient| (float bits)
+    uint32_t* flags;         // [0] the step has stray particles, [1] max |midpoint coefficient| (float bits),
+                             // [2] some face coefficient or velocity is not finite
     float4* mid;             // midpoint step: per particle {qm.xyz, _}, {gfin/W at qm per axis, _}
     unsigned long long* gmid[3];  // midpoint-stencil face gradients, 64-bit fixed point
 };

@@ -1191,7 +1191,7 @@ fl_status fl_tape_create(fl_handle* h, uint32_t max_steps, fl_tape** out) {
         o_gm[a] = pl.take<unsigned long long>(h->F3[a]);
         o_gp[a] = pl.take<double>((h->F3[a] + 255) / 256);
     }
-    const size_t o_coef = pl.take<float4>(3 * cap), o_mid = pl.take<float4>(2 * cap), o_flags = pl.take<uint32_t>(2);
+    const size_t o_coef = pl.take<float4>(3 * cap), o_mid = pl.take<float4>(2 * cap), o_flags = pl.take<uint32_t>(3);
     size_t o_rhs = pl.take<float>(C), o_lam = pl.take<float>(C), o_r = pl.take<float>(C), o_dA = pl.take<float>(C),
            o_dB = pl.take<float>(C), o_q = pl.take<float>(C), o_ci = pl.take<uint16_t>(C), o_fl = pl.take<uint8_t>(nch),
            o_prr = pl.take<float>(nch), o_c64 = pl.take<float2>(nch), o_plan = pl.take<uint32_t>(nch),
@@ -1372,7 +1372,7 @@ fl_status fl_step_adjoint(fl_handle* h, fl_tape* t, const void* dL_dout_dev, voi
     a.coef = t->coef;
     a.mid = t->mid;
     a.flags = t->flags;
-    FL_CUDA(h, cudaMemsetAsync(t->flags, 0, 2 * sizeof(uint32_t), st));
+    FL_CUDA(h, cudaMemsetAsync(t->flags, 0, 3 * sizeof(uint32_t), st));
     a.g_out = (const float4*)dL_dout_dev;
     a.g_sorted = t->g_sorted;
     a.g_in = (float4*)dL_din_dev;

@@ -223,7 +223,8 @@ fl_status mg_alloc(fl_handle* h, uint32_t nx, uint32_t ny, uint32_t nz, float* r
     return FL_OK;
 }
 
-fl_status device_check(fl_handle* h) {
+// cg: the caller goes on to launch a CG (its kernels' occupancy is asked for).
+fl_status device_check(fl_handle* h, bool cg = true) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return set_err(h, FL_NO_DEVICE, std::string("no CUDA device: ") + cudaGetErrorString(e));
@@ -235,6 +236,7 @@ fl_status device_check(fl_handle* h) {
                                             std::to_string(prop.minor));
     if (!prop.cooperativeLaunch) return set_err(h, FL_NO_DEVICE, "device does not support cooperative launch");
     g_num_sms = prop.multiProcessorCount;
+    if (!cg) return FL_OK;
     g_cg_per_sm = fl::cg_max_blocks_per_sm();
     if (g_cg_per_sm < 1) return set_err(h, FL_INTERNAL, "CG kernel cannot be resident (occupancy 0)");
     return FL_OK;
@@ -1007,7 +1009,7 @@ fl_status fl_relax_pressure(uint32_t nx, uint32_t ny, uint32_t nz, const uint8_t
         return set_err(nullptr, FL_INVALID_ARG, "bad grid size");
     if (!(h > 0.0f) || !(rho > 0.0f) || !(dt > 0.0f)) return set_err(nullptr, FL_INVALID_ARG, "h, rho, dt must be > 0");
     if (method > 1u) return set_err(nullptr, FL_INVALID_ARG, "method must be FL_RELAX_JACOBI or FL_RELAX_RBGS");
-    fl_status s = device_check(nullptr);
+    fl_status s = device_check(nullptr, false);
     if (s != FL_OK) return s;
     const size_t C = (size_t)nx * ny * nz;
     const float scale = rho * h * h / dt;  // ProjectionParams::rhs_scale (sim/pressure.rs:31-33)
@@ -1027,23 +1029,21 @@ fl_status fl_relax_pressure(uint32_t nx, uint32_t ny, uint32_t nz, const uint8_t
     float* pb = (float*)(base + o_b);
     uint32_t* bars = (uint32_t*)(base + o_bar);
     float* res = pa;
-    uint32_t status = 0;
     cudaStream_t st = nullptr;
     do {
         if ((e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking)) != cudaSuccess) break;
         if ((e = cudaMemsetAsync(pool, 0, pl.off, st)) != cudaSuccess) break;
         if ((e = cudaMemcpyAsync(dct, cell_type, C, cudaMemcpyHostToDevice, st)) != cudaSuccess) break;
         if ((e = cudaMemcpyAsync(ddiv, divergence, 4 * C, cudaMemcpyHostToDevice, st)) != cudaSuccess) break;
-        if ((e = fl::launch_relax(dct, ddiv, scale, pa, pb, bars, nx, ny, nz, method, iters, g_num_sms, st, &res)) != cudaSuccess)
+        if ((e = fl::solve_relax(dct, ddiv, scale, pa, pb, bars, nx, ny, nz, method, iters, g_num_sms, 2000000000ull, st,
+                                 &res)) != cudaSuccess)
             break;
         if ((e = cudaMemcpyAsync(pressure_out, res, 4 * C, cudaMemcpyDeviceToHost, st)) != cudaSuccess) break;
-        if ((e = cudaMemcpyAsync(&status, bars + fl::BAR_BYTES / 4, 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess) break;
         e = cudaStreamSynchronize(st);
     } while (0);
     fl_status rs = e != cudaSuccess ? cuda_err(nullptr, e, "fl_relax_pressure") : FL_OK;
     if (st) cudaStreamDestroy(st);
     cudaFree(pool);
-    if (rs == FL_OK && status) return set_err(nullptr, (fl_status)status, "a device-side wait expired");
     return rs;
 }
 

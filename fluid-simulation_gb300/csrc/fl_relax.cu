@@ -79,7 +79,7 @@ struct RelaxShared {
 template <bool JACOBI>
 __global__ void __launch_bounds__(RELAX_THREADS, 1) k_relax(const uint8_t* __restrict__ ct, const float* __restrict__ div,
                                                              float scale, float* pa, float* pb, uint32_t* bars, uint32_t nx,
-                                                             uint32_t ny, uint32_t C, uint32_t iters) {
+                                                             uint32_t ny, uint32_t C, uint32_t iters, uint64_t wait_ns) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     RelaxShared& sh = *reinterpret_cast<RelaxShared*>(smem_raw);
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nxy = nx * ny;
@@ -147,16 +147,16 @@ __global__ void __launch_bounds__(RELAX_THREADS, 1) k_relax(const uint8_t* __res
                 out[c] = cnt ? __fdiv_rn(__fsub_rn(sum, sh.rhs[at]), (float)cnt) : 0.0f;
             }
             if (it + 1 == iters && (JACOBI || colour == 1u)) return;
-            if (!grid_barrier(bars, ++epoch, 2000000000ull, bars + BAR_BYTES / 4, &sh.ok)) return;
+            if (!grid_barrier(bars, ++epoch, wait_ns, bars + BAR_BYTES / 4, &sh.ok)) return;
         }
     }
 }
 
 }  // namespace
 
-cudaError_t launch_relax(const uint8_t* ct, const float* div, float scale, float* pa, float* pb, uint32_t* bars,
-                         uint32_t nx, uint32_t ny, uint32_t nz, uint32_t method, uint32_t iters, int num_sms,
-                         cudaStream_t s, float** result) {
+cudaError_t solve_relax(const uint8_t* ct, const float* div, float scale, float* pa, float* pb, uint32_t* bars,
+                        uint32_t nx, uint32_t ny, uint32_t nz, uint32_t method, uint32_t iters, int num_sms,
+                        uint64_t wait_ns, cudaStream_t s, float** result) {
     const uint32_t C = nx * ny * nz, grid = (C + 255) / 256;
     if (iters && (uint64_t)C + 32ull * num_sms <= (uint64_t)RELAX_CELLS * num_sms) {
         const bool jacobi = method == 0u;
@@ -176,10 +176,18 @@ cudaError_t launch_relax(const uint8_t* ct, const float* div, float scale, float
         for (uint32_t done = 0; e == cudaSuccess && done < iters; done += RELAX_SWEEPS) {
             if (done) e = cudaMemsetAsync(bars, 0, BAR_BYTES, s);
             const uint32_t now = iters - done < RELAX_SWEEPS ? iters - done : RELAX_SWEEPS;
-            if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, f, ct, div, scale, pa, pb, bars, nx, ny, C, now);
+            if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, f, ct, div, scale, pa, pb, bars, nx, ny, C, now, wait_ns);
         }
+        uint32_t status = 0;
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&status, bars + BAR_BYTES / 4, 4, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         *result = jacobi && (iters & 1u) ? pb : pa;
-        return e;
+        if (e == cudaErrorCooperativeLaunchTooLarge) (void)cudaGetLastError();
+        else if (e != cudaSuccess || status == 0) return e;
+        // The blocks cannot all be resident, or one waited too long for another (a GPU
+        // shared with other work): a launch per sweep needs neither.
+        if ((e = cudaMemsetAsync(pa, 0, 4 * (size_t)C, s)) != cudaSuccess) return e;
+        if ((e = cudaMemsetAsync(pb, 0, 4 * (size_t)C, s)) != cudaSuccess) return e;
     }
     float* cur = pa;
     for (uint32_t it = 0; it < iters; it++) {

@@ -1194,11 +1194,27 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
     auto edge = [&](uint32_t c0, uint32_t e0, uint32_t c1, uint32_t e1) -> uint32_t {
         return lane == 0 && (e0 & 1u) ? c0 - 1u : lane == 31 && (e1 & 8u) ? c1 + 3u * CSTEP + 1u : 0u;
     };
+    // x . y of a quad; every lane of the warp calls it.
     auto acc_quad = [&](Acc& a, Quad x, Quad y) {
-        acc_add(a, lo2(x.a), lo2(y.a));
-        acc_add(a, hi2(x.a), hi2(y.a));
-        acc_add(a, lo2(x.b), lo2(y.b));
-        acc_add(a, hi2(x.b), hi2(y.b));
+        const float xs[4] = {lo2(x.a), hi2(x.a), lo2(x.b), hi2(x.b)}, ys[4] = {lo2(y.a), hi2(y.a), lo2(y.b), hi2(y.b)};
+        // The FP64 pipe bounds the phases of FL_CG_F64_IEEE, and it takes 16 clocks for a warp
+        // whatever number of lanes holds a liquid cell.  With its two conversions per term
+        // on that pipe a chunk half full took as long as a full one (128^3 with liquid below
+        // x = 0.5: 2,586 us per solve, with the listed cells before 2,482; 191 x 151 x 170:
+        // 2,243 and 1,668); converted by integer operations 2,015 and 1,717 (256^3: 5,308
+        // against 7,335).  Subnormal, infinite or NaN terms take the instruction.
+        if constexpr (ieee) {
+            bool plain = true;
+#pragma unroll
+            for (int k = 0; k < 4; k++) plain = plain && is_plain(xs[k]) && is_plain(ys[k]);
+            if (__all_sync(0xffffffffu, plain)) {
+#pragma unroll
+                for (int k = 0; k < 4; k++) a = __fma_rn(plain_double(xs[k]), plain_double(ys[k]), a);
+                return;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) acc_add(a, xs[k], ys[k]);
     };
     // The exchange after a phase: post 1 alpha, post 2 beta and the stopping test.
     // `meanwhile` (extended forms) is done while the words travel.

@@ -1,4 +1,4 @@
-// fl_df.cuh — float-float sums and products.
+// fl_df.cuh — float-float sums and products, exact conversion to double.
 //
 // Float-float ("double-single") arithmetic: a value is hi + lo with two f32,
 // |lo| <= ulp(hi)/2, about 48 significand bits.  GB300's FP64 pipe has a
@@ -42,5 +42,17 @@ __device__ __forceinline__ Df df_tree(Df (&v)[N]) {
 // FL_CG_F64 were up to 1.4 times as far from exact ones; normalised the solve of the
 // full-depth 128^3 dam takes 1,849 us instead of 1,757.)
 __device__ __forceinline__ Df df_acc(Df a, float x, float y) { return df_add(a, df_prod(x, y)); }
+
+// (double)x by integer operations, for x zero or normal (is_plain): sign, exponent and
+// mantissa moved to their places, the exponent's bias raised by 896.  The conversion
+// instruction shares the FP64 pipe, two lanes per clock and SM.
+__device__ __forceinline__ bool is_plain(float x) {
+    const unsigned a = __float_as_uint(x) & 0x7fffffffu;
+    return a == 0u || a - 0x00800000u < 0x7f000000u;
+}
+__device__ __forceinline__ double plain_double(float x) {
+    const unsigned b = __float_as_uint(x), hi = (unsigned)((int)b >> 3) & 0x8fffffffu;
+    return __hiloint2double((int)(hi + (b << 1 ? 0x38000000u : 0u)), (int)(b << 29));
+}
 
 }  // namespace fl

@@ -1,7 +1,7 @@
 """Float-float sums (csrc/fl_df.cuh, the header that the kernels compile) on the host's
 C++ compiler: accumulated products and a tree of 32 accumulators lose no more than
 Dekker's normalised additions one after the other do, against exact sums, for terms of
-one sign and of both."""
+one sign and of both.  The conversion to double by integer operations is exact."""
 import ctypes
 import os
 import subprocess
@@ -14,12 +14,20 @@ CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 
 SHIM = r"""
 #include <cmath>
+#include <cstring>
 #define __device__
 #define __forceinline__ inline
 static float __fadd_rn(float a, float b) { return a + b; }
 static float __fsub_rn(float a, float b) { return a - b; }
 static float __fmul_rn(float a, float b) { return a * b; }
 static float __fmaf_rn(float a, float b, float c) { return std::fma(a, b, c); }
+static unsigned __float_as_uint(float x) { unsigned b; std::memcpy(&b, &x, 4); return b; }
+static double __hiloint2double(int hi, int lo) {
+    const unsigned long long b = (unsigned long long)(unsigned)hi << 32 | (unsigned)lo;
+    double d;
+    std::memcpy(&d, &b, 8);
+    return d;
+}
 #include "fl_df.cuh"
 using namespace fl;
 // Dekker 1971 with Knuth's two-sum: every sum normalised
@@ -42,6 +50,16 @@ extern "C" void dots(const float* x, const float* y, int n, Df* out) {
     }
     out[0] = df_tree(a);
     out[1] = all;
+}
+"""
+
+
+SHIM += r"""
+extern "C" void doubles(const float* x, int n, unsigned char* plain, double* out) {
+    for (int i = 0; i < n; i++) {
+        plain[i] = is_plain(x[i]);
+        out[i] = plain_double(x[i]);
+    }
 }
 """
 
@@ -76,3 +94,15 @@ def test_no_less_exact_than_one_by_one(lib, n, signs):
         assert abs(err[0]) <= 3 * 2.0**-48 * (n + 5)  # at most that of its operands per addition, n + 5 in a row
         squares += err**2
     assert squares[0] <= squares[1]
+
+
+def test_conversion_to_double(lib):
+    rng = np.random.default_rng(1)
+    mant = np.concatenate([[0, 1, 2, 2**22, 2**23 - 1], rng.integers(0, 2**23, 40)]).astype(np.uint32)
+    bits = (np.arange(512, dtype=np.uint32)[:, None] << np.uint32(23)) | mant  # every sign and exponent
+    x = np.ascontiguousarray(bits.ravel()).view(np.float32)
+    plain, out = np.zeros(x.size, np.uint8), np.zeros(x.size)
+    lib.doubles(ctypes.c_void_p(x.ctypes.data), x.size, ctypes.c_void_p(plain.ctypes.data), ctypes.c_void_p(out.ctypes.data))
+    normal = np.isfinite(x) & ((x == 0) | (np.abs(x) >= np.finfo(np.float32).tiny))
+    assert np.array_equal(plain.astype(bool), normal)
+    assert np.array_equal(out[normal].view(np.uint64), x[normal].astype(np.float64).view(np.uint64))

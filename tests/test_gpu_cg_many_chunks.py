@@ -41,6 +41,19 @@ def test_f32_equals_the_oracle(oracle, dims, fill):
     assert np.array_equal(got, want)
 
 
+@pytest.mark.parametrize("dims", [(33, 30, 31), (128, 40, 30)])
+def test_subnormal_terms(oracle, dims):
+    # FL_CG_F64_IEEE converts such terms in another way than normal ones
+    ct, div, p0 = field(dims, (1, 1, 1))
+    div = np.where(np.random.default_rng(8).uniform(size=div.shape) < 0.3, div * np.float32(1e-40), div).astype(np.float32)
+    assert ((div != 0) & (np.abs(div) < 1e-38)).any()
+    for iters in (1, 8):
+        args = (ct, div, dims, 1.0, 1.0, 1.0, iters, False, p0)
+        got, sg = solve_pressure(*args, tolerance=0.0, precision=FL_CG_F64_IEEE)
+        want, so = oracle.solve_pressure(*args, tolerance=0.0, precision=FL_CG_F64)
+        assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
+
+
 @pytest.mark.parametrize("dims", LARGE)
 def test_more_chunks_than_the_table_holds(oracle, dims):
     ct, div, p0 = field(dims, (1, 1, 1))

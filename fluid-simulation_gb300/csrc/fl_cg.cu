@@ -112,7 +112,7 @@ struct CgShared {
     uint32_t segslot[CHUNK];   // exchange words of the segments, ~0 for an empty one
     float seg[CHUNK];          // segment sums (cg_reduce_final.wgsl thread accumulators)
     float red[2 * CG_THREADS / 32];   // extended forms: warp partials
-    float scal[4];             // scalars of an exchange, broadcast by warp 0
+    float scal[2];             // alpha or beta, and whether the solve is done; broadcast by warp 0
     unsigned long long* area[6];  // exchange areas (see k_cg)
     // Block-uniform values read where they are used: the cell loops are at the
     // 128-register limit of a 512-thread block, and a spilled register costs an
@@ -332,11 +332,6 @@ __device__ __forceinline__ double warp_sum_d(double v) {  // result in lane 0
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     return v;
 }
-__device__ __forceinline__ double warp_allsum_d(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
 // a double's bits in two f32 slots (shared-memory staging and tagged words)
 __device__ __forceinline__ float d_lo(double v) { return __int_as_float(__double2loint(v)); }
 __device__ __forceinline__ float d_hi(double v) { return __int_as_float(__double2hiint(v)); }
@@ -382,8 +377,10 @@ __device__ __forceinline__ uint32_t seg_line(uint32_t nact) { return ((CHUNK + n
 // are 256 chunks apart: FL_CG_F64 1,976 -> 1,890 us on the full-depth 128^3 dam,
 // 4,126 -> 3,990 at 256^3, multigrid 1,584 -> 1,555; tiles of 2 x 8 and 8 x 2 give
 // the same within 1 %.  Blocks of one chunk per warp (or half of that) where there
-// are enough blocks.  For split segments the order did not pay: a block's partials
-// then belong to many segments (256^3: 5,183 -> 5,238 us).
+// are enough blocks.  For split segments the order was tried at 256^3 alone (5,183 ->
+// 5,238 us: a block's partials then belong to many segments), where a plane is 256
+// chunks and a segment's neighbours are z neighbours anyway; on other planes, where
+// they share nothing, it has not been measured.
 __global__ void __launch_bounds__(CHUNK) k_cg_plan(DevBufs b, uint32_t G, int form) {
     after_previous();
     const bool ranges_only = form == PLAN_RANGES;
@@ -848,9 +845,8 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
             sc = rs_old > 1e-30f ? __fdiv_rn(v, rs_old) : 0.0f;
             dn = v <= sh.thr_f;
         }
-        sh.scal[0] = v;
-        sh.scal[1] = sc;
-        sh.scal[2] = dn ? 1.0f : 0.0f;
+        sh.scal[0] = sc;
+        sh.scal[1] = dn ? 1.0f : 0.0f;
     };
     auto wait_word = [&](const unsigned long long* w, uint32_t tag, bool acq, bool& ok) -> float {
         unsigned long long v = ld_tag(w, acq);
@@ -989,8 +985,8 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
             if (lane == 0) post_f32(post, v);
         }
         __syncthreads();
-        sc = sh.scal[1];
-        dn = sh.scal[2] != 0.0f;
+        sc = sh.scal[0];
+        dn = sh.scal[1] != 0.0f;
         return true;
     };
     // Extended forms: the blocks' partials (two words of block bb at 16*bb),
@@ -1016,8 +1012,8 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
                     d2 = v <= sh.thr_d;
                     sh.rs_d = v;
                 }
-                sh.scal[1] = scv;
-                sh.scal[2] = d2 ? 1.0f : 0.0f;
+                sh.scal[0] = scv;
+                sh.scal[1] = d2 ? 1.0f : 0.0f;
             }
         } else if (warp == 0) {
             // a lane's up to MAX_CG_BLOCKS / 32 blocks, loaded first and added in pairs (one
@@ -1041,13 +1037,13 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DevBufs b) {
                     sh.rs_hi = acc.hi;
                     sh.rs_lo = acc.lo;
                 }
-                sh.scal[1] = scv;
-                sh.scal[2] = d2 ? 1.0f : 0.0f;
+                sh.scal[0] = scv;
+                sh.scal[1] = d2 ? 1.0f : 0.0f;
             }
         }
         __syncthreads();
-        sc = sh.scal[1];
-        dn = sh.scal[2] != 0.0f;
+        sc = sh.scal[0];
+        dn = sh.scal[1] != 0.0f;
         return true;
     };
     // Block partial published as two tagged words on the block's line: the

@@ -585,8 +585,12 @@ cudaError_t launch_p2g(const DevBufs& b, const LaunchCfg& L, uint32_t nx, uint32
     // A grid of few tiles takes flat ones: with 8^3 tiles a 64^3 half-tank has some
     // 100 blocks with particles, and the kernel took as long as one block (38 us at
     // 32^3, 46 us at 64^3; tiles of 8 x 8 x 2: 17 and 29 us, of 8 x 8 x 4: 19 and 37).
-    // A larger one fills the chip either way, and flat tiles add more rim sums to
-    // the face arrays (128^3: 77 us with 8^3, 95 us with 8 x 8 x 2; 256^3: 530 and 735).
+    // A larger one fills the chip either way, flat tiles add more rim sums to the face
+    // arrays (128^3: 77 us with 8^3, 95 us with 8 x 8 x 2; 256^3: 530 and 735), and the
+    // tiles without particles cost a block each, so the line follows the grid and not
+    // the liquid.  Flat / 8^3, us, half-full tanks: 56^3 38 / 54, 72^3 55 / 68, 80^3
+    // 75 / 75, 84^3 86 / 84, 112^3 178 / 168; a splash of 0.15 of each edge: 64^3
+    // 15 / 26, 84^3 16 / 26, 128^3 37 / 33, 200^3 149 / 49, 256^3 313 / 98.
     if (tx * ty * ((nz + 7) / 8) < 8u * (uint32_t)L.num_sms)
         launch_after(k_p2g_own<2>, dim3(tx * ty * ((nz + 1) / 2)), 256, s, b, (int)tx, (int)ty);
     else
